@@ -42,6 +42,47 @@ k_rmsnorm(const bf16* __restrict__ X, const bf16* __restrict__ G, bf16* __restri
   }
 }
 
+// The same for whole matrices (the prompt pass): one warp per row, the row in registers, all of
+// its 16-byte loads in flight together and no block barrier. cols a multiple of 8, at most
+// 256 * VECS, 16-byte aligned rows.
+template <int VECS>
+__global__ void __launch_bounds__(256)
+k_rmsnorm_rows(const bf16* __restrict__ X, const bf16* __restrict__ G, bf16* __restrict__ O,
+               int rows, int cols, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const uint4* x = reinterpret_cast<const uint4*>(X + (size_t)row * cols);
+  const uint4* g = reinterpret_cast<const uint4*>(G);
+  uint4* o = reinterpret_cast<uint4*>(O + (size_t)row * cols);
+  const int vecs = cols >> 3;
+  uint4 r[VECS];
+  float ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < VECS; ++j) r[j] = lane + 32 * j < vecs ? x[lane + 32 * j] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+  for (int j = 0; j < VECS; ++j) {
+    const uint32_t w[4] = {r[j].x, r[j].y, r[j].z, r[j].w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) ss += bf_lo(w[e]) * bf_lo(w[e]) + bf_hi(w[e]) * bf_hi(w[e]);
+  }
+  ss = warp_sum(ss);
+  const float inv = rsqrtf(ss / (float)cols + eps);
+#pragma unroll
+  for (int j = 0; j < VECS; ++j) {
+    if (lane + 32 * j >= vecs) continue;
+    const uint4 gv = __ldg(g + lane + 32 * j);
+    const uint32_t w[4] = {r[j].x, r[j].y, r[j].z, r[j].w}, gw[4] = {gv.x, gv.y, gv.z, gv.w};
+    uint32_t q[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      q[e] = pack_bf16(bf16_round(bf_lo(w[e]) * inv) * bf_lo(gw[e]), bf16_round(bf_hi(w[e]) * inv) * bf_hi(gw[e]));
+    o[lane + 32 * j] = make_uint4(q[0], q[1], q[2], q[3]);
+  }
+}
+
 // ---- embedding gather + RMSNorm --------------------------------------------
 // The table is the (tied) lm_head weight in the tiled GEMM layout: element
 // (row, c) lives in unit (row/16, c/32), half (row%16)/8, piece (row%8)*4 + (c%32)/8.
@@ -715,6 +756,18 @@ extern "C" int q_rmsnorm(const void* d_x, const void* d_gain, void* d_out, int r
                          float eps, void* stream) {
   Q_CHECK_ARG(d_x && d_gain && d_out && rows >= 1 && cols >= 1, "q_rmsnorm: bad argument");
   Q_CHECK_ALIGN(d_x, 2, "q_rmsnorm"); Q_CHECK_ALIGN(d_gain, 2, "q_rmsnorm"); Q_CHECK_ALIGN(d_out, 2, "q_rmsnorm");
+  // Many rows: a warp each (k_rmsnorm_rows). Few rows leave most SMs idle that way, so up to two
+  // rows per SM keep a whole CTA; so do odd widths and unaligned rows.
+  if (rows > 296 && cols % 8 == 0 && cols <= 4096 &&
+      (((uintptr_t)d_x | (uintptr_t)d_gain | (uintptr_t)d_out) & 15) == 0) {
+    if (cols <= 2560)
+      Q_CHECK_CUDA(q_launch(k_rmsnorm_rows<10>, dim3((rows + 7) / 8), dim3(256), 0, S(stream), (const bf16*)d_x,
+                            (const bf16*)d_gain, (bf16*)d_out, rows, cols, eps));
+    else
+      Q_CHECK_CUDA(q_launch(k_rmsnorm_rows<16>, dim3((rows + 7) / 8), dim3(256), 0, S(stream), (const bf16*)d_x,
+                            (const bf16*)d_gain, (bf16*)d_out, rows, cols, eps));
+    return Q_OK;
+  }
   Q_CHECK_CUDA(q_launch(k_rmsnorm, dim3(rows), dim3(256), 0, S(stream), (const bf16*)d_x,
                         (const bf16*)d_gain, (bf16*)d_out, cols, eps));
   return Q_OK;
