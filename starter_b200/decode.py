@@ -254,27 +254,28 @@ class DecodeState:
         return weights + kv_token * self.batch * visible_keys + kv_token * self.batch
 
     # ---- prefill: the prompt pass ----
-    PREFILL_ROWS = 2048        # prompt rows processed together (bounds the fp32 partial scratch)
+    PREFILL_ROWS = 8192        # prompt rows processed together (bounds the activation scratch)
+    PROMPT_GEMM_ROWS = 257     # rows from which the projections run on the CTA-pair kernel
 
     def _prefill_scratch(self, rows: int):
-        """Buffers of the prompt pass for `rows` rows, kept for the next call of the same size."""
-        if getattr(self, "_pf", None) is not None and self._pf["rows"] == rows:
+        """Buffers of the prompt pass for up to `rows` rows, kept for the next call."""
+        if getattr(self, "_pf", None) is not None and self._pf["rows"] >= rows:
             return self._pf
         cfg, w, dev = self.cfg, self.w, self.device
         nq, nkv, inter = w.local_q_heads, w.local_kv_heads, w.local_inter
-        plans = {"qkv": _lib.plan(rows, (nq + 2 * nkv) * HEAD_DIM, cfg.hidden, tc=True),
-                 "o": _lib.plan(rows, cfg.hidden, nq * HEAD_DIM, tc=True),
-                 "gu": _lib.plan(rows, 2 * inter, cfg.hidden, tc=True),
-                 "down": _lib.plan(rows, cfg.hidden, inter, tc=True)}
-        n_part = max(p.slots * p.M * p.N for p in plans.values())
         bf = dict(dtype=torch.bfloat16, device=dev)
         self._pf = None                    # release the previous size first
+        few = min(rows, self.PROMPT_GEMM_ROWS - 1)       # chunks of so many rows run on split-K partials
+        shapes = (((nq + 2 * nkv) * HEAD_DIM, cfg.hidden), (cfg.hidden, nq * HEAD_DIM), (2 * inter, cfg.hidden),
+                  (cfg.hidden, inter))
+        plans = [_lib.plan(few, n, k, tc=True) for n, k in shapes]
         self._pf = {
-            "rows": rows, "plans": plans, "partials": torch.empty(n_part, dtype=torch.float32, device=dev),
+            "rows": rows,
             "x": torch.empty((rows, cfg.hidden), **bf), "normed": torch.empty((rows, cfg.hidden), **bf),
             "q": torch.empty((rows, nq, HEAD_DIM), **bf), "att": torch.empty((rows, nq * HEAD_DIM), **bf),
             "act": torch.empty((rows, inter), **bf), "zero": torch.zeros(1, dtype=torch.int32, device=dev),
             "reduced": torch.empty((rows, cfg.hidden), dtype=torch.float32, device=dev) if self.tp > 1 else None,
+            "partials": torch.empty(max(p.slots * p.M * p.N for p in plans), dtype=torch.float32, device=dev),
         }
         return self._pf
 
@@ -284,11 +285,11 @@ class DecodeState:
         [B, V_local].
 
         The prompt pass of the reference (engine/prefill.py:26-62) on this library's own
-        kernels: every projection on the tcgen05 kernel over the tiled weights (256 prompt rows
-        per weight pass), embedding + norm, add + norm, SwiGLU and head norm + RoPE + page write
-        (engine/kernels/prefill.py:19-63) as the fused consumers of the decode step, the causal
+        kernels: from PROMPT_GEMM_ROWS rows on every projection on the CTA-pair tcgen05 kernel with
+        the residual add, SwiGLU or head norm + RoPE + page write (engine/kernels/prefill.py:19-63)
+        as its epilogue, below that on the decode step's projections and consumers; the causal
         attention over the prompt as q_attention_prefill reading the pages just written, lm_head
-        and argmax likewise; no library kernel runs. Sequences are processed PREFILL_ROWS prompt
+        and argmax as in the step; no library kernel runs. Sequences are processed PREFILL_ROWS prompt
         rows at a time. Under tensor
         parallelism the two row-parallel projections are summed over the ranks in fp32 by an
         NCCL all-reduce before the single rounding (the prompt pass is outside the per-step
@@ -300,39 +301,21 @@ class DecodeState:
         if input_ids.dtype != torch.int64 or not input_ids.is_cuda:
             raise ValueError("prompt ids must be an int64 CUDA tensor")
         w.ensure_tc()
-        nq, nkv, inter = w.local_q_heads, w.local_kv_heads, w.local_inter
         H, eps = cfg.hidden, float(cfg.rms_eps)
         per = max(1, self.PREFILL_ROWS // T)                 # sequences per pass
         stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
         ids = input_ids.contiguous()
         logits = torch.empty((B, w.local_vocab), dtype=torch.bfloat16, device=self.device)
         last = torch.empty((B, H), dtype=torch.bfloat16, device=self.device)
+        pf = self._prefill_scratch(min(per, B) * T)
         for b0 in range(0, B, per):
             nb = min(per, B - b0)
-            rows = nb * T
-            pf = self._prefill_scratch(rows)
-            pl, part = pf["plans"], pf["partials"]
-            x, normed, act = pf["x"], pf["normed"], pf["act"]
             table = self.block_table.data_ptr() + b0 * self.pages_per_seq * 4
-            check(lib.q_embed_rmsnorm(_p(ids[b0:b0 + nb]), _p(w.embed), _p(w.layers[0].ln_in), _p(x), _p(normed),
-                                      rows, H, cfg.vocab, eps, stream))
-            for i, lt in enumerate(w.layers):
-                check(lib.q_gemm_tc(_p(normed), _p(lt.wqkv.tc()), _p(part), rows, pl["qkv"].N, H, stream))
-                layout = _lib.KVLayout(self.kpools[i].data_ptr(), self.vpools[i].data_ptr(), table,
-                                       self.pages_per_seq, nkv)
-                check(lib.q_qkv_norm_rope_cache(_p(part), C.byref(pl["qkv"]), _p(lt.q_gain), _p(lt.k_gain),
-                                                _p(self.cos), _p(self.sin), _p(pf["zero"]), _p(pf["q"]),
-                                                C.byref(layout), nb, T, nq, eps, stream))
-                check(lib.q_attention_prefill(_p(pf["q"]), C.byref(layout), _p(pf["zero"]), _p(pf["att"]),
-                                              nb, T, nq, float(HEAD_DIM) ** -0.5, stream))
-                check(lib.q_gemm_tc(_p(pf["att"]), _p(lt.wo.tc()), _p(part), rows, H, nq * HEAD_DIM, stream))
-                self._prefill_add_norm(pf, pl["o"], lt.ln_post, rows, stream)
-                check(lib.q_gemm_tc(_p(normed), _p(lt.wgu.tc()), _p(part), rows, 2 * inter, H, stream))
-                check(lib.q_swiglu(_p(part), C.byref(pl["gu"]), _p(act), rows, inter, stream))
-                check(lib.q_gemm_tc(_p(act), _p(lt.wdown.tc()), _p(part), rows, H, inter, stream))
-                gain = w.layers[i + 1].ln_in if i + 1 < len(w.layers) else w.ln_final
-                self._prefill_add_norm(pf, pl["down"], gain, rows, stream)
-            last[b0:b0 + nb].copy_(normed.view(nb, T, H)[:, -1])
+            check(lib.q_embed_rmsnorm(_p(ids[b0:b0 + nb]), _p(w.embed), _p(w.layers[0].ln_in), _p(pf["x"]),
+                                      _p(pf["normed"]), nb * T, H, cfg.vocab, eps, stream))
+            layers = self._prefill_layers if nb * T >= self.PROMPT_GEMM_ROWS else self._prefill_layers_few_rows
+            layers(pf, nb, T, table, stream)
+            last[b0:b0 + nb].copy_(pf["normed"][:nb * T].view(nb, T, H)[:, -1])
         # lm_head on the last position of every sequence, logits rounded once to bf16
         hp = _lib.plan(B, w.local_vocab, H, tc=True)
         head_part = torch.empty((hp.slots, B, w.local_vocab), dtype=torch.float32, device=self.device)
@@ -352,17 +335,64 @@ class DecodeState:
         self.position.fill_(T)
         return logits
 
-    def _prefill_add_norm(self, pf, plan, gain, rows: int, stream) -> None:
-        """x, normed <- add + RMSNorm of the projection partials in pf['partials'] (summed over
-        the tensor-parallel ranks first, in fp32)."""
-        H, eps = self.cfg.hidden, float(self.cfg.rms_eps)
-        x, normed, part = pf["x"], pf["normed"], pf["partials"]
-        if self.tp == 1:
-            check(lib.q_add_rmsnorm(_p(x), _p(part), C.byref(plan), _p(gain), _p(x), _p(normed), rows, H, eps, stream))
-            return
-        check(lib.q_reduce_partials(_p(part), C.byref(plan), _p(pf["reduced"]), stream))
-        torch.distributed.all_reduce(pf["reduced"], group=self.group)
-        check(lib.q_add_rmsnorm(_p(x), _p(pf["reduced"]), None, _p(gain), _p(x), _p(normed), rows, H, eps, stream))
+    def _prefill_layers(self, pf, nb: int, T: int, table: int, stream) -> None:
+        """All layers over nb * T prompt rows: projections on the CTA-pair kernel with the
+        element-wise work in their epilogues."""
+        cfg, w = self.cfg, self.w
+        nq, nkv, inter = w.local_q_heads, w.local_kv_heads, w.local_inter
+        H, eps, rows = cfg.hidden, float(cfg.rms_eps), nb * T
+        x, normed, q, att, act = (_p(pf[n]) for n in ("x", "normed", "q", "att", "act"))
+        zero, scale = _p(pf["zero"]), float(HEAD_DIM) ** -0.5
+
+        def add_norm(inp, weight, K, gain):
+            if self.tp == 1:
+                check(lib.q_gemm_prompt_add(inp, _p(weight.tc()), x, rows, H, K, stream))
+                check(lib.q_rmsnorm(x, _p(gain), normed, rows, H, eps, stream))
+                return
+            check(lib.q_gemm_prompt_f32(inp, _p(weight.tc()), _p(pf["reduced"]), rows, H, K, stream))
+            torch.distributed.all_reduce(pf["reduced"][:rows], group=self.group)
+            check(lib.q_add_rmsnorm(x, _p(pf["reduced"]), None, _p(gain), x, normed, rows, H, eps, stream))
+
+        for i, lt in enumerate(w.layers):
+            layout = _lib.KVLayout(self.kpools[i].data_ptr(), self.vpools[i].data_ptr(), table, self.pages_per_seq, nkv)
+            check(lib.q_gemm_prompt_qkv(normed, _p(lt.wqkv.tc()), _p(lt.q_gain), _p(lt.k_gain), _p(self.cos),
+                                        _p(self.sin), zero, q, C.byref(layout), nb, T, nq, H, eps, stream))
+            check(lib.q_attention_prefill(q, C.byref(layout), zero, att, nb, T, nq, scale, stream))
+            add_norm(att, lt.wo, nq * HEAD_DIM, lt.ln_post)
+            check(lib.q_gemm_prompt_swiglu(normed, _p(lt.wgu.tc()), act, rows, inter, H, stream))
+            add_norm(act, lt.wdown, inter, w.layers[i + 1].ln_in if i + 1 < len(w.layers) else w.ln_final)
+
+    def _prefill_layers_few_rows(self, pf, nb: int, T: int, table: int, stream) -> None:
+        """The same on the split-K projections of the decode step and their fused consumers."""
+        cfg, w = self.cfg, self.w
+        nq, nkv, inter = w.local_q_heads, w.local_kv_heads, w.local_inter
+        H, eps, rows = cfg.hidden, float(cfg.rms_eps), nb * T
+        x, normed, q, att, act, part = (_p(pf[n]) for n in ("x", "normed", "q", "att", "act", "partials"))
+        zero, scale = _p(pf["zero"]), float(HEAD_DIM) ** -0.5
+        p_qkv = _lib.plan(rows, (nq + 2 * nkv) * HEAD_DIM, H, tc=True)
+        p_o = _lib.plan(rows, H, nq * HEAD_DIM, tc=True)
+        p_gu = _lib.plan(rows, 2 * inter, H, tc=True)
+        p_down = _lib.plan(rows, H, inter, tc=True)
+
+        def add_norm(inp, weight, plan, gain):
+            check(lib.q_gemm_tc(inp, _p(weight.tc()), part, rows, H, plan.K, stream))
+            if self.tp == 1:
+                check(lib.q_add_rmsnorm(x, part, C.byref(plan), _p(gain), x, normed, rows, H, eps, stream))
+                return
+            check(lib.q_reduce_partials(part, C.byref(plan), _p(pf["reduced"]), stream))
+            torch.distributed.all_reduce(pf["reduced"][:rows], group=self.group)
+            check(lib.q_add_rmsnorm(x, _p(pf["reduced"]), None, _p(gain), x, normed, rows, H, eps, stream))
+
+        for i, lt in enumerate(w.layers):
+            layout = _lib.KVLayout(self.kpools[i].data_ptr(), self.vpools[i].data_ptr(), table, self.pages_per_seq, nkv)
+            check(lib.q_gemm_tc(normed, _p(lt.wqkv.tc()), part, rows, p_qkv.N, H, stream))
+            check(lib.q_qkv_norm_rope_cache(part, C.byref(p_qkv), _p(lt.q_gain), _p(lt.k_gain), _p(self.cos),
+                                            _p(self.sin), zero, q, C.byref(layout), nb, T, nq, eps, stream))
+            check(lib.q_attention_prefill(q, C.byref(layout), zero, att, nb, T, nq, scale, stream))
+            add_norm(att, lt.wo, p_o, lt.ln_post)
+            check(lib.q_gemm_tc(normed, _p(lt.wgu.tc()), part, rows, 2 * inter, H, stream))
+            check(lib.q_swiglu(part, C.byref(p_gu), act, rows, inter, stream))
+            add_norm(act, lt.wdown, p_down, w.layers[i + 1].ln_in if i + 1 < len(w.layers) else w.ln_final)
 
     # ---- one decode step (the hot path) ----
     def step(self) -> None:
