@@ -247,25 +247,29 @@ typedef struct q_kv_layout_t {
 
 /* ---- projections of the prompt pass (hundreds to thousands of rows) ----------------
  * engine/prefill.py:40-52 with the layer's element-wise work in the projection's epilogue; the
- * weight in the tiling of q_pack_weight_tc. One accumulator holds a tile's whole K range (fp32),
- * the rounding points are those of the consumers above. N (inter) and K multiples of 32, x
- * 16-byte, outputs 32-byte aligned.
+ * weight in the tiling of q_pack_weight_tc. fp32 accumulation over all of K, the rounding points
+ * are those of the consumers above. N (inter) and K multiples of 32, x 16-byte, outputs 32-byte
+ * aligned.
  *   q_gemm_prompt_f32     out[M][N] = fp32 sums
  *   q_gemm_prompt_add     resid[M][N] = bf16(resid + bf16(sum)), in place
  *   q_gemm_prompt_swiglu  act[M][inter] = q_swiglu of the [gate | up] sums (weight 2*inter rows)
  *   q_gemm_prompt_qkv     q_qkv_norm_rope_cache of the [q | k | v] sums: q_out [rows][n_q][128],
  *                         k and v rows of positions *d_pos .. *d_pos+T-1 into their pages (cos /
- *                         sin tables and pools 32-byte aligned) */
+ *                         sin tables and pools 32-byte aligned)
+ * d_scratch: q_gemm_prompt_scratch_bytes() bytes, 16-byte aligned, the first 8 KB zeroed once by the
+ * caller (every launch leaves them zero), for the parts of tiles that several SM pairs share; one
+ * per stream, since calls that overlap on the GPU may not share it. Null: whole tiles only. */
+int64_t q_gemm_prompt_scratch_bytes(void);
 int q_gemm_prompt_f32(const void* d_x, const void* d_w_tc, float* d_out, int M, int N, int K,
-                      void* stream);
+                      void* d_scratch, void* stream);
 int q_gemm_prompt_add(const void* d_x, const void* d_w_tc, void* d_resid, int M, int N, int K,
-                      void* stream);
+                      void* d_scratch, void* stream);
 int q_gemm_prompt_swiglu(const void* d_x, const void* d_w_tc, void* d_act, int M, int inter, int K,
-                         void* stream);
+                         void* d_scratch, void* stream);
 int q_gemm_prompt_qkv(const void* d_x, const void* d_w_tc, const void* d_q_gain, const void* d_k_gain,
                       const void* d_cos, const void* d_sin, const int32_t* d_pos, void* d_q_out,
                       const q_kv_layout_t* kv, int batch, int T, int n_q_heads, int K, float eps,
-                      void* stream);
+                      void* d_scratch, void* stream);
 
 /* engine/kernels/decode_fused.py:172-210 (qkv_norm_rope_cache), generalised to
  * T consecutive query tokens per sequence (row m = b*T + t sits at absolute

@@ -102,10 +102,11 @@ SIGNATURES = {
     "q_unpack_weight_tc": (_I, [_P, _P, _I, _I, _P]),
     "q_gemm_tc_plan": (_I, [_I, _I, _I, _PLAN]),
     "q_gemm_tc": (_I, [_P, _P, _P, _I, _I, _I, _P]),
-    "q_gemm_prompt_f32": (_I, [_P, _P, _P, _I, _I, _I, _P]),
-    "q_gemm_prompt_add": (_I, [_P, _P, _P, _I, _I, _I, _P]),
-    "q_gemm_prompt_swiglu": (_I, [_P, _P, _P, _I, _I, _I, _P]),
-    "q_gemm_prompt_qkv": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _KV, _I, _I, _I, _I, _F, _P]),
+    "q_gemm_prompt_scratch_bytes": (C.c_int64, []),
+    "q_gemm_prompt_f32": (_I, [_P, _P, _P, _I, _I, _I, _P, _P]),
+    "q_gemm_prompt_add": (_I, [_P, _P, _P, _I, _I, _I, _P, _P]),
+    "q_gemm_prompt_swiglu": (_I, [_P, _P, _P, _I, _I, _I, _P, _P]),
+    "q_gemm_prompt_qkv": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _KV, _I, _I, _I, _I, _F, _P, _P]),
     "q_peer_flag_bytes": (C.c_int64, []),
     "q_argmax_merge_peers": (_I, [_P, _P, C.POINTER(Peers), _I, _P, _P, _I, _P]),
     "q_step_merge": (_I, [_P, _P, _P, _P]),

@@ -2,21 +2,20 @@
 // activation rows, on CTA pairs (tcgen05.mma.cta_group::2), with the layer's element-wise work
 // as the epilogue (reference: engine/prefill.py:40-52 calls library GEMMs and separate kernels).
 //
-// A pair of CTAs (a cluster of two, one SM each) owns an output tile of 256 rows x `bn` columns:
+// A pair of CTAs (a cluster of two, one SM each) owns an output tile of 256 rows x 256 columns:
 // each CTA brings in its 128 activation rows and HALF of the tile's weight rows per 64-k step,
 // the leader's one MMA thread multiplies over both shared memories, and each CTA's tensor memory
-// ends up with its own 128 rows x bn columns in fp32. What bounds this kernel is operand traffic
-// from L2 into shared memory: per 64 k an SM reads 16 KB + bn/2 x 128 B for 128 x bn outputs, at
-// bn = 256 two thirds of the bytes per product of the one-CTA kernel of gemm_tc.cu (weights 128 x
-// rows 256 per SM), which is why prompts leave that kernel.
+// ends up with its own 128 rows x 256 columns in fp32. What bounds this kernel is operand traffic
+// from L2 into shared memory: per 64 k an SM reads 32 KB for 128 x 256 outputs, two thirds of the
+// bytes per product of the one-CTA kernel of gemm_tc.cu (weights 128 x rows 256 per SM), which is
+// why prompts leave that kernel: 1.4 - 1.5 PFLOP/s against 1.0. (Narrower tiles to fill a wave
+// measured worse: 0.66 PFLOP/s at 160 columns, whose weight rows take five copies per stage.)
 //
-// One accumulator holds the whole K range of a tile, so nothing is split, no fp32 partials
-// travel through memory, and the epilogue can apply the consumer right away. Its thread owns one
-// activation row (tensor-memory lane) and walks the columns, so all of these are thread-local:
+// The epilogue's thread owns one activation row (tensor-memory lane) and walks the columns, so all of these are thread-local:
 //   EPI_F32     fp32 sums                          (before a tensor-parallel all-reduce)
 //   EPI_RESID   x = bf16(x + bf16(sum))            (O and down projections, in place)
-//   EPI_SWIGLU  act = bf16(bf16(silu(bf16 g)) * bf16 u): the tile's columns are bn/2 gate columns
-//               (the leader's weight half) and the matching bn/2 up columns (the peer's half)
+//   EPI_SWIGLU  act = bf16(bf16(silu(bf16 g)) * bf16 u): the tile's columns are 128 gate columns
+//               (the leader's weight half) and the matching 128 up columns (the peer's half)
 //   EPI_ROPE    bf16 q|k|v, head norm + RoPE on q and k heads (128 columns each), q to
 //               [row][head][128], k and v rows into their pages
 // The rounding points are those of the consumers in fused_ops.cu.
@@ -27,8 +26,14 @@
 // bytes); commits release stages and hand over accumulators in both CTAs at once. Every wait is
 // bounded as in gemm_tc.cu and reports in the same status word (codes 5-8).
 //
-// Tiles go to pairs in a fixed order (tile = pair + i * pairs): row tiles fastest inside groups of
-// eight, so that the tiles in flight share both operands in L2.
+// Work split: tiles in raster order (row tiles fastest inside groups of eight, so that the tiles in
+// flight share both operands in L2). Whole waves of one tile per pair come first; what is left over
+// - up to two tiles' work per pair - is cut evenly by k steps over all pairs (`split`), since a
+// projection with N = 2560 has 40 tiles at 1024 rows and 80 at 2048 for 74 pairs. A pair that ends
+// up with a part of a tile stores its fp32 accumulator in the caller's scratch, draws a ticket, and
+// the LAST of a tile's pairs adds the parts in k order (its own included, so the sum does not depend
+// on who is last), puts the total back into tensor memory and runs the epilogue. Nobody waits. The
+// unit of all this is a warp: 32 rows of one CTA.
 #include "tc.cuh"
 
 int* q_tc_status_addr();
@@ -38,17 +43,51 @@ namespace {
 constexpr int PG_THREADS = 192;
 constexpr int PG_TILE_K = 64;
 constexpr int PG_A_BYTES = 128 * PG_TILE_K * 2;            // 16 KB of activations per CTA and stage
-constexpr int PG_SMEM_BUDGET = 224 * 1024;
+constexpr int PG_BN = 256, PG_HALF = 128;                  // columns of a tile, weight rows per CTA
+constexpr uint32_t PG_STAGE = PG_A_BYTES + PG_HALF * PG_TILE_K * 2;
+constexpr int PG_STAGES = 7;                               // 224 KB
+constexpr size_t PG_SMEM = 1024 + PG_STAGES * PG_STAGE + (2 * PG_STAGES + 4) * 8 + 16;
 constexpr int PG_GROUP = 8;                                // row tiles per raster group
+constexpr int PG_MAX_PAIRS = 128;
+constexpr int PG_SPLIT_STEPS = 20;
+// scratch: tickets (8 warps per tile, at most two tiles per pair), then two parts per pair
+constexpr size_t PG_TICKET_BYTES = PG_MAX_PAIRS * 2 * 8 * 4;
+constexpr size_t PG_PART_FLOATS = 256 * 256;
 
 enum { EPI_F32 = 0, EPI_RESID = 1, EPI_SWIGLU = 2, EPI_ROPE = 3 };
 
 struct PromptShape {
   int M, N, KT;         // rows, output columns (EPI_SWIGLU: inter), k tiles
-  int mt, nt;           // tiles along rows (256) and columns (bn; EPI_SWIGLU bn/2)
-  int bn;               // MMA N: 128 .. 256, multiple of 32
+  int mt, nt;           // tiles along rows (256) and columns (256; EPI_SWIGLU 128 gate + 128 up)
   int wrows;            // weight rows per copy (a power of two that divides every copy's start)
-  int stages;
+  int waves;            // tiles that each pair takes whole
+  int share;            // k steps of the remaining tiles per pair: whole tiles, or an even split
+};
+
+// The pieces of a pair in order: (tile, k steps [k0, k1)).
+struct Walk {
+  int i, u, u1;
+  __device__ __forceinline__ void start(const PromptShape& sh, int pair, int pairs) {
+    i = 0;
+    const int rest = (sh.mt * sh.nt - sh.waves * pairs) * sh.KT;
+    u = min(rest, pair * sh.share);
+    u1 = min(rest, u + sh.share);
+  }
+  __device__ __forceinline__ bool next(const PromptShape& sh, int pair, int pairs, int& t, int& k0, int& k1) {
+    if (i < sh.waves) {
+      t = pair + i++ * pairs;
+      k0 = 0;
+      k1 = sh.KT;
+      return true;
+    }
+    if (u >= u1) return false;
+    const int rel = u / sh.KT;
+    t = sh.waves * pairs + rel;
+    k0 = u - rel * sh.KT;
+    k1 = min(sh.KT, k0 + u1 - u);
+    u += k1 - k0;
+    return true;
+  }
 };
 
 struct RopeArgs {
@@ -121,6 +160,15 @@ __device__ __forceinline__ void tc_ld16x2(uint32_t a, uint32_t b, float (&v)[16]
       : "r"(a), "r"(b) : "memory");
 #pragma unroll
   for (int i = 0; i < 16; ++i) { v[i] = __uint_as_float(r[i]); w[i] = __uint_as_float(s[i]); }
+}
+
+__device__ __forceinline__ void tc_st16x2(uint32_t a, uint32_t b, const float (&v)[16], const float (&w)[16]) {
+#define Q_R(x, i) "f"(x[i]), "f"(x[i + 1]), "f"(x[i + 2]), "f"(x[i + 3]), "f"(x[i + 4]), "f"(x[i + 5]), "f"(x[i + 6]), "f"(x[i + 7])
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+               ::"r"(a), Q_R(v, 0), Q_R(v, 8) : "memory");
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+               ::"r"(b), Q_R(w, 0), Q_R(w, 8) : "memory");
+#undef Q_R
 }
 
 // 32 bytes (16 bf16) at a 32-byte boundary: whole sectors, since neighbouring lanes hold other rows.
@@ -225,21 +273,85 @@ __device__ __forceinline__ void rope_head(uint32_t taddr, const RopeArgs& ra, bf
   }
 }
 
+// A warp's part (32 rows x 256 columns at `taddr`) of tile `rel` of the split ones. True: this was
+// the tile's last part and tensor memory now holds the sum of all parts, added in k order.
+__device__ __forceinline__ bool merge_parts(const PromptShape& sh, unsigned char* scratch, uint32_t taddr, int pair,
+                                            int rel, int k0, int warp_of_tile, int lane) {
+  const int first = rel * sh.KT / sh.share, last = ((rel + 1) * sh.KT - 1) / sh.share;
+  int* ticket = reinterpret_cast<int*>(scratch) + rel * 8 + warp_of_tile;
+  float* parts = reinterpret_cast<float*>(scratch + PG_TICKET_BYTES);
+  // a pair has at most two parts: the rest of a tile it did not begin, the beginning of its last one;
+  // element (column 4 j + e, lane) of a warp's part sits at (j * 32 + lane) * 4 + e
+  auto part = [&](int p) {
+    return reinterpret_cast<float4*>(parts + (size_t)(2 * p + (p * sh.share > rel * sh.KT ? 0 : 1)) * PG_PART_FLOATS +
+                                     warp_of_tile * (32 * 256)) + lane;
+  };
+  int drawn = 0;
+  if (lane == 0) drawn = *reinterpret_cast<volatile int*>(ticket);
+  drawn = __shfl_sync(0xffffffffu, drawn, 0);
+  if (drawn != last - first) {                    // not known to be the last one: leave the part in memory
+    float4* dst = part(pair);
+#pragma unroll 1
+    for (int c = 0; c < 256; c += 32) {
+      float v[16], w[16];
+      tc_ld16x2(taddr + c, taddr + c + 16, v, w);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        dst[(c / 4 + j) * 32] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        dst[(c / 4 + 4 + j) * 32] = make_float4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+      }
+    }
+    __threadfence();
+    __syncwarp();
+    if (lane == 0) drawn = atomicAdd(ticket, 1);
+    drawn = __shfl_sync(0xffffffffu, drawn, 0);
+    if (drawn != last - first) return false;
+  }
+  __syncwarp();
+  __threadfence();
+  if (lane == 0) *ticket = 0;                     // ready for the next launch
+#pragma unroll 1
+  for (int c = 0; c < 256; c += 32) {
+    float v[16], w[16], own_v[16], own_w[16];
+    tc_ld16x2(taddr + c, taddr + c + 16, own_v, own_w);
+#pragma unroll
+    for (int e = 0; e < 16; ++e) v[e] = w[e] = 0.f;
+    for (int p = first; p <= last; ++p) {
+      if (p == pair) {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) { v[e] += own_v[e]; w[e] += own_w[e]; }
+        continue;
+      }
+      const float4* src = part(p);
+      float4 a[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) a[j] = __ldcg(src + (c / 4 + j) * 32);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        v[4 * j] += a[j].x; v[4 * j + 1] += a[j].y; v[4 * j + 2] += a[j].z; v[4 * j + 3] += a[j].w;
+        w[4 * j] += a[4 + j].x; w[4 * j + 1] += a[4 + j].y; w[4 * j + 2] += a[4 + j].z; w[4 * j + 3] += a[4 + j].w;
+      }
+    }
+    tc_st16x2(taddr + c, taddr + c + 16, v, w);
+  }
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+  return true;
+}
+
 template <int EPI>
 __global__ void __launch_bounds__(PG_THREADS, 1)
 k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, void* __restrict__ out,
-              PromptShape sh, const __grid_constant__ RopeArgs ra, int* status, unsigned long long* tl) {
+              PromptShape sh, const __grid_constant__ RopeArgs ra, unsigned char* scratch, int* status,
+              unsigned long long* tl) {
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   unsigned char* smem = smem_raw + (base - raw);
-  const int half = sh.bn >> 1;                              // weight rows per CTA and stage
-  const uint32_t stage_bytes = PG_A_BYTES + (uint32_t)half * 128u;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)sh.stages * stage_bytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + PG_STAGES * PG_STAGE);
   // full[stages] (leader's) | empty[stages] | acc_full[2] | acc_empty[2] (leader's)
-  const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8u * sh.stages;
-  const uint32_t bar_acc_full = bar_empty + 8u * sh.stages, bar_acc_empty = bar_acc_full + 16u;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * sh.stages + 4);
+  const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8u * PG_STAGES;
+  const uint32_t bar_acc_full = bar_empty + 8u * PG_STAGES, bar_acc_empty = bar_acc_full + 16u;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * PG_STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   tl_begin(tl);
@@ -247,10 +359,9 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_rank();
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-  const int total = sh.mt * sh.nt;
 
   if (tid == 0) {
-    for (int s = 0; s < sh.stages; ++s) {
+    for (int s = 0; s < PG_STAGES; ++s) {
       mbar_init(bar_full + 8 * s, 1);
       mbar_init(bar_empty + 8 * s, 1);
     }
@@ -286,27 +397,31 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
     // ---------------- producer ----------------
     if (lane == 0) {
       const uint32_t full0 = leader_addr(bar_full);
-      const int nload = half / sh.wrows;
+      const int nload = PG_HALF / sh.wrows;
       const uint32_t wbytes = (uint32_t)sh.wrows * 128u;
       int st = 0;
       uint32_t parity = 1;                                  // an untouched stage is free
       bool ok = true, waited = false;
       int issued = 0;
-      for (int t = pair; ok && t < total; t += pairs) {
+      Walk walk;
+      walk.start(sh, pair, pairs);
+      int t, k0, k1;
+      while (ok && walk.next(sh, pair, pairs, t, k0, k1)) {
         int mi, ni;
         locate(t, mi, ni);
-        const int row = mi * 256 + (int)rank * 128;
+        // (rows that do not exist are not worth a copy of zeros, which is slow: any rows will do)
+        const int row0 = mi * 256 + (int)rank * 128, row = row0 < sh.M ? row0 : 0;
         // first weight row of this CTA's half
-        const int n0 = EPI == EPI_SWIGLU ? (int)rank * sh.N + ni * half : ni * sh.bn + (int)rank * half;
-        for (int kt = 0; kt < sh.KT; ++kt) {
+        const int n0 = EPI == EPI_SWIGLU ? (int)rank * sh.N + ni * PG_HALF : ni * PG_BN + (int)rank * PG_HALF;
+        for (int kt = k0; kt < k1; ++kt) {
           if (!mbar_wait(bar_empty + 8 * st, parity, abort_flag)) {
             atomicExch(status, 5);
             *abort_flag = 1;
             ok = false;
             break;
           }
-          const uint32_t full = full0 + 8u * st, dst = base + st * stage_bytes;
-          if (rank == 0) mbar_expect_tx(bar_full + 8 * st, 2 * stage_bytes);
+          const uint32_t full = full0 + 8u * st, dst = base + st * PG_STAGE;
+          if (rank == 0) mbar_expect_tx(bar_full + 8 * st, 2 * PG_STAGE);
           for (int j = 0; j < nload; ++j) {
             const int n = n0 + j * sh.wrows;
             pair_load_4d(dst + PG_A_BYTES + j * wbytes, &wmap, 0, n & 127, kt, n >> 7, full);
@@ -318,41 +433,44 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
           }
           pair_load_2d(dst, &xmap, kt * PG_TILE_K, row, full);
           ++issued;
-          if (++st == sh.stages) { st = 0; parity ^= 1u; }
+          if (++st == PG_STAGES) { st = 0; parity ^= 1u; }
         }
       }
       // Every copy must have landed before the CTAs may leave: the leader waits for the last fill
       // of each stage (both CTAs' bytes), the cluster barrier at the end holds the peer.
       if (rank == 0)
-        for (int s = 0; s < sh.stages && s < issued; ++s) {
-          const int last = (issued - 1 - s) / sh.stages;
+        for (int s = 0; s < PG_STAGES && s < issued; ++s) {
+          const int last = (issued - 1 - s) / PG_STAGES;
           if (!mbar_wait_plain(bar_full + 8 * s, last & 1)) atomicExch(status, 8);
         }
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader) ----------------
     if (rank == 0 && lane == 0) {
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(sh.bn >> 3) << 17) | (16u << 24);
-      const uint32_t stage_units = stage_bytes >> 4;
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(PG_BN >> 3) << 17) | (16u << 24);
+      const uint32_t stage_units = PG_STAGE >> 4;
       const uint64_t desc0 = smem_desc(base);
       int st = 0, seg = 0;
       uint32_t parity = 0;
       bool ok = true;
-      for (int t = pair; ok && t < total; t += pairs, ++seg) {
+      Walk walk;
+      walk.start(sh, pair, pairs);
+      int t, k0, k1;
+      for (; ok && walk.next(sh, pair, pairs, t, k0, k1); ++seg) {
         const int buf = seg & 1;
         if (!mbar_wait(bar_acc_empty + 8 * buf, ((seg >> 1) & 1) ^ 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t dacc = tmem_base + (uint32_t)buf * 256u;
-        for (int kt = 0; kt < sh.KT; ++kt) {
+        for (int kt = k0; kt < k1; ++kt) {
           if (!mbar_wait(bar_full + 8 * st, parity, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint64_t a_desc = desc0 + (uint64_t)(st * stage_units);
           const uint64_t b_desc = a_desc + (PG_A_BYTES >> 4);
 #pragma unroll
           for (int k = 0; k < PG_TILE_K / 16; ++k)
-            pair_mma(dacc, a_desc + 2u * k, b_desc + 2u * k, idesc, (kt | k) ? 1u : 0u);
+            pair_mma(dacc, a_desc + 2u * k, b_desc + 2u * k, idesc, (kt > k0 || k) ? 1u : 0u);
           pair_commit(bar_empty + 8 * st);
-          if (++st == sh.stages) { st = 0; parity ^= 1u; }
+          if (++st == PG_STAGES) { st = 0; parity ^= 1u; }
         }
         if (ok) pair_commit(bar_acc_full + 8 * buf);
       }
@@ -367,7 +485,10 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
     const int q = warp & 3;
     const uint32_t acc_empty0 = leader_addr(bar_acc_empty);
     int seg = 0;
-    for (int t = pair; t < total; t += pairs, ++seg) {
+    Walk walk;
+    walk.start(sh, pair, pairs);
+    int t, k0, k1;
+    for (; walk.next(sh, pair, pairs, t, k0, k1); ++seg) {
       const int buf = seg & 1;
       int mi, ni;
       locate(t, mi, ni);
@@ -383,9 +504,16 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
       }
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)buf * 256u;
+      if (k1 - k0 < sh.KT && !merge_parts(sh, scratch, taddr, pair, t - sh.waves * pairs, k0, (int)rank * 4 + q, lane)) {
+        // a part of a tile, and not the last one: another pair finishes the tile
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(acc_empty0 + 8 * buf);
+        continue;
+      }
       if (EPI == EPI_F32) {
-        float* dst = reinterpret_cast<float*>(out) + (size_t)m * sh.N + ni * sh.bn;
-        for (int c = 0; c < sh.bn && ni * sh.bn + c < sh.N; c += 32) {   // N is a multiple of 32
+        float* dst = reinterpret_cast<float*>(out) + (size_t)m * sh.N + ni * PG_BN;
+        for (int c = 0; c < PG_BN && ni * PG_BN + c < sh.N; c += 32) {   // N is a multiple of 32
           float v[16], w[16];
           tc_ld16x2(taddr + c, taddr + c + 16, v, w);
           if (live) {
@@ -400,9 +528,9 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
           }
         }
       } else if (EPI == EPI_RESID) {
-        bf16* x = reinterpret_cast<bf16*>(out) + (size_t)(live ? m : 0) * sh.N + ni * sh.bn;
+        bf16* x = reinterpret_cast<bf16*>(out) + (size_t)(live ? m : 0) * sh.N + ni * PG_BN;
 #pragma unroll 2
-        for (int c = 0; c < sh.bn && ni * sh.bn + c < sh.N; c += 32) {
+        for (int c = 0; c < PG_BN && ni * PG_BN + c < sh.N; c += 32) {
           float v[16], w[16], a[16];
           uint32_t r0[8], r1[8];
           ld32B(x + c, r0);
@@ -422,11 +550,11 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
           }
         }
       } else if (EPI == EPI_SWIGLU) {
-        bf16* act = reinterpret_cast<bf16*>(out) + (size_t)m * sh.N + ni * half;
-        for (int c = 0; c < half && ni * half + c < sh.N; c += 16) {     // inter is a multiple of 16
+        bf16* act = reinterpret_cast<bf16*>(out) + (size_t)m * sh.N + ni * PG_HALF;
+        for (int c = 0; c < PG_HALF && ni * PG_HALF + c < sh.N; c += 16) {     // inter is a multiple of 16
           float g[16], u[16];
           uint32_t r[8];
-          tc_ld16x2(taddr + c, taddr + half + c, g, u);
+          tc_ld16x2(taddr + c, taddr + PG_HALF + c, g, u);
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
             const float gb = bf16_round(g[e]);
@@ -441,8 +569,8 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
         const int page = ra.block_table[(size_t)b * ra.pages_per_seq + pos / Q_PAGE_TOKENS];
         const int r = pos % Q_PAGE_TOKENS;
         const size_t row = (size_t)page * ra.nkv * (Q_PAGE_TOKENS * 256) + (size_t)r * 256;
-        for (int c = 0; c < sh.bn && ni * sh.bn + c < sh.N; c += 128)
-          rope_head(taddr + c, ra, reinterpret_cast<bf16*>(out), m, live, (ni * sh.bn + c) >> 7, pos, ra.kpool + row,
+        for (int c = 0; c < PG_BN && ni * PG_BN + c < sh.N; c += 128)
+          rope_head(taddr + c, ra, reinterpret_cast<bf16*>(out), m, live, (ni * PG_BN + c) >> 7, pos, ra.kpool + row,
                     ra.vpool + row, r);
       }
       tc_fence_before();
@@ -462,29 +590,16 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
   tl_end(tl);
 }
 
-// Column width of a tile: 256 unless a narrower tile saves waves. `sms`/2 pairs take one tile
-// each per wave, and a tile costs about its operand traffic, 256 + bn rows of 128 bytes per 64 k.
-int pick_bn(int mt, int N, int sms, int step) {
-  int best = 256;
-  long long cost = -1;
-  for (int bn = 256; bn >= 128; bn -= step) {
-    const long long tiles = (long long)mt * ((N + bn - 1) / bn);
-    const long long waves = (tiles + sms / 2 - 1) / (sms / 2);
-    const long long c = waves * (256 + bn);
-    if (cost < 0 || c < cost) { cost = c; best = bn; }
-  }
-  return best;
-}
-
 // `N` as in PromptShape; the weight has `wN` rows.
 template <int EPI>
 int launch_prompt(const void* x, const void* w_tc, void* out, int M, int N, int wN, int K, const RopeArgs& ra,
-                  void* stream, const char* who) {
+                  void* scratch, void* stream, const char* who) {
   Q_CHECK_ARG(x && w_tc && out, "%s: null pointer", who);
   Q_CHECK_ARG(M >= 1 && N >= 32 && N % 32 == 0 && K >= 32 && K % 32 == 0,
               "%s: need rows, N and K multiples of 32 (M=%d N=%d K=%d)", who, M, N, K);
-  Q_CHECK_ARG(((uintptr_t)x & 15) == 0 && ((uintptr_t)w_tc & 1023) == 0 && ((uintptr_t)out & 31) == 0,
-              "%s: x must be 16-byte, the output 32-byte and the tiled weight 1024-byte aligned", who);
+  Q_CHECK_ARG(((uintptr_t)x & 15) == 0 && ((uintptr_t)w_tc & 1023) == 0 && ((uintptr_t)out & 31) == 0 &&
+                  ((uintptr_t)scratch & 15) == 0,
+              "%s: x and scratch must be 16-byte, the output 32-byte and the tiled weight 1024-byte aligned", who);
   int* status = q_tc_status_addr();
   if (!status) { q_set_error("%s: could not locate the device status word", who); return Q_ERR_CUDA; }
   const int sms = q_sm_count();
@@ -492,16 +607,28 @@ int launch_prompt(const void* x, const void* w_tc, void* out, int M, int N, int 
   sh.M = M; sh.N = N;
   sh.KT = (K + PG_TILE_K - 1) / PG_TILE_K;
   sh.mt = (M + 255) / 256;
-  // gate and up halves stay whole 128-row blocks; heads are 128 columns
-  sh.bn = EPI == EPI_SWIGLU ? 256 : pick_bn(sh.mt, N, sms, EPI == EPI_ROPE ? 128 : 32);
-  const int cols = EPI == EPI_SWIGLU ? sh.bn / 2 : sh.bn;
+  const int cols = EPI == EPI_SWIGLU ? PG_HALF : PG_BN;
   sh.nt = (N + cols - 1) / cols;
-  Q_CHECK_ARG((long long)sh.mt * sh.nt < (1ll << 30), "%s: too many tiles", who);
+  const long long tiles = (long long)sh.mt * sh.nt;
+  Q_CHECK_ARG(tiles * sh.KT < (1ll << 30), "%s: too many tiles", who);
   sh.wrows = 128;
-  while ((sh.bn / 2) % sh.wrows || (EPI == EPI_SWIGLU && N % sh.wrows)) sh.wrows >>= 1;
-  const uint32_t stage = PG_A_BYTES + sh.bn / 2 * 128;
-  sh.stages = PG_SMEM_BUDGET / stage;
-  if (sh.stages > 12) sh.stages = 12;
+  while (EPI == EPI_SWIGLU && N % sh.wrows) sh.wrows >>= 1;
+  int pairs = sms / 2 < PG_MAX_PAIRS ? sms / 2 : PG_MAX_PAIRS;
+  // Whole tiles only, or the last wave and the remainder cut evenly: the split saves the idle part of
+  // a wave (k steps of ~0.4 us each) and costs parts through L2 and a late epilogue, PG_SPLIT_STEPS.
+  const int full = (int)(tiles / pairs), rest = (int)(tiles % pairs);
+  sh.waves = full;
+  sh.share = sh.KT;
+  if (scratch && rest) {
+    const int whole = full > 0 ? full - 1 : 0;
+    const int left = (int)(tiles - (long long)whole * pairs);
+    const int share = (left * sh.KT + pairs - 1) / pairs;
+    if (share + PG_SPLIT_STEPS < (full - whole + 1) * sh.KT) {
+      sh.waves = whole;
+      sh.share = share;
+    }
+  }
+  if (sh.share == sh.KT && tiles < pairs) pairs = (int)tiles;
   CUtensorMap xmap, wmap;
   {
     const cuuint64_t dim[2] = {(cuuint64_t)K, (cuuint64_t)M};
@@ -518,39 +645,40 @@ int launch_prompt(const void* x, const void* w_tc, void* out, int M, int N, int 
     int rc = tc_encode(&wmap, w_tc, 4, dim, stride, box, CU_TENSOR_MAP_SWIZZLE_NONE, who);
     if (rc) return rc;
   }
-  const size_t smem = 1024 + (size_t)sh.stages * stage + (2 * sh.stages + 4) * 8 + 16;
   static size_t smem_done[64] = {0};
-  Q_CHECK_CUDA(q_ensure_smem(k_gemm_prompt<EPI>, smem, smem_done));
-  const int tiles = sh.mt * sh.nt;
-  const int pairs = tiles < sms / 2 ? tiles : sms / 2;
-  Q_CHECK_CUDA(q_launch_cluster(k_gemm_prompt<EPI>, dim3(2 * pairs), dim3(PG_THREADS), smem, (cudaStream_t)stream, 2,
-                                xmap, wmap, out, sh, ra, status, q_tl_next(Q_TL_GEMM_TC)));
+  Q_CHECK_CUDA(q_ensure_smem(k_gemm_prompt<EPI>, PG_SMEM, smem_done));
+  Q_CHECK_CUDA(q_launch_cluster(k_gemm_prompt<EPI>, dim3(2 * pairs), dim3(PG_THREADS), PG_SMEM, (cudaStream_t)stream, 2,
+                                xmap, wmap, out, sh, ra, (unsigned char*)scratch, status, q_tl_next(Q_TL_GEMM_TC)));
   return Q_OK;
 }
 
 }  // namespace
 
+extern "C" int64_t q_gemm_prompt_scratch_bytes(void) {
+  return (int64_t)(PG_TICKET_BYTES + (size_t)PG_MAX_PAIRS * 2 * PG_PART_FLOATS * 4);
+}
+
 extern "C" int q_gemm_prompt_f32(const void* d_x, const void* d_w_tc, float* d_out, int M, int N, int K,
-                                 void* stream) {
-  return launch_prompt<EPI_F32>(d_x, d_w_tc, d_out, M, N, N, K, RopeArgs(), stream, "q_gemm_prompt_f32");
+                                 void* d_scratch, void* stream) {
+  return launch_prompt<EPI_F32>(d_x, d_w_tc, d_out, M, N, N, K, RopeArgs(), d_scratch, stream, "q_gemm_prompt_f32");
 }
 
 extern "C" int q_gemm_prompt_add(const void* d_x, const void* d_w_tc, void* d_resid, int M, int N, int K,
-                                 void* stream) {
+                                 void* d_scratch, void* stream) {
   Q_CHECK_ARG(d_x != d_resid, "q_gemm_prompt_add: the residual cannot be the projection's input");
-  return launch_prompt<EPI_RESID>(d_x, d_w_tc, d_resid, M, N, N, K, RopeArgs(), stream, "q_gemm_prompt_add");
+  return launch_prompt<EPI_RESID>(d_x, d_w_tc, d_resid, M, N, N, K, RopeArgs(), d_scratch, stream, "q_gemm_prompt_add");
 }
 
 extern "C" int q_gemm_prompt_swiglu(const void* d_x, const void* d_w_tc, void* d_act, int M, int inter, int K,
-                                    void* stream) {
-  return launch_prompt<EPI_SWIGLU>(d_x, d_w_tc, d_act, M, inter, 2 * inter, K, RopeArgs(), stream,
+                                    void* d_scratch, void* stream) {
+  return launch_prompt<EPI_SWIGLU>(d_x, d_w_tc, d_act, M, inter, 2 * inter, K, RopeArgs(), d_scratch, stream,
                                    "q_gemm_prompt_swiglu");
 }
 
 extern "C" int q_gemm_prompt_qkv(const void* d_x, const void* d_w_tc, const void* d_q_gain, const void* d_k_gain,
                                  const void* d_cos, const void* d_sin, const int32_t* d_pos, void* d_q_out,
                                  const q_kv_layout_t* kv, int batch, int T, int n_q_heads, int K, float eps,
-                                 void* stream) {
+                                 void* d_scratch, void* stream) {
   const char* who = "q_gemm_prompt_qkv";
   Q_CHECK_ARG(d_q_gain && d_k_gain && d_cos && d_sin && d_pos && kv, "%s: null pointer", who);
   Q_CHECK_ARG(kv->d_kpool && kv->d_vpool && kv->d_block_table && kv->pages_per_seq >= 1 && kv->n_kv_heads >= 1,
@@ -566,5 +694,5 @@ extern "C" int q_gemm_prompt_qkv(const void* d_x, const void* d_w_tc, const void
   ra.kpool = (char*)kv->d_kpool; ra.vpool = (char*)kv->d_vpool; ra.block_table = kv->d_block_table;
   ra.pages_per_seq = kv->pages_per_seq; ra.T = T; ra.nq = n_q_heads; ra.nkv = kv->n_kv_heads; ra.eps = eps;
   const int N = (n_q_heads + 2 * kv->n_kv_heads) * 128;
-  return launch_prompt<EPI_ROPE>(d_x, d_w_tc, d_q_out, batch * T, N, N, K, ra, stream, who);
+  return launch_prompt<EPI_ROPE>(d_x, d_w_tc, d_q_out, batch * T, N, N, K, ra, d_scratch, stream, who);
 }

@@ -275,6 +275,7 @@ class DecodeState:
             "q": torch.empty((rows, nq, HEAD_DIM), **bf), "att": torch.empty((rows, nq * HEAD_DIM), **bf),
             "act": torch.empty((rows, inter), **bf), "zero": torch.zeros(1, dtype=torch.int32, device=dev),
             "reduced": torch.empty((rows, cfg.hidden), dtype=torch.float32, device=dev) if self.tp > 1 else None,
+            "split": torch.zeros(lib.q_gemm_prompt_scratch_bytes(), dtype=torch.uint8, device=dev),
             "partials": torch.empty(max(p.slots * p.M * p.N for p in plans), dtype=torch.float32, device=dev),
         }
         return self._pf
@@ -341,25 +342,25 @@ class DecodeState:
         cfg, w = self.cfg, self.w
         nq, nkv, inter = w.local_q_heads, w.local_kv_heads, w.local_inter
         H, eps, rows = cfg.hidden, float(cfg.rms_eps), nb * T
-        x, normed, q, att, act = (_p(pf[n]) for n in ("x", "normed", "q", "att", "act"))
+        x, normed, q, att, act, split = (_p(pf[n]) for n in ("x", "normed", "q", "att", "act", "split"))
         zero, scale = _p(pf["zero"]), float(HEAD_DIM) ** -0.5
 
         def add_norm(inp, weight, K, gain):
             if self.tp == 1:
-                check(lib.q_gemm_prompt_add(inp, _p(weight.tc()), x, rows, H, K, stream))
+                check(lib.q_gemm_prompt_add(inp, _p(weight.tc()), x, rows, H, K, split, stream))
                 check(lib.q_rmsnorm(x, _p(gain), normed, rows, H, eps, stream))
                 return
-            check(lib.q_gemm_prompt_f32(inp, _p(weight.tc()), _p(pf["reduced"]), rows, H, K, stream))
+            check(lib.q_gemm_prompt_f32(inp, _p(weight.tc()), _p(pf["reduced"]), rows, H, K, split, stream))
             torch.distributed.all_reduce(pf["reduced"][:rows], group=self.group)
             check(lib.q_add_rmsnorm(x, _p(pf["reduced"]), None, _p(gain), x, normed, rows, H, eps, stream))
 
         for i, lt in enumerate(w.layers):
             layout = _lib.KVLayout(self.kpools[i].data_ptr(), self.vpools[i].data_ptr(), table, self.pages_per_seq, nkv)
             check(lib.q_gemm_prompt_qkv(normed, _p(lt.wqkv.tc()), _p(lt.q_gain), _p(lt.k_gain), _p(self.cos),
-                                        _p(self.sin), zero, q, C.byref(layout), nb, T, nq, H, eps, stream))
+                                        _p(self.sin), zero, q, C.byref(layout), nb, T, nq, H, eps, split, stream))
             check(lib.q_attention_prefill(q, C.byref(layout), zero, att, nb, T, nq, scale, stream))
             add_norm(att, lt.wo, nq * HEAD_DIM, lt.ln_post)
-            check(lib.q_gemm_prompt_swiglu(normed, _p(lt.wgu.tc()), act, rows, inter, H, stream))
+            check(lib.q_gemm_prompt_swiglu(normed, _p(lt.wgu.tc()), act, rows, inter, H, split, stream))
             add_norm(act, lt.wdown, inter, w.layers[i + 1].ln_in if i + 1 < len(w.layers) else w.ln_final)
 
     def _prefill_layers_few_rows(self, pf, nb: int, T: int, table: int, stream) -> None:

@@ -33,44 +33,56 @@ def stream():
 
 
 def P(t):
-    return C.c_void_p(t.data_ptr())
+    return None if t is None else C.c_void_p(t.data_ptr())
+
+
+@pytest.fixture(scope="module", params=["split", "whole"])
+def scratch(request, ops):
+    """Parts of tiles shared by several SM pairs, or (no scratch) whole tiles only."""
+    from starter_b200._lib import lib
+    if request.param == "whole":
+        return None
+    return torch.zeros(lib.q_gemm_prompt_scratch_bytes(), dtype=torch.uint8, device="cuda")
 
 
 # one row; rows around one CTA, one tile and a raster group of eight row tiles; columns of less than
-# a tile, narrow tiles (few row tiles) and wide ones; K of less than a 64-k step, odd and long
-SHAPES = [(256, 256, 512), (1, 32, 32), (128, 128, 64), (129, 160, 96), (257, 2560, 416), (700, 96, 1024),
-          (2103, 2560, 4096), (2305, 4896, 160)]
+# a tile; K of less than a 64-k step, odd and long. With scratch: one tile cut over many pairs, few
+# tiles over all pairs, one wave and a remainder, and shapes that stay whole.
+SHAPES = [(256, 256, 512), (1, 32, 32), (128, 128, 64), (129, 160, 96), (257, 2560, 416), (700, 96, 4096),
+          (1000, 2560, 9728), (2103, 2560, 4096), (2305, 4896, 160)]
 
 
 @pytest.mark.parametrize("M,N,K", SHAPES)
-def test_sums_and_residual(ops, M, N, K):
+def test_sums_and_residual(ops, scratch, M, N, K):
     """fp32 sums within the bar of the decode projections (rtol = atol = 2e-3), rows past M untouched;
     the residual form equals the two roundings of that sum bit for bit."""
     from starter_b200._lib import check, lib
     x, w, res = rand((M, K), 1, 1.0), rand((N, K), 2, 0.02), rand((M, N), 3, 1.0)
     xd, tiled = x.cuda(), ops.pack_weight_tc(w.cuda())
     out = torch.full((M + 3, N), float("nan"), dtype=torch.float32, device="cuda")
-    check(lib.q_gemm_prompt_f32(P(xd), P(tiled.data), P(out), M, N, K, stream()))
+    check(lib.q_gemm_prompt_f32(P(xd), P(tiled.data), P(out), M, N, K, P(scratch), stream()))
     total = torch.full((M + 3, N), float("nan"), dtype=torch.bfloat16, device="cuda")
     total[:M] = res.cuda()
-    check(lib.q_gemm_prompt_add(P(xd), P(tiled.data), P(total), M, N, K, stream()))
+    check(lib.q_gemm_prompt_add(P(xd), P(tiled.data), P(total), M, N, K, P(scratch), stream()))
     got = out.cpu()
     torch.testing.assert_close(got[:M], O.linear_fp32(x, w), rtol=2e-3, atol=2e-3)
     assert torch.isnan(got[M:]).all() and torch.isnan(total[M:].float()).all()
     want = (res.float() + got[:M].to(torch.bfloat16).float()).to(torch.bfloat16)
     assert torch.equal(total[:M].cpu(), want)
+    if scratch is not None:
+        assert not scratch[:8192].any()                       # every ticket is back to zero
     assert ops.device_status() == [0, 0, 0, 0]
 
 
-@pytest.mark.parametrize("M,inter,K", [(1, 32, 32), (300, 96, 128), (257, 1184, 416), (600, 9728, 256)])
-def test_swiglu(ops, M, inter, K):
+@pytest.mark.parametrize("M,inter,K", [(1, 32, 32), (300, 96, 128), (257, 1184, 416), (600, 9728, 256), (900, 1312, 2560)])
+def test_swiglu(ops, scratch, M, inter, K):
     """Within one bf16 rounding of the oracle's SwiGLU of the fp32 sums (inter not a multiple of 128
     puts the up rows across the 128-row weight blocks)."""
     from starter_b200._lib import check, lib
     x, w = rand((M, K), 4, 1.0), rand((2 * inter, K), 5, 0.05)
     xd, tiled = x.cuda(), ops.pack_weight_tc(w.cuda())
     act = torch.full((M + 2, inter), float("nan"), dtype=torch.bfloat16, device="cuda")
-    check(lib.q_gemm_prompt_swiglu(P(xd), P(tiled.data), P(act), M, inter, K, stream()))
+    check(lib.q_gemm_prompt_swiglu(P(xd), P(tiled.data), P(act), M, inter, K, P(scratch), stream()))
     ref = O.swiglu(O.linear_fp32(x, w))
     torch.testing.assert_close(act[:M].cpu().float(), ref.float(), rtol=0.02, atol=2e-3)
     assert bit_equal_fraction(act[:M].cpu(), ref) > 0.98
@@ -78,12 +90,12 @@ def test_swiglu(ops, M, inter, K):
     assert ops.device_status() == [0, 0, 0, 0]
 
 
-@pytest.mark.parametrize("B,T,nq,nkv,pos", [(1, 1, 1, 1, 0), (2, 130, 4, 2, 70), (3, 301, 8, 1, 0), (1, 1000, 32, 8, 5)])
-def test_qkv_norm_rope_pages(ops, B, T, nq, nkv, pos):
+@pytest.mark.parametrize("B,T,nq,nkv,pos", [(1, 1, 1, 1, 0), (2, 130, 4, 2, 70), (3, 301, 8, 1, 0), (1, 1000, 32, 8, 5), (1, 2000, 32, 8, 0)])
+def test_qkv_norm_rope_pages(ops, scratch, B, T, nq, nkv, pos):
     """q, k within the bar of the separate kernel, v exact; only the slots of this block are written
     in the NaN-poisoned pages."""
     from starter_b200._lib import check, lib
-    width, K, rows = (nq + 2 * nkv) * 128, 128, B * T
+    width, K, rows = (nq + 2 * nkv) * 128, 2560 if T == 2000 else 128, B * T
     w, x = rand((width, K), 6, 0.02), rand((rows, K), 7, 4.0)
     qg, kg = gain(128, 8), gain(128, 9)
     capacity = pos + T + 70
@@ -94,9 +106,9 @@ def test_qkv_norm_rope_pages(ops, B, T, nq, nkv, pos):
     q = torch.full((rows + 1, nq, 128), float("nan"), dtype=torch.bfloat16, device="cuda")
     dev = [t.cuda() for t in (qg, kg, cos, sin)]
     check(lib.q_gemm_prompt_qkv(P(xd), P(tiled.data), P(dev[0]), P(dev[1]), P(dev[2]), P(dev[3]), P(position), P(q),
-                                C.byref(cache.layout), B, T, nq, K, 1e-6, stream()))
+                                C.byref(cache.layout), B, T, nq, K, 1e-6, P(scratch), stream()))
     sums = torch.empty((rows, width), dtype=torch.float32, device="cuda")
-    check(lib.q_gemm_prompt_f32(P(xd), P(tiled.data), P(sums), rows, width, K, stream()))
+    check(lib.q_gemm_prompt_f32(P(xd), P(tiled.data), P(sums), rows, width, K, P(scratch), stream()))
     at = (pos + torch.arange(T)).repeat(B)
     eq, ek, ev = O.qkv_norm_rope(sums.cpu(), qg, kg, 1e-6, cos[at], sin[at], nq, nkv)
     got = q.cpu()
