@@ -20,8 +20,11 @@
 //               [row][head][128], k and v rows into their pages
 // The rounding points are those of the consumers in fused_ops.cu.
 //
-// Roles per CTA (192 threads): warp 0 producer (one lane), warp 1 MMA issuer (the leader's one
-// lane), warps 2-5 epilogue, which drains one of two accumulators while the MMAs fill the other.
+// Roles per CTA (320 threads): warp 0 producer (one lane), warp 1 MMA issuer (the leader's one
+// lane), warps 2-9 epilogue, which drain one of two accumulators while the MMAs fill the other: two
+// warps per 32 rows, each for two runs of 64 columns (four warps took as long for head norm + RoPE
+// as the MMAs for a tile with K = 2560). What the epilogue reads besides the accumulator is
+// requested before it waits for it, or one step ahead.
 // The `full` barriers live in the leader: both CTAs' copies complete there (a stage is 2 x its
 // bytes); commits release stages and hand over accumulators in both CTAs at once. Every wait is
 // bounded as in gemm_tc.cu and reports in the same status word (codes 5-8).
@@ -33,14 +36,15 @@
 // up with a part of a tile stores its fp32 accumulator in the caller's scratch, draws a ticket, and
 // the LAST of a tile's pairs adds the parts in k order (its own included, so the sum does not depend
 // on who is last), puts the total back into tensor memory and runs the epilogue. Nobody waits. The
-// unit of all this is a warp: 32 rows of one CTA.
+// unit of all this is a warp: 32 rows x 2 x 64 columns.
 #include "tc.cuh"
 
 int* q_tc_status_addr();
 
 namespace {
 
-constexpr int PG_THREADS = 192;
+constexpr int PG_THREADS = 320;
+constexpr int PG_EPI_WARPS = 8;
 constexpr int PG_TILE_K = 64;
 constexpr int PG_A_BYTES = 128 * PG_TILE_K * 2;            // 16 KB of activations per CTA and stage
 constexpr int PG_BN = 256, PG_HALF = 128;                  // columns of a tile, weight rows per CTA
@@ -50,8 +54,8 @@ constexpr size_t PG_SMEM = 1024 + PG_STAGES * PG_STAGE + (2 * PG_STAGES + 4) * 8
 constexpr int PG_GROUP = 8;                                // row tiles per raster group
 constexpr int PG_MAX_PAIRS = 128;
 constexpr int PG_SPLIT_STEPS = 20;
-// scratch: tickets (8 warps per tile, at most two tiles per pair), then two parts per pair
-constexpr size_t PG_TICKET_BYTES = PG_MAX_PAIRS * 2 * 8 * 4;
+// scratch: tickets (16 warps per tile, at most two tiles per pair), then two parts per pair
+constexpr size_t PG_TICKET_BYTES = PG_MAX_PAIRS * 2 * 16 * 4;
 constexpr size_t PG_PART_FLOATS = 256 * 256;
 
 enum { EPI_F32 = 0, EPI_RESID = 1, EPI_SWIGLU = 2, EPI_ROPE = 3 };
@@ -63,6 +67,11 @@ struct PromptShape {
   int waves;            // tiles that each pair takes whole
   int share;            // k steps of the remaining tiles per pair: whole tiles, or an even split
 };
+
+// First row of the 128 that a CTA loads for rows [row0, row0 + 128): the last block is moved up so
+// that it holds no rows past M (copies that fill in zeros are slow), and a block that has no rows at
+// all loads some others; neither computes anything twice that is stored.
+__device__ __forceinline__ int first_row(int row0, int M) { return row0 >= M ? 0 : max(0, min(row0, M - 128)); }
 
 // The pieces of a pair in order: (tile, k steps [k0, k1)).
 struct Walk {
@@ -175,7 +184,7 @@ __device__ __forceinline__ void tc_st16x2(uint32_t a, uint32_t b, const float (&
 __device__ __forceinline__ void ld32B(const void* p, uint32_t (&r)[8]) {
   asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "l"(p) : "memory");
+               : "l"(p));
 }
 __device__ __forceinline__ void st32B(void* p, const uint32_t (&r)[8]) {
   asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
@@ -208,13 +217,24 @@ __device__ __forceinline__ void st_page16(char* row, int r, int d, const float (
   st32B(row + (((d >> 3) ^ (r & 6)) << 4), b);
 }
 
-// One 128-column head of one row: `taddr` is the head's first column in tensor memory.
+// Rotary rows of 16 dims and of their partners 64 on.
+struct RotRow { uint32_t c0[8], c1[8], s0[8], s1[8]; };
+__device__ __forceinline__ void ld_rot(RotRow& r, const bf16* cs, const bf16* sn) {
+  ld32B(cs, r.c0);
+  ld32B(cs + 64, r.c1);
+  ld32B(sn, r.s0);
+  ld32B(sn + 64, r.s1);
+}
+
+// One 128-column head of one row: `taddr` is the head's first column in tensor memory, `rot` already
+// holds the rotary rows of dims 0..15 and 64..79.
 __device__ __forceinline__ void rope_head(uint32_t taddr, const RopeArgs& ra, bf16* Q, int m, bool live, int head,
-                                          int pos, char* krow, char* vrow, int r) {
+                                          RotRow& rot, const bf16* cs, const bf16* sn, char* krow, char* vrow, int r) {
   const bool is_q = head < ra.nq, is_v = head >= ra.nq + ra.nkv;     // warp-uniform
   const int kh = is_v ? head - ra.nq - ra.nkv : head - ra.nq;
   const size_t hoff = is_q ? 0 : (size_t)kh * (Q_PAGE_TOKENS * 256);
   if (is_v) {
+#pragma unroll 1
     for (int d = 0; d < 64; d += 16) {
       float lo[16], hi[16];
       tc_ld16x2(taddr + d, taddr + 64 + d, lo, hi);
@@ -238,67 +258,70 @@ __device__ __forceinline__ void rope_head(uint32_t taddr, const RopeArgs& ra, bf
   }
   const float inv = rsqrtf(ss / 128.f + ra.eps);
   const bf16* gain = is_q ? ra.q_gain : ra.k_gain;
-  const bf16* cs = ra.cos + (size_t)pos * 128;
-  const bf16* sn = ra.sin + (size_t)pos * 128;
 #pragma unroll 1
   for (int d = 0; d < 64; d += 16) {
-    float lo[16], hi[16], g[16], c[16], s[16], o[16];
-    uint32_t w[8];
+    float lo[16], hi[16], g[16];
     tc_ld16x2(taddr + d, taddr + 64 + d, lo, hi);
+    const RotRow cur = rot;
+    if (d < 48) ld_rot(rot, cs + d + 16, sn + d + 16);
     ld_gain16(gain + d, g);
 #pragma unroll
     for (int e = 0; e < 16; ++e) lo[e] = bf16_round(bf16_round(bf16_round(lo[e]) * inv) * g[e]);
     ld_gain16(gain + 64 + d, g);
 #pragma unroll
     for (int e = 0; e < 16; ++e) hi[e] = bf16_round(bf16_round(bf16_round(hi[e]) * inv) * g[e]);
+    float o[16], p[16];                                      // rounded once more at the store
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      ld32B(cs + 64 * h + d, w);
-      unpack16(w, c);
-      ld32B(sn + 64 * h + d, w);
-      unpack16(w, s);
-#pragma unroll
-      for (int e = 0; e < 16; ++e)
-        o[e] = h == 0 ? bf16_round(lo[e] * c[e]) + bf16_round(-hi[e] * s[e])
-                      : bf16_round(hi[e] * c[e]) + bf16_round(lo[e] * s[e]);   // rounded at the store
-      if (live) {
-        if (is_q) {
-          pack16(o, w);
-          st32B(Q + ((size_t)m * ra.nq + head) * 128 + 64 * h + d, w);
-        } else {
-          st_page16(krow + hoff, r, 64 * h + d, o);
-        }
+    for (int e = 0; e < 16; ++e) {
+      const float c0 = e & 1 ? bf_hi(cur.c0[e >> 1]) : bf_lo(cur.c0[e >> 1]);
+      const float c1 = e & 1 ? bf_hi(cur.c1[e >> 1]) : bf_lo(cur.c1[e >> 1]);
+      const float s0 = e & 1 ? bf_hi(cur.s0[e >> 1]) : bf_lo(cur.s0[e >> 1]);
+      const float s1 = e & 1 ? bf_hi(cur.s1[e >> 1]) : bf_lo(cur.s1[e >> 1]);
+      o[e] = bf16_round(lo[e] * c0) + bf16_round(-hi[e] * s0);
+      p[e] = bf16_round(hi[e] * c1) + bf16_round(lo[e] * s1);
+    }
+    if (live) {
+      if (is_q) {
+        bf16* dst = Q + ((size_t)m * ra.nq + head) * 128 + d;
+        uint32_t w[8];
+        pack16(o, w);
+        st32B(dst, w);
+        pack16(p, w);
+        st32B(dst + 64, w);
+      } else {
+        st_page16(krow + hoff, r, d, o);
+        st_page16(krow + hoff, r, 64 + d, p);
       }
     }
   }
 }
 
-// A warp's part (32 rows x 256 columns at `taddr`) of tile `rel` of the split ones. True: this was
-// the tile's last part and tensor memory now holds the sum of all parts, added in k order.
-__device__ __forceinline__ bool merge_parts(const PromptShape& sh, unsigned char* scratch, uint32_t taddr, int pair,
-                                            int rel, int k0, int warp_of_tile, int lane) {
+// A warp's part (32 rows x 64 columns at `ta` and at `tb`) of tile `rel` of the split ones. True: this
+// was the tile's last part and tensor memory now holds the sum of all parts, added in k order.
+__device__ __forceinline__ bool merge_parts(const PromptShape& sh, unsigned char* scratch, uint32_t ta, uint32_t tb,
+                                            int pair, int rel, int warp_of_tile, int lane) {
   const int first = rel * sh.KT / sh.share, last = ((rel + 1) * sh.KT - 1) / sh.share;
-  int* ticket = reinterpret_cast<int*>(scratch) + rel * 8 + warp_of_tile;
+  int* ticket = reinterpret_cast<int*>(scratch) + rel * 16 + warp_of_tile;
   float* parts = reinterpret_cast<float*>(scratch + PG_TICKET_BYTES);
   // a pair has at most two parts: the rest of a tile it did not begin, the beginning of its last one;
-  // element (column 4 j + e, lane) of a warp's part sits at (j * 32 + lane) * 4 + e
+  // columns 4 j .. 4 j + 3 of run b of a lane are the float4 at ((b * 16 + j) * 32 + lane)
   auto part = [&](int p) {
     return reinterpret_cast<float4*>(parts + (size_t)(2 * p + (p * sh.share > rel * sh.KT ? 0 : 1)) * PG_PART_FLOATS +
-                                     warp_of_tile * (32 * 256)) + lane;
+                                     warp_of_tile * (32 * 128)) + lane;
   };
   int drawn = 0;
   if (lane == 0) drawn = *reinterpret_cast<volatile int*>(ticket);
   drawn = __shfl_sync(0xffffffffu, drawn, 0);
   if (drawn != last - first) {                    // not known to be the last one: leave the part in memory
     float4* dst = part(pair);
-#pragma unroll 1
-    for (int c = 0; c < 256; c += 32) {
+#pragma unroll
+    for (int c = 0; c < 64; c += 16) {
       float v[16], w[16];
-      tc_ld16x2(taddr + c, taddr + c + 16, v, w);
+      tc_ld16x2(ta + c, tb + c, v, w);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        dst[(c / 4 + j) * 32] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-        dst[(c / 4 + 4 + j) * 32] = make_float4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+        __stcg(dst + (c / 4 + j) * 32, make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
+        __stcg(dst + (16 + c / 4 + j) * 32, make_float4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]));
       }
     }
     __threadfence();
@@ -311,28 +334,38 @@ __device__ __forceinline__ bool merge_parts(const PromptShape& sh, unsigned char
   __threadfence();
   if (lane == 0) *ticket = 0;                     // ready for the next launch
 #pragma unroll 1
-  for (int c = 0; c < 256; c += 32) {
-    float v[16], w[16], own_v[16], own_w[16];
-    tc_ld16x2(taddr + c, taddr + c + 16, own_v, own_w);
+  for (int b = 0; b < 2; ++b) {
+    // 64 columns at a time: 16 loads of a part are in flight together
+    const uint32_t t = b ? tb : ta;
+    float v[4][16];
 #pragma unroll
-    for (int e = 0; e < 16; ++e) v[e] = w[e] = 0.f;
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int e = 0; e < 16; ++e) v[c][e] = 0.f;
+#pragma unroll 1
     for (int p = first; p <= last; ++p) {
       if (p == pair) {
 #pragma unroll
-        for (int e = 0; e < 16; ++e) { v[e] += own_v[e]; w[e] += own_w[e]; }
+        for (int c = 0; c < 4; c += 2) {
+          float x[16], y[16];
+          tc_ld16x2(t + 16 * c, t + 16 * c + 16, x, y);
+#pragma unroll
+          for (int e = 0; e < 16; ++e) { v[c][e] += x[e]; v[c + 1][e] += y[e]; }
+        }
         continue;
       }
-      const float4* src = part(p);
-      float4 a[8];
+      const float4* src = part(p) + b * (16 * 32);
+      float4 a[16];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) a[j] = __ldcg(src + (c / 4 + j) * 32);
+      for (int j = 0; j < 16; ++j) a[j] = __ldcg(src + j * 32);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        v[4 * j] += a[j].x; v[4 * j + 1] += a[j].y; v[4 * j + 2] += a[j].z; v[4 * j + 3] += a[j].w;
-        w[4 * j] += a[4 + j].x; w[4 * j + 1] += a[4 + j].y; w[4 * j + 2] += a[4 + j].z; w[4 * j + 3] += a[4 + j].w;
+      for (int j = 0; j < 16; ++j) {
+        float* d = v[j >> 2] + 4 * (j & 3);
+        d[0] += a[j].x; d[1] += a[j].y; d[2] += a[j].z; d[3] += a[j].w;
       }
     }
-    tc_st16x2(taddr + c, taddr + c + 16, v, w);
+    tc_st16x2(t, t + 16, v[0], v[1]);
+    tc_st16x2(t + 32, t + 48, v[2], v[3]);
   }
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
   return true;
@@ -367,7 +400,7 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(bar_acc_full + 8 * b, 1);
-      mbar_init(bar_acc_empty + 8 * b, 8);                  // four epilogue warps of each CTA
+      mbar_init(bar_acc_empty + 8 * b, 2 * PG_EPI_WARPS);   // of both CTAs
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -409,8 +442,7 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
       while (ok && walk.next(sh, pair, pairs, t, k0, k1)) {
         int mi, ni;
         locate(t, mi, ni);
-        // (rows that do not exist are not worth a copy of zeros, which is slow: any rows will do)
-        const int row0 = mi * 256 + (int)rank * 128, row = row0 < sh.M ? row0 : 0;
+        const int row = first_row(mi * 256 + (int)rank * 128, sh.M);
         // first weight row of this CTA's half
         const int n0 = EPI == EPI_SWIGLU ? (int)rank * sh.N + ni * PG_HALF : ni * PG_BN + (int)rank * PG_HALF;
         for (int kt = k0; kt < k1; ++kt) {
@@ -480,9 +512,11 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
       }
     }
   } else {
-    // ---------------- epilogue (warps 2..5) ----------------
+    // ---------------- epilogue (warps 2..9) ----------------
     pdl_wait();
-    const int q = warp & 3;
+    const int q = warp & 3, h = (warp - 2) >> 2;
+    // the warp's two runs of 64 columns: gate and up columns that belong together, or one head
+    const int ca = EPI == EPI_SWIGLU ? 64 * h : 128 * h, cb = EPI == EPI_SWIGLU ? PG_HALF + 64 * h : ca + 64;
     const uint32_t acc_empty0 = leader_addr(bar_acc_empty);
     int seg = 0;
     Walk walk;
@@ -492,8 +526,34 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
       const int buf = seg & 1;
       int mi, ni;
       locate(t, mi, ni);
-      const int m = mi * 256 + (int)rank * 128 + q * 32 + lane;
-      const bool live = m < sh.M;
+      const int row0 = mi * 256 + (int)rank * 128;
+      const int m = first_row(row0, sh.M) + q * 32 + lane;
+      const bool live = m >= row0 && m < sh.M;
+      const int n0 = EPI == EPI_SWIGLU ? ni * PG_HALF + ca : ni * PG_BN + ca;      // output column of run a
+      // operands besides the accumulator: requested now, used after the wait
+      uint32_t res[EPI == EPI_RESID ? 8 : 1][8];
+      bf16* x = reinterpret_cast<bf16*>(out) + (size_t)(live ? m : 0) * sh.N + n0;
+      if (EPI == EPI_RESID) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (n0 + 16 * j < sh.N) ld32B(x + 16 * j, res[j]);
+      }
+      RotRow rot;
+      const bf16 *cs = nullptr, *sn = nullptr;
+      char *krow = nullptr, *vrow = nullptr;
+      int r = 0;
+      if (EPI == EPI_ROPE) {
+        const int mm = live ? m : 0;
+        const int b = mm / ra.T, pos = ra.pos[0] + mm - b * ra.T;
+        const int page = ra.block_table[(size_t)b * ra.pages_per_seq + pos / Q_PAGE_TOKENS];
+        r = pos % Q_PAGE_TOKENS;
+        const size_t row = (size_t)page * ra.nkv * (Q_PAGE_TOKENS * 256) + (size_t)r * 256;
+        krow = ra.kpool + row;
+        vrow = ra.vpool + row;
+        cs = ra.cos + (size_t)pos * 128;
+        sn = ra.sin + (size_t)pos * 128;
+        ld_rot(rot, cs, sn);
+      }
       const int landed = mbar_wait(bar_acc_full + 8 * buf, (seg >> 1) & 1, abort_flag) ? 1 : 0;
       if (!__all_sync(0xffffffffu, landed)) {
         if (lane == 0) {
@@ -504,74 +564,67 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
       }
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)buf * 256u;
-      if (k1 - k0 < sh.KT && !merge_parts(sh, scratch, taddr, pair, t - sh.waves * pairs, k0, (int)rank * 4 + q, lane)) {
-        // a part of a tile, and not the last one: another pair finishes the tile
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(acc_empty0 + 8 * buf);
-        continue;
-      }
-      if (EPI == EPI_F32) {
-        float* dst = reinterpret_cast<float*>(out) + (size_t)m * sh.N + ni * PG_BN;
-        for (int c = 0; c < PG_BN && ni * PG_BN + c < sh.N; c += 32) {   // N is a multiple of 32
-          float v[16], w[16];
-          tc_ld16x2(taddr + c, taddr + c + 16, v, w);
-          if (live) {
+      const uint32_t ta = taddr + ca, tb = taddr + cb;
+      // (a part of a tile that is not the last one: another pair finishes the tile)
+      const bool whole = k1 - k0 == sh.KT ||
+                         merge_parts(sh, scratch, ta, tb, pair, t - sh.waves * pairs, ((int)rank * 4 + q) * 2 + h, lane);
+      if (whole && n0 < sh.N) {
+        if (EPI == EPI_F32) {
+          float* dst = reinterpret_cast<float*>(out) + (size_t)m * sh.N + n0;
+#pragma unroll 2
+          for (int c = 0; c < 128 && n0 + c < sh.N; c += 32) {             // N is a multiple of 32
+            float v[16], w[16];
+            tc_ld16x2(ta + c, ta + c + 16, v, w);
+            if (live) {
 #pragma unroll
-            for (int j = 0; j < 16; j += 8) {
-              uint32_t a[8], b[8];
+              for (int j = 0; j < 16; j += 8) {
+                uint32_t a[8], b[8];
 #pragma unroll
-              for (int e = 0; e < 8; ++e) { a[e] = __float_as_uint(v[j + e]); b[e] = __float_as_uint(w[j + e]); }
-              st32B(dst + c + j, a);
-              st32B(dst + c + 16 + j, b);
+                for (int e = 0; e < 8; ++e) { a[e] = __float_as_uint(v[j + e]); b[e] = __float_as_uint(w[j + e]); }
+                st32B(dst + c + j, a);
+                st32B(dst + c + 16 + j, b);
+              }
             }
           }
-        }
-      } else if (EPI == EPI_RESID) {
-        bf16* x = reinterpret_cast<bf16*>(out) + (size_t)(live ? m : 0) * sh.N + ni * PG_BN;
-#pragma unroll 2
-        for (int c = 0; c < PG_BN && ni * PG_BN + c < sh.N; c += 32) {
-          float v[16], w[16], a[16];
-          uint32_t r0[8], r1[8];
-          ld32B(x + c, r0);
-          ld32B(x + c + 16, r1);
-          tc_ld16x2(taddr + c, taddr + c + 16, v, w);
-          unpack16(r0, a);
+        } else if (EPI == EPI_RESID) {
 #pragma unroll
-          for (int e = 0; e < 16; ++e) v[e] = a[e] + bf16_round(v[e]);
-          unpack16(r1, a);
+          for (int j = 0; j < 8; j += 2) {
+            if (n0 + 16 * j < sh.N) {
+              float v[16], w[16], a[16];
+              tc_ld16x2(ta + 16 * j, ta + 16 * j + 16, v, w);
+              unpack16(res[j], a);
 #pragma unroll
-          for (int e = 0; e < 16; ++e) w[e] = a[e] + bf16_round(w[e]);
-          pack16(v, r0);
-          pack16(w, r1);
-          if (live) {
-            st32B(x + c, r0);
-            st32B(x + c + 16, r1);
+              for (int e = 0; e < 16; ++e) v[e] = a[e] + bf16_round(v[e]);
+              unpack16(res[j + 1], a);
+#pragma unroll
+              for (int e = 0; e < 16; ++e) w[e] = a[e] + bf16_round(w[e]);
+              uint32_t o0[8], o1[8];
+              pack16(v, o0);
+              pack16(w, o1);
+              if (live) {
+                st32B(x + 16 * j, o0);
+                st32B(x + 16 * j + 16, o1);
+              }
+            }
           }
-        }
-      } else if (EPI == EPI_SWIGLU) {
-        bf16* act = reinterpret_cast<bf16*>(out) + (size_t)m * sh.N + ni * PG_HALF;
-        for (int c = 0; c < PG_HALF && ni * PG_HALF + c < sh.N; c += 16) {     // inter is a multiple of 16
-          float g[16], u[16];
-          uint32_t r[8];
-          tc_ld16x2(taddr + c, taddr + PG_HALF + c, g, u);
+        } else if (EPI == EPI_SWIGLU) {
+          bf16* act = reinterpret_cast<bf16*>(out) + (size_t)m * sh.N + n0;
+#pragma unroll 1
+          for (int c = 0; c < 64 && n0 + c < sh.N; c += 16) {              // inter is a multiple of 16
+            float g[16], u[16];
+            uint32_t w[8];
+            tc_ld16x2(ta + c, tb + c, g, u);
 #pragma unroll
-          for (int e = 0; e < 16; ++e) {
-            const float gb = bf16_round(g[e]);
-            g[e] = bf16_round(gb / (1.0f + expf(-gb))) * bf16_round(u[e]);
+            for (int e = 0; e < 16; ++e) {
+              const float gb = bf16_round(g[e]);
+              g[e] = bf16_round(gb / (1.0f + expf(-gb))) * bf16_round(u[e]);
+            }
+            pack16(g, w);
+            if (live) st32B(act + c, w);
           }
-          pack16(g, r);
-          if (live) st32B(act + c, r);
+        } else {
+          rope_head(ta, ra, reinterpret_cast<bf16*>(out), m, live, n0 >> 7, rot, cs, sn, krow, vrow, r);
         }
-      } else {
-        const int mm = live ? m : 0;
-        const int b = mm / ra.T, pos = ra.pos[0] + mm - b * ra.T;
-        const int page = ra.block_table[(size_t)b * ra.pages_per_seq + pos / Q_PAGE_TOKENS];
-        const int r = pos % Q_PAGE_TOKENS;
-        const size_t row = (size_t)page * ra.nkv * (Q_PAGE_TOKENS * 256) + (size_t)r * 256;
-        for (int c = 0; c < PG_BN && ni * PG_BN + c < sh.N; c += 128)
-          rope_head(taddr + c, ra, reinterpret_cast<bf16*>(out), m, live, (ni * PG_BN + c) >> 7, pos, ra.kpool + row,
-                    ra.vpool + row, r);
       }
       tc_fence_before();
       __syncwarp();
