@@ -14,7 +14,9 @@
 // products under the current one's last softmax, since an item is only ~9 tiles long at 1-2 K keys.
 //
 // Warps 0-3 / 4-7: softmax and epilogue of query tile 0 / 1 (a thread owns a row: no shuffles).
-// Warp 8: producer lane. Warp 9: MMA lane.
+// Warp 8: producer lane. Warp 9: MMA issue; the whole warp walks the loop and one elected lane
+// issues, so that descriptors live in uniform registers: an MMA of 128 x 128 x 16 takes 64 cycles,
+// about what a single diverged lane needs to assemble its operands.
 // The running maximum is only moved (and O rescaled) when a row's maximum grew by more than 2^8:
 // the scale of P and of the row sum is free, so results keep their precision, and most tiles skip
 // the pass over O. Cast boundaries as in attention.cu: fp32 scores and statistics, P rounded to
@@ -121,6 +123,15 @@ __device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t* r) {
       : "memory");
 }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -217,7 +228,8 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
     }
   } else if (warp == 9) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    {
+      const bool leader = elect_one();
       const uint32_t f16 = (1u << 4) | (1u << 7) | (1u << 10) | (16u << 17) | (8u << 24);   // 128 x 128, fp32 sums
       const uint32_t idesc_s = f16, idesc_pv = f16 | (1u << 16);      // V: the non-contracted dimension is contiguous
       const uint64_t q_desc = smem_desc(base + AP_Q), k_desc = smem_desc(base + AP_K);
@@ -227,12 +239,17 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
       uint32_t kstep = 0, vstep = 0, nitems = 0;
       bool ok = true;
       auto wait = [&](uint32_t b, uint32_t parity) {
-        if (ok && !mbar_wait(b, parity, abort_flag)) { atomicExch(status, 8); *abort_flag = 1; ok = false; }
+        const int landed = mbar_wait(b, parity, abort_flag) ? 1 : 0;
+        if (!__all_sync(0xffffffffu, landed)) {
+          if (leader) { atomicExch(status, 8); *abort_flag = 1; }
+          ok = false;
+        }
         tc_fence_after();
         return ok;
       };
       auto scores = [&](int i) {                           // S_i = Q_i K^T of the K tile at kstep
         const uint64_t a = q_desc + (uint64_t)(i * (AP_TILE >> 4)), b = k_desc + (uint64_t)((kstep & 1) * (AP_TILE >> 4));
+        if (!leader) return;
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
           const uint32_t off = (uint32_t)(ks >> 2) * (AP_HALF >> 4) + (ks & 3) * 2;
@@ -245,9 +262,13 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
       for (int i = 0; i < 2 && ok; ++i) {
         if (!wait(bar(B_QF, i), 0) || (i == 0 && !wait(bar(B_KF, 0), 0))) break;
         scores(i);
-        if (cur.n == 1) tc_commit(bar(B_QE, i));
+        if (leader && cur.n == 1) tc_commit(bar(B_QE, i));
+        __syncwarp();
       }
-      if (ok) { tc_commit(bar(B_KE, 0)); ++kstep; }
+      if (ok) {
+        if (leader) tc_commit(bar(B_KE, 0));
+        ++kstep;
+      }
       while (ok) {
         // the item after this one
         bool more = false;
@@ -264,26 +285,34 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
             if (j == 0 && !wait(bar(B_OE, i), (nitems & 1) ^ 1)) break;
             for (int h = 0; h < 2; ++h) {                  // P comes in two halves of 64 keys
               if (!wait(bar(B_P, 2 * i + h), vstep & 1)) break;
+              if (leader) {
 #pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                const int ks = 4 * h + k;
-                tc_mma_ta(tmem + 256u + 128u * i, tmem + 128u * i + 8u * ks,
-                          v_desc + (uint64_t)(vs * (AP_TILE >> 4) + ks * (2048 >> 4)), idesc_pv, (j | ks) ? 1u : 0u);
+                for (int k = 0; k < 4; ++k) {
+                  const int ks = 4 * h + k;
+                  tc_mma_ta(tmem + 256u + 128u * i, tmem + 128u * i + 8u * ks,
+                            v_desc + (uint64_t)(vs * (AP_TILE >> 4) + ks * (2048 >> 4)), idesc_pv, (j | ks) ? 1u : 0u);
+                }
               }
+              __syncwarp();
             }
             if (!ok) break;
-            if (last) tc_commit(bar(B_OF, i));
+            if (last && leader) tc_commit(bar(B_OF, i));
             if (ahead) {
               if (i == 0 && !wait(bar(B_KF, kstep & 1), (kstep >> 1) & 1)) break;
               if (last && !wait(bar(B_QF, i), (nitems + 1) & 1)) break;
               scores(i);
-              if (last ? nxt.n == 1 : j + 2 == cur.n) tc_commit(bar(B_QE, i));
+              if (leader && (last ? nxt.n == 1 : j + 2 == cur.n)) tc_commit(bar(B_QE, i));
+              __syncwarp();
             }
           }
           if (!ok) break;
-          tc_commit(bar(B_VE, vs));
+          if (leader) {
+            tc_commit(bar(B_VE, vs));
+            if (ahead) tc_commit(bar(B_KE, kstep & 1));
+          }
+          __syncwarp();
           ++vstep;
-          if (ahead) { tc_commit(bar(B_KE, kstep & 1)); ++kstep; }
+          if (ahead) ++kstep;
         }
         ++nitems;
         if (!more) break;

@@ -200,17 +200,19 @@ __device__ __forceinline__ void unpack16(const uint32_t (&r)[8], float (&v)[16])
   for (int i = 0; i < 8; ++i) { v[2 * i] = bf_lo(r[i]); v[2 * i + 1] = bf_hi(r[i]); }
 }
 // 16 gains, the same for all lanes
-__device__ __forceinline__ void ld_gain16(const bf16* p, float (&v)[16]) {
+__device__ __forceinline__ void ld_gain16(const bf16* p, uint32_t (&r)[8]) {
   const uint4 a = __ldg(reinterpret_cast<const uint4*>(p)), b = __ldg(reinterpret_cast<const uint4*>(p) + 1);
-  const uint32_t r[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-  unpack16(r, v);
+  r[0] = a.x; r[1] = a.y; r[2] = a.z; r[3] = a.w; r[4] = b.x; r[5] = b.y; r[6] = b.z; r[7] = b.w;
+}
+__device__ __forceinline__ uint32_t mul2(uint32_t a, uint32_t b) {
+  const __nv_bfloat162 p = __hmul2_rn(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<__nv_bfloat162*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&p);
 }
 
 // k / v row of a page: the 32 bytes of dims d..d+15 (d a multiple of 16) are one aligned pair of
 // 16-byte chunks whose order depends on the token's parity (chunk index XOR-ed with r & 7).
-__device__ __forceinline__ void st_page16(char* row, int r, int d, const float (&v)[16]) {
-  uint32_t a[8], b[8];
-  pack16(v, a);
+__device__ __forceinline__ void st_page16(char* row, int r, int d, const uint32_t (&a)[8]) {
+  uint32_t b[8];
   const bool swap = r & 1;
 #pragma unroll
   for (int i = 0; i < 4; ++i) { b[i] = swap ? a[i + 4] : a[i]; b[i + 4] = swap ? a[i] : a[i + 4]; }
@@ -238,56 +240,55 @@ __device__ __forceinline__ void rope_head(uint32_t taddr, const RopeArgs& ra, bf
     for (int d = 0; d < 64; d += 16) {
       float lo[16], hi[16];
       tc_ld16x2(taddr + d, taddr + 64 + d, lo, hi);
+      uint32_t a[8], b[8];
+      pack16(lo, a);
+      pack16(hi, b);
       if (live) {
-        st_page16(vrow + hoff, r, d, lo);
-        st_page16(vrow + hoff, r, 64 + d, hi);
+        st_page16(vrow + hoff, r, d, a);
+        st_page16(vrow + hoff, r, 64 + d, b);
       }
     }
     return;
   }
+  // The head as bf16 pairs: one pass over tensor memory. The products below are of two bf16 values
+  // and rounded to bf16, which the packed multiply does in one instruction.
+  uint32_t xl[4][8], xh[4][8];
   float ss = 0.f;
-#pragma unroll 1
-  for (int d = 0; d < 64; d += 16) {
-    float lo[16], hi[16];
-    tc_ld16x2(taddr + d, taddr + 64 + d, lo, hi);
 #pragma unroll
-    for (int e = 0; e < 16; ++e) {
-      const float a = bf16_round(lo[e]), b = bf16_round(hi[e]);
-      ss += a * a + b * b;
+  for (int i = 0; i < 4; ++i) {
+    float lo[16], hi[16];
+    tc_ld16x2(taddr + 16 * i, taddr + 64 + 16 * i, lo, hi);
+    pack16(lo, xl[i]);
+    pack16(hi, xh[i]);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      ss += bf_lo(xl[i][e]) * bf_lo(xl[i][e]) + bf_hi(xl[i][e]) * bf_hi(xl[i][e]);
+      ss += bf_lo(xh[i][e]) * bf_lo(xh[i][e]) + bf_hi(xh[i][e]) * bf_hi(xh[i][e]);
     }
   }
   const float inv = rsqrtf(ss / 128.f + ra.eps);
   const bf16* gain = is_q ? ra.q_gain : ra.k_gain;
-#pragma unroll 1
-  for (int d = 0; d < 64; d += 16) {
-    float lo[16], hi[16], g[16];
-    tc_ld16x2(taddr + d, taddr + 64 + d, lo, hi);
-    const RotRow cur = rot;
-    if (d < 48) ld_rot(rot, cs + d + 16, sn + d + 16);
-    ld_gain16(gain + d, g);
 #pragma unroll
-    for (int e = 0; e < 16; ++e) lo[e] = bf16_round(bf16_round(bf16_round(lo[e]) * inv) * g[e]);
-    ld_gain16(gain + 64 + d, g);
+  for (int i = 0; i < 4; ++i) {
+    const int d = 16 * i;
+    uint32_t g0[8], g1[8], o[8], p[8];
+    ld_gain16(gain + d, g0);
+    ld_gain16(gain + 64 + d, g1);
 #pragma unroll
-    for (int e = 0; e < 16; ++e) hi[e] = bf16_round(bf16_round(bf16_round(hi[e]) * inv) * g[e]);
-    float o[16], p[16];                                      // rounded once more at the store
-#pragma unroll
-    for (int e = 0; e < 16; ++e) {
-      const float c0 = e & 1 ? bf_hi(cur.c0[e >> 1]) : bf_lo(cur.c0[e >> 1]);
-      const float c1 = e & 1 ? bf_hi(cur.c1[e >> 1]) : bf_lo(cur.c1[e >> 1]);
-      const float s0 = e & 1 ? bf_hi(cur.s0[e >> 1]) : bf_lo(cur.s0[e >> 1]);
-      const float s1 = e & 1 ? bf_hi(cur.s1[e >> 1]) : bf_lo(cur.s1[e >> 1]);
-      o[e] = bf16_round(lo[e] * c0) + bf16_round(-hi[e] * s0);
-      p[e] = bf16_round(hi[e] * c1) + bf16_round(lo[e] * s1);
+    for (int e = 0; e < 8; ++e) {
+      const uint32_t lo = mul2(pack_bf16(bf_lo(xl[i][e]) * inv, bf_hi(xl[i][e]) * inv), g0[e]);
+      const uint32_t hi = mul2(pack_bf16(bf_lo(xh[i][e]) * inv, bf_hi(xh[i][e]) * inv), g1[e]);
+      const uint32_t a = mul2(lo, rot.c0[e]), b = mul2(hi, rot.s0[e]);
+      const uint32_t c = mul2(hi, rot.c1[e]), f = mul2(lo, rot.s1[e]);
+      o[e] = pack_bf16(bf_lo(a) - bf_lo(b), bf_hi(a) - bf_hi(b));
+      p[e] = pack_bf16(bf_lo(c) + bf_lo(f), bf_hi(c) + bf_hi(f));
     }
+    if (i < 3) ld_rot(rot, cs + d + 16, sn + d + 16);
     if (live) {
       if (is_q) {
         bf16* dst = Q + ((size_t)m * ra.nq + head) * 128 + d;
-        uint32_t w[8];
-        pack16(o, w);
-        st32B(dst, w);
-        pack16(p, w);
-        st32B(dst + 64, w);
+        st32B(dst, o);
+        st32B(dst + 64, p);
       } else {
         st_page16(krow + hoff, r, d, o);
         st_page16(krow + hoff, r, 64 + d, p);
