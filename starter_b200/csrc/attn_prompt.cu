@@ -132,6 +132,30 @@ __device__ __forceinline__ bool elect_one() {
       : "=r"(p));
   return p != 0;
 }
+// Two fp32 lanes per instruction, each rounded like the scalar one; and the largest of three.
+__device__ __forceinline__ unsigned long long pair2(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpair2(unsigned long long r, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r));
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -383,11 +407,10 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
         }
         float mx[4] = {v[0], v[1], v[2], v[3]};
 #pragma unroll
-        for (int k = 4; k < 128; k += 4) {
-          mx[0] = fmaxf(mx[0], v[k]); mx[1] = fmaxf(mx[1], v[k + 1]);
-          mx[2] = fmaxf(mx[2], v[k + 2]); mx[3] = fmaxf(mx[3], v[k + 3]);
-        }
-        const float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+        for (int k = 4; k < 124; k += 8)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) mx[e] = max3(mx[e], v[k + e], v[k + 4 + e]);
+        const float m_tile = max3(max3(mx[0], mx[1], mx[2]), mx[3], fmaxf(max3(v[124], v[125], v[126]), v[127]));
         if (j == 0) {
           m = m_tile;
         } else {
@@ -413,15 +436,18 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
           }
         }
         const float mc = m == -INFINITY ? 0.f : m * c;
-        float sum[4] = {0.f, 0.f, 0.f, 0.f};
+        const unsigned long long c2 = pair2(c, c), mc2 = pair2(-mc, -mc);
+        unsigned long long sum[2] = {0ull, 0ull};
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           uint32_t p[32];
 #pragma unroll
           for (int k = 0; k < 32; ++k) {
-            const float a = ex2(fmaf(v[64 * h + 2 * k], c, -mc)), b = ex2(fmaf(v[64 * h + 2 * k + 1], c, -mc));
-            sum[(2 * k) & 3] += a;
-            sum[(2 * k + 1) & 3] += b;
+            float a, b;
+            unpair2(fma2(pair2(v[64 * h + 2 * k], v[64 * h + 2 * k + 1]), c2, mc2), a, b);
+            a = ex2(a);
+            b = ex2(b);
+            sum[k & 1] = add2(sum[k & 1], pair2(a, b));
             p[k] = pack_bf16(a, b);
           }
           tc_st32(s_addr + 32 * h, p);
@@ -431,7 +457,9 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
           if (lane == 0) mbar_arrive(bar(B_P, 2 * i + h));
           __syncwarp();
         }
-        l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+        float s_lo, s_hi;
+        unpair2(add2(sum[0], sum[1]), s_lo, s_hi);
+        l += s_lo + s_hi;
       }
       if (!ok || !wait(bar(B_OF, i), nitems & 1)) break;
       const float inv = l > 0.f ? 1.f / l : (l == 0.f ? 0.f : l);      // NaN stays NaN
