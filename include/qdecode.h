@@ -385,6 +385,33 @@ typedef struct q_layer_weights_t {
   const void* wdown_tc;
 } q_layer_weights_t;
 
+/* The prompt pass of one GPU in one call (engine/prefill.py:26-62): batch * T prompt tokens through
+ * all layers, K and V rows of positions *pos .. *pos+T-1 into the pages, the final norm of every
+ * sequence's last position into d_last [batch][hidden]. From few_rows rows on the projections are
+ * q_gemm_prompt_*, below that q_gemm_tc and its consumers (partials: enough for every plan of up to
+ * few_rows - 1 rows). x, normed [rows][hidden], q, attended [rows][n_q*128], act [rows][inter] are
+ * scratch of the caller (32-byte aligned), split as in q_gemm_prompt_* (cleared by every call).
+ * layers: wqkv_tc .. wdown_tc, gains and pools are read; only enqueues on `stream`. */
+typedef struct q_prompt_t {
+  int32_t hidden, inter, n_layers, n_q_heads, n_kv_heads, vocab, few_rows;
+  float rms_eps, attn_scale;
+  const void* embed;       /* tiled like q_embed_rmsnorm's */
+  const void* ln_final;
+  const void* cos;
+  const void* sin;
+  const int32_t* pos;
+  void* x;
+  void* normed;
+  void* q;
+  void* attended;
+  void* act;
+  float* partials;
+  void* split;
+} q_prompt_t;
+int q_prompt_pass(const q_prompt_t* p, const q_layer_weights_t* layers, const int64_t* d_tokens,
+                  const int32_t* d_block_table, int pages_per_seq, int batch, int T, void* d_last,
+                  void* stream);
+
 typedef struct q_state_t {
   const void* embed;        /* [full_vocab][hidden], tiled layout */
   const void* lm_head;      /* [vocab][hidden] tiled (local shard; == embed when tied, tp 1) */

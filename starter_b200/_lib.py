@@ -71,6 +71,13 @@ class State(C.Structure):
     ]
 
 
+class Prompt(C.Structure):
+    _fields_ = ([(n, C.c_int32) for n in ("hidden", "inter", "n_layers", "n_q_heads", "n_kv_heads", "vocab", "few_rows")]
+                + [(n, C.c_float) for n in ("rms_eps", "attn_scale")]
+                + [(n, C.c_void_p) for n in ("embed", "ln_final", "cos", "sin", "pos", "x", "normed", "q", "attended",
+                                             "act", "partials", "split")])
+
+
 _P = C.c_void_p
 _I = C.c_int
 _F = C.c_float
@@ -107,6 +114,7 @@ SIGNATURES = {
     "q_gemm_prompt_add": (_I, [_P, _P, _P, _I, _I, _I, _P, _P]),
     "q_gemm_prompt_swiglu": (_I, [_P, _P, _P, _I, _I, _I, _P, _P]),
     "q_gemm_prompt_qkv": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _KV, _I, _I, _I, _I, _F, _P, _P]),
+    "q_prompt_pass": (_I, [C.POINTER(Prompt), C.POINTER(LayerWeights), _P, _P, _I, _I, _I, _P, _P]),
     "q_peer_flag_bytes": (C.c_int64, []),
     "q_argmax_merge_peers": (_I, [_P, _P, C.POINTER(Peers), _I, _P, _P, _I, _P]),
     "q_step_merge": (_I, [_P, _P, _P, _P]),

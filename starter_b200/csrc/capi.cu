@@ -643,3 +643,72 @@ extern "C" int q_verify_step(q_engine* e, void* stream) {
   Q_CHECK_ARG(e->cfg.tp_size == 1, "q_verify_step: single GPU only");
   return run_layers(e, false, stream);
 }
+
+// The prompt pass: the same launches as the steps above, seven a layer (eight on split-K partials),
+// enqueued from here because a host loop over the ABI costs more than the kernels of a short prompt.
+extern "C" int q_prompt_pass(const q_prompt_t* p, const q_layer_weights_t* layers, const int64_t* d_tokens,
+                             const int32_t* d_block_table, int pages_per_seq, int batch, int T, void* d_last,
+                             void* stream) {
+  const char* who = "q_prompt_pass";
+  Q_CHECK_ARG(p && layers && d_tokens && d_block_table && d_last, "%s: null pointer", who);
+  Q_CHECK_ARG(p->embed && p->ln_final && p->cos && p->sin && p->pos && p->x && p->normed && p->q && p->attended &&
+                  p->act && p->partials && p->split,
+              "%s: a required pointer is null", who);
+  Q_CHECK_ARG(p->n_layers >= 1 && p->n_q_heads >= 1 && p->n_kv_heads >= 1 && batch >= 1 && T >= 1 &&
+                  (long long)batch * T < (1ll << 30),
+              "%s: bad sizes", who);
+  const int rows = batch * T, H = p->hidden, I = p->inter;
+  const int nq = p->n_q_heads, nkv = p->n_kv_heads;
+  for (int l = 0; l < p->n_layers; ++l)
+    Q_CHECK_ARG(layers[l].wqkv_tc && layers[l].wo_tc && layers[l].wgu_tc && layers[l].wdown_tc && layers[l].ln_in &&
+                    layers[l].ln_post && layers[l].q_gain && layers[l].k_gain && layers[l].kpool && layers[l].vpool,
+                "%s: layer %d has a null tensor", who, l);
+  const bool few = rows < p->few_rows;
+  cudaStream_t st = (cudaStream_t)stream;
+  q_gemm_plan_t p_qkv, p_o, p_gu, p_down;
+  if (few) {
+    TRY(q_gemm_tc_plan(rows, (nq + 2 * nkv) * 128, H, &p_qkv));
+    TRY(q_gemm_tc_plan(rows, H, nq * 128, &p_o));
+    TRY(q_gemm_tc_plan(rows, 2 * I, H, &p_gu));
+    TRY(q_gemm_tc_plan(rows, H, I, &p_down));
+  } else {
+    // tickets are zero after every finished launch; this also covers one that gave up
+    Q_CHECK_CUDA(cudaMemsetAsync(p->split, 0, (size_t)q_gemm_prompt_ticket_bytes(), st));
+  }
+  TRY(q_embed_rmsnorm(d_tokens, p->embed, layers[0].ln_in, p->x, p->normed, rows, H, p->vocab, p->rms_eps, stream));
+  for (int l = 0; l < p->n_layers; ++l) {
+    const q_layer_weights_t& w = layers[l];
+    const bool last = l + 1 == p->n_layers;
+    const void* gain = last ? p->ln_final : layers[l + 1].ln_in;
+    q_kv_layout_t kv;
+    kv.d_kpool = w.kpool; kv.d_vpool = w.vpool; kv.d_block_table = d_block_table;
+    kv.pages_per_seq = pages_per_seq; kv.n_kv_heads = nkv;
+    if (few) {
+      TRY(q_gemm_tc_launch(p->normed, w.wqkv_tc, p->partials, &p_qkv, stream));
+      TRY(q_qkv_norm_rope_cache(p->partials, &p_qkv, w.q_gain, w.k_gain, p->cos, p->sin, p->pos, p->q, &kv, batch, T,
+                                nq, p->rms_eps, stream));
+      TRY(q_attention_prefill(p->q, &kv, p->pos, p->attended, batch, T, nq, p->attn_scale, stream));
+      TRY(q_gemm_tc_launch(p->attended, w.wo_tc, p->partials, &p_o, stream));
+      TRY(q_add_rmsnorm(p->x, p->partials, &p_o, w.ln_post, p->x, p->normed, rows, H, p->rms_eps, stream));
+      TRY(q_gemm_tc_launch(p->normed, w.wgu_tc, p->partials, &p_gu, stream));
+      TRY(q_swiglu(p->partials, &p_gu, p->act, rows, I, stream));
+      TRY(q_gemm_tc_launch(p->act, w.wdown_tc, p->partials, &p_down, stream));
+      TRY(q_add_rmsnorm(p->x, p->partials, &p_down, gain, p->x, p->normed, rows, H, p->rms_eps, stream));
+      continue;
+    }
+    TRY(q_gemm_prompt_qkv(p->normed, w.wqkv_tc, w.q_gain, w.k_gain, p->cos, p->sin, p->pos, p->q, &kv, batch, T, nq, H,
+                          p->rms_eps, p->split, stream));
+    TRY(q_attention_prefill(p->q, &kv, p->pos, p->attended, batch, T, nq, p->attn_scale, stream));
+    TRY(q_gemm_prompt_add(p->attended, w.wo_tc, p->x, rows, H, nq * 128, p->split, stream));
+    TRY(q_rmsnorm(p->x, w.ln_post, p->normed, rows, H, p->rms_eps, stream));
+    TRY(q_gemm_prompt_swiglu(p->normed, w.wgu_tc, p->act, rows, I, H, p->split, stream));
+    TRY(q_gemm_prompt_add(p->act, w.wdown_tc, p->x, rows, H, I, p->split, stream));
+    if (!last) TRY(q_rmsnorm(p->x, gain, p->normed, rows, H, p->rms_eps, stream));
+  }
+  // the last position of every sequence (only these rows need the final norm)
+  const size_t row = (size_t)H * 2;
+  const char* src = (const char*)(few ? p->normed : p->x) + (size_t)(T - 1) * row;
+  Q_CHECK_CUDA(cudaMemcpy2DAsync(d_last, row, src, (size_t)T * row, row, batch, cudaMemcpyDeviceToDevice, st));
+  if (!few) TRY(q_rmsnorm(d_last, p->ln_final, d_last, batch, H, p->rms_eps, stream));
+  return Q_OK;
+}

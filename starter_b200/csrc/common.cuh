@@ -132,6 +132,9 @@ int q_gemm_launch_planned(const void* d_x, const void* d_w_tiled, float* d_parti
 int q_gemm_tc_launch(const void* d_x, const void* d_w_tc, float* d_partials, const q_gemm_plan_t* plan,
                      void* stream);
 
+// Leading bytes of q_gemm_prompt_*'s scratch that have to be zero before a launch.
+int64_t q_gemm_prompt_ticket_bytes();
+
 // q_swiglu on partials whose columns are in q_gemm_swiglu's interleaved gate/up order
 // (interleaved = 1) or in [gate | up] order (0).
 int q_swiglu_layout(const float* d_branch, const q_gemm_plan_t* plan, void* d_out, int rows, int inter,

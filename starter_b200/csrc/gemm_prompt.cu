@@ -708,6 +708,8 @@ int launch_prompt(const void* x, const void* w_tc, void* out, int M, int N, int 
 
 }  // namespace
 
+int64_t q_gemm_prompt_ticket_bytes() { return (int64_t)PG_TICKET_BYTES; }
+
 extern "C" int64_t q_gemm_prompt_scratch_bytes(void) {
   return (int64_t)(PG_TICKET_BYTES + (size_t)PG_MAX_PAIRS * 2 * PG_PART_FLOATS * 4);
 }

@@ -258,27 +258,45 @@ class DecodeState:
     PROMPT_GEMM_ROWS = 257     # rows from which the projections run on the CTA-pair kernel
 
     def _prefill_scratch(self, rows: int):
-        """Buffers of the prompt pass for up to `rows` rows, kept for the next call."""
+        """Buffers of the prompt pass for up to `rows` rows at a time, kept for the next call."""
         if getattr(self, "_pf", None) is not None and self._pf["rows"] >= rows:
             return self._pf
-        cfg, w, dev = self.cfg, self.w, self.device
-        nq, nkv, inter = w.local_q_heads, w.local_kv_heads, w.local_inter
-        bf = dict(dtype=torch.bfloat16, device=dev)
+        cfg, w, dev, B = self.cfg, self.w, self.device, self.batch
+        nq, nkv, inter, vocab = w.local_q_heads, w.local_kv_heads, w.local_inter, w.local_vocab
+        bf, f32, i32 = (dict(dtype=t, device=dev) for t in (torch.bfloat16, torch.float32, torch.int32))
+        u8 = dict(dtype=torch.uint8, device=dev)
         self._pf = None                    # release the previous size first
         few = min(rows, self.PROMPT_GEMM_ROWS - 1)       # chunks of so many rows run on split-K partials
         shapes = (((nq + 2 * nkv) * HEAD_DIM, cfg.hidden), (cfg.hidden, nq * HEAD_DIM), (2 * inter, cfg.hidden),
                   (cfg.hidden, inter))
         plans = [_lib.plan(few, n, k, tc=True) for n, k in shapes]
-        self._pf = {
+        hp = _lib.plan(B, vocab, cfg.hidden, tc=True)
+        pf = {
             "rows": rows,
             "x": torch.empty((rows, cfg.hidden), **bf), "normed": torch.empty((rows, cfg.hidden), **bf),
             "q": torch.empty((rows, nq, HEAD_DIM), **bf), "att": torch.empty((rows, nq * HEAD_DIM), **bf),
-            "act": torch.empty((rows, inter), **bf), "zero": torch.zeros(1, dtype=torch.int32, device=dev),
-            "reduced": torch.empty((rows, cfg.hidden), dtype=torch.float32, device=dev) if self.tp > 1 else None,
-            "split": torch.zeros(lib.q_gemm_prompt_scratch_bytes(), dtype=torch.uint8, device=dev),
-            "partials": torch.empty(max(p.slots * p.M * p.N for p in plans), dtype=torch.float32, device=dev),
+            "act": torch.empty((rows, inter), **bf), "zero": torch.zeros(1, **i32),
+            "reduced": torch.empty((rows, cfg.hidden), **f32) if self.tp > 1 else None,
+            "split": torch.zeros(lib.q_gemm_prompt_scratch_bytes(), **u8),
+            "partials": torch.empty(max(p.slots * p.M * p.N for p in plans), **f32),
+            "last": torch.empty((B, cfg.hidden), **bf), "head_plan": hp,
+            "head": torch.empty((hp.slots, B, vocab), **f32), "val": torch.empty(B, **f32), "idx": torch.empty(B, **i32),
+            "arg_scratch": torch.zeros(lib.q_argmax_scratch_bytes(B, vocab), **u8),
         }
-        return self._pf
+        if self.tp == 1:
+            pf["layers"] = (_lib.LayerWeights * cfg.n_layers)(*[
+                _lib.LayerWeights(lt.wqkv.data_ptr(), lt.wo.data_ptr(), lt.wgu.data_ptr(), lt.wdown.data_ptr(),
+                                  lt.ln_in.data_ptr(), lt.ln_post.data_ptr(), lt.q_gain.data_ptr(), lt.k_gain.data_ptr(),
+                                  self.kpools[i].data_ptr(), self.vpools[i].data_ptr(), lt.wqkv.tc().data_ptr(),
+                                  lt.wo.tc().data_ptr(), lt.wgu.tc().data_ptr(), lt.wdown.tc().data_ptr())
+                for i, lt in enumerate(w.layers)])
+            pf["prompt"] = _lib.Prompt(cfg.hidden, inter, cfg.n_layers, nq, nkv, cfg.vocab, self.PROMPT_GEMM_ROWS,
+                                       cfg.rms_eps, float(HEAD_DIM) ** -0.5, w.embed.data_ptr(), w.ln_final.data_ptr(),
+                                       self.cos.data_ptr(), self.sin.data_ptr(),
+                                       *(pf[n].data_ptr() for n in ("zero", "x", "normed", "q", "att", "act",
+                                                                    "partials", "split")))
+        self._pf = pf
+        return pf
 
     def prefill(self, input_ids: torch.Tensor) -> torch.Tensor:
         """Runs the whole prompt, fills the KV pages, leaves the first generated token in
@@ -291,7 +309,7 @@ class DecodeState:
         as its epilogue, below that on the decode step's projections and consumers; the causal
         attention over the prompt as q_attention_prefill reading the pages just written, lm_head
         and argmax as in the step; no library kernel runs. Sequences are processed PREFILL_ROWS prompt
-        rows at a time. Under tensor
+        rows at a time (one q_prompt_pass call each). Under tensor
         parallelism the two row-parallel projections are summed over the ranks in fp32 by an
         NCCL all-reduce before the single rounding (the prompt pass is outside the per-step
         path)."""
@@ -307,25 +325,25 @@ class DecodeState:
         stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
         ids = input_ids.contiguous()
         logits = torch.empty((B, w.local_vocab), dtype=torch.bfloat16, device=self.device)
-        last = torch.empty((B, H), dtype=torch.bfloat16, device=self.device)
         pf = self._prefill_scratch(min(per, B) * T)
+        last, hp = pf["last"], pf["head_plan"]
         for b0 in range(0, B, per):
             nb = min(per, B - b0)
             table = self.block_table.data_ptr() + b0 * self.pages_per_seq * 4
+            if self.tp == 1:
+                check(lib.q_prompt_pass(C.byref(pf["prompt"]), pf["layers"], _p(ids[b0:b0 + nb]), table,
+                                        self.pages_per_seq, nb, T, _p(last[b0:b0 + nb]), stream))
+                continue
             check(lib.q_embed_rmsnorm(_p(ids[b0:b0 + nb]), _p(w.embed), _p(w.layers[0].ln_in), _p(pf["x"]),
                                       _p(pf["normed"]), nb * T, H, cfg.vocab, eps, stream))
             layers = self._prefill_layers if nb * T >= self.PROMPT_GEMM_ROWS else self._prefill_layers_few_rows
             layers(pf, nb, T, table, stream)
             last[b0:b0 + nb].copy_(pf["normed"][:nb * T].view(nb, T, H)[:, -1])
         # lm_head on the last position of every sequence, logits rounded once to bf16
-        hp = _lib.plan(B, w.local_vocab, H, tc=True)
-        head_part = torch.empty((hp.slots, B, w.local_vocab), dtype=torch.float32, device=self.device)
-        check(lib.q_gemm_tc(_p(last), _p(w.lm_head.tc()), _p(head_part), B, w.local_vocab, H, stream))
-        val = torch.empty(B, dtype=torch.float32, device=self.device)
-        idx = torch.empty(B, dtype=torch.int32, device=self.device)
-        scratch = torch.zeros(lib.q_argmax_scratch_bytes(B, w.local_vocab), dtype=torch.uint8, device=self.device)
-        check(lib.q_logits_argmax(_p(head_part), C.byref(hp), _p(logits), _p(val), _p(idx),
-                                  _p(self.tokens) if self.tp == 1 else None, None, 0, _p(scratch), B,
+        val, idx = pf["val"], pf["idx"]
+        check(lib.q_gemm_tc(_p(last), _p(w.lm_head.tc()), _p(pf["head"]), B, w.local_vocab, H, stream))
+        check(lib.q_logits_argmax(_p(pf["head"]), C.byref(hp), _p(logits), _p(val), _p(idx),
+                                  _p(self.tokens) if self.tp == 1 else None, None, 0, _p(pf["arg_scratch"]), B,
                                   w.local_vocab, w.vocab_offset, stream))
         if self.tp > 1:
             gv = torch.empty((self.tp, B), dtype=torch.float32, device=self.device)
@@ -337,8 +355,7 @@ class DecodeState:
         return logits
 
     def _prefill_layers(self, pf, nb: int, T: int, table: int, stream) -> None:
-        """All layers over nb * T prompt rows: projections on the CTA-pair kernel with the
-        element-wise work in their epilogues."""
+        """All layers over nb * T prompt rows under tensor parallelism (one GPU: q_prompt_pass)."""
         cfg, w = self.cfg, self.w
         nq, nkv, inter = w.local_q_heads, w.local_kv_heads, w.local_inter
         H, eps, rows = cfg.hidden, float(cfg.rms_eps), nb * T
@@ -346,10 +363,6 @@ class DecodeState:
         zero, scale = _p(pf["zero"]), float(HEAD_DIM) ** -0.5
 
         def add_norm(inp, weight, K, gain):
-            if self.tp == 1:
-                check(lib.q_gemm_prompt_add(inp, _p(weight.tc()), x, rows, H, K, split, stream))
-                check(lib.q_rmsnorm(x, _p(gain), normed, rows, H, eps, stream))
-                return
             check(lib.q_gemm_prompt_f32(inp, _p(weight.tc()), _p(pf["reduced"]), rows, H, K, split, stream))
             torch.distributed.all_reduce(pf["reduced"][:rows], group=self.group)
             check(lib.q_add_rmsnorm(x, _p(pf["reduced"]), None, _p(gain), x, normed, rows, H, eps, stream))
@@ -377,9 +390,6 @@ class DecodeState:
 
         def add_norm(inp, weight, plan, gain):
             check(lib.q_gemm_tc(inp, _p(weight.tc()), part, rows, H, plan.K, stream))
-            if self.tp == 1:
-                check(lib.q_add_rmsnorm(x, part, C.byref(plan), _p(gain), x, normed, rows, H, eps, stream))
-                return
             check(lib.q_reduce_partials(part, C.byref(plan), _p(pf["reduced"]), stream))
             torch.distributed.all_reduce(pf["reduced"][:rows], group=self.group)
             check(lib.q_add_rmsnorm(x, _p(pf["reduced"]), None, _p(gain), x, normed, rows, H, eps, stream))
