@@ -970,13 +970,19 @@ extern "C" int q_attention_decode(const float* d_qkv_partials, const q_gemm_plan
   // most tiles one split can be handed: ceil(tiles / splits) over the page capacity
   int ring = (kv->pages_per_seq + splits - 1) / splits;
   ring = ring < 1 ? 1 : (ring > NS ? NS : ring);
+  // Two stages leave room for a third CTA on an SM (registers allow three). Worth it exactly where
+  // that saves the second wave; a step of 12 layers with three / two stages, us: 320 CTAs x 8 tiles
+  // 1203 / 1121, 384 x 11 1315 / 1237, but 512 x 6 1263 / 1297 (two waves either way) and 256 x 32
+  // 1403 / 1417 (one wave either way).
+  int sms = q_sm_count();
+  if (sms <= 0) sms = 148;
+  const long long ctas = (long long)splits * batch * nkv;
+  if (ring == 3 && ctas > 2 * sms && ctas <= 3 * sms) ring = 2;
   // Three warp groups (one tile each at a time) when every CTA of the launch gets an SM of its
   // own; otherwise one group, so that two CTAs still fit on an SM. A ring stage must always be
   // consumed by the same group (its mbarrier parity is tracked per group), so the three groups
   // need the three-stage ring.
-  int sms = q_sm_count();
-  if (sms <= 0) sms = 148;
-  const bool wide = splits > 1 && (long long)splits * batch * nkv <= sms && ring == 3 && NS == 3;
+  const bool wide = splits > 1 && ctas <= sms && ring == 3 && NS == 3;
   const int dc = wide ? 12 : 4;
   const dim3 block((dc + 1) * 32);
   static size_t done[4][64] = {{0}};

@@ -45,6 +45,7 @@ enum { B_QF = 0, B_QE = 2, B_KF = 4, B_KE = 6, B_VF = 8, B_VE = 10, B_SF = 12, B
 struct AttnShape {
   int batch, T, G, gshift, nq, nkv, pages_per_seq;
   int tokens;        // prompt tokens per query tile: 128 / G
+  int tiles;         // query tiles per work item: 2, or 1 when there are SMs enough for all tiles
   int blocks;        // work items per (sequence, kv head)
   int items;
   int wide;          // the output is 32-byte aligned
@@ -59,8 +60,8 @@ __device__ __forceinline__ Item item_at(const AttnShape& sh, int w, int pos) {
   const int blk = w / heads, bh = w - blk * heads;
   it.b = bh / sh.nkv;
   it.kh = bh - it.b * sh.nkv;
-  it.q0 = (sh.blocks - 1 - blk) * 2 * sh.tokens;           // latest blocks (most keys) first
-  it.max_limit = pos + min(it.q0 + 2 * sh.tokens, sh.T);
+  it.q0 = (sh.blocks - 1 - blk) * sh.tiles * sh.tokens;           // latest blocks (most keys) first
+  it.max_limit = pos + min(it.q0 + sh.tiles * sh.tokens, sh.T);
   it.n = (it.max_limit + AP_KEYS - 1) / AP_KEYS;
   return it;
 }
@@ -186,6 +187,11 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  if (warp == 8 && lane == 0) {
+    prefetch_map(&qmap);
+    prefetch_map(&kmap);
+    prefetch_map(&vmap);
+  }
   if (warp == 9) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                  ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
@@ -209,7 +215,7 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
         const int w = item_of(r);
         if (w >= sh.items) continue;
         const Item it = item_at(sh, w, pos);
-        for (int i = 0; ok && i < 2; ++i) {
+        for (int i = 0; ok && i < sh.tiles; ++i) {
           if (!mbar_wait(bar(B_QE, i), (nitems & 1) ^ 1, abort_flag)) { fail(); break; }
           const int tok = it.b * sh.T + it.q0 + i * sh.tokens;
           mbar_expect_tx(bar(B_QF, i), AP_TILE);
@@ -238,7 +244,7 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
       }
       // copies in flight must land before the CTA may leave
       for (int i = 0; i < 2; ++i) {
-        if (nitems > 0) mbar_wait_plain(bar(B_QF, i), (nitems - 1) & 1);
+        if (nitems > 0 && i < sh.tiles) mbar_wait_plain(bar(B_QF, i), (nitems - 1) & 1);
         if (step > (uint32_t)i) {
           const uint32_t last = ((step - 1 - i) >> 1) & 1;
           mbar_wait_plain(bar(B_KF, (step - 1 - i) & 1), last);
@@ -283,7 +289,7 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
       };
       int r = 0;
       Item cur = item_at(sh, item_of(0), pos);             // the grid has at most one CTA per item
-      for (int i = 0; i < 2 && ok; ++i) {
+      for (int i = 0; i < sh.tiles && ok; ++i) {
         if (!wait(bar(B_QF, i), 0) || (i == 0 && !wait(bar(B_KF, 0), 0))) break;
         scores(i);
         if (leader && cur.n == 1) tc_commit(bar(B_QE, i));
@@ -305,7 +311,7 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
           const bool last = j + 1 == cur.n, ahead = !last || more;
           const int vs = vstep & 1;
           if (!wait(bar(B_VF, vs), (vstep >> 1) & 1)) break;
-          for (int i = 0; i < 2 && ok; ++i) {
+          for (int i = 0; i < sh.tiles && ok; ++i) {
             if (j == 0 && !wait(bar(B_OE, i), (nitems & 1) ^ 1)) break;
             for (int h = 0; h < 2; ++h) {                  // P comes in two halves of 64 keys
               if (!wait(bar(B_P, 2 * i + h), vstep & 1)) break;
@@ -343,7 +349,7 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
         cur = nxt;
       }
     }
-  } else {
+  } else if ((warp >> 2) < sh.tiles) {
     // ---------------- softmax and epilogue: query tile `i`, one row per thread ----------------
     const int i = warp >> 2;
     const int row = tid & 127;
@@ -532,7 +538,11 @@ extern "C" int q_attention_prefill(const void* d_q, const q_kv_layout_t* kv, con
   sh.gshift = 0;
   while ((1 << sh.gshift) < G) ++sh.gshift;
   sh.tokens = 128 >> sh.gshift;
-  sh.blocks = (T + 2 * sh.tokens - 1) / (2 * sh.tokens);
+  // Two tiles of a CTA hide each other's latencies, but also share its exponentials: while every
+  // tile can have an SM of its own, one per CTA is faster.
+  const int sms = q_sm_count();
+  sh.tiles = (long long)((T + sh.tokens - 1) / sh.tokens) * batch * nkv <= sms ? 1 : 2;
+  sh.blocks = (T + sh.tiles * sh.tokens - 1) / (sh.tiles * sh.tokens);
   const long long items = (long long)sh.blocks * batch * nkv;
   Q_CHECK_ARG(items < (1ll << 30) && (long long)batch * T < (1ll << 31), "q_attention_prefill: too many rows");
   sh.items = (int)items;
@@ -557,7 +567,6 @@ extern "C" int q_attention_prefill(const void* d_q, const q_kv_layout_t* kv, con
   }
   static size_t done[64] = {0};
   Q_CHECK_CUDA(q_ensure_smem(k_attn_prompt, AP_SMEM, done));
-  const int sms = q_sm_count();
   const int grid = sh.items < sms ? sh.items : sms;
   Q_CHECK_CUDA(q_launch(k_attn_prompt, dim3(grid), dim3(AP_THREADS), AP_SMEM, (cudaStream_t)stream, qmap, kmap, vmap,
                         kv->d_block_table, d_pos, (bf16*)d_out, sh, status));

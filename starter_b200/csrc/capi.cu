@@ -368,10 +368,13 @@ static float* hidden_partials(const q_engine* e, bool second) {
   return second ? e->st.partials + max_plan_floats(e) : e->st.partials;
 }
 
-// Up to 8 rows on one GPU: residual add + RMSNorm run as the prologue of the projection
-// that consumes them, the residual alternating between st.x and st.normed.
+// One and two rows on one GPU: residual add + RMSNorm run as the prologue of the projection
+// that consumes them, the residual alternating between st.x and st.normed. Every CTA of the
+// projection reads all rows' partials there (25 KB a row from L2 at 2560 columns), so above that one
+// k_add_rmsnorm launch is cheaper. Step of 12 layers at 700 keys, prologue / launch, us:
+// 1 row 725 / 765, 2 rows 764 / 772, 3 rows 802 / 779, 5 rows 945 / 859, 8 rows 1008 / 878.
 static bool norm_in_gemm(const q_engine* e) {
-  return e->cfg.tp_size == 1 && !e->tc && e->T == 1 && e->rows <= 8 && e->cfg.hidden % 4 == 0 &&
+  return e->cfg.tp_size == 1 && !e->tc && e->T == 1 && e->rows <= 2 && e->cfg.hidden % 4 == 0 &&
          e->cfg.hidden <= 3072 && g_norm_in_gemm;
 }
 

@@ -407,6 +407,10 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  if (warp == 0 && lane == 0) {
+    prefetch_map(&wmap);
+    prefetch_map(&xmap);
+  }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
                  ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
