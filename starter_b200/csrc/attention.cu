@@ -893,6 +893,65 @@ extern "C" int q_attention_splits(int batch, int n_kv_heads, int capacity) {
   return s;
 }
 
+// Clusters of `splits` CTAs of the decode kernel that the current device holds at once (a cluster
+// stays inside one GPC, so this is less than SMs / splits), asked once per device; without a device
+// the count that the SMs alone would allow.
+static int resident_clusters(bool wide, int splits, int sms) {
+  static int cached[64][2][9];
+  const int dev = q_device_index();
+  if (dev < 0) return (wide ? sms : 2 * sms) / splits;
+  int& n = cached[dev][wide][splits];
+  if (n == 0) {
+    static size_t done[2][64] = {{0}};
+    int got = 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(splits, 1);
+    cfg.blockDim = dim3(wide ? 13 * 32 : 5 * 32);
+    cfg.dynamicSmemBytes = attn_decode_smem(NS);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = splits; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    cudaError_t e = wide ? q_ensure_smem(k_attn_decode<true, 3>, attn_decode_smem(NS), done[0])
+                         : q_ensure_smem(k_attn_decode<true, 1>, attn_decode_smem(NS), done[1]);
+    if (e == cudaSuccess)
+      e = wide ? cudaOccupancyMaxActiveClusters(&got, k_attn_decode<true, 3>, &cfg)
+               : cudaOccupancyMaxActiveClusters(&got, k_attn_decode<true, 1>, &cfg);
+    if (e != cudaSuccess) { cudaGetLastError(); got = (wide ? sms : 2 * sms) / splits; }
+    n = got > 0 ? got : -1;
+  }
+  return n;
+}
+
+extern "C" int q_attention_decode_splits(int batch, int n_kv_heads, int capacity) {
+  if (batch < 1 || n_kv_heads < 1 || capacity < 1) return 1;
+  int sms = q_sm_count();
+  if (sms <= 0) sms = 148;
+  const int vh = batch * n_kv_heads;
+  const int tiles = (capacity + Q_PAGE_TOKENS - 1) / Q_PAGE_TOKENS;
+  // One sequence of a very long context: every SM takes a split (merged through global memory).
+  // Step of 4 layers, 8 kv heads, 18 splits / 8: 357 / 361 us at 8 K keys, but 340 / 331 at 2 K.
+  if (tiles > 96 && sms / vh > MAX_CLUSTER) return sms / vh < 32 ? sms / vh : 32;
+  // One CTA of three warp groups per SM, its splits merging in a cluster, as long as all clusters
+  // are resident at once and a split can see three tiles (fewer: the three groups have no work).
+  // Two smaller CTAs per SM, which hold more splits, measured slower up to 9 sequences of 8 kv heads
+  // - 5 sequences, 3 / 7 splits: 350 / 367 us at 700 keys, 368 / 416 at 2 K, 448 / 523 at 8 K - and
+  // clusters that have to wait for a place cost a second pass: 6 sequences, 2 / 3 splits 352 / 378.
+  int s = sms / vh;
+  if (s > 8) s = 8;
+  if (s > (tiles - 1) / 2) s = (tiles - 1) / 2;
+  for (; s >= 2; --s)
+    if (resident_clusters(true, s, sms) >= vh) return s;
+  // Otherwise two CTAs per SM: 12 sequences, 2 / 3 splits (288 CTAs, not all resident): 421 / 446.
+  s = 2 * sms / vh;
+  if (s > 8) s = 8;
+  if (s > tiles) s = tiles;
+  // (with a tenth to spare above pairs, which place anywhere: 11 sequences, 2 / 3 splits 422 / 439)
+  for (; s >= 2; --s)
+    if (resident_clusters(false, s, sms) * (s > 2 ? 9 : 10) >= vh * 10) return s;
+  return 1;
+}
+
 extern "C" int q_attention(const void* d_q, const q_kv_layout_t* kv, const int32_t* d_pos,
                            float* d_scratch_o, float* d_scratch_ml, void* d_out, int batch, int T,
                            int n_q_heads, int splits, float scale, void* stream) {

@@ -124,7 +124,8 @@ class DecodeState:
             raise _lib.QDecodeError("could not size the split-K partial buffer")
         self.partials = torch.empty(n_part, **f32)
         self.reduced = torch.zeros((rows, cfg.hidden), **f32) if self.tp > 1 else None
-        self.attn_splits = lib.q_attention_splits(batch, nkv, self.capacity)
+        splits = lib.q_attention_decode_splits if q_tokens == 1 else lib.q_attention_splits
+        self.attn_splits = splits(batch, nkv, self.capacity)
         g = nq // nkv
         self.attn_o = torch.empty((batch * nkv, self.attn_splits, q_tokens * g, HEAD_DIM), **f32)
         self.attn_ml = torch.empty((batch * nkv, self.attn_splits, q_tokens * g, 2), **f32)
