@@ -13,8 +13,11 @@
 // while the softmax of the other runs; a CTA is persistent and starts the next item's first
 // products under the current one's last softmax, since an item is only ~9 tiles long at 1-2 K keys.
 //
-// Warps 0-3 / 4-7: softmax and epilogue of query tile 0 / 1 (a thread owns a row: no shuffles).
-// Warp 8: producer lane. Warp 9: MMA issue; the whole warp walks the loop and one elected lane
+// Warps 0-7 / 8-15: softmax and epilogue of query tile 0 / 1. Two threads share a row (64 scores, then
+// 64 dims of O each) and exchange its maximum through shared memory: a step is a chain - scores,
+// softmax, P V, next scores - and with one thread per row it took 4500 cycles, of which the softmax
+// of 128 scores was more than half.
+// Warp 16: producer lane. Warp 17: MMA issue; the whole warp walks the loop and one elected lane
 // issues, so that descriptors live in uniform registers: an MMA of 128 x 128 x 16 takes 64 cycles,
 // about what a single diverged lane needs to assemble its operands.
 // The running maximum is only moved (and O rescaled) when a row's maximum grew by more than 2^8:
@@ -31,13 +34,14 @@ int* q_attn_status_addr();
 
 namespace {
 
-constexpr int AP_THREADS = 320;
+constexpr int AP_THREADS = 576;                            // 16 softmax warps, producer, MMA
 constexpr int AP_KEYS = 128;                               // keys per tile
 constexpr uint32_t AP_HALF = 128 * 128;                    // bytes of 128 rows x 64 dims
 constexpr uint32_t AP_TILE = 2 * AP_HALF;                  // 128 rows x 128 dims
 constexpr uint32_t AP_Q = 0, AP_K = 2 * AP_TILE, AP_V = AP_K + 2 * AP_TILE;
 constexpr uint32_t AP_BARS = AP_V + 2 * AP_TILE;           // 192 KB in
-constexpr size_t AP_SMEM = 1024 + AP_BARS + 24 * 8 + 16;
+constexpr uint32_t AP_RED = AP_BARS + 24 * 8 + 16;         // row exchange: [3][2 tiles][2 halves][128] floats
+constexpr size_t AP_SMEM = 1024 + AP_RED + 3 * 2 * 2 * 128 * 4;
 constexpr float AP_GROWTH = 8.f;                           // log2 of the growth that moves the maximum
 
 enum { B_QF = 0, B_QE = 2, B_KF = 4, B_KE = 6, B_VF = 8, B_VE = 10, B_SF = 12, B_P = 14, B_OF = 18, B_OE = 20 };
@@ -113,26 +117,14 @@ __device__ __forceinline__ void tc_pin32(float* v) {
     asm volatile("" : "+f"(v[i]), "+f"(v[i + 1]), "+f"(v[i + 2]), "+f"(v[i + 3]), "+f"(v[i + 4]), "+f"(v[i + 5]),
                       "+f"(v[i + 6]), "+f"(v[i + 7]));
 }
-__device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t* r) {
+__device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
-      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
       ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
-        "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
-        "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "elect.sync _|p, 0xffffffff;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(p));
-  return p != 0;
-}
 // Two fp32 lanes per instruction, each rounded like the scalar one; and the largest of three.
 __device__ __forceinline__ unsigned long long pair2(float a, float b) {
   unsigned long long r;
@@ -180,19 +172,19 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     for (int i = 0; i < 24; ++i) {
-      const bool warps = (i >= B_P && i < B_P + 4) || (i >= B_OE && i < B_OE + 2);   // four softmax warps arrive
-      mbar_init(bars + 8u * i, warps ? 4 : 1);
+      const bool warps = i >= B_P && i < B_P + 4;          // four softmax warps arrive (eight at the epilogue)
+      mbar_init(bars + 8u * i, i >= B_OE && i < B_OE + 2 ? 8 : warps ? 4 : 1);
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (warp == 8 && lane == 0) {
+  if (warp == 16 && lane == 0) {
     prefetch_map(&qmap);
     prefetch_map(&kmap);
     prefetch_map(&vmap);
   }
-  if (warp == 9) {
+  if (warp == 17) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                  ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -200,11 +192,12 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;                        // columns: S0 0, S1 128, O0 256, O1 384
+  // All 512 columns are this CTA's, so its tensor memory starts at column 0.
+  constexpr uint32_t tmem = 0;
   pdl_wait();                                              // q and this pass's K/V rows
   const int pos = pos_ptr[0];
 
-  if (warp == 8) {
+  if (warp == 16) {
     // ---------------- producer ----------------
     if (lane == 0) {
       uint32_t step = 0;                                   // K/V tiles requested so far
@@ -256,10 +249,9 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
         while (clock64() - t0 < 2000000) __nanosleep(1000);
       }
     }
-  } else if (warp == 9) {
+  } else if (warp == 17) {
     // ---------------- MMA issuer ----------------
     {
-      const bool leader = elect_one();
       const uint32_t f16 = (1u << 4) | (1u << 7) | (1u << 10) | (16u << 17) | (8u << 24);   // 128 x 128, fp32 sums
       const uint32_t idesc_s = f16, idesc_pv = f16 | (1u << 16);      // V: the non-contracted dimension is contiguous
       const uint64_t q_desc = smem_desc(base + AP_Q), k_desc = smem_desc(base + AP_K);
@@ -271,7 +263,7 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
       auto wait = [&](uint32_t b, uint32_t parity) {
         const int landed = mbar_wait(b, parity, abort_flag) ? 1 : 0;
         if (!__all_sync(0xffffffffu, landed)) {
-          if (leader) { atomicExch(status, 8); *abort_flag = 1; }
+          if (elect_one()) { atomicExch(status, 8); *abort_flag = 1; }
           ok = false;
         }
         tc_fence_after();
@@ -279,7 +271,7 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
       };
       auto scores = [&](int i) {                           // S_i = Q_i K^T of the K tile at kstep
         const uint64_t a = q_desc + (uint64_t)(i * (AP_TILE >> 4)), b = k_desc + (uint64_t)((kstep & 1) * (AP_TILE >> 4));
-        if (!leader) return;
+        if (!elect_one()) return;
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
           const uint32_t off = (uint32_t)(ks >> 2) * (AP_HALF >> 4) + (ks & 3) * 2;
@@ -292,11 +284,11 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
       for (int i = 0; i < sh.tiles && ok; ++i) {
         if (!wait(bar(B_QF, i), 0) || (i == 0 && !wait(bar(B_KF, 0), 0))) break;
         scores(i);
-        if (leader && cur.n == 1) tc_commit(bar(B_QE, i));
+        if (elect_one() && cur.n == 1) tc_commit(bar(B_QE, i));
         __syncwarp();
       }
       if (ok) {
-        if (leader) tc_commit(bar(B_KE, 0));
+        if (elect_one()) tc_commit(bar(B_KE, 0));
         ++kstep;
       }
       while (ok) {
@@ -315,7 +307,7 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
             if (j == 0 && !wait(bar(B_OE, i), (nitems & 1) ^ 1)) break;
             for (int h = 0; h < 2; ++h) {                  // P comes in two halves of 64 keys
               if (!wait(bar(B_P, 2 * i + h), vstep & 1)) break;
-              if (leader) {
+              if (elect_one()) {
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                   const int ks = 4 * h + k;
@@ -326,17 +318,17 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
               __syncwarp();
             }
             if (!ok) break;
-            if (last && leader) tc_commit(bar(B_OF, i));
+            if (last && elect_one()) tc_commit(bar(B_OF, i));
             if (ahead) {
               if (i == 0 && !wait(bar(B_KF, kstep & 1), (kstep >> 1) & 1)) break;
               if (last && !wait(bar(B_QF, i), (nitems + 1) & 1)) break;
               scores(i);
-              if (leader && (last ? nxt.n == 1 : j + 2 == cur.n)) tc_commit(bar(B_QE, i));
+              if (elect_one() && (last ? nxt.n == 1 : j + 2 == cur.n)) tc_commit(bar(B_QE, i));
               __syncwarp();
             }
           }
           if (!ok) break;
-          if (leader) {
+          if (elect_one()) {
             tc_commit(bar(B_VE, vs));
             if (ahead) tc_commit(bar(B_KE, kstep & 1));
           }
@@ -349,27 +341,31 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
         cur = nxt;
       }
     }
-  } else if ((warp >> 2) < sh.tiles) {
-    // ---------------- softmax and epilogue: query tile `i`, one row per thread ----------------
-    const int i = warp >> 2;
+  } else if ((warp >> 3) < sh.tiles) {
+    // ---------------- softmax and epilogue: query tile `i`, half a row per thread ----------------
+    const int i = warp >> 3, half = (warp >> 2) & 1;
     const int row = tid & 127;
+    float* red = reinterpret_cast<float*>(smem + AP_RED) + i * 256;        // [buffer * 512 + half * 128 + row]
+    auto tile_sync = [&]() { asm volatile("bar.sync %0, 256;" ::"r"(1 + i) : "memory"); };
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t s_addr = tmem + lanes + 128u * i, o_addr = tmem + lanes + 256u + 128u * i;
+    const uint32_t s_addr = tmem + lanes + 128u * i + 64u * half, p_addr = tmem + lanes + 128u * i + 32u * half;
+    const uint32_t o_addr = tmem + lanes + 256u + 128u * i + 64u * half;
     // A scale that is not positive (the maximum would sit elsewhere) is multiplied in first.
     const bool plain = sh.scale_log2 > 0.f;
     const float c = plain ? sh.scale_log2 : 1.f;
     uint32_t step = 0, nitems = 0;
-    bool ok = true;
+    // A warp whose wait ran out keeps coming to the tile's barriers; at the item's end all eight
+    // warps learn of it and leave together.
+    bool broken = false;
     auto wait = [&](uint32_t b, uint32_t parity) {
-      const int landed = mbar_wait(b, parity, abort_flag) ? 1 : 0;
+      const int landed = broken || mbar_wait(b, parity, abort_flag) ? 1 : 0;
       if (!__all_sync(0xffffffffu, landed)) {
         if (lane == 0) { atomicExch(status, 9); *abort_flag = 1; }
-        ok = false;
+        broken = true;
       }
       tc_fence_after();
-      return ok;
     };
-    for (int r = 0; ok && r * (int)gridDim.x < sh.items; ++r) {
+    for (int r = 0; r * (int)gridDim.x < sh.items; ++r) {
       const int w = item_of(r);
       if (w >= sh.items) continue;
       const Item it = item_at(sh, w, pos);
@@ -381,30 +377,30 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
       const int free_keys = t_last < sh.T ? pos + t_first + 1 : 0;
       float m = -INFINITY, l = 0.f;
       for (int j = 0; j < it.n; ++j, ++step) {
-        if (!wait(bar(B_SF, i), step & 1)) break;
-        float v[128];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) tc_ld32(s_addr + 32 * k, v + 32 * k);
+        wait(bar(B_SF, i), step & 1);
+        float v[64];
+        tc_ld32(s_addr, v);
+        tc_ld32(s_addr + 32, v + 32);
         tc_wait_ld();
-#pragma unroll
-        for (int k = 0; k < 4; ++k) tc_pin32(v + 32 * k);
+        tc_pin32(v);
+        tc_pin32(v + 32);
         const int key_base = j * AP_KEYS;
         if (!plain) {
 #pragma unroll
-          for (int k = 0; k < 128; ++k) v[k] *= sh.scale_log2;
+          for (int k = 0; k < 64; ++k) v[k] *= sh.scale_log2;
         }
         if (key_base + AP_KEYS > free_keys) {
-          const int vis = limit - key_base;
+          const int vis = limit - key_base - 64 * half;
 #pragma unroll
-          for (int k = 0; k < 128; ++k) v[k] = k < vis ? v[k] : -INFINITY;
+          for (int k = 0; k < 64; ++k) v[k] = k < vis ? v[k] : -INFINITY;
         }
-        if (i == 0 && key_base + AP_KEYS > it.max_limit) {
+        if (tid < 128 && key_base + AP_KEYS > it.max_limit) {
           // V rows past the newest key hold stale bits (0 * garbage could be NaN): clear them
           // before the first product with this tile may start
-          if (!wait(bar(B_VF, step & 1), (step >> 1) & 1)) break;
+          wait(bar(B_VF, step & 1), (step >> 1) & 1);
           unsigned char* vt = smem + AP_V + (step & 1) * AP_TILE;
           const int live = it.max_limit - key_base;
-          for (int q = tid; q < (128 - live) * 16; q += 128) {
+          for (int q = tid; !broken && q < (128 - live) * 16; q += 128) {
             const int kr = live + (q >> 4);
             *reinterpret_cast<uint4*>(vt + (q & 8 ? AP_HALF : 0u) + kr * 128 + ((q & 7) << 4)) = make_uint4(0, 0, 0, 0);
           }
@@ -413,10 +409,17 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
         }
         float mx[4] = {v[0], v[1], v[2], v[3]};
 #pragma unroll
-        for (int k = 4; k < 124; k += 8)
+        for (int k = 4; k < 60; k += 8)
 #pragma unroll
           for (int e = 0; e < 4; ++e) mx[e] = max3(mx[e], v[k + e], v[k + 4 + e]);
-        const float m_tile = max3(max3(mx[0], mx[1], mx[2]), mx[3], fmaxf(max3(v[124], v[125], v[126]), v[127]));
+        float m_tile = max3(max3(mx[0], mx[1], mx[2]), mx[3], fmaxf(max3(v[60], v[61], v[62]), v[63]));
+        // the row's other half; this barrier also says that both halves of S are in registers, so
+        // that P may overwrite them
+        red[(step & 1) * 512 + half * 128 + row] = m_tile;
+        tc_fence_before();
+        tile_sync();
+        tc_fence_after();
+        m_tile = fmaxf(m_tile, red[(step & 1) * 512 + (half ^ 1) * 128 + row]);
         if (j == 0) {
           m = m_tile;
         } else {
@@ -429,14 +432,12 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
             m = m_new;
 #pragma unroll 1
             for (int k = 0; k < 4; ++k) {
-              float o[32];
-              tc_ld32(o_addr + 32 * k, o);
-              tc_wait_ld();
-              tc_pin32(o);
-              uint32_t u[32];
+              float o[16];
+              uint32_t u[16];
+              tc_ld16(o_addr + 16 * k, o);
 #pragma unroll
-              for (int e = 0; e < 32; ++e) u[e] = __float_as_uint(o[e] * f);
-              tc_st32(o_addr + 32 * k, u);
+              for (int e = 0; e < 16; ++e) u[e] = __float_as_uint(o[e] * f);
+              tc_st16(o_addr + 16 * k, u);
             }
             tc_wait_st();
           }
@@ -446,50 +447,56 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
         unsigned long long sum[2] = {0ull, 0ull};
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          uint32_t p[32];
+          uint32_t p[16];
 #pragma unroll
-          for (int k = 0; k < 32; ++k) {
+          for (int k = 0; k < 16; ++k) {
             float a, b;
-            unpair2(fma2(pair2(v[64 * h + 2 * k], v[64 * h + 2 * k + 1]), c2, mc2), a, b);
+            unpair2(fma2(pair2(v[32 * h + 2 * k], v[32 * h + 2 * k + 1]), c2, mc2), a, b);
             a = ex2(a);
             b = ex2(b);
             sum[k & 1] = add2(sum[k & 1], pair2(a, b));
             p[k] = pack_bf16(a, b);
           }
-          tc_st32(s_addr + 32 * h, p);
-          tc_wait_st();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar(B_P, 2 * i + h));
-          __syncwarp();
+          tc_st16(p_addr + 16 * h, p);
         }
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(B_P, 2 * i + half));
+        __syncwarp();
         float s_lo, s_hi;
         unpair2(add2(sum[0], sum[1]), s_lo, s_hi);
         l += s_lo + s_hi;
       }
-      if (!ok || !wait(bar(B_OF, i), nitems & 1)) break;
+      red[1024 + half * 128 + row] = l;
+      int give_up;
+      asm volatile(
+          "{\n\t.reg .pred p, q;\n\t"
+          "setp.ne.u32 q, %1, 0;\n\t"
+          "barrier.cta.red.or.pred p, %2, 256, q;\n\t"
+          "selp.u32 %0, 1, 0, p;\n\t}"
+          : "=r"(give_up) : "r"((int)broken), "r"(1 + i) : "memory");
+      if (give_up) break;
+      l += red[1024 + (half ^ 1) * 128 + row];
+      wait(bar(B_OF, i), nitems & 1);
+      if (broken) { ++nitems; continue; }
       const float inv = l > 0.f ? 1.f / l : (l == 0.f ? 0.f : l);      // NaN stays NaN
-      bf16* dst = out + (((size_t)it.b * sh.T + t) * sh.nq + it.kh * sh.G + (row & (sh.G - 1))) * 128;
+      bf16* dst = out + (((size_t)it.b * sh.T + t) * sh.nq + it.kh * sh.G + (row & (sh.G - 1))) * 128 + 64 * half;
 #pragma unroll 1
       for (int k = 0; k < 4; ++k) {
-        float o[32];
-        tc_ld32(o_addr + 32 * k, o);
-        tc_wait_ld();
-        tc_pin32(o);
+        float o[16];
+        tc_ld16(o_addr + 16 * k, o);
         if (t < sh.T) {
+          uint32_t u[8];
 #pragma unroll
-          for (int e = 0; e < 32; e += 16) {
-            uint32_t u[8];
+          for (int q = 0; q < 8; ++q) u[q] = pack_bf16(o[2 * q] * inv, o[2 * q + 1] * inv);
+          if (sh.wide) {
+            asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                         ::"l"(dst + 16 * k), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]),
+                         "r"(u[6]), "r"(u[7]) : "memory");
+          } else {
 #pragma unroll
-            for (int q = 0; q < 8; ++q) u[q] = pack_bf16(o[e + 2 * q] * inv, o[e + 2 * q + 1] * inv);
-            if (sh.wide) {
-              asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-                           ::"l"(dst + 32 * k + e), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]),
-                           "r"(u[6]), "r"(u[7]) : "memory");
-            } else {
-#pragma unroll
-              for (int q = 0; q < 8; ++q) *reinterpret_cast<uint32_t*>(dst + 32 * k + e + 2 * q) = u[q];
-            }
+            for (int q = 0; q < 8; ++q) *reinterpret_cast<uint32_t*>(dst + 16 * k + 2 * q) = u[q];
           }
         }
         __syncwarp();
@@ -505,7 +512,7 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
   __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (warp == 9) {
+  if (warp == 17) {
     __syncwarp();
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");

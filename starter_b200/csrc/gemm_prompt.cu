@@ -483,10 +483,15 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader) ----------------
-    if (rank == 0 && lane == 0) {
+    // (the whole warp walks the loop and one elected lane issues, so that descriptors live in uniform
+    // registers)
+    if (rank == 0) {
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(PG_BN >> 3) << 17) | (16u << 24);
       const uint32_t stage_units = PG_STAGE >> 4;
       const uint64_t desc0 = smem_desc(base);
+      auto warp_wait = [&](uint32_t b, uint32_t par) {
+        return __all_sync(0xffffffffu, mbar_wait(b, par, abort_flag) ? 1 : 0) != 0;
+      };
       int st = 0, seg = 0;
       uint32_t parity = 0;
       bool ok = true;
@@ -495,23 +500,27 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
       int t, k0, k1;
       for (; ok && walk.next(sh, pair, pairs, t, k0, k1); ++seg) {
         const int buf = seg & 1;
-        if (!mbar_wait(bar_acc_empty + 8 * buf, ((seg >> 1) & 1) ^ 1, abort_flag)) { ok = false; break; }
+        if (!warp_wait(bar_acc_empty + 8 * buf, ((seg >> 1) & 1) ^ 1)) { ok = false; break; }
         tc_fence_after();
         const uint32_t dacc = tmem_base + (uint32_t)buf * 256u;
         for (int kt = k0; kt < k1; ++kt) {
-          if (!mbar_wait(bar_full + 8 * st, parity, abort_flag)) { ok = false; break; }
+          if (!warp_wait(bar_full + 8 * st, parity)) { ok = false; break; }
           tc_fence_after();
           const uint64_t a_desc = desc0 + (uint64_t)(st * stage_units);
           const uint64_t b_desc = a_desc + (PG_A_BYTES >> 4);
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < PG_TILE_K / 16; ++k)
-            pair_mma(dacc, a_desc + 2u * k, b_desc + 2u * k, idesc, (kt > k0 || k) ? 1u : 0u);
-          pair_commit(bar_empty + 8 * st);
+            for (int k = 0; k < PG_TILE_K / 16; ++k)
+              pair_mma(dacc, a_desc + 2u * k, b_desc + 2u * k, idesc, (kt > k0 || k) ? 1u : 0u);
+            pair_commit(bar_empty + 8 * st);
+          }
+          __syncwarp();
           if (++st == PG_STAGES) { st = 0; parity ^= 1u; }
         }
-        if (ok) pair_commit(bar_acc_full + 8 * buf);
+        if (ok && elect_one()) pair_commit(bar_acc_full + 8 * buf);
+        __syncwarp();
       }
-      if (!ok) {
+      if (!ok && lane == 0) {
         atomicExch(status, 6);
         *abort_flag = 1;
       }

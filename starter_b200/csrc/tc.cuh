@@ -45,6 +45,17 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 __device__ __forceinline__ bool mbar_wait_plain(uint32_t bar, uint32_t parity) {
   return mbar_wait(bar, parity, nullptr);
 }
+// One lane of a converged warp. Asked for where it branches: the compiler then knows that a single
+// lane runs what follows and keeps MMA operands in uniform registers.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ uint64_t stream_policy() {
   uint64_t p;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
