@@ -392,7 +392,8 @@ typedef struct q_layer_weights_t {
  * sequence's last position into d_last [batch][hidden]. From few_rows rows on the projections are
  * q_gemm_prompt_*, below that q_gemm_tc and its consumers (partials: enough for every plan of up to
  * few_rows - 1 rows). x, normed [rows][hidden], q, attended [rows][n_q*128], act [rows][inter] are
- * scratch of the caller (32-byte aligned), split as in q_gemm_prompt_* (cleared by every call).
+ * scratch of the caller (32-byte aligned), split as in q_gemm_prompt_* (its tickets are cleared by
+ * every call; null if no call has few_rows rows).
  * layers: wqkv_tc .. wdown_tc, gains and pools are read; only enqueues on `stream`. */
 typedef struct q_prompt_t {
   int32_t hidden, inter, n_layers, n_q_heads, n_kv_heads, vocab, few_rows;

@@ -305,18 +305,15 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
           if (!wait(bar(B_VF, vs), (vstep >> 1) & 1)) break;
           for (int i = 0; i < sh.tiles && ok; ++i) {
             if (j == 0 && !wait(bar(B_OE, i), (nitems & 1) ^ 1)) break;
-            for (int h = 0; h < 2; ++h) {                  // P comes in two halves of 64 keys
-              if (!wait(bar(B_P, 2 * i + h), vstep & 1)) break;
-              if (elect_one()) {
+            // P comes in two halves of 64 keys, from different warps
+            if (!wait(bar(B_P, 2 * i), vstep & 1) || !wait(bar(B_P, 2 * i + 1), vstep & 1)) break;
+            if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                  const int ks = 4 * h + k;
-                  tc_mma_ta(tmem + 256u + 128u * i, tmem + 128u * i + 8u * ks,
-                            v_desc + (uint64_t)(vs * (AP_TILE >> 4) + ks * (2048 >> 4)), idesc_pv, (j | ks) ? 1u : 0u);
-                }
-              }
-              __syncwarp();
+              for (int ks = 0; ks < 8; ++ks)
+                tc_mma_ta(tmem + 256u + 128u * i, tmem + 128u * i + 8u * ks,
+                          v_desc + (uint64_t)(vs * (AP_TILE >> 4) + ks * (2048 >> 4)), idesc_pv, (j | ks) ? 1u : 0u);
             }
+            __syncwarp();
             if (!ok) break;
             if (last && elect_one()) tc_commit(bar(B_OF, i));
             if (ahead) {

@@ -655,7 +655,7 @@ extern "C" int q_prompt_pass(const q_prompt_t* p, const q_layer_weights_t* layer
   const char* who = "q_prompt_pass";
   Q_CHECK_ARG(p && layers && d_tokens && d_block_table && d_last, "%s: null pointer", who);
   Q_CHECK_ARG(p->embed && p->ln_final && p->cos && p->sin && p->pos && p->x && p->normed && p->q && p->attended &&
-                  p->act && p->partials && p->split,
+                  p->act && p->partials && (p->split || batch * T < p->few_rows),
               "%s: a required pointer is null", who);
   Q_CHECK_ARG(p->n_layers >= 1 && p->n_q_heads >= 1 && p->n_kv_heads >= 1 && batch >= 1 && T >= 1 &&
                   (long long)batch * T < (1ll << 30),
@@ -709,9 +709,7 @@ extern "C" int q_prompt_pass(const q_prompt_t* p, const q_layer_weights_t* layer
     if (!last) TRY(q_rmsnorm(p->x, gain, p->normed, rows, H, p->rms_eps, stream));
   }
   // the last position of every sequence (only these rows need the final norm)
-  const size_t row = (size_t)H * 2;
-  const char* src = (const char*)(few ? p->normed : p->x) + (size_t)(T - 1) * row;
-  Q_CHECK_CUDA(cudaMemcpy2DAsync(d_last, row, src, (size_t)T * row, row, batch, cudaMemcpyDeviceToDevice, st));
-  if (!few) TRY(q_rmsnorm(d_last, p->ln_final, d_last, batch, H, p->rms_eps, stream));
+  TRY(q_rmsnorm_strided((const char*)p->x + (size_t)(T - 1) * H * 2, (long long)T * H, p->ln_final, d_last, batch, H,
+                        p->rms_eps, stream));
   return Q_OK;
 }

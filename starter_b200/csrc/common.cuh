@@ -132,6 +132,10 @@ int q_gemm_launch_planned(const void* d_x, const void* d_w_tiled, float* d_parti
 int q_gemm_tc_launch(const void* d_x, const void* d_w_tc, float* d_partials, const q_gemm_plan_t* plan,
                      void* stream);
 
+// RMSNorm of `rows` rows that lie `stride` elements apart, into consecutive rows.
+int q_rmsnorm_strided(const void* d_x, long long stride, const void* d_gain, void* d_out, int rows, int cols,
+                      float eps, void* stream);
+
 // Leading bytes of q_gemm_prompt_*'s scratch that have to be zero before a launch.
 int64_t q_gemm_prompt_ticket_bytes();
 

@@ -23,12 +23,12 @@ __device__ __forceinline__ void arg_better(float& bv, int& bi, float v, int i) {
 // ---- RMSNorm (plain) -------------------------------------------------------
 __global__ void __launch_bounds__(256)
 k_rmsnorm(const bf16* __restrict__ X, const bf16* __restrict__ G, bf16* __restrict__ O,
-          int cols, float eps) {
+          int cols, long long stride, float eps) {
   __shared__ float red[32];
   pdl_launch_dependents();
   pdl_wait();
   const size_t row = blockIdx.x;
-  const bf16* x = X + row * cols;
+  const bf16* x = X + row * stride;
   float ss = 0.f;
   for (int c = threadIdx.x; c < cols; c += blockDim.x) {
     float v = __bfloat162float(x[c]);
@@ -637,9 +637,11 @@ k_logits_argmax(const float* __restrict__ P, PlanView pv, bf16* __restrict__ log
     const bool two = pv.u != 0;
     for (int c = c0 + 4 * threadIdx.x; c < c0 + ARG_COLS && c < vocab; c += 1024) {
       const float4 a = *reinterpret_cast<const float4*>(p0 + c);
-      const float4 b = two ? *reinterpret_cast<const float4*>(p0 + c + pv.slot_stride)
-                           : make_float4(0.f, 0.f, 0.f, 0.f);
+      // Few rows: the second slot is asked for without looking (one round trip). Many rows: a slot
+      // is 39 MB at 64 rows, only what holds a partial is read.
       const int extra = plan_count(pv, c, row) - 1;
+      const float4 b = two && (gridDim.y <= 8 || extra > 0) ? *reinterpret_cast<const float4*>(p0 + c + pv.slot_stride)
+                                                            : make_float4(0.f, 0.f, 0.f, 0.f);
       float s[4] = {a.x, a.y, a.z, a.w};
       if (extra > 0) { s[0] += b.x; s[1] += b.y; s[2] += b.z; s[3] += b.w; }
       for (int k = 2; k <= extra; ++k) {
@@ -769,7 +771,14 @@ extern "C" int q_rmsnorm(const void* d_x, const void* d_gain, void* d_out, int r
     return Q_OK;
   }
   Q_CHECK_CUDA(q_launch(k_rmsnorm, dim3(rows), dim3(256), 0, S(stream), (const bf16*)d_x,
-                        (const bf16*)d_gain, (bf16*)d_out, cols, eps));
+                        (const bf16*)d_gain, (bf16*)d_out, cols, (long long)cols, eps));
+  return Q_OK;
+}
+
+int q_rmsnorm_strided(const void* d_x, long long stride, const void* d_gain, void* d_out, int rows, int cols,
+                      float eps, void* stream) {
+  Q_CHECK_CUDA(q_launch(k_rmsnorm, dim3(rows), dim3(256), 0, S(stream), (const bf16*)d_x,
+                        (const bf16*)d_gain, (bf16*)d_out, cols, stride, eps));
   return Q_OK;
 }
 

@@ -657,6 +657,12 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
   tl_end(tl);
 }
 
+int pair_count() {
+  const int sms = q_sm_count();
+  const int pairs = (sms > 0 ? sms : 148) / 2;
+  return pairs < PG_MAX_PAIRS ? pairs : PG_MAX_PAIRS;
+}
+
 // `N` as in PromptShape; the weight has `wN` rows.
 template <int EPI>
 int launch_prompt(const void* x, const void* w_tc, void* out, int M, int N, int wN, int K, const RopeArgs& ra,
@@ -669,7 +675,6 @@ int launch_prompt(const void* x, const void* w_tc, void* out, int M, int N, int 
               "%s: x and scratch must be 16-byte, the output 32-byte and the tiled weight 1024-byte aligned", who);
   int* status = q_tc_status_addr();
   if (!status) { q_set_error("%s: could not locate the device status word", who); return Q_ERR_CUDA; }
-  const int sms = q_sm_count();
   PromptShape sh;
   sh.M = M; sh.N = N;
   sh.KT = (K + PG_TILE_K - 1) / PG_TILE_K;
@@ -680,7 +685,7 @@ int launch_prompt(const void* x, const void* w_tc, void* out, int M, int N, int 
   Q_CHECK_ARG(tiles * sh.KT < (1ll << 30), "%s: too many tiles", who);
   sh.wrows = 128;
   while (EPI == EPI_SWIGLU && N % sh.wrows) sh.wrows >>= 1;
-  int pairs = sms / 2 < PG_MAX_PAIRS ? sms / 2 : PG_MAX_PAIRS;
+  int pairs = pair_count();
   // Whole tiles only, or the last wave and the remainder cut evenly: the split saves the idle part of
   // a wave (k steps of ~0.4 us each) and costs parts through L2 and a late epilogue, PG_SPLIT_STEPS.
   const int full = (int)(tiles / pairs), rest = (int)(tiles % pairs);
@@ -724,7 +729,7 @@ int launch_prompt(const void* x, const void* w_tc, void* out, int M, int N, int 
 int64_t q_gemm_prompt_ticket_bytes() { return (int64_t)PG_TICKET_BYTES; }
 
 extern "C" int64_t q_gemm_prompt_scratch_bytes(void) {
-  return (int64_t)(PG_TICKET_BYTES + (size_t)PG_MAX_PAIRS * 2 * PG_PART_FLOATS * 4);
+  return (int64_t)(PG_TICKET_BYTES + (size_t)pair_count() * 2 * PG_PART_FLOATS * 4);
 }
 
 extern "C" int q_gemm_prompt_f32(const void* d_x, const void* d_w_tc, float* d_out, int M, int N, int K,

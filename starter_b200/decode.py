@@ -278,13 +278,15 @@ class DecodeState:
             "q": torch.empty((rows, nq, HEAD_DIM), **bf), "att": torch.empty((rows, nq * HEAD_DIM), **bf),
             "act": torch.empty((rows, inter), **bf), "zero": torch.zeros(1, **i32),
             "reduced": torch.empty((rows, cfg.hidden), **f32) if self.tp > 1 else None,
-            "split": torch.zeros(lib.q_gemm_prompt_scratch_bytes(), **u8),
+            "split": torch.empty(lib.q_gemm_prompt_scratch_bytes() if rows >= self.PROMPT_GEMM_ROWS else 0, **u8),
             "partials": torch.empty(max(p.slots * p.M * p.N for p in plans), **f32),
             "last": torch.empty((B, cfg.hidden), **bf), "head_plan": hp,
             "head": torch.empty((hp.slots, B, vocab), **f32), "val": torch.empty(B, **f32), "idx": torch.empty(B, **i32),
             "arg_scratch": torch.zeros(lib.q_argmax_scratch_bytes(B, vocab), **u8),
         }
-        if self.tp == 1:
+        if self.tp > 1:
+            pf["split"].zero_()
+        else:
             pf["layers"] = (_lib.LayerWeights * cfg.n_layers)(*[
                 _lib.LayerWeights(lt.wqkv.data_ptr(), lt.wo.data_ptr(), lt.wgu.data_ptr(), lt.wdown.data_ptr(),
                                   lt.ln_in.data_ptr(), lt.ln_post.data_ptr(), lt.q_gain.data_ptr(), lt.k_gain.data_ptr(),
