@@ -194,8 +194,17 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
   tc_fence_after();
   // All 512 columns are this CTA's, so its tensor memory starts at column 0.
   constexpr uint32_t tmem = 0;
-  pdl_wait();                                              // q and this pass's K/V rows
+  // Position and block table were written by earlier steps: read before the wait, like the decode
+  // kernel does (two round trips that a short prompt would see in full).
   const int pos = pos_ptr[0];
+  int first_page[2] = {0, 0};
+  if (warp == 16) {
+    const Item it = item_at(sh, item_of(0), pos);          // the grid has at most one CTA per item
+    const int32_t* table = block_table + (size_t)it.b * sh.pages_per_seq;
+    first_page[0] = table[0];
+    if (it.max_limit > Q_PAGE_TOKENS) first_page[1] = table[1];
+  }
+  pdl_wait();                                              // q and this pass's K/V rows
 
   if (warp == 16) {
     // ---------------- producer ----------------
@@ -221,7 +230,8 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
           const int s = step & 1;
           const uint32_t parity = ((step >> 1) & 1) ^ 1;
           const int np = min(2, npages - 2 * j);
-          const int page0 = table[2 * j], page1 = np > 1 ? table[2 * j + 1] : 0;
+          const int page0 = step ? table[2 * j] : first_page[0];
+          const int page1 = np < 2 ? 0 : step ? table[2 * j + 1] : first_page[1];
           for (int kv = 0; kv < 2; ++kv) {
             if (!mbar_wait(bar(kv ? B_VE : B_KE, s), parity, abort_flag)) { fail(); break; }
             const uint32_t full = bar(kv ? B_VF : B_KF, s);

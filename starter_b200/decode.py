@@ -103,6 +103,7 @@ class DecodeState:
         handle = C.c_void_p()
         check(lib.q_create(C.byref(ccfg), C.byref(handle)))
         self.handle = handle
+        self.layer_structs = []
         for i, lt in enumerate(weights.layers):
             lw = _lib.LayerWeights(lt.wqkv.data_ptr(), lt.wo.data_ptr(), lt.wgu.data_ptr(),
                                    lt.wdown.data_ptr(), lt.ln_in.data_ptr(), lt.ln_post.data_ptr(),
@@ -111,6 +112,7 @@ class DecodeState:
                                    *((lt.wqkv.tc().data_ptr(), lt.wo.tc().data_ptr(), lt.wgu.tc().data_ptr(),
                                       lt.wdown.tc().data_ptr()) if use_tc else (0, 0, 0, 0)))
             check(lib.q_bind_layer(handle, i, C.byref(lw)))
+            self.layer_structs.append(lw)
 
         bf = dict(dtype=torch.bfloat16, device=dev)
         f32 = dict(dtype=torch.float32, device=dev)
@@ -287,12 +289,9 @@ class DecodeState:
         if self.tp > 1:
             pf["split"].zero_()
         else:
-            pf["layers"] = (_lib.LayerWeights * cfg.n_layers)(*[
-                _lib.LayerWeights(lt.wqkv.data_ptr(), lt.wo.data_ptr(), lt.wgu.data_ptr(), lt.wdown.data_ptr(),
-                                  lt.ln_in.data_ptr(), lt.ln_post.data_ptr(), lt.q_gain.data_ptr(), lt.k_gain.data_ptr(),
-                                  self.kpools[i].data_ptr(), self.vpools[i].data_ptr(), lt.wqkv.tc().data_ptr(),
-                                  lt.wo.tc().data_ptr(), lt.wgu.tc().data_ptr(), lt.wdown.tc().data_ptr())
-                for i, lt in enumerate(w.layers)])
+            pf["layers"] = (_lib.LayerWeights * cfg.n_layers)(*self.layer_structs)
+            for lw, tiled in zip(pf["layers"], w.tc_layers):
+                lw.wqkv_tc, lw.wo_tc, lw.wgu_tc, lw.wdown_tc = (t.data_ptr() for t in tiled)
             pf["prompt"] = _lib.Prompt(cfg.hidden, inter, cfg.n_layers, nq, nkv, cfg.vocab, self.PROMPT_GEMM_ROWS,
                                        cfg.rms_eps, float(HEAD_DIM) ** -0.5, w.embed.data_ptr(), w.ln_final.data_ptr(),
                                        self.cos.data_ptr(), self.sin.data_ptr(),

@@ -217,6 +217,7 @@ class PackedWeights:
     ln_final: torch.Tensor
     device: torch.device = None
     layers: list[LayerTensors] = field(default_factory=list)
+    tc_layers: "list | None" = None     # per layer (wqkv, wo, wgu, wdown) in the tcgen05 tiling, once built
 
     @property
     def local_q_heads(self) -> int:
@@ -261,10 +262,11 @@ class PackedWeights:
     def ensure_tc(self) -> None:
         """Builds the tcgen05 tiling of every matrix (steps with 9 rows and more, the prompt
         pass). Doubles the weight bytes held in HBM."""
-        for lt in self.layers:
-            for name in ("wqkv", "wo", "wgu", "wdown"):
-                getattr(lt, name).tc()
+        if self.tc_layers is not None:
+            return
+        layers = [tuple(getattr(lt, name).tc() for name in ("wqkv", "wo", "wgu", "wdown")) for lt in self.layers]
         self.lm_head.tc()
+        self.tc_layers = layers
 
     @property
     def has_tc(self) -> bool:
