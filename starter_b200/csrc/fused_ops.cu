@@ -48,13 +48,13 @@ k_rmsnorm(const bf16* __restrict__ X, const bf16* __restrict__ G, bf16* __restri
 template <int VECS>
 __global__ void __launch_bounds__(256)
 k_rmsnorm_rows(const bf16* __restrict__ X, const bf16* __restrict__ G, bf16* __restrict__ O,
-               int rows, int cols, float eps) {
+               int rows, int cols, long long stride, float eps) {
   pdl_launch_dependents();
   pdl_wait();
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (row >= rows) return;
-  const uint4* x = reinterpret_cast<const uint4*>(X + (size_t)row * cols);
+  const uint4* x = reinterpret_cast<const uint4*>(X + (size_t)row * stride);
   const uint4* g = reinterpret_cast<const uint4*>(G);
   uint4* o = reinterpret_cast<uint4*>(O + (size_t)row * cols);
   const int vecs = cols >> 3;
@@ -760,25 +760,28 @@ extern "C" int q_rmsnorm(const void* d_x, const void* d_gain, void* d_out, int r
   Q_CHECK_ALIGN(d_x, 2, "q_rmsnorm"); Q_CHECK_ALIGN(d_gain, 2, "q_rmsnorm"); Q_CHECK_ALIGN(d_out, 2, "q_rmsnorm");
   // Many rows: a warp each (k_rmsnorm_rows). Few rows leave most SMs idle that way, so up to two
   // rows per SM keep a whole CTA; so do odd widths and unaligned rows.
-  if (rows > 296 && cols % 8 == 0 && cols <= 4096 &&
-      (((uintptr_t)d_x | (uintptr_t)d_gain | (uintptr_t)d_out) & 15) == 0) {
-    if (cols <= 2560)
-      Q_CHECK_CUDA(q_launch(k_rmsnorm_rows<10>, dim3((rows + 7) / 8), dim3(256), 0, S(stream), (const bf16*)d_x,
-                            (const bf16*)d_gain, (bf16*)d_out, rows, cols, eps));
-    else
-      Q_CHECK_CUDA(q_launch(k_rmsnorm_rows<16>, dim3((rows + 7) / 8), dim3(256), 0, S(stream), (const bf16*)d_x,
-                            (const bf16*)d_gain, (bf16*)d_out, rows, cols, eps));
-    return Q_OK;
-  }
+  if (rows > 296) return q_rmsnorm_strided(d_x, cols, d_gain, d_out, rows, cols, eps, stream);
   Q_CHECK_CUDA(q_launch(k_rmsnorm, dim3(rows), dim3(256), 0, S(stream), (const bf16*)d_x,
                         (const bf16*)d_gain, (bf16*)d_out, cols, (long long)cols, eps));
   return Q_OK;
 }
 
+// (the prompt pass norms one row per sequence with it: 16-byte loads in one round trip, where the
+// CTA per row of k_rmsnorm took 10 us for one cold row of 2560)
 int q_rmsnorm_strided(const void* d_x, long long stride, const void* d_gain, void* d_out, int rows, int cols,
                       float eps, void* stream) {
-  Q_CHECK_CUDA(q_launch(k_rmsnorm, dim3(rows), dim3(256), 0, S(stream), (const bf16*)d_x,
-                        (const bf16*)d_gain, (bf16*)d_out, cols, stride, eps));
+  const bool vec = cols % 8 == 0 && stride % 8 == 0 && cols <= 4096 &&
+                   (((uintptr_t)d_x | (uintptr_t)d_gain | (uintptr_t)d_out) & 15) == 0;
+  const dim3 grid((rows + 7) / 8);
+  if (vec && cols <= 2560)
+    Q_CHECK_CUDA(q_launch(k_rmsnorm_rows<10>, grid, dim3(256), 0, S(stream), (const bf16*)d_x, (const bf16*)d_gain,
+                          (bf16*)d_out, rows, cols, stride, eps));
+  else if (vec)
+    Q_CHECK_CUDA(q_launch(k_rmsnorm_rows<16>, grid, dim3(256), 0, S(stream), (const bf16*)d_x, (const bf16*)d_gain,
+                          (bf16*)d_out, rows, cols, stride, eps));
+  else
+    Q_CHECK_CUDA(q_launch(k_rmsnorm, dim3(rows), dim3(256), 0, S(stream), (const bf16*)d_x, (const bf16*)d_gain,
+                          (bf16*)d_out, cols, stride, eps));
   return Q_OK;
 }
 
