@@ -317,11 +317,19 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
             if (j == 0 && !wait(bar(B_OE, i), (nitems & 1) ^ 1)) break;
             // P comes in two halves of 64 keys, from different warps
             if (!wait(bar(B_P, 2 * i), vstep & 1) || !wait(bar(B_P, 2 * i + 1), vstep & 1)) break;
+            const int keys = cur.max_limit - j * AP_KEYS;      // in the last tile, k steps past the newest key are left out
             if (elect_one()) {
+              if (keys >= AP_KEYS) {
 #pragma unroll
-              for (int ks = 0; ks < 8; ++ks)
-                tc_mma_ta(tmem + 256u + 128u * i, tmem + 128u * i + 8u * ks,
-                          v_desc + (uint64_t)(vs * (AP_TILE >> 4) + ks * (2048 >> 4)), idesc_pv, (j | ks) ? 1u : 0u);
+                for (int ks = 0; ks < 8; ++ks)
+                  tc_mma_ta(tmem + 256u + 128u * i, tmem + 128u * i + 8u * ks,
+                            v_desc + (uint64_t)(vs * (AP_TILE >> 4) + ks * (2048 >> 4)), idesc_pv, (j | ks) ? 1u : 0u);
+              } else {
+#pragma unroll 1
+                for (int ks = 0; 16 * ks < keys; ++ks)
+                  tc_mma_ta(tmem + 256u + 128u * i, tmem + 128u * i + 8u * ks,
+                            v_desc + (uint64_t)(vs * (AP_TILE >> 4) + ks * (2048 >> 4)), idesc_pv, (j | ks) ? 1u : 0u);
+              }
             }
             __syncwarp();
             if (!ok) break;
@@ -401,13 +409,13 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
 #pragma unroll
           for (int k = 0; k < 64; ++k) v[k] = k < vis ? v[k] : -INFINITY;
         }
-        if (tid < 128 && key_base + AP_KEYS > it.max_limit) {
-          // V rows past the newest key hold stale bits (0 * garbage could be NaN): clear them
-          // before the first product with this tile may start
+        if (tid < 128 && key_base + AP_KEYS > it.max_limit && (it.max_limit & 15)) {
+          // V rows past the newest key hold stale bits (0 * garbage could be NaN): clear those of its
+          // k step before the first product with this tile may start
           wait(bar(B_VF, step & 1), (step >> 1) & 1);
           unsigned char* vt = smem + AP_V + (step & 1) * AP_TILE;
           const int live = it.max_limit - key_base;
-          for (int q = tid; !broken && q < (128 - live) * 16; q += 128) {
+          for (int q = tid; !broken && q < ((16 - live) & 15) * 16; q += 128) {
             const int kr = live + (q >> 4);
             *reinterpret_cast<uint4*>(vt + (q & 8 ? AP_HALF : 0u) + kr * 128 + ((q & 7) << 4)) = make_uint4(0, 0, 0, 0);
           }

@@ -283,9 +283,12 @@ class DecodeState:
             "split": torch.empty(lib.q_gemm_prompt_scratch_bytes() if rows >= self.PROMPT_GEMM_ROWS else 0, **u8),
             "partials": torch.empty(max(p.slots * p.M * p.N for p in plans), **f32),
             "last": torch.empty((B, cfg.hidden), **bf), "head_plan": hp,
-            "head": torch.empty((hp.slots, B, vocab), **f32), "val": torch.empty(B, **f32), "idx": torch.empty(B, **i32),
-            "arg_scratch": torch.zeros(lib.q_argmax_scratch_bytes(B, vocab), **u8),
+            "head": torch.empty((hp.slots, B, vocab), **f32),
+            "val": self.arg_val, "idx": self.arg_idx, "arg_scratch": self.arg_scratch,
         }
+        if self.rows != B:                 # (the scratch layout goes by the row count)
+            pf.update(val=torch.empty(B, **f32), idx=torch.empty(B, **i32),
+                      arg_scratch=torch.zeros(lib.q_argmax_scratch_bytes(B, vocab), **u8))
         if self.tp > 1:
             pf["split"].zero_()
         else:
