@@ -371,10 +371,13 @@ def kernels_per_step(state) -> int:
     """Launches of this library's kernels in one decode step (NCCL's are not counted)."""
     L, rows = state.cfg.n_layers, state.rows
     if state.tp == 1:
-        if rows <= 8:
+        if rows <= 2:
             # embed, first QKV | attention, O, gate|up (add+norm prologue, SwiGLU epilogue), down,
             # next QKV or lm_head (add+norm prologue) | argmax
             return 2 + 5 * L + 1
+        if rows <= 8:
+            # embed | QKV, attention, O, add+norm, gate|up (SwiGLU epilogue), down, add+norm | lm_head, argmax
+            return 1 + 7 * L + 2
         # embed | QKV, attention, O, add+norm, gate|up, SwiGLU, down, add+norm | lm_head, argmax
         return 1 + 8 * L + 2
     if state.peers:

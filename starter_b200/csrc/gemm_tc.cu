@@ -1,5 +1,6 @@
 // Weight-streaming GEMM on the 5th-generation tensor cores (tcgen05.mma, accumulators in
-// tensor memory) for 9 .. 256 activation rows.
+// tensor memory) for 9 .. 256 activation rows (more run as row chunks of 256; the prompt pass uses
+// gemm_prompt.cu from 257 rows on).
 //
 // Y[M,N] = X[M,K] . W[N,K]^T, bf16 operands, fp32 accumulation, written as the same fp32
 // split-K partial slots that the stream-K kernel of gemm_streamk.cu produces, so the fused
