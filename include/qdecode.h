@@ -298,6 +298,8 @@ int q_kv_scatter(const void* d_k, const void* d_v, const q_kv_layout_t* kv,
  *   d_scratch_ml: float[batch*n_kv][splits][T*G][2]
  * q_attention_splits returns the split count to size those for a capacity. */
 int q_attention_splits(int batch, int n_kv_heads, int capacity);
+/* The same for q_attention with `rows` = T*G query rows per kv head. */
+int q_attention_block_splits(int batch, int n_kv_heads, int capacity, int rows);
 /* The same for q_attention_decode, whose splits merge in thread-block clusters. */
 int q_attention_decode_splits(int batch, int n_kv_heads, int capacity);
 

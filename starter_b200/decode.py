@@ -126,9 +126,9 @@ class DecodeState:
             raise _lib.QDecodeError("could not size the split-K partial buffer")
         self.partials = torch.empty(n_part, **f32)
         self.reduced = torch.zeros((rows, cfg.hidden), **f32) if self.tp > 1 else None
-        splits = lib.q_attention_decode_splits if q_tokens == 1 else lib.q_attention_splits
-        self.attn_splits = splits(batch, nkv, self.capacity)
         g = nq // nkv
+        self.attn_splits = (lib.q_attention_decode_splits(batch, nkv, self.capacity) if q_tokens == 1 else
+                            lib.q_attention_block_splits(batch, nkv, self.capacity, q_tokens * g))
         self.attn_o = torch.empty((batch * nkv, self.attn_splits, q_tokens * g, HEAD_DIM), **f32)
         self.attn_ml = torch.empty((batch * nkv, self.attn_splits, q_tokens * g, 2), **f32)
         self.attn_tickets = torch.zeros(batch * nkv, dtype=torch.int32, device=dev)
@@ -265,7 +265,7 @@ class DecodeState:
         if getattr(self, "_pf", None) is not None and self._pf["rows"] >= rows:
             return self._pf
         cfg, w, dev, B = self.cfg, self.w, self.device, self.batch
-        nq, nkv, inter, vocab = w.local_q_heads, w.local_kv_heads, w.local_inter, w.local_vocab
+        nq, nkv, inter = w.local_q_heads, w.local_kv_heads, w.local_inter
         bf, f32, i32 = (dict(dtype=t, device=dev) for t in (torch.bfloat16, torch.float32, torch.int32))
         u8 = dict(dtype=torch.uint8, device=dev)
         self._pf = None                    # release the previous size first
@@ -273,7 +273,6 @@ class DecodeState:
         shapes = (((nq + 2 * nkv) * HEAD_DIM, cfg.hidden), (cfg.hidden, nq * HEAD_DIM), (2 * inter, cfg.hidden),
                   (cfg.hidden, inter))
         plans = [_lib.plan(few, n, k, tc=True) for n, k in shapes]
-        hp = _lib.plan(B, vocab, cfg.hidden, tc=True)
         pf = {
             "rows": rows,
             "x": torch.empty((rows, cfg.hidden), **bf), "normed": torch.empty((rows, cfg.hidden), **bf),
@@ -282,19 +281,14 @@ class DecodeState:
             "reduced": torch.empty((rows, cfg.hidden), **f32) if self.tp > 1 else None,
             "split": torch.empty(lib.q_gemm_prompt_scratch_bytes() if rows >= self.PROMPT_GEMM_ROWS else 0, **u8),
             "partials": torch.empty(max(p.slots * p.M * p.N for p in plans), **f32),
-            "last": torch.empty((B, cfg.hidden), **bf), "head_plan": hp,
-            "head": torch.empty((hp.slots, B, vocab), **f32),
-            "val": self.arg_val, "idx": self.arg_idx, "arg_scratch": self.arg_scratch,
+            "last": torch.empty((B, cfg.hidden), **bf),
         }
-        if self.rows != B:                 # (the scratch layout goes by the row count)
-            pf.update(val=torch.empty(B, **f32), idx=torch.empty(B, **i32),
-                      arg_scratch=torch.zeros(lib.q_argmax_scratch_bytes(B, vocab), **u8))
         if self.tp > 1:
             pf["split"].zero_()
         else:
             pf["layers"] = (_lib.LayerWeights * cfg.n_layers)(*self.layer_structs)
             for lw, tiled in zip(pf["layers"], w.tc_layers):
-                lw.wqkv_tc, lw.wo_tc, lw.wgu_tc, lw.wdown_tc = (t.data_ptr() for t in tiled)
+                lw.wqkv_tc, lw.wo_tc, lw.wgu_tc, lw.wdown_tc = tiled
             pf["prompt"] = _lib.Prompt(cfg.hidden, inter, cfg.n_layers, nq, nkv, cfg.vocab, self.PROMPT_GEMM_ROWS,
                                        cfg.rms_eps, float(HEAD_DIM) ** -0.5, w.embed.data_ptr(), w.ln_final.data_ptr(),
                                        self.cos.data_ptr(), self.sin.data_ptr(),
@@ -302,6 +296,17 @@ class DecodeState:
                                                                     "partials", "split")))
         self._pf = pf
         return pf
+
+    def _prefill_head(self, pf) -> None:
+        """The lm_head buffers of the prompt pass: made while the layers already run."""
+        B, vocab, dev = self.batch, self.w.local_vocab, self.device
+        hp = pf["head_plan"] = _lib.plan(B, vocab, self.cfg.hidden, tc=True)
+        pf["head"] = torch.empty((hp.slots, B, vocab), dtype=torch.float32, device=dev)
+        pf.update(val=self.arg_val, idx=self.arg_idx, arg_scratch=self.arg_scratch)
+        if self.rows != B:                 # (the scratch layout goes by the row count)
+            pf.update(val=torch.empty(B, dtype=torch.float32, device=dev),
+                      idx=torch.empty(B, dtype=torch.int32, device=dev),
+                      arg_scratch=torch.zeros(lib.q_argmax_scratch_bytes(B, vocab), dtype=torch.uint8, device=dev))
 
     def prefill(self, input_ids: torch.Tensor) -> torch.Tensor:
         """Runs the whole prompt, fills the KV pages, leaves the first generated token in
@@ -329,9 +334,8 @@ class DecodeState:
         per = max(1, self.PREFILL_ROWS // T)                 # sequences per pass
         stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
         ids = input_ids.contiguous()
-        logits = torch.empty((B, w.local_vocab), dtype=torch.bfloat16, device=self.device)
         pf = self._prefill_scratch(min(per, B) * T)
-        last, hp = pf["last"], pf["head_plan"]
+        last = pf["last"]
         for b0 in range(0, B, per):
             nb = min(per, B - b0)
             table = self.block_table.data_ptr() + b0 * self.pages_per_seq * 4
@@ -345,7 +349,10 @@ class DecodeState:
             layers(pf, nb, T, table, stream)
             last[b0:b0 + nb].copy_(pf["normed"][:nb * T].view(nb, T, H)[:, -1])
         # lm_head on the last position of every sequence, logits rounded once to bf16
-        val, idx = pf["val"], pf["idx"]
+        logits = torch.empty((B, w.local_vocab), dtype=torch.bfloat16, device=self.device)
+        if "head" not in pf:
+            self._prefill_head(pf)
+        hp, val, idx = pf["head_plan"], pf["val"], pf["idx"]
         check(lib.q_gemm_tc(_p(last), _p(w.lm_head.tc()), _p(pf["head"]), B, w.local_vocab, H, stream))
         check(lib.q_logits_argmax(_p(pf["head"]), C.byref(hp), _p(logits), _p(val), _p(idx),
                                   _p(self.tokens) if self.tp == 1 else None, None, 0, _p(pf["arg_scratch"]), B,

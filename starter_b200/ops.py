@@ -323,8 +323,8 @@ class SmallQueryAttention:
         self.batch, self.hq, self.hk, self.capacity = batch, query_heads, kv_heads, capacity
         self.T = tokens_per_seq
         self.groups = query_heads // kv_heads
-        self.splits = lib.q_attention_splits(batch, kv_heads, capacity)
         rows = self.T * self.groups
+        self.splits = lib.q_attention_block_splits(batch, kv_heads, capacity, rows)
         self.partials = torch.empty((batch * kv_heads, self.splits, rows, HEAD_DIM),
                                     dtype=torch.float32, device=device)
         self.stats = torch.empty((batch * kv_heads, self.splits, rows, 2),

@@ -217,7 +217,7 @@ class PackedWeights:
     ln_final: torch.Tensor
     device: torch.device = None
     layers: list[LayerTensors] = field(default_factory=list)
-    tc_layers: "list | None" = None     # per layer (wqkv, wo, wgu, wdown) in the tcgen05 tiling, once built
+    tc_layers: "list | None" = None     # per layer the addresses of (wqkv, wo, wgu, wdown) in the tcgen05 tiling, once built
 
     @property
     def local_q_heads(self) -> int:
@@ -264,7 +264,7 @@ class PackedWeights:
         pass). Doubles the weight bytes held in HBM."""
         if self.tc_layers is not None:
             return
-        layers = [tuple(getattr(lt, name).tc() for name in ("wqkv", "wo", "wgu", "wdown")) for lt in self.layers]
+        layers = [tuple(getattr(lt, name).tc().data_ptr() for name in ("wqkv", "wo", "wgu", "wdown")) for lt in self.layers]
         self.lm_head.tc()
         self.tc_layers = layers
 

@@ -17,6 +17,9 @@ def test_split_count_is_usable(batch, kv_heads):
         s = lib.q_attention_decode_splits(batch, kv_heads, capacity)
         assert 1 <= s <= 32 and s <= max(1, (capacity + 63) // 64)
         assert s == 1 or s * batch * kv_heads <= 2 * 148
+        assert lib.q_attention_block_splits(batch, kv_heads, capacity, 16) == lib.q_attention_splits(batch, kv_heads, capacity)
+        b = lib.q_attention_block_splits(batch, kv_heads, capacity, 17)      # one CTA per SM
+        assert 1 <= b <= 32 and b <= max(1, (capacity + 63) // 64) and (b == 1 or b * batch * kv_heads <= 148)
 
 
 def test_prompt_entry_points_reject_bad_arguments():
