@@ -53,7 +53,7 @@ constexpr int PG_STAGES = 7;                               // 224 KB
 constexpr size_t PG_SMEM = 1024 + PG_STAGES * PG_STAGE + (2 * PG_STAGES + 4) * 8 + 16;
 constexpr int PG_GROUP = 8;                                // row tiles per raster group
 constexpr int PG_MAX_PAIRS = 128;
-constexpr int PG_SPLIT_STEPS = 20;
+constexpr int PG_SPLIT_STEPS = 60;                         // what a split costs, in k steps
 // scratch: tickets (16 warps per tile, at most two tiles per pair), then two parts per pair
 constexpr size_t PG_TICKET_BYTES = PG_MAX_PAIRS * 2 * 16 * 4;
 constexpr size_t PG_PART_FLOATS = 256 * 256;
@@ -687,7 +687,9 @@ int launch_prompt(const void* x, const void* w_tc, void* out, int M, int N, int 
   while (EPI == EPI_SWIGLU && N % sh.wrows) sh.wrows >>= 1;
   int pairs = pair_count();
   // Whole tiles only, or the last wave and the remainder cut evenly: the split saves the idle part of
-  // a wave (k steps of ~0.4 us each) and costs parts through L2 and a late epilogue, PG_SPLIT_STEPS.
+  // a wave (k steps of ~0.4 us each) and costs parts through L2, tickets, the merge and a late epilogue.
+  // Split / whole, us: QKV at 1024 rows (52 against 80 steps) 39.3 / 34.9, O at 400 (9 against 64)
+  // 29.4 / 25.3, down at 1500 (123 against 152) 70.2 / 58.8, but down at 1024 (83 against 152) 50.3 / 57.0.
   const int full = (int)(tiles / pairs), rest = (int)(tiles % pairs);
   sh.waves = full;
   sh.share = sh.KT;

@@ -46,10 +46,10 @@ def scratch(request, ops):
 
 
 # one row; rows around one CTA, one tile and a raster group of eight row tiles; columns of less than
-# a tile; K of less than a 64-k step, odd and long. With scratch: one tile cut over many pairs, few
-# tiles over all pairs, one wave and a remainder, and shapes that stay whole.
+# a tile; K of less than a 64-k step, odd and long. With scratch: few tiles cut over all pairs,
+# shares of more than a tile, a whole wave before the split, and shapes that stay whole.
 SHAPES = [(256, 256, 512), (1, 32, 32), (128, 128, 64), (129, 160, 96), (257, 2560, 416), (700, 96, 4096),
-          (1000, 2560, 9728), (2103, 2560, 4096), (2305, 4896, 160)]
+          (1000, 2560, 9728), (2048, 2560, 9728), (3800, 2560, 8192), (2103, 2560, 4096), (2305, 4896, 160)]
 
 
 @pytest.mark.parametrize("M,N,K", SHAPES)
@@ -74,12 +74,15 @@ def test_sums_and_residual(ops, scratch, M, N, K):
     assert ops.device_status() == [0, 0, 0, 0]
 
 
-@pytest.mark.parametrize("M,inter,K", [(1, 32, 32), (300, 96, 128), (257, 1184, 416), (600, 9728, 256), (900, 1312, 2560)])
+@pytest.mark.parametrize("M,inter,K", [(1, 32, 32), (300, 96, 128), (257, 1184, 416), (600, 9728, 256), (600, 1312, 9728)])
 def test_swiglu(ops, scratch, M, inter, K):
     """Within one bf16 rounding of the oracle's SwiGLU of the fp32 sums (inter not a multiple of 128
     puts the up rows across the 128-row weight blocks)."""
     from starter_b200._lib import check, lib
-    x, w = rand((M, K), 4, 1.0), rand((2 * inter, K), 5, 0.05)
+    # Gate sums of standard deviation 0.8, so |g| < 4: where the two fp32 sums round to neighbouring bf16
+    # values of g, silu moves by at most ulp(g) * |silu'(g) / silu(g)| <= 2^-7 * 1.02 of itself there
+    # (at g = -16 one step of g already moves silu by 6 %, whatever the kernel does).
+    x, w = rand((M, K), 4, 1.0), rand((2 * inter, K), 5, 0.8 * K ** -0.5)
     xd, tiled = x.cuda(), ops.pack_weight_tc(w.cuda())
     act = torch.full((M + 2, inter), float("nan"), dtype=torch.bfloat16, device="cuda")
     check(lib.q_gemm_prompt_swiglu(P(xd), P(tiled.data), P(act), M, inter, K, P(scratch), stream()))
@@ -90,12 +93,12 @@ def test_swiglu(ops, scratch, M, inter, K):
     assert ops.device_status() == [0, 0, 0, 0]
 
 
-@pytest.mark.parametrize("B,T,nq,nkv,pos", [(1, 1, 1, 1, 0), (2, 130, 4, 2, 70), (3, 301, 8, 1, 0), (1, 1000, 32, 8, 5), (1, 2000, 32, 8, 0)])
+@pytest.mark.parametrize("B,T,nq,nkv,pos", [(1, 1, 1, 1, 0), (2, 130, 4, 2, 70), (3, 301, 8, 1, 0), (1, 1000, 32, 8, 5), (1, 250, 32, 8, 0)])
 def test_qkv_norm_rope_pages(ops, scratch, B, T, nq, nkv, pos):
     """q, k within the bar of the separate kernel, v exact; only the slots of this block are written
     in the NaN-poisoned pages."""
     from starter_b200._lib import check, lib
-    width, K, rows = (nq + 2 * nkv) * 128, 2560 if T == 2000 else 128, B * T
+    width, K, rows = (nq + 2 * nkv) * 128, 9728 if T == 250 else 128, B * T
     w, x = rand((width, K), 6, 0.02), rand((rows, K), 7, 4.0)
     qg, kg = gain(128, 8), gain(128, 9)
     capacity = pos + T + 70
