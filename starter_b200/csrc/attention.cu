@@ -925,17 +925,21 @@ static int resident_clusters(bool wide, int splits, int sms) {
 
 extern "C" int q_attention_block_splits(int batch, int n_kv_heads, int capacity, int rows) {
   // More than 16 query rows per kv head take k_attn_split<2>, whose registers leave room for one CTA
-  // per SM: splits beyond that are a second wave. Verification step of 4 layers, new / old count, us:
-  // 3 x 5 tokens at 4 K keys 445 / 466, 6 x 8 at 500 457 / 482, 1 x 6 at 8 K 389 / 409, 8 x 8 at 4 K
-  // 571 / 594, 2 x 8 at 1 K 420 / 423.
+  // per SM: the count with the fewest (waves x pages of a split), where starting and merging a CTA
+  // costs about four pages. Verification step of 4 layers, this count / two CTAs per SM, us: 3 x 5
+  // tokens at 4 K keys 445 / 466, 6 x 8 at 500 457 / 482, 1 x 6 at 8 K 389 / 409, 8 x 8 at 4 K 571 / 594.
   const int s = q_attention_splits(batch, n_kv_heads, capacity);
   if (rows <= 16 || batch < 1 || n_kv_heads < 1 || capacity < 1) return s;
   int sms = q_sm_count();
   if (sms <= 0) sms = 148;
-  const int tiles = (capacity + Q_PAGE_TOKENS - 1) / Q_PAGE_TOKENS;
-  int n = sms / (batch * n_kv_heads);
-  n = n < 1 ? 1 : n > 32 ? 32 : n;
-  return n < tiles ? n : tiles;
+  const long long tiles = ((long long)capacity + Q_PAGE_TOKENS - 1) / Q_PAGE_TOKENS;
+  long long best = 1, cost = -1;
+  for (long long n = 1; n <= 32 && n <= tiles; ++n) {
+    const long long waves = (n * batch * n_kv_heads + sms - 1) / sms;
+    const long long c = waves * ((tiles + n - 1) / n + 4);
+    if (cost < 0 || c < cost) { cost = c; best = n; }
+  }
+  return (int)best;
 }
 
 extern "C" int q_attention_decode_splits(int batch, int n_kv_heads, int capacity) {

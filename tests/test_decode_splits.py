@@ -18,8 +18,16 @@ def test_split_count_is_usable(batch, kv_heads):
         assert 1 <= s <= 32 and s <= max(1, (capacity + 63) // 64)
         assert s == 1 or s * batch * kv_heads <= 2 * 148
         assert lib.q_attention_block_splits(batch, kv_heads, capacity, 16) == lib.q_attention_splits(batch, kv_heads, capacity)
-        b = lib.q_attention_block_splits(batch, kv_heads, capacity, 17)      # one CTA per SM
-        assert 1 <= b <= 32 and b <= max(1, (capacity + 63) // 64) and (b == 1 or b * batch * kv_heads <= 148)
+        b = lib.q_attention_block_splits(batch, kv_heads, capacity, 17)
+        assert 1 <= b <= 32 and b <= max(1, (capacity + 63) // 64)
+
+
+@pytest.mark.parametrize("batch,capacity,splits", [(6, 512, 3), (6, 10240, 3), (3, 14080, 6), (8, 4096, 2), (7, 16384, 5)])
+def test_block_splits_fill_waves(batch, capacity, splits):
+    """One CTA per SM for more than 16 query rows: one full wave, or two where one would leave a
+    quarter of the SMs idle (148 SMs, 8 kv heads)."""
+    from starter_b200._lib import lib
+    assert lib.q_attention_block_splits(batch, 8, capacity, 32) == splits
 
 
 def test_prompt_entry_points_reject_bad_arguments():
