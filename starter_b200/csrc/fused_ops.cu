@@ -637,11 +637,9 @@ k_logits_argmax(const float* __restrict__ P, PlanView pv, bf16* __restrict__ log
     const bool two = pv.u != 0;
     for (int c = c0 + 4 * threadIdx.x; c < c0 + ARG_COLS && c < vocab; c += 1024) {
       const float4 a = *reinterpret_cast<const float4*>(p0 + c);
-      // Few rows: the second slot is asked for without looking (one round trip). Many rows: a slot
-      // is 39 MB at 64 rows, only what holds a partial is read.
+      const float4 b = two ? *reinterpret_cast<const float4*>(p0 + c + pv.slot_stride)
+                           : make_float4(0.f, 0.f, 0.f, 0.f);
       const int extra = plan_count(pv, c, row) - 1;
-      const float4 b = two && (gridDim.y <= 8 || extra > 0) ? *reinterpret_cast<const float4*>(p0 + c + pv.slot_stride)
-                                                            : make_float4(0.f, 0.f, 0.f, 0.f);
       float s[4] = {a.x, a.y, a.z, a.w};
       if (extra > 0) { s[0] += b.x; s[1] += b.y; s[2] += b.z; s[3] += b.w; }
       for (int k = 2; k <= extra; ++k) {
