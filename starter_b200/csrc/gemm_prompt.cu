@@ -486,6 +486,7 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
     // (the whole warp walks the loop and one elected lane issues, so that descriptors live in uniform
     // registers)
     if (rank == 0) {
+      pdl_wait();                                           // as in gemm_tc.cu: the wait limit starts here
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(PG_BN >> 3) << 17) | (16u << 24);
       const uint32_t stage_units = PG_STAGE >> 4;
       const uint64_t desc0 = smem_desc(base);

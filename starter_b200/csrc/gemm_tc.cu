@@ -187,6 +187,9 @@ k_gemm_tc(const __grid_constant__ CUtensorMap xmap, const unsigned char* __restr
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     if (lane == 0) {
+      // Nothing can land in `full` before the activations exist, and the kernel before may wait for a
+      // peer longer than WAIT_CYCLES: the limit starts when that kernel is done.
+      pdl_wait();
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(sh.m_pad >> 3) << 17) |
                              ((uint32_t)(TILE_ROWS >> 4) << 24);     // f32 accum, bf16 x bf16, K-major both
       // Like the producer, this thread's instruction count per tile matters (a loop with

@@ -6,7 +6,10 @@
 
 namespace {
 
-constexpr long long WAIT_CYCLES = 1000000000ll;            // about half a second: the limit of every wait
+// About half a second: the limit of every wait on an mbarrier. It has to cover this kernel's own work
+// only: a kernel before it may wait for a late peer much longer (option peer_wait_iters, about 4 s), so
+// every role passes the dependency wait before its first wait that the previous kernel could hold up.
+constexpr long long WAIT_CYCLES = 1000000000ll;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);

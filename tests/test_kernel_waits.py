@@ -1,0 +1,24 @@
+"""Rules that the kernels' waits follow, read from their sources: what goes wrong without them shows
+only under a timing that a test cannot make (or should not make on a GPU)."""
+import re
+from pathlib import Path
+
+CSRC = Path(__file__).resolve().parents[1] / "starter_b200" / "csrc"
+
+
+def source(name):
+    return re.sub(r"//[^\n]*", "", (CSRC / name).read_text())
+
+
+def between(text, start, end):
+    a = text.index(start)
+    return text[a:text.index(end, a)]
+
+
+def test_mma_roles_start_their_limit_after_the_dependency_wait():
+    """A projection launched early behind a kernel that polls a late peer (up to about 4 s) must not
+    count that time against its own half second."""
+    for name in ("gemm_tc.cu", "gemm_prompt.cu"):
+        role = between(source(name), "} else if (warp == 1) {", "  } else {\n")
+        assert "pdl_wait();" in role, f"{name}: the MMA role never passes the dependency wait"
+        assert role.index("pdl_wait();") < role.index("mbar_wait("), f"{name}: a bounded wait comes before it"

@@ -1,5 +1,7 @@
 """The tcgen05 projection (q_gemm_tc, 9 rows and more) through the C ABI against the CPU
 oracle: the 128 x 64 weight tiling, the partial slots, and the fused consumers reading them."""
+from types import SimpleNamespace
+
 import pytest
 import torch
 
@@ -156,3 +158,54 @@ def test_tc_gemm_rejects_bad_operands(ops):
     with pytest.raises(ValueError, match="aligned"):       # a weight that is not 1024-byte aligned
         _lib.check(_lib.lib.q_gemm_tc(C.c_void_p(x.data_ptr()), C.c_void_p(wt.data_ptr() + 16),
                                       C.c_void_p(out.data_ptr()), 12, 16, 64, None))
+
+
+@pytest.mark.parametrize("form", ["rows", "pairs"])
+def test_projection_behind_a_kernel_that_waits_for_a_late_peer(ops, form):
+    """The add+norm exchange may poll a late peer for about 4 s; the projection after it, whose CTAs
+    are already resident then, must not count that against its own half second. On one GPU, with a
+    world of two whose second rank never writes: the exchange gives up after a second or two (word
+    3), the projection behind it reports nothing and multiplies what the exchange left."""
+    import ctypes as C
+    from starter_b200 import _lib
+    lib, check = _lib.lib, _lib.check
+    rows, K, N = 9, 2560, 256                                  # few CTAs: both kernels fit on the GPU together
+    recv = 2 * 2 * 2 * rows * K
+    buf = torch.zeros(recv + lib.q_peer_flag_bytes() // 4, dtype=torch.float32, device="cuda")
+    counters = torch.zeros(4, dtype=torch.int32, device="cuda")
+    peers = _lib.Peers()
+    peers.rank, peers.world = 0, 2
+    for r in range(2):
+        peers.partials[r] = buf.data_ptr()
+        peers.flags[r] = buf.data_ptr() + recv * 4
+    peers.epoch = counters.data_ptr()
+    P = lambda t: C.c_void_p(t.data_ptr())
+    x, own = torch.zeros((rows, K), dtype=torch.bfloat16, device="cuda"), randx(rows, K, 11).float().cuda()
+    gain = torch.ones(K, dtype=torch.bfloat16, device="cuda")
+    total, normed = torch.empty_like(x), torch.empty_like(x)
+    w = randw(N, K, 12)
+    tiled = ops.pack_weight_tc(w.cuda())
+    plan = _lib.plan(rows, N, K, tc=True)
+    part = torch.empty((plan.slots if form == "rows" else 1, rows, N), dtype=torch.float32, device="cuda")
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    ops.clear_status()
+    check(lib.q_set_option(b"peer_wait_iters", 700_000))
+    try:
+        begin.record()
+        check(lib.q_add_rmsnorm_peers(P(x), C.byref(peers), P(own), None, P(gain), P(total), P(normed), rows, K, 1e-6,
+                                      stream))
+        if form == "rows":
+            check(lib.q_gemm_tc(P(normed), P(tiled.data), P(part), rows, N, K, stream))
+        else:
+            check(lib.q_gemm_prompt_f32(P(normed), P(tiled.data), P(part), rows, N, K, None, stream))
+        end.record()
+        torch.cuda.synchronize()
+    finally:
+        check(lib.q_set_option(b"peer_wait_iters", 1 << 21))
+    status = ops.device_status()
+    ops.clear_status()
+    assert begin.elapsed_time(end) > 800.0                     # longer than the projection's own limit
+    assert status == [0, 0, 0, 1]
+    got = sum_slots(SimpleNamespace(data=part, plan=plan)) if form == "rows" else part[0].cpu()
+    torch.testing.assert_close(got, O.linear_fp32(normed.cpu(), w), rtol=2e-3, atol=2e-3)
