@@ -256,9 +256,10 @@ typedef struct q_kv_layout_t {
  *   q_gemm_prompt_qkv     q_qkv_norm_rope_cache of the [q | k | v] sums: q_out [rows][n_q][128],
  *                         k and v rows of positions *d_pos .. *d_pos+T-1 into their pages (cos /
  *                         sin tables and pools 32-byte aligned)
- * d_scratch: q_gemm_prompt_scratch_bytes() bytes, 16-byte aligned, the first 16 KB zeroed once by the
- * caller (every launch leaves them zero), for the parts of tiles that several SM pairs share; one
- * per stream, since calls that overlap on the GPU may not share it. Null: whole tiles only. */
+ * d_scratch: q_gemm_prompt_scratch_bytes() bytes, 16-byte aligned, the first 16 KB zeroed by the
+ * caller before the first launch and after one that gave up (device status word 2; every other
+ * launch leaves them zero), for the parts of tiles that several SM pairs share; one per stream,
+ * since calls that overlap on the GPU may not share it. Null: whole tiles only. */
 int64_t q_gemm_prompt_scratch_bytes(void);
 int q_gemm_prompt_f32(const void* d_x, const void* d_w_tc, float* d_out, int M, int N, int K,
                       void* d_scratch, void* stream);

@@ -36,7 +36,8 @@
 // up with a part of a tile stores its fp32 accumulator in the caller's scratch, draws a ticket, and
 // the LAST of a tile's pairs adds the parts in k order (its own included, so the sum does not depend
 // on who is last), puts the total back into tensor memory and runs the epilogue. Nobody waits. The
-// unit of all this is a warp: 32 rows x 2 x 64 columns.
+// unit of all this is a warp: 32 rows x 2 x 64 columns. A launch that gives up leaves tickets drawn, so
+// the prompt pass clears them before each run of layers.
 #include "tc.cuh"
 
 int* q_tc_status_addr();
@@ -56,6 +57,7 @@ constexpr int PG_MAX_PAIRS = 128;
 constexpr int PG_SPLIT_STEPS = 60;                         // what a split costs, in k steps
 // scratch: tickets (16 warps per tile, at most two tiles per pair), then two parts per pair
 constexpr size_t PG_TICKET_BYTES = PG_MAX_PAIRS * 2 * 16 * 4;
+static_assert(PG_TICKET_BYTES == 16384, "stated in qdecode.h");
 constexpr size_t PG_PART_FLOATS = 256 * 256;
 
 enum { EPI_F32 = 0, EPI_RESID = 1, EPI_SWIGLU = 2, EPI_ROPE = 3 };

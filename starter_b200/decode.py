@@ -259,6 +259,7 @@ class DecodeState:
     # ---- prefill: the prompt pass ----
     PREFILL_ROWS = 8192        # prompt rows processed together (bounds the activation scratch)
     PROMPT_GEMM_ROWS = 257     # rows from which the projections run on the CTA-pair kernel
+    PROMPT_TICKET_BYTES = 16384    # leading bytes of q_gemm_prompt_*'s scratch that have to be zero
 
     def _prefill_scratch(self, rows: int):
         """Buffers of the prompt pass for up to `rows` rows at a time, kept for the next call."""
@@ -283,9 +284,7 @@ class DecodeState:
             "partials": torch.empty(max(p.slots * p.M * p.N for p in plans), **f32),
             "last": torch.empty((B, cfg.hidden), **bf),
         }
-        if self.tp > 1:
-            pf["split"].zero_()
-        else:
+        if self.tp == 1:
             pf["layers"] = (_lib.LayerWeights * cfg.n_layers)(*self.layer_structs)
             for lw, tiled in zip(pf["layers"], w.tc_layers):
                 lw.wqkv_tc, lw.wo_tc, lw.wgu_tc, lw.wdown_tc = tiled
@@ -372,6 +371,8 @@ class DecodeState:
         nq, nkv, inter = w.local_q_heads, w.local_kv_heads, w.local_inter
         H, eps, rows = cfg.hidden, float(cfg.rms_eps), nb * T
         x, normed, q, att, act, split = (_p(pf[n]) for n in ("x", "normed", "q", "att", "act", "split"))
+        # (as q_prompt_pass does: a launch that gave up leaves tickets drawn)
+        pf["split"][:self.PROMPT_TICKET_BYTES].zero_()
         zero, scale = _p(pf["zero"]), float(HEAD_DIM) ** -0.5
 
         def add_norm(inp, weight, K, gain):

@@ -197,3 +197,39 @@ def test_a_wrong_shard_fails_every_rank():
 def test_a_rank_that_never_arrives_is_named():
     out = _run_failure_case("absent")
     assert "rank(s) [1] of 2 did not arrive at 'step0'" in out[0], out
+
+
+def test_prompt_pass_clears_tickets_of_a_launch_that_gave_up(monkeypatch):
+    """The tensor-parallel prompt pass hands q_gemm_prompt_* a scratch whose tickets are zero in every
+    run of layers, whatever an earlier launch that gave up left there; the rest of the scratch stays.
+    (The library's calls are recorded, nothing runs.)"""
+    from types import SimpleNamespace as NS
+    from starter_b200 import decode
+    cfg = NS(n_layers=2, hidden=64, rms_eps=1e-6)
+    weight = NS(tc=lambda: torch.zeros(1))
+    layer = NS(wqkv=weight, wo=weight, wgu=weight, wdown=weight, q_gain=torch.zeros(1), k_gain=torch.zeros(1),
+               ln_in=torch.zeros(1), ln_post=torch.zeros(1))
+    pool = [torch.zeros(1)] * cfg.n_layers
+    state = NS(cfg=cfg, w=NS(local_q_heads=2, local_kv_heads=1, local_inter=64, layers=[layer] * 2, ln_final=torch.zeros(1)),
+               kpools=pool, vpools=pool, pages_per_seq=1, cos=torch.zeros(1), sin=torch.zeros(1), group=None,
+               PROMPT_TICKET_BYTES=16384)
+    pf = {n: torch.zeros(4) for n in ("x", "normed", "q", "att", "act", "zero")}
+    pf["reduced"] = torch.zeros((300, cfg.hidden))
+    pf["split"] = torch.empty(decode.lib.q_gemm_prompt_scratch_bytes(), dtype=torch.uint8)
+    seen = []
+
+    class Recorder:
+        def __getattr__(self, name):
+            def call(*args):
+                if name.startswith("q_gemm_prompt"):
+                    seen.append((name, bool(pf["split"][:16384].any()), bool(pf["split"][16384:].all())))
+                return 0
+            return call
+
+    monkeypatch.setattr(decode, "lib", Recorder())
+    monkeypatch.setattr(torch.distributed, "all_reduce", lambda t, group=None: None)
+    for _ in range(2):
+        pf["split"].fill_(3)                                   # what a launch that gave up may leave
+        decode.DecodeState._prefill_layers(state, pf, 1, 300, 0, None)
+    assert len(seen) == 2 * 4 * cfg.n_layers
+    assert all(not drawn and kept for _, drawn, kept in seen)
