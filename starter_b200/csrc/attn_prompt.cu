@@ -343,9 +343,11 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
             }
           }
           if (!ok) break;
-          if (elect_one()) {
+          // (not after the last tile: nobody waits for it any more, and the arrival could find that the
+          // CTA has left)
+          if (ahead && elect_one()) {
             tc_commit(bar(B_VE, vs));
-            if (ahead) tc_commit(bar(B_KE, kstep & 1));
+            tc_commit(bar(B_KE, kstep & 1));
           }
           __syncwarp();
           ++vstep;

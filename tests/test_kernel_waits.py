@@ -22,3 +22,15 @@ def test_mma_roles_start_their_limit_after_the_dependency_wait():
         role = between(source(name), "} else if (warp == 1) {", "  } else {\n")
         assert "pdl_wait();" in role, f"{name}: the MMA role never passes the dependency wait"
         assert role.index("pdl_wait();") < role.index("mbar_wait("), f"{name}: a bounded wait comes before it"
+
+
+def test_prompt_attention_commits_nothing_that_nobody_waits_for():
+    """The softmax warps wait for the last products' B_OF commit and then the CTA leaves: a commit issued
+    after it would arrive in shared memory that may be another CTA's by then. The stage releases come
+    after it, so the last tile has none."""
+    text = source("attn_prompt.cu")
+    loop = text[text.index("tc_commit(bar(B_OF, i))"):]
+    release = loop.index("tc_commit(bar(B_VE, vs))")
+    guard = loop.rindex("if (", 0, release)
+    assert loop[guard:].startswith("if (ahead && elect_one()) {")
+    assert loop.count("tc_commit(bar(B_VE") == 1
