@@ -34,3 +34,17 @@ def test_prompt_attention_commits_nothing_that_nobody_waits_for():
     guard = loop.rindex("if (", 0, release)
     assert loop[guard:].startswith("if (ahead && elect_one()) {")
     assert loop.count("tc_commit(bar(B_VE") == 1
+
+
+def test_tensor_memory_loads_are_tied_to_their_wait():
+    """A memory clobber does not order register arithmetic: the registers of a tensor-memory load are
+    safe only if the wait is part of the same statement, or if they are pinned after it."""
+    statements = [s.split(");\n")[0] for name in ("tc.cuh", "gemm_tc.cu", "gemm_prompt.cu", "attn_prompt.cu")
+                  for s in source(name).split("asm volatile(")[1:]]
+    loads = [s for s in statements if "tcgen05.ld." in s]
+    waiting = [s for s in loads if "tcgen05.wait::ld" in s]
+    assert len(loads) == 3 and len(waiting) == 2, "a tensor-memory load without its wait"
+    # the third, tc_ld32 of the prompt attention: two loads in flight, one wait, both arrays pinned behind it
+    text = re.sub(r"\s+", " ", source("attn_prompt.cu"))
+    assert text.count("tc_ld32(") == 3
+    assert "tc_ld32(s_addr, v); tc_ld32(s_addr + 32, v + 32); tc_wait_ld(); tc_pin32(v); tc_pin32(v + 32);" in text
