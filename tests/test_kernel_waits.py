@@ -48,3 +48,12 @@ def test_tensor_memory_loads_are_tied_to_their_wait():
     text = re.sub(r"\s+", " ", source("attn_prompt.cu"))
     assert text.count("tc_ld32(") == 3
     assert "tc_ld32(s_addr, v); tc_ld32(s_addr + 32, v + 32); tc_wait_ld(); tc_pin32(v); tc_pin32(v + 32);" in text
+
+
+def test_prompt_attention_reads_its_inputs_after_the_dependency_wait():
+    """*d_pos and the block table may come from the caller's kernel right before, which may have released
+    its dependents early: nothing is read from global memory before the dependency wait."""
+    text = source("attn_prompt.cu")
+    kernel = text[text.index("__global__"):]
+    before = kernel[kernel.index("pdl_launch_dependents();"):kernel.index("pdl_wait();")]
+    assert not re.search(r"pos_ptr|block_table|table\[", before)
