@@ -102,10 +102,9 @@ def test_live_random_models(cuda, tmp_path, nq, nkv, hidden, inter, vocab, layer
 
 
 def test_long_prompts_through_the_prompt_pass(cuda, tmp_path):
-    """Prompts longer than one row chunk of the tcgen05 projection (256), longer than the
-    prompt-pass row budget (2048: one sequence per pass then) and several sequences per pass,
-    with 8 query heads per kv head: the own causal attention and the many-row partial plans
-    against native Hugging Face."""
+    """Prompts of more than 256 rows (the projections on CTA pairs), one and several sequences, with
+    8 query heads per kv head, against native Hugging Face. (In several passes:
+    test_prompt_pass_in_several_chunks.)"""
     from transformers import Qwen3Config, Qwen3ForCausalLM
     from starter_b200 import Engine
     torch.manual_seed(77)
@@ -121,6 +120,49 @@ def test_long_prompts_through_the_prompt_pass(cuda, tmp_path):
         prompt = torch.randint(0, 300, (batch, length), generator=gen).tolist()
         tokens, logits = stepwise_logits(engine, prompt, count)
         assert_parity(native, prompt, tokens, logits)
+
+
+@pytest.mark.parametrize("batch,length,budget", [
+    (3, 250, 600),       # 500 rows on CTA pairs, then 250 on split-K partials
+    (5, 257, 600),       # 514, 514, and one sequence of the fewest rows on CTA pairs
+    (3, 700, 1500),      # 1400 and 700 rows
+    (4, 100, 150),       # a sequence at a time, each on split-K partials
+])
+def test_prompt_pass_in_several_chunks(cuda, tmp_path, batch, length, budget):
+    """A prompt whose rows exceed PREFILL_ROWS goes through the layers a few sequences at a time: the
+    later chunks' block tables and last rows, a last chunk on the other projection route, and buffers
+    kept from a larger chunk. Against the pass in one piece and against native Hugging Face."""
+    from starter_b200 import Engine
+    from starter_b200.decode import DecodeState
+    path = _live_model(tmp_path, 8, 1, 256, 384, 300, 2, 78, positions=1024)
+    engine, native = Engine(path), O.native_model(path)
+    prompt = torch.randint(0, 300, (batch, length), generator=torch.Generator().manual_seed(length))
+    ids = prompt.cuda()
+
+    def run(state):
+        for pool in state.kpools + state.vpools:
+            pool.fill_(float("nan"))
+        logits = state.prefill(ids).float().cpu()
+        assert int(state.position.item()) == length
+        pages = [p.view(batch, -1, 1, 64, 128)[:, :, 0].reshape(batch, -1, 128) for p in state.kpools + state.vpools]
+        assert all(torch.isnan(p[:, length:].float()).all() for p in pages)
+        return logits, state.tokens.cpu(), torch.stack([p[:, :length] for p in pages]).cpu()
+
+    with torch.inference_mode():
+        whole = DecodeState(engine.weights, batch, length, 1)
+        want, tokens, pages = run(whole)
+        whole.PREFILL_ROWS = budget
+        kept, kept_tokens, kept_pages = run(whole)             # in chunks, on the buffers of the whole pass
+        chunked = DecodeState(engine.weights, batch, length, 1)
+        chunked.PREFILL_ROWS = budget
+        got, got_tokens, got_pages = run(chunked)
+    assert torch.equal(got, kept) and torch.equal(got_tokens, kept_tokens)
+    assert torch.equal(got_pages.view(torch.int16), kept_pages.view(torch.int16))
+    # another split of K in the projections: two roundings of bf16 (2^-8 each) either way, twice over
+    torch.testing.assert_close(got_pages.float(), pages.float(), rtol=2 ** -6, atol=2 ** -6)
+    assert float((got - want).abs().max()) <= TOL
+    for t, lg in ((tokens, want), (got_tokens, got)):
+        assert_parity(native, prompt.tolist(), [t.tolist()], lg[None])
 
 
 def test_generate_contract_and_graph_replay(cuda, golden_dir):
@@ -167,14 +209,14 @@ def test_zero_lm_head_yields_token_zero_and_never_stops(cuda, golden_dir, tmp_pa
 
 
 def test_norm_prologue_step_matches_separate_add_norm_kernels(cuda, golden_dir):
-    """Default step (add + norm inside the consuming projection, up to 8 rows) against the
+    """Default step of one and two rows (add + norm inside the consuming projection) against the
     step with separate add+norm launches: same tokens, logits equal up to the reduction
     order of the sum of squares."""
     from starter_b200 import Engine, _lib
     from starter_b200.ops import device_status
     engine = Engine(str(golden_dir / "tiny_qwen3"), keep_logits=True)
     gen = torch.Generator().manual_seed(22)
-    for batch, length, count in ((1, 9, 12), (4, 70, 8), (8, 5, 6)):
+    for batch, length, count in ((1, 9, 12), (2, 70, 8)):
         prompt = torch.randint(0, 127, (batch, length), generator=gen).tolist()
         new_tokens, new_logits = stepwise_logits(engine, prompt, count)
         _lib.check(_lib.lib.q_set_option(b"norm_in_gemm", 0))
@@ -185,6 +227,19 @@ def test_norm_prologue_step_matches_separate_add_norm_kernels(cuda, golden_dir):
         assert new_tokens == old_tokens
         torch.testing.assert_close(new_logits, old_logits, rtol=1.6e-2, atol=2e-3)
     assert device_status() == [0, 0, 0, 0]
+
+
+def test_steps_of_2_to_8_rows_match_native(cuda, golden_dir):
+    """Both sides of the row count from which add + norm is a launch of its own (3), and the most rows
+    of the stream-K projections (8), against native Hugging Face."""
+    from starter_b200 import Engine
+    path = str(golden_dir / "tiny_qwen3")
+    engine, native = Engine(path, keep_logits=True), O.native_model(path)
+    gen = torch.Generator().manual_seed(23)
+    for batch, length, count in ((2, 70, 6), (3, 70, 6), (8, 5, 6)):
+        prompt = torch.randint(0, 127, (batch, length), generator=gen).tolist()
+        tokens, logits = stepwise_logits(engine, prompt, count)
+        assert_parity(native, prompt, tokens, logits)
 
 
 def test_pdl_off_gives_identical_tokens(cuda, golden_dir):
@@ -200,12 +255,12 @@ def test_pdl_off_gives_identical_tokens(cuda, golden_dir):
     assert a == b
 
 
-def _live_model(tmp_path, nq, nkv, hidden, inter, vocab, layers, seed):
+def _live_model(tmp_path, nq, nkv, hidden, inter, vocab, layers, seed, positions=512):
     from transformers import Qwen3Config, Qwen3ForCausalLM
     torch.manual_seed(seed)
     cfg = Qwen3Config(vocab_size=vocab, hidden_size=hidden, intermediate_size=inter,
                       num_hidden_layers=layers, num_attention_heads=nq, num_key_value_heads=nkv,
-                      head_dim=128, max_position_embeddings=512, rope_theta=1_000_000.0,
+                      head_dim=128, max_position_embeddings=positions, rope_theta=1_000_000.0,
                       tie_word_embeddings=True, sliding_window=None)
     Qwen3ForCausalLM(cfg).eval().to(torch.bfloat16).save_pretrained(tmp_path, safe_serialization=True)
     return str(tmp_path)
