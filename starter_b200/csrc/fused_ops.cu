@@ -756,9 +756,12 @@ extern "C" int q_rmsnorm(const void* d_x, const void* d_gain, void* d_out, int r
                          float eps, void* stream) {
   Q_CHECK_ARG(d_x && d_gain && d_out && rows >= 1 && cols >= 1, "q_rmsnorm: bad argument");
   Q_CHECK_ALIGN(d_x, 2, "q_rmsnorm"); Q_CHECK_ALIGN(d_gain, 2, "q_rmsnorm"); Q_CHECK_ALIGN(d_out, 2, "q_rmsnorm");
-  // Many rows: a warp each (k_rmsnorm_rows). Few rows leave most SMs idle that way, so up to two
-  // rows per SM keep a whole CTA; so do odd widths and unaligned rows.
-  if (rows > 296) return q_rmsnorm_strided(d_x, cols, d_gain, d_out, rows, cols, eps, stream);
+  // Many rows: a warp each (k_rmsnorm_rows); odd widths and unaligned rows keep a CTA per row. So do up
+  // to two rows per SM, not for speed - CTA / warp, 2560 columns, us: 16 rows 4.9 / 3.8, 256 6.5 / 4.0,
+  // 400 6.8 / 4.2, 2048 10.2 / 4.4 - but because the two forms add the squares in another order and few
+  // rows are the operator's own use, where there is about a microsecond in it.
+  const int sms = q_sm_count();
+  if (rows > 2 * (sms > 0 ? sms : 148)) return q_rmsnorm_strided(d_x, cols, d_gain, d_out, rows, cols, eps, stream);
   Q_CHECK_CUDA(q_launch(k_rmsnorm, dim3(rows), dim3(256), 0, S(stream), (const bf16*)d_x,
                         (const bf16*)d_gain, (bf16*)d_out, cols, (long long)cols, eps));
   return Q_OK;
