@@ -893,21 +893,23 @@ extern "C" int q_attention_splits(int batch, int n_kv_heads, int capacity) {
   return s;
 }
 
-// Clusters of `splits` CTAs of the decode kernel that the current device holds at once (a cluster
-// stays inside one GPC, so this is less than SMs / splits), asked once per device; without a device
-// the count that the SMs alone would allow.
-static int resident_clusters(bool wide, int splits, int sms) {
-  static int cached[64][2][9];
+// Clusters of `splits` CTAs of the decode kernel (three warp groups or one, with three ring stages or
+// at most two) that the current device holds at once (a cluster stays inside one GPC, so this is less
+// than SMs / splits), asked once per device; without a device the count that the SMs alone would allow.
+static int resident_clusters(bool wide, bool deep, int splits, int sms) {
+  static int cached[64][3][9];
+  const int form = wide ? 0 : deep ? 1 : 2;
+  const int fallback = (wide ? sms : deep ? 2 * sms : 3 * sms) / splits;
   const int dev = q_device_index();
-  if (dev < 0) return (wide ? sms : 2 * sms) / splits;
-  int& n = cached[dev][wide][splits];
+  if (dev < 0) return fallback;
+  int& n = cached[dev][form][splits];
   if (n == 0) {
     static size_t done[2][64] = {{0}};
     int got = 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(splits, 1);
     cfg.blockDim = dim3(wide ? 13 * 32 : 5 * 32);
-    cfg.dynamicSmemBytes = attn_decode_smem(NS);
+    cfg.dynamicSmemBytes = attn_decode_smem(wide || deep ? NS : 2);
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = splits; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
@@ -917,7 +919,7 @@ static int resident_clusters(bool wide, int splits, int sms) {
     if (e == cudaSuccess)
       e = wide ? cudaOccupancyMaxActiveClusters(&got, k_attn_decode<true, 3>, &cfg)
                : cudaOccupancyMaxActiveClusters(&got, k_attn_decode<true, 1>, &cfg);
-    if (e != cudaSuccess) { cudaGetLastError(); got = (wide ? sms : 2 * sms) / splits; }
+    if (e != cudaSuccess) { cudaGetLastError(); got = fallback; }
     n = got > 0 ? got : -1;
   }
   return n;
@@ -943,31 +945,49 @@ extern "C" int q_attention_block_splits(int batch, int n_kv_heads, int capacity,
 }
 
 extern "C" int q_attention_decode_splits(int batch, int n_kv_heads, int capacity) {
+  // Figures: a step of 4 layers, us, contexts in keys; "vh" = sequences x kv heads, the clusters of a launch.
   if (batch < 1 || n_kv_heads < 1 || capacity < 1) return 1;
   int sms = q_sm_count();
   if (sms <= 0) sms = 148;
   const int vh = batch * n_kv_heads;
   const int tiles = (capacity + Q_PAGE_TOKENS - 1) / Q_PAGE_TOKENS;
   // One sequence of a very long context: every SM takes a split (merged through global memory).
-  // Step of 4 layers, 8 kv heads, 18 splits / 8: 357 / 361 us at 8 K keys, but 340 / 331 at 2 K.
+  // 8 kv heads, 18 splits / 8: 247 / 248 at 8 K, 299 / 345 at 30 K, but 226 / 224 at 4 K.
   if (tiles > 96 && sms / vh > MAX_CLUSTER) return sms / vh < 32 ? sms / vh : 32;
+  // From 9 rows on the projections run on k_gemm_tc, whose CTAs leave no room on their SM: all of the
+  // attention starts at once when they end, and clusters of three and more need a tenth of the places
+  // to spare (44 clusters of 3, 45 would fit an idle GPU: 389 at 4 K; of 6 narrow CTAs, 45 again: 348; of 5: 310).
+  const bool after_tc = batch >= 9;
   // One CTA of three warp groups per SM, its splits merging in a cluster, as long as all clusters
   // are resident at once and a split can see three tiles (fewer: the three groups have no work).
-  // Two smaller CTAs per SM, which hold more splits, measured slower up to 9 sequences of 8 kv heads
-  // - 5 sequences, 3 / 7 splits: 350 / 367 us at 700 keys, 368 / 416 at 2 K, 448 / 523 at 8 K - and
-  // clusters that have to wait for a place cost a second pass: 6 sequences, 2 / 3 splits 352 / 378.
+  // Clusters that have to wait for a place cost a second pass: 6 sequences, 2 / 3 splits 352 / 378.
   int s = sms / vh;
   if (s > 8) s = 8;
   if (s > (tiles - 1) / 2) s = (tiles - 1) / 2;
-  for (; s >= 2; --s)
-    if (resident_clusters(true, s, sms) >= vh) return s;
-  // Otherwise two CTAs per SM: 12 sequences, 2 / 3 splits (288 CTAs, not all resident): 421 / 446.
+  while (s >= 2 && resident_clusters(true, true, s, sms) * 10 < vh * (after_tc && s > 2 ? 11 : 10)) --s;
+  if (s >= 2) {
+    // Few clusters of a long context leave a third of the SMs idle; two narrow CTAs on every SM, merged
+    // through memory, pay from 20 tiles a split on. 2 sequences of 8 kv heads, 6 / 18 splits: 253 / 257 at
+    // 4 K, 279 / 273 at 8 K, 415 / 376 at 30 K (more than MAX_CLUSTER splits only: clusters of 9 to 16
+    // find few places, 3 sequences with 12 splits 550 at 30 K against 461 with 5).
+    if (tiles > 20 * s && 2 * sms / vh > MAX_CLUSTER) return 2 * sms / vh;
+    // Behind the stream-K projections, whose CTAs leave room, the wide CTAs start early and win up to 8
+    // sequences - 5 of 8 kv heads, 3 / 7 splits: 231 / 243 at 700, 256 / 292 at 2 K, 335 / 399 at 8 K. Behind
+    // k_gemm_tc they win while a split's tiles go around the three groups once (9 sequences of 4 kv heads,
+    // 3 / 7 splits: 251 / 253 at 400, but 3 / 6 splits 283 / 280 at 2 K, 311 / 301 at 4 K) or where they
+    // fill the SMs (9 sequences of 8 kv heads, 2 / 3 splits: 300 / 304 at 1 K).
+    if (!after_tc || tiles < 3 * s || (s * vh * 10 >= sms * 9 && tiles >= 6 * s)) return s;
+  }
+  // Otherwise two narrow CTAs per SM, three where a split is at most two tiles (a smaller ring), with a
+  // tenth to spare above pairs, which place anywhere: 12 sequences of 8 kv heads, 2 / 3 splits 343 / 387 at
+  // 2 K; 8 at 200 keys, 4 splits of one tile / 3 of two: 227 / 245.
   s = 2 * sms / vh;
   if (s > 8) s = 8;
   if (s > tiles) s = tiles;
-  // (with a tenth to spare above pairs, which place anywhere: 11 sequences, 2 / 3 splits 422 / 439)
-  for (; s >= 2; --s)
-    if (resident_clusters(false, s, sms) * (s > 2 ? 9 : 10) >= vh * 10) return s;
+  for (; s >= 2; --s) {
+    const bool deep = tiles > 2 * s, wide = deep && s * vh <= sms;      // as q_attention_decode launches them
+    if (resident_clusters(wide, deep, s, sms) * 10 >= vh * (s > 2 ? 11 : 10)) return s;
+  }
   return 1;
 }
 

@@ -52,7 +52,24 @@ def test_prompt_entry_points_reject_bad_arguments():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("B,nq,nkv,pos", [(1, 32, 8, 7000), (2, 8, 2, 90), (3, 32, 8, 2000), (5, 32, 8, 700), (6, 32, 8, 700),
+@pytest.mark.parametrize("batch,kv_heads,capacity,splits", [
+    (5, 8, 712, 3), (2, 8, 4012, 6),                    # wide CTAs, their clusters resident
+    (2, 8, 8012, 18), (3, 4, 16012, 24),                # a long context on few clusters: merged through memory
+    (11, 4, 4012, 5), (16, 4, 2012, 4),                 # behind the tcgen05 projections: narrow CTAs
+    (9, 4, 412, 3), (9, 8, 1012, 2),                    # ... but wide ones for few tiles, or where they fill the SMs
+    (8, 8, 212, 4), (9, 8, 412, 4),                     # splits of one or two tiles: three CTAs per SM
+    (12, 8, 2012, 2), (64, 8, 345, 1)])
+def test_split_counts_of_the_measured_rule(batch, kv_heads, capacity, splits):
+    """One shape per line of q_attention_decode_splits, with the count that measured best there or within
+    one per cent of it (148 SMs)."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs CUDA")
+    from starter_b200._lib import lib
+    assert lib.q_attention_decode_splits(batch, kv_heads, capacity) == splits
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,nq,nkv,pos", [(2, 32, 8, 7700), (11, 16, 4, 700), (9, 32, 8, 400), (1, 32, 8, 7000), (2, 8, 2, 90), (3, 32, 8, 2000), (5, 32, 8, 700), (6, 32, 8, 700),
                                           (11, 32, 8, 500), (40, 32, 8, 430), (64, 32, 8, 333)])
 def test_decode_attention_at_its_split_count(B, nq, nkv, pos):
     """The fused decode attention with the splits and the ring it is given in a step - one wide CTA
