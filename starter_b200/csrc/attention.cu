@@ -928,8 +928,10 @@ static int resident_clusters(bool wide, bool deep, int splits, int sms) {
 extern "C" int q_attention_block_splits(int batch, int n_kv_heads, int capacity, int rows) {
   // More than 16 query rows per kv head take k_attn_split<2>, whose registers leave room for one CTA
   // per SM: the count with the fewest (waves x pages of a split), where starting and merging a CTA
-  // costs about four pages. Verification step of 4 layers, this count / two CTAs per SM, us: 3 x 5
+  // costs about seven pages. Verification step of 4 layers, this count / two CTAs per SM, us: 3 x 5
   // tokens at 4 K keys 445 / 466, 6 x 8 at 500 457 / 482, 1 x 6 at 8 K 389 / 409, 8 x 8 at 4 K 571 / 594.
+  // (Seven and not four: waves that gain a page or two lose - 8 x 8 tokens at 16 K keys, 2 splits in one
+  // wave / 9 in four: 100 / 111 us, 16 x 8 1 / 8 splits 190 / 209, 4 x 8 4 / 9 splits 55 / 58.)
   const int s = q_attention_splits(batch, n_kv_heads, capacity);
   if (rows <= 16 || batch < 1 || n_kv_heads < 1 || capacity < 1) return s;
   int sms = q_sm_count();
@@ -938,7 +940,7 @@ extern "C" int q_attention_block_splits(int batch, int n_kv_heads, int capacity,
   long long best = 1, cost = -1;
   for (long long n = 1; n <= 32 && n <= tiles; ++n) {
     const long long waves = (n * batch * n_kv_heads + sms - 1) / sms;
-    const long long c = waves * ((tiles + n - 1) / n + 4);
+    const long long c = waves * ((tiles + n - 1) / n + 7);
     if (cost < 0 || c < cost) { cost = c; best = n; }
   }
   return (int)best;

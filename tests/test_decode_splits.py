@@ -22,10 +22,11 @@ def test_split_count_is_usable(batch, kv_heads):
         assert 1 <= b <= 32 and b <= max(1, (capacity + 63) // 64)
 
 
-@pytest.mark.parametrize("batch,capacity,splits", [(6, 512, 3), (6, 10240, 3), (3, 14080, 6), (8, 4096, 2), (7, 16384, 5)])
+@pytest.mark.parametrize("batch,capacity,splits", [(6, 512, 3), (6, 10240, 3), (3, 14080, 6), (8, 4096, 2), (7, 16384, 5),
+                                                   (8, 16000, 2), (4, 16000, 4), (16, 16000, 1), (5, 32000, 7)])
 def test_block_splits_fill_waves(batch, capacity, splits):
     """One CTA per SM for more than 16 query rows: one full wave, or two where one would leave a
-    quarter of the SMs idle (148 SMs, 8 kv heads)."""
+    quarter of the SMs idle, but no further wave for a page or two (148 SMs, 8 kv heads)."""
     from starter_b200._lib import lib
     assert lib.q_attention_block_splits(batch, 8, capacity, 32) == splits
 
