@@ -297,12 +297,16 @@ int q_kv_scatter(const void* d_k, const void* d_v, const q_kv_layout_t* kv,
  * merges them and rounds once to bf16. out is [batch*T][n_q*128].
  *   d_scratch_o: float[batch*n_kv][splits][T*G][128]
  *   d_scratch_ml: float[batch*n_kv][splits][T*G][2]
- * q_attention_splits returns the split count to size those for a capacity. */
-int q_attention_splits(int batch, int n_kv_heads, int capacity);
-/* The same for q_attention with `rows` = T*G query rows per kv head. */
+ * Any split count from 1 to 32 gives the result; the next two functions return the measured choice
+ * for a capacity, q_attention_block_splits for q_attention with `rows` = T*G query rows per kv head
+ * and q_attention_decode_splits for q_attention_decode (batch = its rows), whose splits can merge in
+ * thread-block clusters. q_attention_splits counts two CTAs per SM and is what the first returns up
+ * to 16 rows. q_attention and q_attention_decode read *d_pos and the block table before their
+ * dependency wait: a kernel of the caller in front of them that writes either must not release its
+ * dependents (programmatic dependent launch) before the write. */
 int q_attention_block_splits(int batch, int n_kv_heads, int capacity, int rows);
-/* The same for q_attention_decode, whose splits merge in thread-block clusters. */
 int q_attention_decode_splits(int batch, int n_kv_heads, int capacity);
+int q_attention_splits(int batch, int n_kv_heads, int capacity);
 
 int q_attention(const void* d_q, const q_kv_layout_t* kv, const int32_t* d_pos,
                 float* d_scratch_o, float* d_scratch_ml, void* d_out,
@@ -313,8 +317,8 @@ int q_attention(const void* d_q, const q_kv_layout_t* kv, const int32_t* d_pos,
  * engine/prefill.py:45-52 calls the library's scaled-dot-product attention there). d_q is
  * [batch*T][n_q][128] bf16 (normed, rotated); the keys and values are read from the pages,
  * which must already hold positions *d_pos .. *d_pos+T-1 of every sequence; row (b,t,head)
- * sees keys [0, *d_pos + t + 1). No split scratch: one CTA per (sequence, kv head, block of
- * 128/G tokens). G = n_q_heads / n_kv_heads must be 1, 2, 4 or 8. out is [batch*T][n_q*128]. */
+ * sees keys [0, *d_pos + t + 1). No split scratch: persistent CTAs walk (sequence, kv head, block
+ * of one or two times 128/G tokens). G = n_q_heads / n_kv_heads must be 1, 2, 4 or 8. out is [batch*T][n_q*128]. */
 int q_attention_prefill(const void* d_q, const q_kv_layout_t* kv, const int32_t* d_pos,
                         void* d_out, int batch, int T, int n_q_heads, float scale,
                         void* stream);

@@ -258,7 +258,10 @@ class DecodeState:
 
     # ---- prefill: the prompt pass ----
     PREFILL_ROWS = 8192        # prompt rows processed together (bounds the activation scratch)
-    PROMPT_GEMM_ROWS = 257     # rows from which the projections run on the CTA-pair kernel
+    # Rows from which the projections run on the CTA-pair kernel: the first that k_gemm_tc cannot hold in
+    # one pass over the weight (256). Prompt pass of 12 layers, k_gemm_tc / pairs, us: 64 rows 1133 / 2091,
+    # 192 1615 / 2058, 256 1856 / 2064, but 257 2232 / 2128, 300 2336 / 2118, 512 2641 / 2220, 1024 4548 / 3230.
+    PROMPT_GEMM_ROWS = 257
     PROMPT_TICKET_BYTES = 16384    # leading bytes of q_gemm_prompt_*'s scratch that have to be zero
 
     def _prefill_scratch(self, rows: int):

@@ -1,5 +1,5 @@
 """The prompt attention kernel where it can go wrong: one and two query tiles per CTA, several items
-per CTA, every head grouping, a maximum that keeps growing (the lazy rescale), scales that are not
+per CTA, every head grouping, a maximum that keeps growing (a rescale of O in every tile), scales that are not
 positive, an output that is only 4-byte aligned."""
 import ctypes as C
 
