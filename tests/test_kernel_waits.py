@@ -57,3 +57,11 @@ def test_prompt_attention_reads_its_inputs_after_the_dependency_wait():
     kernel = text[text.index("__global__"):]
     before = kernel[kernel.index("pdl_launch_dependents();"):kernel.index("pdl_wait();")]
     assert not re.search(r"pos_ptr|block_table|table\[", before)
+
+
+def test_the_wait_on_an_mbarrier_is_one_loop_bounded_by_the_clock():
+    """Every role of the tcgen05 kernels inlines it: a second loop for flag and clock cost a prompt of 64
+    tokens 2 %. Its limit counts cycles, since a try may itself sleep."""
+    body = between(source("tc.cuh"), "bool mbar_wait(", "__device__ __forceinline__ bool mbar_wait_plain(")
+    assert len(re.findall(r"\bfor \(|\bwhile \(", body)) == 1
+    assert "clock64()" in body and "> WAIT_CYCLES" in body and "*abort_flag" in body
