@@ -182,6 +182,27 @@ int q_gemm_tc_plan(int M, int N, int K, q_gemm_plan_t* plan);
 int q_gemm_tc(const void* d_x, const void* d_w_tc, float* d_partials, int M, int N, int K,
               void* stream);
 
+/* ---- whole projections of 1..64 rows with the layer's element-wise work inside -------------
+ * Same weight tiling as q_gemm_tc; N and K multiples of 8 and 64, x, gain and outputs 16-byte
+ * aligned. No partial slots: K is split inside a thread-block cluster and added there.
+ *   q_gemm_rows_f32     out = n @ W^T in fp32                          (W [N][K])
+ *   q_gemm_rows_add     resid = bf16(resid + bf16(x @ W^T)) in place, and into
+ *                       d_ss[q_gemm_rows_parts(M, N, K)][M] the sums of squares of parts of its rows
+ *   q_gemm_rows_swiglu  act = silu(n @ gate^T) * (n @ up^T), W [gate; up] = [2 inter][K]
+ * n = RMSNorm(x) * gain with the row's sum of squares from the `parts` parts in d_ss
+ * (engine/kernels/decode_fused.py:19-44 split between the two projections around it); a null gain
+ * takes x as it is (q_gemm_rows_f32 only).
+ * q_gemm_rows_supported: 1 if the four projections of a layer are all taken at this row count;
+ * q_gemm_rows_parts: 0 if the shape is not. */
+int q_gemm_rows_supported(int M, int hidden, int inter, int q_cols, int qkv_cols);
+int q_gemm_rows_parts(int M, int N, int K);
+int q_gemm_rows_f32(const void* d_x, const void* d_gain, const float* d_ss, int parts,
+                    const void* d_w_tc, float* d_out, int M, int N, int K, float eps, void* stream);
+int q_gemm_rows_add(const void* d_x, const void* d_w_tc, void* d_resid, float* d_ss, int M, int N, int K,
+                    void* stream);
+int q_gemm_rows_swiglu(const void* d_x, const void* d_gain, const float* d_ss, int parts,
+                       const void* d_w_tc, void* d_act, int M, int inter, int K, float eps, void* stream);
+
 /* No counterpart in the reference. d_out[M][N] (fp32) = X . W^T, i.e. q_gemm_splitk
  * followed by q_reduce_partials, for callers that may not allocate device memory
  * (their own pool owns all of it, their runtime forbids allocator calls, or they

@@ -109,6 +109,11 @@ SIGNATURES = {
     "q_unpack_weight_tc": (_I, [_P, _P, _I, _I, _P]),
     "q_gemm_tc_plan": (_I, [_I, _I, _I, _PLAN]),
     "q_gemm_tc": (_I, [_P, _P, _P, _I, _I, _I, _P]),
+    "q_gemm_rows_supported": (_I, [_I, _I, _I, _I, _I]),
+    "q_gemm_rows_parts": (_I, [_I, _I, _I]),
+    "q_gemm_rows_f32": (_I, [_P, _P, _P, _I, _P, _P, _I, _I, _I, _F, _P]),
+    "q_gemm_rows_add": (_I, [_P, _P, _P, _P, _I, _I, _I, _P]),
+    "q_gemm_rows_swiglu": (_I, [_P, _P, _P, _I, _P, _P, _I, _I, _I, _F, _P]),
     "q_gemm_prompt_scratch_bytes": (C.c_int64, []),
     "q_gemm_prompt_f32": (_I, [_P, _P, _P, _I, _I, _I, _P, _P]),
     "q_gemm_prompt_add": (_I, [_P, _P, _P, _I, _I, _I, _P, _P]),

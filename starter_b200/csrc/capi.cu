@@ -384,24 +384,39 @@ static bool peer_exchange_in_gemm(const q_engine* e) {
          e->cfg.hidden <= 3072 && e->p_o.slots <= 2 && e->p_down.slots <= 2 && e->cfg.tp_size <= g_peer_in_gemm;
 }
 
-// attention .. O projection, from the QKV partials in st.partials. o_partials == nullptr: the O
-// projection pushes its partials to the tensor-parallel peers instead (1-8 rows).
-static int attn_after_qkv(q_engine* e, int layer, float* o_partials, void* stream) {
+// Up to 64 rows on one GPU behind the tcgen05 tiling: five launches a layer (gemm_rows.cu).
+static bool rows_path(const q_config_t& c, int rows) {
+  return c.tp_size == 1 && q_gemm_rows_supported(rows, c.hidden, c.inter, c.n_q_heads * 128,
+                                                 (c.n_q_heads + 2 * c.n_kv_heads) * 128);
+}
+
+// Head norm, RoPE, K/V write and attention, from the QKV sums in st.partials (p_qkv null: complete sums,
+// not partial slots).
+static int attention(q_engine* e, int layer, const q_gemm_plan_t* p_qkv, void* stream) {
   const q_config_t& c = e->cfg;
   const q_state_t& s = e->st;
   const q_layer_weights_t& w = e->layers[layer];
   q_kv_layout_t kv = kv_of(e, layer);
   if (e->T == 1 && s.attn_tickets && c.n_q_heads / c.n_kv_heads <= 8) {
     // head norm + RoPE + K/V write + attention + split merge in one launch
-    TRY(q_attention_decode(s.partials, &e->p_qkv, w.q_gain, w.k_gain, s.cos, s.sin, s.pos, &kv, s.attn_o,
+    TRY(q_attention_decode(s.partials, p_qkv, w.q_gain, w.k_gain, s.cos, s.sin, s.pos, &kv, s.attn_o,
                            s.attn_ml, s.attn_tickets, s.attended, s.batch, c.n_q_heads, s.attn_splits,
                            c.attn_scale, c.rms_eps, stream));
   } else {
-    TRY(q_qkv_norm_rope_cache(s.partials, &e->p_qkv, w.q_gain, w.k_gain, s.cos, s.sin, s.pos, s.q, &kv,
+    TRY(q_qkv_norm_rope_cache(s.partials, p_qkv, w.q_gain, w.k_gain, s.cos, s.sin, s.pos, s.q, &kv,
                               s.batch, e->T, c.n_q_heads, c.rms_eps, stream));
     TRY(q_attention(s.q, &kv, s.pos, s.attn_o, s.attn_ml, s.attended, s.batch, e->T, c.n_q_heads,
                     s.attn_splits, c.attn_scale, stream));
   }
+  return Q_OK;
+}
+
+// attention .. O projection, from the QKV partials in st.partials. o_partials == nullptr: the O
+// projection pushes its partials to the tensor-parallel peers instead (1-8 rows).
+static int attn_after_qkv(q_engine* e, int layer, float* o_partials, void* stream) {
+  const q_state_t& s = e->st;
+  const q_layer_weights_t& w = e->layers[layer];
+  TRY(attention(e, layer, &e->p_qkv, stream));
   if (!o_partials) return q_gemm_push(s.attended, w.wo, &e->p_o, &e->peers, stream);
   return project(e, s.attended, w.wo, w.wo_tc, o_partials, e->p_o, stream);
 }
@@ -616,6 +631,24 @@ static int run_layers(q_engine* e, bool advance, void* stream) {
     }
     return head_argmax(e, advance, stream);
   }
+  if (e->tc && rows_path(c, e->rows)) {
+    // The sums of squares of the residual's rows lie behind the QKV sums: their buffer holds two slots of them,
+    // and a row has fewer parts than QKV columns (q_gemm_rows_supported).
+    const int rows = e->rows, q_cols = c.n_q_heads * 128, qkv_cols = e->p_qkv.N;
+    float* ss = s.partials + (size_t)rows * qkv_cols;
+    const int o_parts = q_gemm_rows_parts(rows, c.hidden, q_cols), down_parts = q_gemm_rows_parts(rows, c.hidden, c.inter);
+    for (int l = 0; l < c.n_layers; ++l) {
+      const q_layer_weights_t& w = e->layers[l];
+      TRY(q_gemm_rows_f32(l ? s.x : s.normed, l ? w.ln_in : nullptr, ss, down_parts, w.wqkv_tc, s.partials, rows,
+                          qkv_cols, c.hidden, c.rms_eps, stream));
+      TRY(attention(e, l, nullptr, stream));
+      TRY(q_gemm_rows_add(s.attended, w.wo_tc, s.x, ss, rows, c.hidden, q_cols, stream));
+      TRY(q_gemm_rows_swiglu(s.x, w.ln_post, ss, o_parts, w.wgu_tc, s.act, rows, c.inter, c.hidden, c.rms_eps, stream));
+      TRY(q_gemm_rows_add(s.act, w.wdown_tc, s.x, ss, rows, c.hidden, c.inter, stream));
+    }
+    TRY(q_rmsnorm_strided(s.x, c.hidden, s.ln_final, s.normed, rows, c.hidden, c.rms_eps, stream));
+    return head(e, advance, stream);
+  }
   for (int l = 0; l < c.n_layers; ++l) {
     TRY(attn_block(e, l, s.partials, stream));
     TRY(q_add_rmsnorm(s.x, s.partials, &e->p_o, e->layers[l].ln_post, s.x, s.normed, e->rows,
@@ -679,6 +712,10 @@ extern "C" int q_prompt_pass(const q_prompt_t* p, const q_layer_weights_t* layer
     Q_CHECK_CUDA(cudaMemsetAsync(p->split, 0, (size_t)q_gemm_prompt_ticket_bytes(), st));
   }
   TRY(q_embed_rmsnorm(d_tokens, p->embed, layers[0].ln_in, p->x, p->normed, rows, H, p->vocab, p->rms_eps, stream));
+  const int qkv_cols = (nq + 2 * nkv) * 128;
+  const bool whole = few && q_gemm_rows_supported(rows, H, I, nq * 128, qkv_cols);
+  const int o_parts = whole ? q_gemm_rows_parts(rows, H, nq * 128) : 0, down_parts = whole ? q_gemm_rows_parts(rows, H, I) : 0;
+  float* ss = whole ? p->partials + (size_t)rows * qkv_cols : nullptr;      // as in run_layers
   for (int l = 0; l < p->n_layers; ++l) {
     const q_layer_weights_t& w = layers[l];
     const bool last = l + 1 == p->n_layers;
@@ -686,6 +723,17 @@ extern "C" int q_prompt_pass(const q_prompt_t* p, const q_layer_weights_t* layer
     q_kv_layout_t kv;
     kv.d_kpool = w.kpool; kv.d_vpool = w.vpool; kv.d_block_table = d_block_table;
     kv.pages_per_seq = pages_per_seq; kv.n_kv_heads = nkv;
+    if (whole) {
+      TRY(q_gemm_rows_f32(l ? p->x : p->normed, l ? w.ln_in : nullptr, ss, down_parts, w.wqkv_tc, p->partials, rows,
+                          qkv_cols, H, p->rms_eps, stream));
+      TRY(q_qkv_norm_rope_cache(p->partials, nullptr, w.q_gain, w.k_gain, p->cos, p->sin, p->pos, p->q, &kv, batch, T, nq,
+                                p->rms_eps, stream));
+      TRY(q_attention_prefill(p->q, &kv, p->pos, p->attended, batch, T, nq, p->attn_scale, stream));
+      TRY(q_gemm_rows_add(p->attended, w.wo_tc, p->x, ss, rows, H, nq * 128, stream));
+      TRY(q_gemm_rows_swiglu(p->x, w.ln_post, ss, o_parts, w.wgu_tc, p->act, rows, I, H, p->rms_eps, stream));
+      TRY(q_gemm_rows_add(p->act, w.wdown_tc, p->x, ss, rows, H, I, stream));
+      continue;
+    }
     if (few) {
       TRY(q_gemm_tc_launch(p->normed, w.wqkv_tc, p->partials, &p_qkv, stream));
       TRY(q_qkv_norm_rope_cache(p->partials, &p_qkv, w.q_gain, w.k_gain, p->cos, p->sin, p->pos, p->q, &kv, batch, T,
