@@ -44,20 +44,27 @@ k_rmsnorm(const bf16* __restrict__ X, const bf16* __restrict__ G, bf16* __restri
 
 // The same for whole matrices (the prompt pass): one warp per row, the row in registers, all of
 // its 16-byte loads in flight together and no block barrier. cols a multiple of 8, at most
-// 256 * VECS, 16-byte aligned rows.
-template <int VECS>
+// 256 * VECS, 16-byte aligned rows. EARLY: the gains, which are weights, are asked for before the dependency
+// wait and held (they are cold in a step that streams all weights between two uses): where an SM has no second
+// CTA to run those registers cost nothing.
+template <int VECS, bool EARLY>
 __global__ void __launch_bounds__(256)
 k_rmsnorm_rows(const bf16* __restrict__ X, const bf16* __restrict__ G, bf16* __restrict__ O,
                int rows, int cols, long long stride, float eps) {
   pdl_launch_dependents();
-  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const uint4* g = reinterpret_cast<const uint4*>(G);
+  const int vecs = cols >> 3;
+  uint4 gr[EARLY ? VECS : 1];
+  if (EARLY) {
+#pragma unroll
+    for (int j = 0; j < VECS; ++j) gr[j] = lane + 32 * j < vecs ? __ldg(g + lane + 32 * j) : make_uint4(0, 0, 0, 0);
+  }
+  pdl_wait();
   if (row >= rows) return;
   const uint4* x = reinterpret_cast<const uint4*>(X + (size_t)row * stride);
-  const uint4* g = reinterpret_cast<const uint4*>(G);
   uint4* o = reinterpret_cast<uint4*>(O + (size_t)row * cols);
-  const int vecs = cols >> 3;
   uint4 r[VECS];
   float ss = 0.f;
 #pragma unroll
@@ -73,7 +80,7 @@ k_rmsnorm_rows(const bf16* __restrict__ X, const bf16* __restrict__ G, bf16* __r
 #pragma unroll
   for (int j = 0; j < VECS; ++j) {
     if (lane + 32 * j >= vecs) continue;
-    const uint4 gv = __ldg(g + lane + 32 * j);
+    const uint4 gv = EARLY ? gr[j] : __ldg(g + lane + 32 * j);
     const uint32_t w[4] = {r[j].x, r[j].y, r[j].z, r[j].w}, gw[4] = {gv.x, gv.y, gv.z, gv.w};
     uint32_t q[4];
 #pragma unroll
@@ -774,15 +781,19 @@ int q_rmsnorm_strided(const void* d_x, long long stride, const void* d_gain, voi
   const bool vec = cols % 8 == 0 && stride % 8 == 0 && cols <= 4096 &&
                    (((uintptr_t)d_x | (uintptr_t)d_gain | (uintptr_t)d_out) & 15) == 0;
   const dim3 grid((rows + 7) / 8);
-  if (vec && cols <= 2560)
-    Q_CHECK_CUDA(q_launch(k_rmsnorm_rows<10>, grid, dim3(256), 0, S(stream), (const bf16*)d_x, (const bf16*)d_gain,
-                          (bf16*)d_out, rows, cols, stride, eps));
-  else if (vec)
-    Q_CHECK_CUDA(q_launch(k_rmsnorm_rows<16>, grid, dim3(256), 0, S(stream), (const bf16*)d_x, (const bf16*)d_gain,
-                          (bf16*)d_out, rows, cols, stride, eps));
-  else
+  // Gains held from before the wait / fetched after the sum, cols 2560, us: 300 rows 3.0 / 4.3, 1024 3.4 / 4.8, but
+  // 2048 (256 CTAs) 6.2 / 5.3, 8192 20.5 / 16.4; the one norm of a 64-row decode step 4.1 / 8.7.
+  const int sms = q_sm_count();
+  const bool early = (int)grid.x <= (sms > 0 ? sms : 148);
+  if (vec) {
+    auto kern = cols <= 2560 ? (early ? k_rmsnorm_rows<10, true> : k_rmsnorm_rows<10, false>)
+                             : (early ? k_rmsnorm_rows<16, true> : k_rmsnorm_rows<16, false>);
+    Q_CHECK_CUDA(q_launch(kern, grid, dim3(256), 0, S(stream), (const bf16*)d_x, (const bf16*)d_gain, (bf16*)d_out,
+                          rows, cols, stride, eps));
+  } else {
     Q_CHECK_CUDA(q_launch(k_rmsnorm, dim3(rows), dim3(256), 0, S(stream), (const bf16*)d_x, (const bf16*)d_gain,
                           (bf16*)d_out, cols, stride, eps));
+  }
   return Q_OK;
 }
 
