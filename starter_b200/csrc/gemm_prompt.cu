@@ -8,8 +8,9 @@
 // ends up with its own 128 rows x 256 columns in fp32. What bounds this kernel is operand traffic
 // from L2 into shared memory: per 64 k an SM reads 32 KB for 128 x 256 outputs, two thirds of the
 // bytes per product of the one-CTA kernel of gemm_tc.cu (weights 128 x rows 256 per SM), which is
-// why prompts leave that kernel: 1.4 - 1.5 PFLOP/s against 1.0. (Narrower tiles to fill a wave
-// measured worse: 0.66 PFLOP/s at 160 columns, whose weight rows take five copies per stage.)
+// why prompts leave that kernel: 1.4 - 1.5 PFLOP/s against 1.0. O and down, whose 2560 columns are ten such tiles
+// only, take tiles of 160 columns where these fill the last wave better (a CTA's 80 weight rows come in one or two
+// copies, with a tensor map for each multiple of 16 rows; in five copies of 16 rows they ran at 0.66 PFLOP/s).
 //
 // The epilogue's thread owns one activation row (tensor-memory lane) and walks the columns, so all of these are thread-local:
 //   EPI_F32     fp32 sums                          (before a tensor-parallel all-reduce)
@@ -49,9 +50,10 @@ constexpr int PG_EPI_WARPS = 8;
 constexpr int PG_TILE_K = 64;
 constexpr int PG_A_BYTES = 128 * PG_TILE_K * 2;            // 16 KB of activations per CTA and stage
 constexpr int PG_BN = 256, PG_HALF = 128;                  // columns of a tile, weight rows per CTA
-constexpr uint32_t PG_STAGE = PG_A_BYTES + PG_HALF * PG_TILE_K * 2;
-constexpr int PG_STAGES = 7;                               // 224 KB
-constexpr size_t PG_SMEM = 1024 + PG_STAGES * PG_STAGE + (2 * PG_STAGES + 4) * 8 + 16;
+constexpr int PG_NARROW = 160;                             // ... of a narrow tile: weight rows in runs of 16, see launch_prompt
+__host__ __device__ constexpr uint32_t pg_stage(int bn) { return PG_A_BYTES + bn / 2 * PG_TILE_K * 2; }
+__host__ __device__ constexpr int pg_stages(int bn) { return bn == PG_BN ? 7 : 8; }                     // 224 KB, 208 KB
+constexpr size_t pg_smem(int bn) { return 1024 + pg_stages(bn) * pg_stage(bn) + (2 * pg_stages(bn) + 4) * 8 + 16; }
 constexpr int PG_GROUP = 8;                                // row tiles per raster group
 constexpr int PG_MAX_PAIRS = 128;
 constexpr int PG_SPLIT_STEPS = 60;                         // what a split costs, in k steps
@@ -100,6 +102,11 @@ struct Walk {
     return true;
   }
 };
+
+// The tiled weight with boxes of wrows rows; narrow tiles: of 16, 32, .. 80 rows, since a run of 80 weight rows
+// crosses at most one boundary of a 128-row block.
+template <int BN>
+struct WeightMaps { CUtensorMap m[BN == PG_BN ? 1 : BN / 32]; };
 
 struct RopeArgs {
   const bf16* q_gain; const bf16* k_gain; const bf16* cos; const bf16* sin;
@@ -374,11 +381,14 @@ __device__ __forceinline__ bool merge_parts(const PromptShape& sh, unsigned char
   return true;
 }
 
-template <int EPI>
+template <int EPI, int BN>
 __global__ void __launch_bounds__(PG_THREADS, 1)
-k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, void* __restrict__ out,
-              PromptShape sh, const __grid_constant__ RopeArgs ra, unsigned char* scratch, int* status,
+k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ WeightMaps<BN> wmaps,
+              void* __restrict__ out, PromptShape sh, const __grid_constant__ RopeArgs ra, unsigned char* scratch, int* status,
               unsigned long long* tl) {
+  constexpr int PG_STAGES = pg_stages(BN), HALF = BN / 2;
+  constexpr uint32_t PG_STAGE = pg_stage(BN);
+  constexpr bool NARROW = BN != PG_BN;
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -410,7 +420,7 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (warp == 0 && lane == 0) {
-    prefetch_map(&wmap);
+    if (!NARROW) prefetch_map(&wmaps.m[0]);
     prefetch_map(&xmap);
   }
   if (warp == 1) {
@@ -437,7 +447,7 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
     // ---------------- producer ----------------
     if (lane == 0) {
       const uint32_t full0 = leader_addr(bar_full);
-      const int nload = PG_HALF / sh.wrows;
+      const int nload = NARROW ? 0 : PG_HALF / sh.wrows;
       const uint32_t wbytes = (uint32_t)sh.wrows * 128u;
       int st = 0;
       uint32_t parity = 1;                                  // an untouched stage is free
@@ -451,7 +461,9 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
         locate(t, mi, ni);
         const int row = first_row(mi * 256 + (int)rank * 128, sh.M);
         // first weight row of this CTA's half
-        const int n0 = EPI == EPI_SWIGLU ? (int)rank * sh.N + ni * PG_HALF : ni * PG_BN + (int)rank * PG_HALF;
+        const int n0 = EPI == EPI_SWIGLU ? (int)rank * sh.N + ni * PG_HALF : ni * BN + (int)rank * HALF;
+        // narrow: the rows up to the end of their 128-row block, then the rest
+        const int run = min(HALF, 128 - (n0 & 127));
         for (int kt = k0; kt < k1; ++kt) {
           if (!mbar_wait(bar_empty + 8 * st, parity, abort_flag)) {
             atomicExch(status, 5);
@@ -461,9 +473,14 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
           }
           const uint32_t full = full0 + 8u * st, dst = base + st * PG_STAGE;
           if (rank == 0) mbar_expect_tx(bar_full + 8 * st, 2 * PG_STAGE);
+          if (NARROW) {
+            pair_load_4d(dst + PG_A_BYTES, &wmaps.m[(run >> 4) - 1], 0, n0 & 127, kt, n0 >> 7, full);
+            if (run < HALF)
+              pair_load_4d(dst + PG_A_BYTES + run * 128, &wmaps.m[((HALF - run) >> 4) - 1], 0, 0, kt, (n0 >> 7) + 1, full);
+          }
           for (int j = 0; j < nload; ++j) {
             const int n = n0 + j * sh.wrows;
-            pair_load_4d(dst + PG_A_BYTES + j * wbytes, &wmap, 0, n & 127, kt, n >> 7, full);
+            pair_load_4d(dst + PG_A_BYTES + j * wbytes, &wmaps.m[0], 0, n & 127, kt, n >> 7, full);
           }
           if (!waited) {                                    // weights do not depend on the previous kernel
             pdl_wait();
@@ -489,7 +506,7 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
     // registers)
     if (rank == 0) {
       pdl_wait();                                           // as in gemm_tc.cu: the wait limit starts here
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(PG_BN >> 3) << 17) | (16u << 24);
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | (16u << 24);
       const uint32_t stage_units = PG_STAGE >> 4;
       const uint64_t desc0 = smem_desc(base);
       auto warp_wait = [&](uint32_t b, uint32_t par) {
@@ -533,7 +550,8 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
     pdl_wait();
     const int q = warp & 3, h = (warp - 2) >> 2;
     // the warp's two runs of 64 columns: gate and up columns that belong together, or one head
-    const int ca = EPI == EPI_SWIGLU ? 64 * h : 128 * h, cb = EPI == EPI_SWIGLU ? PG_HALF + 64 * h : ca + 64;
+    const int ca = EPI == EPI_SWIGLU ? 64 * h : HALF * h, cb = EPI == EPI_SWIGLU ? PG_HALF + 64 * h : ca + 64;
+    constexpr int RUNS = HALF / 16;                         // runs of 16 columns of a warp (not EPI_SWIGLU)
     const uint32_t acc_empty0 = leader_addr(bar_acc_empty);
     int seg = 0;
     Walk walk;
@@ -546,13 +564,13 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
       const int row0 = mi * 256 + (int)rank * 128;
       const int m = first_row(row0, sh.M) + q * 32 + lane;
       const bool live = m >= row0 && m < sh.M;
-      const int n0 = EPI == EPI_SWIGLU ? ni * PG_HALF + ca : ni * PG_BN + ca;      // output column of run a
+      const int n0 = EPI == EPI_SWIGLU ? ni * PG_HALF + ca : ni * BN + ca;      // output column of run a
       // operands besides the accumulator: requested now, used after the wait
-      uint32_t res[EPI == EPI_RESID ? 8 : 1][8];
+      uint32_t res[EPI == EPI_RESID ? (RUNS + 1) / 2 * 2 : 1][8];
       bf16* x = reinterpret_cast<bf16*>(out) + (size_t)(live ? m : 0) * sh.N + n0;
       if (EPI == EPI_RESID) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
+        for (int j = 0; j < RUNS; ++j)
           if (n0 + 16 * j < sh.N) ld32B(x + 16 * j, res[j]);
       }
       RotRow rot;
@@ -583,15 +601,16 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)buf * 256u;
       const uint32_t ta = taddr + ca, tb = taddr + cb;
       // (a part of a tile that is not the last one: another pair finishes the tile)
-      const bool whole = k1 - k0 == sh.KT ||
+      const bool whole = NARROW || k1 - k0 == sh.KT ||
                          merge_parts(sh, scratch, ta, tb, pair, t - sh.waves * pairs, ((int)rank * 4 + q) * 2 + h, lane);
       if (whole && n0 < sh.N) {
         if (EPI == EPI_F32) {
           float* dst = reinterpret_cast<float*>(out) + (size_t)m * sh.N + n0;
 #pragma unroll 2
-          for (int c = 0; c < 128 && n0 + c < sh.N; c += 32) {             // N is a multiple of 32
+          for (int c = 0; c < HALF && n0 + c < sh.N; c += 32) {            // N is a multiple of 32
             float v[16], w[16];
             tc_ld16x2(ta + c, ta + c + 16, v, w);
+            const bool second = c + 16 < HALF && (!NARROW || n0 + c + 16 < sh.N);
             if (live) {
 #pragma unroll
               for (int j = 0; j < 16; j += 8) {
@@ -599,14 +618,15 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
 #pragma unroll
                 for (int e = 0; e < 8; ++e) { a[e] = __float_as_uint(v[j + e]); b[e] = __float_as_uint(w[j + e]); }
                 st32B(dst + c + j, a);
-                st32B(dst + c + 16 + j, b);
+                if (second) st32B(dst + c + 16 + j, b);
               }
             }
           }
         } else if (EPI == EPI_RESID) {
 #pragma unroll
-          for (int j = 0; j < 8; j += 2) {
+          for (int j = 0; j < RUNS; j += 2) {
             if (n0 + 16 * j < sh.N) {
+              const bool second = j + 1 < RUNS && (!NARROW || n0 + 16 * j + 16 < sh.N);
               float v[16], w[16], a[16];
               tc_ld16x2(ta + 16 * j, ta + 16 * j + 16, v, w);
               unpack16(res[j], a);
@@ -620,7 +640,7 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
               pack16(w, o1);
               if (live) {
                 st32B(x + 16 * j, o0);
-                st32B(x + 16 * j + 16, o1);
+                if (second) st32B(x + 16 * j + 16, o1);
               }
             }
           }
@@ -667,6 +687,34 @@ int pair_count() {
 }
 
 // `N` as in PromptShape; the weight has `wN` rows.
+template <int EPI, int BN>
+int launch_tiles(const void* x, const void* w_tc, void* out, int M, int wN, int K, PromptShape sh, int pairs,
+                 const RopeArgs& ra, void* scratch, int* status, void* stream, const char* who) {
+  CUtensorMap xmap;
+  WeightMaps<BN> wmaps;
+  {
+    const cuuint64_t dim[2] = {(cuuint64_t)K, (cuuint64_t)M};
+    const cuuint64_t stride[1] = {(cuuint64_t)K * 2};
+    const cuuint32_t box[2] = {(cuuint32_t)PG_TILE_K, 128};
+    int rc = tc_encode(&xmap, x, 2, dim, stride, box, CU_TENSOR_MAP_SWIZZLE_128B, who);
+    if (rc) return rc;
+  }
+  for (size_t i = 0; i < sizeof(wmaps.m) / sizeof(wmaps.m[0]); ++i) {
+    // the tiled weight as (64 k, 128 rows, k tiles, row blocks): tiles are already swizzled images
+    const cuuint64_t dim[4] = {64, 128, (cuuint64_t)sh.KT, (cuuint64_t)((wN + 127) / 128)};
+    const cuuint64_t stride[3] = {128, 16384, (cuuint64_t)sh.KT * 16384};
+    const cuuint32_t box[4] = {64, BN == PG_BN ? (cuuint32_t)sh.wrows : 16 * (cuuint32_t)(i + 1), 1, 1};
+    int rc = tc_encode(&wmaps.m[i], w_tc, 4, dim, stride, box, CU_TENSOR_MAP_SWIZZLE_NONE, who);
+    if (rc) return rc;
+  }
+  static size_t smem_done[64] = {0};
+  Q_CHECK_CUDA(q_ensure_smem(k_gemm_prompt<EPI, BN>, pg_smem(BN), smem_done));
+  Q_CHECK_CUDA(q_launch_cluster(k_gemm_prompt<EPI, BN>, dim3(2 * pairs), dim3(PG_THREADS), pg_smem(BN),
+                                (cudaStream_t)stream, 2, xmap, wmaps, out, sh, ra, (unsigned char*)scratch, status,
+                                q_tl_next(Q_TL_GEMM_TC)));
+  return Q_OK;
+}
+
 template <int EPI>
 int launch_prompt(const void* x, const void* w_tc, void* out, int M, int N, int wN, int K, const RopeArgs& ra,
                   void* scratch, void* stream, const char* who) {
@@ -705,28 +753,29 @@ int launch_prompt(const void* x, const void* w_tc, void* out, int M, int N, int 
       sh.share = share;
     }
   }
+  constexpr bool can_be_narrow = EPI == EPI_RESID || EPI == EPI_F32;
+  if (can_be_narrow) {
+    // Narrow tiles where they leave less of a wave idle: whole, in units of one k step x one column. A narrow step
+    // takes 0.69 of a wide one (0.63 the columns, the same activations), a split 45 steps here, 25 behind whole
+    // waves. Wide / narrow, us: O at 257 rows 25.5 / 19.1, 1024 27.1 / 20.4, 2048 44.0 / 36.2, but 1280 27.3 / 33.8,
+    // 4096 66.8 / 70.7, 8192 126 / 130; down at 512 41.0 / 39.6, 1024 51.7 / 42.7, 2103 100 / 90, but 2560
+    // 108 / 117, 8192 298 / 356.
+    PromptShape nr = sh;
+    nr.nt = (N + PG_NARROW - 1) / PG_NARROW;
+    const long long nt = (long long)nr.mt * nr.nt;
+    const int tail = sh.share == sh.KT ? (rest ? sh.KT : 0) : sh.share + (sh.waves ? 25 : 45);
+    const long long wide = (long long)(sh.waves * sh.KT + tail) * PG_BN;
+    const long long narrow = (nt + pairs - 1) / pairs * sh.KT * 175;
+    if (narrow < wide) {
+      nr.waves = (int)(nt / pairs);
+      nr.share = nr.KT;
+      if (nt < pairs) pairs = (int)nt;
+      return launch_tiles<EPI, can_be_narrow ? PG_NARROW : PG_BN>(x, w_tc, out, M, wN, K, nr, pairs, ra, scratch, status,
+                                                                  stream, who);
+    }
+  }
   if (sh.share == sh.KT && tiles < pairs) pairs = (int)tiles;
-  CUtensorMap xmap, wmap;
-  {
-    const cuuint64_t dim[2] = {(cuuint64_t)K, (cuuint64_t)M};
-    const cuuint64_t stride[1] = {(cuuint64_t)K * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)PG_TILE_K, 128};
-    int rc = tc_encode(&xmap, x, 2, dim, stride, box, CU_TENSOR_MAP_SWIZZLE_128B, who);
-    if (rc) return rc;
-  }
-  {
-    // the tiled weight as (64 k, 128 rows, k tiles, row blocks): tiles are already swizzled images
-    const cuuint64_t dim[4] = {64, 128, (cuuint64_t)sh.KT, (cuuint64_t)((wN + 127) / 128)};
-    const cuuint64_t stride[3] = {128, 16384, (cuuint64_t)sh.KT * 16384};
-    const cuuint32_t box[4] = {64, (cuuint32_t)sh.wrows, 1, 1};
-    int rc = tc_encode(&wmap, w_tc, 4, dim, stride, box, CU_TENSOR_MAP_SWIZZLE_NONE, who);
-    if (rc) return rc;
-  }
-  static size_t smem_done[64] = {0};
-  Q_CHECK_CUDA(q_ensure_smem(k_gemm_prompt<EPI>, PG_SMEM, smem_done));
-  Q_CHECK_CUDA(q_launch_cluster(k_gemm_prompt<EPI>, dim3(2 * pairs), dim3(PG_THREADS), PG_SMEM, (cudaStream_t)stream, 2,
-                                xmap, wmap, out, sh, ra, (unsigned char*)scratch, status, q_tl_next(Q_TL_GEMM_TC)));
-  return Q_OK;
+  return launch_tiles<EPI, PG_BN>(x, w_tc, out, M, wN, K, sh, pairs, ra, scratch, status, stream, who);
 }
 
 }  // namespace

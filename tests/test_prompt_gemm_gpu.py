@@ -74,6 +74,13 @@ def test_sums_and_residual(ops, scratch, M, N, K):
     assert ops.device_status() == [0, 0, 0, 0]
 
 
+# Tiles of 160 columns: a last tile of 32 and of 96 columns, weight rows that end inside a 128-row block, one
+# wave with idle pairs and three waves, a K that is no multiple of 64.
+@pytest.mark.parametrize("M,N,K", [(512, 2592, 512), (2100, 2592, 96), (130, 576, 9728), (5000, 672, 160)])
+def test_narrow_tiles(ops, scratch, M, N, K):
+    test_sums_and_residual(ops, scratch, M, N, K)
+
+
 @pytest.mark.parametrize("M,inter,K", [(1, 32, 32), (300, 96, 128), (257, 1184, 416), (600, 9728, 256), (600, 1312, 9728)])
 def test_swiglu(ops, scratch, M, inter, K):
     """Within one bf16 rounding of the oracle's SwiGLU of the fp32 sums (inter not a multiple of 128
