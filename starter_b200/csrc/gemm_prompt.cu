@@ -757,13 +757,14 @@ int launch_prompt(const void* x, const void* w_tc, void* out, int M, int N, int 
   if (can_be_narrow) {
     // Narrow tiles where they leave less of a wave idle: whole, in units of one k step x one column. A narrow step
     // takes 0.69 of a wide one (0.63 the columns, the same activations), a split 45 steps here, 25 behind whole
-    // waves. Wide / narrow, us: O at 257 rows 25.5 / 19.1, 1024 27.1 / 20.4, 2048 44.0 / 36.2, but 1280 27.3 / 33.8,
+    // waves; the tiles of a wave that is nearly empty run faster, down to 0.6 of the time. Wide / narrow, us: O at 257 rows 25.5 / 19.1, 1024 27.1 / 20.4, 2048 44.0 / 36.2, but 1280 27.3 / 33.8,
     // 4096 66.8 / 70.7, 8192 126 / 130; down at 512 41.0 / 39.6, 1024 51.7 / 42.7, 2103 100 / 90, but 2560
     // 108 / 117, 8192 298 / 356.
     PromptShape nr = sh;
     nr.nt = (N + PG_NARROW - 1) / PG_NARROW;
     const long long nt = (long long)nr.mt * nr.nt;
-    const int tail = sh.share == sh.KT ? (rest ? sh.KT : 0) : sh.share + (sh.waves ? 25 : 45);
+    const int tail = sh.share != sh.KT ? sh.share + (sh.waves ? 25 : 45)
+                     : rest ? sh.KT * (6 * pairs + 4 * rest) / (10 * pairs) : 0;
     const long long wide = (long long)(sh.waves * sh.KT + tail) * PG_BN;
     const long long narrow = (nt + pairs - 1) / pairs * sh.KT * 175;
     if (narrow < wide) {
