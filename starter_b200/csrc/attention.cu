@@ -70,6 +70,15 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
       "l"(src), "r"(bytes), "r"(bar)
       : "memory");
 }
+// The first `keys` rows (at most a page) of a K and a V tile. Rows past the newest key are left out: what the ring
+// held there is masked in the scores and cleared in V, like the stale rows of the page would be. (Decode
+// step of 12 layers, whole tiles / this, us: 5 x 701 keys 779 / 775, 8 x 700 810 / 802, 64 x 333 1037 / 1034.)
+__device__ __forceinline__ void copy_tile(unsigned char* stage, const char* k, const char* v, int keys, uint32_t bar) {
+  const uint32_t bytes = (uint32_t)min(keys, Q_PAGE_TOKENS) * 256u;
+  mbar_expect_tx(bar, 2 * bytes);
+  bulk_g2s(smem_u32(stage), k, bytes, bar);
+  bulk_g2s(smem_u32(stage) + TILE_BYTES, v, bytes, bar);
+}
 __device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2,
                                         uint32_t& r3) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -158,10 +167,8 @@ k_attn_split(const bf16* __restrict__ Q, const char* __restrict__ kpool,
         }
         const int page = block_table[(size_t)b * pages_per_seq + tile0 + it];
         const size_t off = ((size_t)page * nkv + kh) * TILE_BYTES;
-        const uint32_t bar = smem_u32(&bars[s]);
-        mbar_expect_tx(bar, STAGE_BYTES);
-        bulk_g2s(smem_u32(stages + s * STAGE_BYTES), kpool + off, TILE_BYTES, bar);
-        bulk_g2s(smem_u32(stages + s * STAGE_BYTES + TILE_BYTES), vpool + off, TILE_BYTES, bar);
+        copy_tile(stages + s * STAGE_BYTES, kpool + off, vpool + off, max_limit - (tile0 + it) * Q_PAGE_TOKENS,
+                  smem_u32(&bars[s]));
       }
       if (!waited) pdl_wait();
     }
@@ -490,10 +497,8 @@ k_attn_decode(const float* __restrict__ PQ, PlanView pv, const bf16* __restrict_
       if (tile >= 32) page = block_table[(size_t)b * pages_per_seq + tile];
       if (lane == 0) {
         const size_t off = ((size_t)page * nkv + kh) * TILE_BYTES;
-        const uint32_t bar = smem_u32(&bars[it]);
-        mbar_expect_tx(bar, STAGE_BYTES);
-        bulk_g2s(smem_u32(stages + it * STAGE_BYTES), kpool + off, TILE_BYTES, bar);
-        bulk_g2s(smem_u32(stages + it * STAGE_BYTES + TILE_BYTES), vpool + off, TILE_BYTES, bar);
+        copy_tile(stages + it * STAGE_BYTES, kpool + off, vpool + off, max_limit - tile * Q_PAGE_TOKENS,
+                  smem_u32(&bars[it]));
       }
     }
   }
@@ -612,10 +617,8 @@ k_attn_decode(const float* __restrict__ PQ, PlanView pv, const bf16* __restrict_
         }
         const int page = block_table[(size_t)b * pages_per_seq + tile0 + it];
         const size_t off = ((size_t)page * nkv + kh) * TILE_BYTES;
-        const uint32_t bar = smem_u32(&bars[s]);
-        mbar_expect_tx(bar, STAGE_BYTES);
-        bulk_g2s(smem_u32(stages + s * STAGE_BYTES), kpool + off, TILE_BYTES, bar);
-        bulk_g2s(smem_u32(stages + s * STAGE_BYTES + TILE_BYTES), vpool + off, TILE_BYTES, bar);
+        copy_tile(stages + s * STAGE_BYTES, kpool + off, vpool + off, max_limit - (tile0 + it) * Q_PAGE_TOKENS,
+                  smem_u32(&bars[s]));
       }
     }
   } else {
