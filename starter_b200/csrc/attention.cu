@@ -27,6 +27,7 @@ constexpr int TILE_BYTES = 64 * 128 * 2;   // one K or V page tile
 constexpr int STAGE_BYTES = 2 * TILE_BYTES;
 constexpr int CONSUMERS = 4;
 constexpr int THREADS = (CONSUMERS + 1) * 32;
+constexpr int MO_LD = 136;                 // floats of a row of the warps' merge area (query rows on other banks)
 constexpr int MAX_CLUSTER = 16;            // most key splits that merge inside one thread-block cluster
 constexpr unsigned WAIT_LIMIT = 1u << 22;
 
@@ -98,6 +99,12 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
       "{%8,%9}, {%0,%1,%2,%3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// 8 x 8 bf16 matrix, a lane's pair (row lane / 4, columns 2 (lane % 4) ..), transposed.
+__device__ __forceinline__ uint32_t transpose8x8(uint32_t a) {
+  uint32_t r;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(a));
+  return r;
 }
 __device__ __forceinline__ void consumer_sync() {
   asm volatile("bar.sync 1, %0;" ::"n"(CONSUMERS * 32) : "memory");
@@ -431,7 +438,7 @@ k_attn_merge(const float* __restrict__ part_o, const float* __restrict__ part_ml
 // memory, the cluster synchronises once, and CTA r of the cluster combines 1/S of the
 // (row, dim) outputs from all S CTAs in split order. No global round trips, no tickets.
 template <bool CL, int DG>
-__global__ void __launch_bounds__((4 * DG + 1) * 32)
+__global__ void __launch_bounds__((4 * DG + 1) * 32, CL && DG == 1 ? 4 : 1)
 k_attn_decode(const float* __restrict__ PQ, PlanView pv, const bf16* __restrict__ QG,
               const bf16* __restrict__ KG, const bf16* __restrict__ COS, const bf16* __restrict__ SIN,
               const int32_t* __restrict__ pos_ptr, char* __restrict__ kpool, char* __restrict__ vpool,
@@ -445,6 +452,7 @@ k_attn_decode(const float* __restrict__ PQ, PlanView pv, const bf16* __restrict_
   const int NS = ring_stages;
   constexpr int DC = 4 * DG;                 // consumer warps: DG groups of four, one tile per group at a time
   constexpr int DT = (DC + 1) * 32;          // threads; warp DC is the producer
+  constexpr int SETS = DG == 3 ? 8 : 4;      // accumulators of Q K^T (one CTA per SM has the registers)
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char* stages = smem;                               // NS * STAGE_BYTES
   unsigned char* qtile = smem + NS * STAGE_BYTES;             // 16 rows * 256 B
@@ -591,7 +599,7 @@ k_attn_decode(const float* __restrict__ PQ, PlanView pv, const bf16* __restrict_
         *reinterpret_cast<uint2*>(knew + 4 * lane) = o;
       }
     }
-    for (int i = tid; i < (16 - G) * 16; i += DT) {       // query rows G..15 are zero
+    for (int i = tid; i < (8 - G) * 16; i += DT) {        // query rows G..7 are zero
       const int r = G + (i >> 4), ch = i & 15;
       *reinterpret_cast<uint4*>(qtile + r * 256 + ((ch ^ (r & 7)) << 4)) = make_uint4(0, 0, 0, 0);
     }
@@ -622,12 +630,21 @@ k_attn_decode(const float* __restrict__ PQ, PlanView pv, const bf16* __restrict_
       }
     }
   } else {
+    // Keys are the M dimension of the MMAs and the (at most 8) query rows the N dimension: S^T = K Q^T, O^T = V^T P^T.
+    // A lane holds keys g, g + 8 and query rows 2 t4, 2 t4 + 1; the other way round half of every accumulator
+    // belonged to query rows 8-15, which do not exist here. Decode step of 12 layers, that way / this, us:
+    // 1 x 1024 keys 709 / 706, 8 x 700 802 / 798, 64 x 333 1034 / 1006, 32 x 2048 1274 / 1265, 3 x 16000 1155 / 1108.
     const int g = lane >> 2, t4 = lane & 3;
-    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
-    float oacc[16][4];
+    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};   // rows 2 t4, 2 t4 + 1 (l: of this lane's keys)
+    float oacc[8][4];                                                 // dims 16 n + g, 16 n + g + 8
 #pragma unroll
-    for (int n = 0; n < 16; ++n) oacc[n][0] = oacc[n][1] = oacc[n][2] = oacc[n][3] = 0.f;
-    const uint32_t q_base = smem_u32(qtile);
+    for (int n = 0; n < 8; ++n) oacc[n][0] = oacc[n][1] = oacc[n][2] = oacc[n][3] = 0.f;
+    uint32_t qf[8][2];                                                // Q^T fragments of the eight k steps
+#pragma unroll
+    for (int kp = 0; kp < 4; ++kp) {
+      const int row = lane & 7, ch = 4 * kp + (lane >> 3);
+      ldsm_x4(smem_u32(qtile) + row * 256 + ((ch ^ row) << 4), qf[2 * kp][0], qf[2 * kp][1], qf[2 * kp + 1][0], qf[2 * kp + 1][1]);
+    }
     const int grp = warp >> 2, wk = warp & 3;       // tile lane of the warp's group, key quarter of the warp
     for (int it = grp; it < ntiles; it += DG) {
       const int s = it % NS;
@@ -653,81 +670,50 @@ k_attn_decode(const float* __restrict__ PQ, PlanView pv, const bf16* __restrict_
       }
       __syncwarp();
       const uint32_t k_base = smem_u32(kt), v_base = smem_u32(vt);
-      // the eight k-steps go to four independent accumulator sets (an MMA's result is ~280
-      // cycles away), added at the end
-      float sset[4][2][4];
+      // the eight k-steps go to independent accumulators (an MMA's result is ~280 cycles away), added at the end
+      float sset[SETS][4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) sset[q][j][0] = sset[q][j][1] = sset[q][j][2] = sset[q][j][3] = 0.f;
+      for (int q = 0; q < SETS; ++q) sset[q][0] = sset[q][1] = sset[q][2] = sset[q][3] = 0.f;
+      const int arow = wk * 16 + (lane & 7) + 8 * ((lane >> 3) & 1);
 #pragma unroll
       for (int ks = 0; ks < 8; ++ks) {
-        uint32_t a0, a1, a2, a3, b0, b1, b2, b3;
-        {
-          const int row = (lane & 7) + 8 * ((lane >> 3) & 1);
-          const int ch = 2 * ks + (lane >> 4);
-          ldsm_x4(q_base + row * 256 + ((ch ^ (row & 7)) << 4), a0, a1, a2, a3);
-        }
-        {
-          const int mi = lane >> 3;
-          const int key = wk * 16 + 8 * (mi >> 1) + (lane & 7);
-          const int ch = 2 * ks + (mi & 1);
-          ldsm_x4(k_base + key * 256 + ((ch ^ (key & 7)) << 4), b0, b1, b2, b3);
-        }
-        mma16816(sset[ks & 3][0], a0, a1, a2, a3, b0, b1);
-        mma16816(sset[ks & 3][1], a0, a1, a2, a3, b2, b3);
+        uint32_t a0, a1, a2, a3;
+        const int ch = 2 * ks + (lane >> 4);
+        ldsm_x4(k_base + arow * 256 + ((ch ^ (arow & 7)) << 4), a0, a1, a2, a3);
+        mma16816(sset[ks % SETS], a0, a1, a2, a3, qf[ks][0], qf[ks][1]);
       }
-      float sacc[2][4];
+      float sc[4];                            // (key g, row 2 t4), (g, 2 t4 + 1), (g + 8, 2 t4), (g + 8, 2 t4 + 1)
 #pragma unroll
-      for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) sacc[j][e] = (sset[0][j][e] + sset[1][j][e]) + (sset[2][j][e] + sset[3][j][e]);
-      float pr[2][4];
+      for (int e = 0; e < 4; ++e) {
+        float v = (sset[0][e] + sset[1][e]) + (sset[2][e] + sset[3][e]);
+        if (SETS == 8) v += (sset[4][e] + sset[5][e]) + (sset[6][e] + sset[7][e]);
+        v *= scale_log2;
+        sc[e] = my_key0 + g + 8 * (e >> 1) < max_limit ? v : -INFINITY;
+      }
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        float mx = -INFINITY;
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int key = my_key0 + 8 * j + 2 * t4 + e;
-            float v = sacc[j][2 * h + e] * scale_log2;
-            v = key < max_limit ? v : -INFINITY;
-            sacc[j][2 * h + e] = v;
-            mx = fmaxf(mx, v);
-          }
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        float mx = fmaxf(sc[h], sc[2 + h]);
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
         const float m_new = fmaxf(m_run[h], mx);
         const float m_safe = m_new == -INFINITY ? 0.f : m_new;
         const float resc = exp2f(m_run[h] - m_safe);
-        float sum = 0.f;
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const float pv2 = exp2f(sacc[j][2 * h + e] - m_safe);
-            pr[j][2 * h + e] = pv2;
-            sum += pv2;
-          }
-        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-        l_run[h] = l_run[h] * resc + sum;
+        sc[h] = exp2f(sc[h] - m_safe);
+        sc[2 + h] = exp2f(sc[2 + h] - m_safe);
+        l_run[h] = l_run[h] * resc + (sc[h] + sc[2 + h]);
         m_run[h] = m_new;
 #pragma unroll
-        for (int n = 0; n < 16; ++n) { oacc[n][2 * h] *= resc; oacc[n][2 * h + 1] *= resc; }
+        for (int n = 0; n < 8; ++n) { oacc[n][h] *= resc; oacc[n][2 + h] *= resc; }
       }
-      const uint32_t pa0 = pack_bf16(pr[0][0], pr[0][1]), pa1 = pack_bf16(pr[0][2], pr[0][3]);
-      const uint32_t pa2 = pack_bf16(pr[1][0], pr[1][1]), pa3 = pack_bf16(pr[1][2], pr[1][3]);
+      const uint32_t pb0 = transpose8x8(pack_bf16(sc[0], sc[1])), pb1 = transpose8x8(pack_bf16(sc[2], sc[3]));
+      const int mi = lane >> 3, vrow = wk * 16 + 8 * (mi >> 1) + (lane & 7);
 #pragma unroll
-      for (int dp = 0; dp < 8; ++dp) {
-        uint32_t b0, b1, b2, b3;
-        const int mi = lane >> 3;
-        const int key = wk * 16 + 8 * (mi & 1) + (lane & 7);
-        const int ch = 2 * dp + (mi >> 1);
-        ldsm_x4_t(v_base + key * 256 + ((ch ^ (key & 7)) << 4), b0, b1, b2, b3);
-        mma16816(oacc[2 * dp], pa0, pa1, pa2, pa3, b0, b1);
-        mma16816(oacc[2 * dp + 1], pa0, pa1, pa2, pa3, b2, b3);
+      for (int n = 0; n < 8; ++n) {
+        uint32_t a0, a1, a2, a3;
+        const int ch = 2 * n + (mi & 1);
+        ldsm_x4_t(v_base + vrow * 256 + ((ch ^ (vrow & 7)) << 4), a0, a1, a2, a3);
+        mma16816(oacc[n], a0, a1, a2, a3, pb0, pb1);
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&bars[NS + s]));
@@ -735,16 +721,23 @@ k_attn_decode(const float* __restrict__ PQ, PlanView pv, const bf16* __restrict_
     if (stamp) g_attn_trace[3] = tl_now();
     // merge the consumer warps' states through shared memory (only the G real query rows)
     asm volatile("bar.sync 1, %0;" ::"n"(DC * 32) : "memory");
-    float* mo = reinterpret_cast<float*>(stages);            // [DC][G][128]
-    float* mml = mo + DC * G * 128;                          // [DC][G][2]
-    if (g < G) {
-      float* dst = mo + ((size_t)warp * G + g) * 128;
+    float* mo = reinterpret_cast<float*>(stages);            // [DC][G][MO_LD]
+    float* mml = mo + DC * G * MO_LD;                        // [DC][G][2]
 #pragma unroll
-      for (int n = 0; n < 16; ++n)
-        *reinterpret_cast<float2*>(dst + 8 * n + 2 * t4) = make_float2(oacc[n][0], oacc[n][1]);
-      if (t4 == 0) {
-        mml[((size_t)warp * G + g) * 2] = m_run[0];
-        mml[((size_t)warp * G + g) * 2 + 1] = l_run[0];
+    for (int h = 0; h < 2; ++h) {
+      float l = l_run[h];
+      l += __shfl_xor_sync(0xffffffffu, l, 4);
+      l += __shfl_xor_sync(0xffffffffu, l, 8);
+      l += __shfl_xor_sync(0xffffffffu, l, 16);
+      const int r = 2 * t4 + h;
+      if (r < G) {
+        float* dst = mo + ((size_t)warp * G + r) * MO_LD + g;
+#pragma unroll
+        for (int n = 0; n < 8; ++n) { dst[16 * n] = oacc[n][h]; dst[16 * n + 8] = oacc[n][2 + h]; }
+        if (g == 0) {
+          mml[((size_t)warp * G + r) * 2] = m_run[h];
+          mml[((size_t)warp * G + r) * 2 + 1] = l;
+        }
       }
     }
     asm volatile("bar.sync 1, %0;" ::"n"(DC * 32) : "memory");
@@ -759,7 +752,7 @@ k_attn_decode(const float* __restrict__ PQ, PlanView pv, const bf16* __restrict_
       for (int w = 0; w < DC; ++w) {
         const float wt = exp2f(mw[w] - Ms);
         Lsum += wt * mml[((size_t)w * G + r) * 2 + 1];
-        O += wt * mo[((size_t)w * G + r) * 128 + d];
+        O += wt * mo[((size_t)w * G + r) * MO_LD + d];
       }
       if (S == 1) {
         out[((size_t)b * nq + kh * G + r) * 128 + d] = __float2bfloat16_rn(Lsum > 0.f ? O / Lsum : 0.f);
@@ -1081,6 +1074,9 @@ extern "C" int q_attention_decode(const float* d_qkv_partials, const q_gemm_plan
   if (sms <= 0) sms = 148;
   const long long ctas = (long long)splits * batch * nkv;
   if (ring == 3 && ctas > 2 * sms && ctas <= 3 * sms) ring = 2;
+  // ... and one stage, with nothing to merge, for a fourth CTA: while one of the four computes, the others' copies
+  // are in flight. Three stages / one, us: 64 x 333 keys 1009 / 999, 64 x 1000 1315 / 1292.
+  if (ring == 3 && splits == 1 && ctas > 3 * sms && ctas <= 4 * sms) ring = 1;
   // Three warp groups (one tile each at a time) when every CTA of the launch gets an SM of its
   // own; otherwise one group, so that two CTAs still fit on an SM. A ring stage must always be
   // consumed by the same group (its mbarrier parity is tracked per group), so the three groups
@@ -1094,7 +1090,7 @@ extern "C" int q_attention_decode(const float* d_qkv_partials, const q_gemm_plan
   Q_CHECK_CUDA(q_ensure_smem(k_attn_decode<false, 3>, attn_decode_smem(NS), done[2]));
   Q_CHECK_CUDA(q_ensure_smem(k_attn_decode<true, 3>, attn_decode_smem(NS), done[3]));
   // the merge scratch (consumer states, then the CTA's own rows) reuses the ring
-  const int scratch_stages = (G * (dc + 1) * 130 * 4 + STAGE_BYTES - 1) / STAGE_BYTES;
+  const int scratch_stages = (G * (dc + 1) * (MO_LD + 2) * 4 + STAGE_BYTES - 1) / STAGE_BYTES;
   if (ring < scratch_stages) ring = scratch_stages;
   Q_CHECK_ARG(ring <= NS, "q_attention_decode: merge scratch does not fit the ring");
   bool cluster = splits >= 2 && splits <= MAX_CLUSTER && !g_attn_no_cluster;
@@ -1139,6 +1135,9 @@ extern "C" int q_attention_decode(const float* d_qkv_partials, const q_gemm_plan
   if (cluster) {
     if (wide) Q_CHECK_CUDA(q_launch_cluster(k_attn_decode<true, 3>, grid, block, smem, st, (unsigned)splits, Q_ATTN_DECODE_ARGS));
     else Q_CHECK_CUDA(q_launch_cluster(k_attn_decode<true, 1>, grid, block, smem, st, (unsigned)splits, Q_ATTN_DECODE_ARGS));
+  } else if (splits == 1) {
+    // nothing to merge: the form without the merge through memory, which needs fewer registers (96, not 128)
+    Q_CHECK_CUDA(q_launch(k_attn_decode<true, 1>, grid, block, smem, st, Q_ATTN_DECODE_ARGS));
   } else {
     if (wide) Q_CHECK_CUDA(q_launch(k_attn_decode<false, 3>, grid, block, smem, st, Q_ATTN_DECODE_ARGS));
     else Q_CHECK_CUDA(q_launch(k_attn_decode<false, 1>, grid, block, smem, st, Q_ATTN_DECODE_ARGS));
