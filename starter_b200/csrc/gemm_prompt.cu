@@ -30,7 +30,7 @@
 // bytes); commits release stages and hand over accumulators in both CTAs at once. Every wait is
 // bounded as in gemm_tc.cu and reports in the same status word (codes 5-8).
 //
-// Work split: tiles in raster order (row tiles fastest inside groups of eight, so that the tiles in
+// Work split: tiles in raster order (row tiles fastest inside groups of `group`, so that the tiles in
 // flight share both operands in L2). Whole waves of one tile per pair come first; what is left over
 // - up to two tiles' work per pair - is cut evenly by k steps over all pairs (`split`), since a
 // projection with N = 2560 has 40 tiles at 1024 rows and 80 at 2048 for 74 pairs. A pair that ends
@@ -54,7 +54,6 @@ constexpr int PG_NARROW = 160;                             // ... of a narrow ti
 __host__ __device__ constexpr uint32_t pg_stage(int bn) { return PG_A_BYTES + bn / 2 * PG_TILE_K * 2; }
 __host__ __device__ constexpr int pg_stages(int bn) { return bn == PG_BN ? 7 : 8; }                     // 224 KB, 208 KB
 constexpr size_t pg_smem(int bn) { return 1024 + pg_stages(bn) * pg_stage(bn) + (2 * pg_stages(bn) + 4) * 8 + 16; }
-constexpr int PG_GROUP = 8;                                // row tiles per raster group
 constexpr int PG_MAX_PAIRS = 128;
 constexpr int PG_SPLIT_STEPS = 60;                         // what a split costs, in k steps
 // scratch: tickets (16 warps per tile, at most two tiles per pair), then two parts per pair
@@ -68,6 +67,7 @@ struct PromptShape {
   int M, N, KT;         // rows, output columns (EPI_SWIGLU: inter), k tiles
   int mt, nt;           // tiles along rows (256) and columns (256; EPI_SWIGLU 128 gate + 128 up)
   int wrows;            // weight rows per copy (a power of two that divides every copy's start)
+  int group;            // row tiles of a raster group
   int waves;            // tiles that each pair takes whole
   int share;            // k steps of the remaining tiles per pair: whole tiles, or an even split
 };
@@ -436,11 +436,11 @@ k_gemm_prompt(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
 
   // (row tile, column tile) of a tile number
   auto locate = [&](int t, int& mi, int& ni) {
-    const int per = PG_GROUP * sh.nt;
+    const int per = sh.group * sh.nt;
     const int g = t / per, in = t - g * per;
-    const int rows = min(PG_GROUP, sh.mt - g * PG_GROUP);
+    const int rows = min(sh.group, sh.mt - g * sh.group);
     ni = in / rows;
-    mi = g * PG_GROUP + in - ni * rows;
+    mi = g * sh.group + in - ni * rows;
   };
 
   if (warp == 0) {
@@ -728,6 +728,11 @@ int launch_prompt(const void* x, const void* w_tc, void* out, int M, int N, int 
   if (!status) { q_set_error("%s: could not locate the device status word", who); return Q_ERR_CUDA; }
   PromptShape sh;
   sh.M = M; sh.N = N;
+  // A raster group reads the whole weight once. Where the weight does not stay in L2 from one group to the next,
+  // fewer and taller groups: gate|up (100 MB) in groups of 4 / 8 / 16 / 32 row tiles 609 / 597 / 586 / 580 us at
+  // 8192 rows, 534 / 527 / 516 / 512 at 7000 (in a loop under the power cap), but down (50 MB) 328 / 333 / 335 / 351
+  // and O (21 MB) 143 / 141 / 143 / 152.
+  sh.group = (long long)wN * K * 2 > (64ll << 20) ? 32 : 8;
   sh.KT = (K + PG_TILE_K - 1) / PG_TILE_K;
   sh.mt = (M + 255) / 256;
   const int cols = EPI == EPI_SWIGLU ? PG_HALF : PG_BN;
