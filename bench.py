@@ -378,6 +378,12 @@ def kernels_per_step(state) -> int:
         if rows <= 8:
             # embed | QKV, attention, O, add+norm, gate|up (SwiGLU epilogue), down, add+norm | lm_head, argmax
             return 1 + 7 * L + 2
+        from starter_b200._lib import lib
+        c = state.cfg
+        q = c.n_q_heads * 128
+        if lib.q_gemm_rows_supported(rows, c.hidden, c.inter, q, q + 2 * c.n_kv_heads * 128):
+            # embed | QKV, attention, O, gate|up, down (norm, add and SwiGLU inside) | final norm, lm_head, argmax
+            return 1 + 5 * L + 3
         # embed | QKV, attention, O, add+norm, gate|up, SwiGLU, down, add+norm | lm_head, argmax
         return 1 + 8 * L + 2
     if state.peers:
