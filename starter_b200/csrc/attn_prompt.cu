@@ -13,8 +13,8 @@
 // while the softmax of the other runs; a CTA is persistent and starts the next item's first
 // products under the current one's last softmax, since an item is only ~9 tiles long at 1-2 K keys.
 //
-// Warps 0-7 / 8-15: softmax and epilogue of query tile 0 / 1. Two threads share a row (64 scores, then
-// 64 dims of O each) and exchange its maximum through shared memory: a step is a chain - scores,
+// Warps 0-7 / 8-15: softmax and epilogue of query tile 0 / 1 (TILES = 1: all of one tile). Two (four) threads
+// share a row (64 or 32 scores, then as many dims of O each) and exchange its maximum through shared memory: a step is a chain - scores,
 // softmax, P V, next scores - and with one thread per row it took 4500 cycles, of which the softmax
 // of 128 scores was more than half.
 // Warp 16: producer lane. Warp 17: MMA issue; the whole warp walks the loop and one elected lane
@@ -41,7 +41,7 @@ constexpr uint32_t AP_HALF = 128 * 128;                    // bytes of 128 rows 
 constexpr uint32_t AP_TILE = 2 * AP_HALF;                  // 128 rows x 128 dims
 constexpr uint32_t AP_Q = 0, AP_K = 2 * AP_TILE, AP_V = AP_K + 2 * AP_TILE;
 constexpr uint32_t AP_BARS = AP_V + 2 * AP_TILE;           // 192 KB in
-constexpr uint32_t AP_RED = AP_BARS + 24 * 8 + 16;         // row exchange: [3][2 tiles][2 halves][128] floats
+constexpr uint32_t AP_RED = AP_BARS + 24 * 8 + 16;         // row exchange: [3][2 tiles x 2 or 4 parts][128] floats
 constexpr size_t AP_SMEM = 1024 + AP_RED + 3 * 2 * 2 * 128 * 4;
 
 enum { B_QF = 0, B_QE = 2, B_KF = 4, B_KE = 6, B_VF = 8, B_VE = 10, B_SF = 12, B_P = 14, B_OF = 18, B_OE = 20 };
@@ -49,7 +49,7 @@ enum { B_QF = 0, B_QE = 2, B_KF = 4, B_KE = 6, B_VF = 8, B_VE = 10, B_SF = 12, B
 struct AttnShape {
   int batch, T, G, gshift, nq, nkv, pages_per_seq;
   int tokens;        // prompt tokens per query tile: 128 / G
-  int tiles;         // query tiles per work item: 2, or 1 when there are SMs enough for all tiles
+  int tiles;         // query tiles per work item: 2, or 1 where there are at most two for an SM
   int blocks;        // work items per (sequence, kv head)
   int items;
   int wide;          // the output is 32-byte aligned
@@ -155,10 +155,13 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
+template <int TILES>
 __global__ void __launch_bounds__(AP_THREADS, 1)
 k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
               const __grid_constant__ CUtensorMap vmap, const int32_t* __restrict__ block_table,
               const int32_t* __restrict__ pos_ptr, bf16* __restrict__ out, AttnShape sh, int* status) {
+  constexpr int WARPS = TILES == 2 ? 8 : 16;               // softmax warps of a query tile
+  constexpr int PER_ROW = WARPS / 4, COLS = 128 / PER_ROW; // threads of a row, scores (and dims of O) of each
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -172,8 +175,8 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     for (int i = 0; i < 24; ++i) {
-      const bool warps = i >= B_P && i < B_P + 4;          // four softmax warps arrive (eight at the epilogue)
-      mbar_init(bars + 8u * i, i >= B_OE && i < B_OE + 2 ? 8 : warps ? 4 : 1);
+      const bool warps = i >= B_P && i < B_P + 4;          // half a tile's softmax warps arrive (all at the epilogue)
+      mbar_init(bars + 8u * i, i >= B_OE && i < B_OE + 2 ? WARPS : warps ? WARPS / 2 : 1);
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -217,7 +220,7 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
         const int w = item_of(r);
         if (w >= sh.items) continue;
         const Item it = item_at(sh, w, pos);
-        for (int i = 0; ok && i < sh.tiles; ++i) {
+        for (int i = 0; ok && i < TILES; ++i) {
           if (!mbar_wait(bar(B_QE, i), (nitems & 1) ^ 1, abort_flag)) { fail(); break; }
           const int tok = it.b * sh.T + it.q0 + i * sh.tokens;
           mbar_expect_tx(bar(B_QF, i), AP_TILE);
@@ -247,7 +250,7 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
       }
       // copies in flight must land before the CTA may leave
       for (int i = 0; i < 2; ++i) {
-        if (nitems > 0 && i < sh.tiles) mbar_wait_plain(bar(B_QF, i), (nitems - 1) & 1);
+        if (nitems > 0 && i < TILES) mbar_wait_plain(bar(B_QF, i), (nitems - 1) & 1);
         if (step > (uint32_t)i) {
           const uint32_t last = ((step - 1 - i) >> 1) & 1;
           mbar_wait_plain(bar(B_KF, (step - 1 - i) & 1), last);
@@ -291,7 +294,7 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
       };
       int r = 0;
       Item cur = item_at(sh, item_of(0), pos);             // the grid has at most one CTA per item
-      for (int i = 0; i < sh.tiles && ok; ++i) {
+      for (int i = 0; i < TILES && ok; ++i) {
         if (!wait(bar(B_QF, i), 0) || (i == 0 && !wait(bar(B_KF, 0), 0))) break;
         scores(i);
         if (elect_one() && cur.n == 1) tc_commit(bar(B_QE, i));
@@ -313,7 +316,7 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
           const bool last = j + 1 == cur.n, ahead = !last || more;
           const int vs = vstep & 1;
           if (!wait(bar(B_VF, vs), (vstep >> 1) & 1)) break;
-          for (int i = 0; i < sh.tiles && ok; ++i) {
+          for (int i = 0; i < TILES && ok; ++i) {
             if (j == 0 && !wait(bar(B_OE, i), (nitems & 1) ^ 1)) break;
             // P comes in two halves of 64 keys, from different warps
             if (!wait(bar(B_P, 2 * i), vstep & 1) || !wait(bar(B_P, 2 * i + 1), vstep & 1)) break;
@@ -358,20 +361,20 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
         cur = nxt;
       }
     }
-  } else if ((warp >> 3) < sh.tiles) {
-    // ---------------- softmax and epilogue: query tile `i`, half a row per thread ----------------
-    const int i = warp >> 3, half = (warp >> 2) & 1;
+  } else {
+    // ---------------- softmax and epilogue: query tile `i`, half (a quarter) of a row per thread ----------------
+    const int i = TILES == 2 ? warp >> 3 : 0, part = TILES == 2 ? (warp >> 2) & 1 : warp >> 2;
     const int row = tid & 127;
-    float* red = reinterpret_cast<float*>(smem + AP_RED) + i * 256;        // [buffer * 512 + half * 128 + row]
-    auto tile_sync = [&]() { asm volatile("bar.sync %0, 256;" ::"r"(1 + i) : "memory"); };
+    float* red = reinterpret_cast<float*>(smem + AP_RED) + i * 256;        // [buffer * 512 + part * 128 + row]
+    auto tile_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + i), "n"(WARPS * 32) : "memory"); };
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t s_addr = tmem + lanes + 128u * i + 64u * half, p_addr = tmem + lanes + 128u * i + 32u * half;
-    const uint32_t o_addr = tmem + lanes + 256u + 128u * i + 64u * half;
+    const uint32_t s_addr = tmem + lanes + 128u * i + (uint32_t)(COLS * part), p_addr = tmem + lanes + 128u * i + (uint32_t)(COLS / 2 * part);
+    const uint32_t o_addr = tmem + lanes + 256u + 128u * i + (uint32_t)(COLS * part);
     // A scale that is not positive (the maximum would sit elsewhere) is multiplied in first.
     const bool plain = sh.scale_log2 > 0.f;
     const float c = plain ? sh.scale_log2 : 1.f;
     uint32_t step = 0, nitems = 0;
-    // A warp whose wait ran out keeps coming to the tile's barriers; at the item's end all eight
+    // A warp whose wait ran out keeps coming to the tile's barriers; at the item's end all its tile's
     // warps learn of it and leave together.
     bool broken = false;
     auto wait = [&](uint32_t b, uint32_t parity) {
@@ -395,21 +398,21 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
       float m = -INFINITY, l = 0.f;
       for (int j = 0; j < it.n; ++j, ++step) {
         wait(bar(B_SF, i), step & 1);
-        float v[64];
-        tc_ld32(s_addr, v);
-        tc_ld32(s_addr + 32, v + 32);
+        float v[COLS];
+#pragma unroll
+        for (int k = 0; k < COLS; k += 32) tc_ld32(s_addr + k, v + k);
         tc_wait_ld();
-        tc_pin32(v);
-        tc_pin32(v + 32);
+#pragma unroll
+        for (int k = 0; k < COLS; k += 32) tc_pin32(v + k);
         const int key_base = j * AP_KEYS;
         if (!plain) {
 #pragma unroll
-          for (int k = 0; k < 64; ++k) v[k] *= sh.scale_log2;
+          for (int k = 0; k < COLS; ++k) v[k] *= sh.scale_log2;
         }
         if (key_base + AP_KEYS > free_keys) {
-          const int vis = limit - key_base - 64 * half;
+          const int vis = limit - key_base - COLS * part;
 #pragma unroll
-          for (int k = 0; k < 64; ++k) v[k] = k < vis ? v[k] : -INFINITY;
+          for (int k = 0; k < COLS; ++k) v[k] = k < vis ? v[k] : -INFINITY;
         }
         if (tid < 128 && key_base + AP_KEYS > it.max_limit && (it.max_limit & 15)) {
           // V rows past the newest key hold stale bits (0 * garbage could be NaN): clear those of its
@@ -426,17 +429,18 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
         }
         float mx[4] = {v[0], v[1], v[2], v[3]};
 #pragma unroll
-        for (int k = 4; k < 60; k += 8)
+        for (int k = 4; k < COLS - 4; k += 8)
 #pragma unroll
           for (int e = 0; e < 4; ++e) mx[e] = max3(mx[e], v[k + e], v[k + 4 + e]);
-        float m_tile = max3(max3(mx[0], mx[1], mx[2]), mx[3], fmaxf(max3(v[60], v[61], v[62]), v[63]));
-        // the row's other half; this barrier also says that both halves of S are in registers, so
-        // that P may overwrite them
-        red[(step & 1) * 512 + half * 128 + row] = m_tile;
+        float m_tile = max3(max3(mx[0], mx[1], mx[2]), mx[3], fmaxf(max3(v[COLS - 4], v[COLS - 3], v[COLS - 2]), v[COLS - 1]));
+        // the row's other parts; this barrier also says that all of S is in registers, so that P may
+        // overwrite it
+        red[(step & 1) * 512 + part * 128 + row] = m_tile;
         tc_fence_before();
         tile_sync();
         tc_fence_after();
-        m_tile = fmaxf(m_tile, red[(step & 1) * 512 + (half ^ 1) * 128 + row]);
+#pragma unroll
+        for (int e = 1; e < PER_ROW; ++e) m_tile = fmaxf(m_tile, red[(step & 1) * 512 + (part ^ e) * 128 + row]);
         if (j == 0) {
           m = m_tile;
         } else {
@@ -447,7 +451,7 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
             l *= f;
             m = m_new;
 #pragma unroll 1
-            for (int k = 0; k < 4; ++k) {
+            for (int k = 0; k < COLS / 16; ++k) {
               float o[16];
               uint32_t u[16];
               tc_ld16(o_addr + 16 * k, o);
@@ -462,7 +466,7 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
         const unsigned long long c2 = pair2(c, c), mc2 = pair2(-mc, -mc);
         unsigned long long sum[2] = {0ull, 0ull};
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+        for (int h = 0; h < COLS / 32; ++h) {
           uint32_t p[16];
 #pragma unroll
           for (int k = 0; k < 16; ++k) {
@@ -478,28 +482,33 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
         tc_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar(B_P, 2 * i + half));
+        if (lane == 0) mbar_arrive(bar(B_P, 2 * i + part / (PER_ROW / 2)));
         __syncwarp();
         float s_lo, s_hi;
         unpair2(add2(sum[0], sum[1]), s_lo, s_hi);
         l += s_lo + s_hi;
       }
-      red[1024 + half * 128 + row] = l;
+      red[1024 + part * 128 + row] = l;
       int give_up;
       asm volatile(
           "{\n\t.reg .pred p, q;\n\t"
           "setp.ne.u32 q, %1, 0;\n\t"
-          "barrier.cta.red.or.pred p, %2, 256, q;\n\t"
+          "barrier.cta.red.or.pred p, %2, %3, q;\n\t"
           "selp.u32 %0, 1, 0, p;\n\t}"
-          : "=r"(give_up) : "r"((int)broken), "r"(1 + i) : "memory");
+          : "=r"(give_up) : "r"((int)broken), "r"(1 + i), "n"(WARPS * 32) : "memory");
       if (give_up) break;
-      l += red[1024 + (half ^ 1) * 128 + row];
+      {
+        float all = red[1024 + row];                       // (in the same order in all threads of a row)
+#pragma unroll
+        for (int e = 1; e < PER_ROW; ++e) all += red[1024 + e * 128 + row];
+        l = all;
+      }
       wait(bar(B_OF, i), nitems & 1);
       if (broken) { ++nitems; continue; }
       const float inv = l > 0.f ? 1.f / l : (l == 0.f ? 0.f : l);      // NaN stays NaN
-      bf16* dst = out + (((size_t)it.b * sh.T + t) * sh.nq + it.kh * sh.G + (row & (sh.G - 1))) * 128 + 64 * half;
+      bf16* dst = out + (((size_t)it.b * sh.T + t) * sh.nq + it.kh * sh.G + (row & (sh.G - 1))) * 128 + COLS * part;
 #pragma unroll 1
-      for (int k = 0; k < 4; ++k) {
+      for (int k = 0; k < COLS / 16; ++k) {
         float o[16];
         tc_ld16(o_addr + 16 * k, o);
         if (t < sh.T) {
@@ -561,10 +570,12 @@ extern "C" int q_attention_prefill(const void* d_q, const q_kv_layout_t* kv, con
   sh.gshift = 0;
   while ((1 << sh.gshift) < G) ++sh.gshift;
   sh.tokens = 128 >> sh.gshift;
-  // Two tiles of a CTA hide each other's latencies, but also share its exponentials: while every
-  // tile can have an SM of its own, one per CTA is faster.
+  // Two tiles of a CTA hide each other's latencies; one tile has all 16 softmax warps, four threads to a row, and a
+  // shorter chain. Up to two tiles per SM the one is faster. One tile / two, us: 1 x 592 tokens 15.5 / 18.8, 1 x 1024
+  // 22.8 / 26.4, 1 x 1184 (296 tiles) 28.8 / 30.7, 3 x 250 10.2 / 12.8, 9 x 128 10.2 / 10.5, but 1 x 1200 32.4 / 31.8,
+  // 3 x 400 (312) 19.4 / 17.0, 2 x 701 26.9 / 22.8. (With half of the warps idle, one tile took 17.1 at 592.)
   const int sms = q_sm_count();
-  sh.tiles = (long long)((T + sh.tokens - 1) / sh.tokens) * batch * nkv <= sms ? 1 : 2;
+  sh.tiles = (long long)((T + sh.tokens - 1) / sh.tokens) * batch * nkv <= 2ll * sms ? 1 : 2;
   sh.blocks = (T + sh.tiles * sh.tokens - 1) / (sh.tiles * sh.tokens);
   const long long items = (long long)sh.blocks * batch * nkv;
   Q_CHECK_ARG(items < (1ll << 30) && (long long)batch * T < (1ll << 31), "q_attention_prefill: too many rows");
@@ -588,10 +599,11 @@ extern "C" int q_attention_prefill(const void* d_q, const q_kv_layout_t* kv, con
                        who);
     if (rc) return rc;
   }
-  static size_t done[64] = {0};
-  Q_CHECK_CUDA(q_ensure_smem(k_attn_prompt, AP_SMEM, done));
+  static size_t done[2][64] = {{0}};
+  auto kern = sh.tiles == 2 ? k_attn_prompt<2> : k_attn_prompt<1>;
+  Q_CHECK_CUDA(q_ensure_smem(kern, AP_SMEM, done[sh.tiles - 1]));
   const int grid = sh.items < sms ? sh.items : sms;
-  Q_CHECK_CUDA(q_launch(k_attn_prompt, dim3(grid), dim3(AP_THREADS), AP_SMEM, (cudaStream_t)stream, qmap, kmap, vmap,
+  Q_CHECK_CUDA(q_launch(kern, dim3(grid), dim3(AP_THREADS), AP_SMEM, (cudaStream_t)stream, qmap, kmap, vmap,
                         kv->d_block_table, d_pos, (bf16*)d_out, sh, status));
   return Q_OK;
 }

@@ -62,3 +62,10 @@ def test_scale_that_is_not_positive(ops, scale):
 
 def test_output_of_4_byte_alignment(ops):
     case(ops, 1, 8, 2, 200, 0, False, 128 ** -0.5, offset=2)
+
+
+# Two query tiles per SM of 148: the last count with one tile per item (two items per CTA, every row's maximum
+# exchanged among four threads), and the first with two.
+@pytest.mark.parametrize("T,base", [(1184, 0), (1185, 0), (1000, 70)])
+def test_where_the_forms_part(ops, T, base):
+    case(ops, 1, 32, 8, T, base, True, 128 ** -0.5)
