@@ -182,7 +182,7 @@ int q_gemm_tc_plan(int M, int N, int K, q_gemm_plan_t* plan);
 int q_gemm_tc(const void* d_x, const void* d_w_tc, float* d_partials, int M, int N, int K,
               void* stream);
 
-/* ---- whole projections of 1..128 rows with the layer's element-wise work inside -------------
+/* ---- whole projections of 1..64 rows with the layer's element-wise work inside -------------
  * Same weight tiling as q_gemm_tc; N and K multiples of 8 and 64, x, gain and outputs 16-byte
  * aligned. No partial slots: K is split inside a thread-block cluster and added there.
  *   q_gemm_rows_f32     out = n @ W^T in fp32                          (W [N][K])

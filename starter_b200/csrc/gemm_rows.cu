@@ -1,4 +1,4 @@
-// Projections of a step (or a short prompt) with 1 .. 128 activation rows whose outputs are complete when the kernel ends: no
+// Projections of a step with 1 .. 64 activation rows whose outputs are complete when the kernel ends: no
 // split-K slots in memory, the layer's element-wise work before and after the product inside the kernel
 // (reference: engine/decode_step.py:43-59 runs norm, projection, add, norm, projection, SwiGLU, projection).
 //
@@ -10,8 +10,8 @@
 // so that a layer is QKV, attention, O, gate|up, down: five launches instead of the eight of gemm_tc.cu with
 // k_add_rmsnorm and k_swiglu between the projections (4 - 5 us each, of which under 1 us is work).
 //
-// What bounds it is the weight stream from HBM. The activations are the A operand (M = 64 or 128 rows of
-// the instruction; rows past the batch hold leftovers of shared memory and are never read back), the weight rows
+// What bounds it is the weight stream from HBM. The activations are the A operand (M = 64 rows of the
+// instruction; rows past the batch hold leftovers of shared memory and are never read back), the weight rows
 // the B operand: there a CTA's share is any number of 8-row atoms (1 KB for 64 k) of the 128 x 64 tiles of
 // gemm_tc.cu, copied as they lie. A cluster of S CTAs owns a run of atoms and splits K; at the end every CTA
 // sends its fp32 sums to the cluster CTA that owns the row (rows are dealt out in S runs) through
@@ -37,14 +37,12 @@ namespace {
 
 constexpr int GR_THREADS = 384;
 constexpr int GR_EPI = 256;                       // threads of warps 4-11
-constexpr int GR_MAX_ROWS = 128;
-constexpr int GR_MISC = (GR_MAX_ROWS + GR_EPI) * 4;        // bytes: 1 / rms of the rows, then partial sums of squares
+constexpr int GR_MISC = (64 + GR_EPI) * 4;        // bytes: 1 / rms of the rows, then partial sums of squares
 constexpr int GR_ATOM = 1024;                     // 8 weight rows x 64 k
 constexpr int GR_TILE = 16 * GR_ATOM;             // one 128 x 64 tile
 constexpr int GR_MAX_COLS = 256;                  // accumulator columns of a CTA
 constexpr int GR_MAX_STAGES = 12;
 constexpr size_t GR_SMEM = 224 * 1024;            // one CTA per SM
-constexpr size_t GR_SMEM_MAX = 227 * 1024;        // what a kernel is allowed (always the same: no launch lowers another's)
 
 enum { EPI_F32 = 0, EPI_RESID = 1, EPI_SWIGLU = 2 };
 
@@ -79,8 +77,7 @@ __device__ __forceinline__ uint32_t norm2(uint32_t x, float inv, uint32_t g) {
   return *reinterpret_cast<const uint32_t*>(&p);
 }
 
-// MR = rows of the MMA.
-template <int EPI, bool NORM, int MR>
+template <int EPI, bool NORM>
 __global__ void __launch_bounds__(GR_THREADS, 1)
 k_gemm_rows(const __grid_constant__ CUtensorMap xmap, const unsigned char* __restrict__ W, void* __restrict__ out,
             float* __restrict__ ss_out, const RowsShape sh, const RowsNorm nm, int* status, unsigned long long* tl) {
@@ -89,7 +86,7 @@ k_gemm_rows(const __grid_constant__ CUtensorMap xmap, const unsigned char* __res
   const uint32_t base = (raw + 1023u) & ~1023u;
   unsigned char* smem = smem_raw + (base - raw);
   float* recv = reinterpret_cast<float*>(smem + sh.recv_off);               // [S][rpr][ld]
-  float* inv_s = reinterpret_cast<float*>(smem + sh.misc_off);              // [GR_MAX_ROWS], then [GR_EPI] partial sums
+  float* inv_s = reinterpret_cast<float*>(smem + sh.misc_off);              // [64], then [GR_EPI] partial sums
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + sh.misc_off + GR_MISC);
   // full[stages] | empty[stages] | ready[stages] | acc_full
   const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8u * GR_MAX_STAGES;
@@ -109,8 +106,7 @@ k_gemm_rows(const __grid_constant__ CUtensorMap xmap, const unsigned char* __res
   const int rot = nk > 0 ? cl % nk : 0;
   const int cols = nu * (EPI == EPI_SWIGLU ? 16 : 8);                        // accumulator columns
   uint32_t tcols = 32;
-  const int mma_cols = MR == 64 ? cols : (cols + 15) / 16 * 16;              // (8 columns of leftovers, never read back)
-  while ((int)tcols < mma_cols) tcols <<= 1;
+  while ((int)tcols < cols) tcols <<= 1;
 
   // Nobody but warp 0 waits for the first weight copies to be issued, and they wait for nothing but the barriers:
   // tensor memory is allocated, and gains are fetched, meanwhile.
@@ -239,7 +235,7 @@ k_gemm_rows(const __grid_constant__ CUtensorMap xmap, const unsigned char* __res
     // ---------------- MMA issuer ----------------
     // (the whole warp walks the loop and one elected lane issues: descriptors stay in uniform registers)
     pdl_wait();                         // as in gemm_tc.cu: the wait limit starts here
-    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(mma_cols >> 3) << 17) | ((uint32_t)(MR >> 4) << 24);
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(cols >> 3) << 17) | (4u << 24);
     const uint64_t desc0 = smem_desc(base);
     const uint32_t stage_units = (uint32_t)sh.stage_bytes >> 4, a_units = a_bytes >> 4, tile_units = (uint32_t)sh.tile_bytes >> 4;
     bool ok = true;
@@ -291,20 +287,20 @@ k_gemm_rows(const __grid_constant__ CUtensorMap xmap, const unsigned char* __res
 #pragma unroll 8
         for (int p = g; p < nm.parts; p += groups) s += nm.ss[p * sh.M + r];
       }
-      inv_s[GR_MAX_ROWS + et] = s;
+      inv_s[64 + et] = s;
       epi_sync();
       if (et < sh.M) {
         float t = 0.f;
-        for (int j = 0; j < groups; ++j) t += inv_s[GR_MAX_ROWS + j * mp + et];
+        for (int j = 0; j < groups; ++j) t += inv_s[64 + j * mp + et];
         inv_s[et] = rsqrtf(t * nm.inv_k + nm.eps);
       }
       epi_sync();
       // A thread has one 16-byte chunk of rows r0, r0 + 16, ...: r0 % 8 is r % 8 of all of them, so that the
       // swizzled position stands for the same 8 columns in each.
       const int r0 = (et & 127) >> 3, pos = et & 7, chunk = pos ^ (r0 & 7);
-      float inv[MR / 16];
+      float inv[4];
 #pragma unroll
-      for (int j = 0; j < MR / 16; ++j) inv[j] = r0 + 16 * j < sh.M ? inv_s[r0 + 16 * j] : 0.f;
+      for (int j = 0; j < 4; ++j) inv[j] = r0 + 16 * j < sh.M ? inv_s[r0 + 16 * j] : 0.f;
       // Each group has one of a stage's two tiles. (Both wait for every stage: a group that skipped a phase of a
       // barrier could take the one before it for the one it waits for.)
       int st = 0, kt = rot;
@@ -317,7 +313,7 @@ k_gemm_rows(const __grid_constant__ CUtensorMap xmap, const unsigned char* __res
           unsigned char* a = smem + st * sh.stage_bytes + half * sh.tile_bytes + r0 * 128 + pos * 16;
           const uint4 gv = *reinterpret_cast<const uint4*>(gain_s + k * 64 + chunk * 8);
 #pragma unroll
-          for (int j = 0; j < MR / 16; ++j) {
+          for (int j = 0; j < 4; ++j) {
             if (r0 + 16 * j < sh.M) {
               uint4* p = reinterpret_cast<uint4*>(a + j * 2048);
               uint4 v = *p;
@@ -362,13 +358,12 @@ k_gemm_rows(const __grid_constant__ CUtensorMap xmap, const unsigned char* __res
       __syncwarp();
       gr_cluster_wait();                                                     // every CTA of the cluster has started
     }
-    // tensor memory -> the receive area of the CTA that finishes the row. With 64 rows a warp's first 16
-    // lanes hold 16 of them.
+    // tensor memory -> the receive area of the CTA that finishes the row. With M = 64 a warp's first 16
+    // lanes hold 16 rows.
     const int q = warp & 3;
-    constexpr int PER_WARP = MR / 4;
-    if (ok && q * PER_WARP < sh.M) {
-      const int m = q * PER_WARP + lane;
-      const bool live = lane < PER_WARP && m < sh.M;
+    if (ok && q * 16 < sh.M) {
+      const int m = q * 16 + lane;
+      const bool live = lane < 16 && m < sh.M;
       const int owner = live ? m / sh.rpr : 0;
       uint32_t dst = smem_u32(recv + ((size_t)rank * sh.rpr + (live ? m - owner * sh.rpr : 0)) * sh.ld);
       if (sh.S > 1) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(dst), "r"(owner));
@@ -473,7 +468,7 @@ k_gemm_rows(const __grid_constant__ CUtensorMap xmap, const unsigned char* __res
 
 // Clusters of S CTAs, one CTA per SM, that the current device holds at once (a cluster stays inside one
 // GPC); without a device what the SM count alone would allow.
-template <int EPI, bool NORM, int MR>
+template <int EPI, bool NORM>
 int rows_clusters(int S, int sms) {
   static int cached[64][5];
   if (S == 1) return sms;
@@ -491,8 +486,8 @@ int rows_clusters(int S, int sms) {
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     cfg.attrs = at; cfg.numAttrs = 1;
-    cudaError_t e = q_ensure_smem(k_gemm_rows<EPI, NORM, MR>, GR_SMEM_MAX, done);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&got, k_gemm_rows<EPI, NORM, MR>, &cfg);
+    cudaError_t e = q_ensure_smem(k_gemm_rows<EPI, NORM>, cfg.dynamicSmemBytes, done);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&got, k_gemm_rows<EPI, NORM>, &cfg);
     if (e != cudaSuccess) { cudaGetLastError(); got = sms / S; }
     n = got < sms / S ? got : sms / S;
     if (n < 1) n = 1;
@@ -501,9 +496,9 @@ int rows_clusters(int S, int sms) {
 }
 
 // N output columns (EPI_SWIGLU: inter) over the device; false where the kernel does not take the shape.
-template <int EPI, bool NORM, int MR>
-bool rows_shape_of(int M, int N, int K, RowsShape* sh, size_t* smem) {
-  if (M < 1 || M > MR || N < 8 || N % 8 || K < 64 || K % 64) return false;
+template <int EPI, bool NORM>
+bool rows_shape(int M, int N, int K, RowsShape* sh, size_t* smem) {
+  if (M < 1 || M > Q_MAX_ROWS || N < 8 || N % 8 || K < 64 || K % 64) return false;
   int sms = q_sm_count();
   if (sms <= 0) sms = 148;
   const int per = EPI == EPI_SWIGLU ? 16 : 8;
@@ -519,7 +514,7 @@ bool rows_shape_of(int M, int N, int K, RowsShape* sh, size_t* smem) {
   long long best = -1;
   for (int S = 1; S <= 4; S *= 2) {
     RowsShape t = *sh;
-    const int ncl = rows_clusters<EPI, NORM, MR>(S, sms);
+    const int ncl = rows_clusters<EPI, NORM>(S, sms);
     t.S = S;
     t.log_s = S == 4 ? 2 : S - 1;
     t.clusters = t.units < ncl ? t.units : ncl;
@@ -538,21 +533,16 @@ bool rows_shape_of(int M, int N, int K, RowsShape* sh, size_t* smem) {
     if (fixed + 3 * (size_t)t.stage_bytes > GR_SMEM) continue;
     t.stages = (int)((GR_SMEM - fixed) / t.stage_bytes);
     if (t.stages > GR_MAX_STAGES) t.stages = GR_MAX_STAGES;
-    size_t ring = (size_t)t.stages * t.stage_bytes + (t.tile_bytes > MR * 128 ? 0 : MR * 128 - t.tile_bytes);
+    size_t ring = (size_t)t.stages * t.stage_bytes + (t.tile_bytes > 8192 ? 0 : 8192 - t.tile_bytes);   // 64 rows are read
     if (S == 1 && ring < recv) ring = recv;
     t.recv_off = S > 1 ? (int)ring : 0;
     t.misc_off = (int)((ring + (S > 1 ? recv : 0) + 15) / 16 * 16);
     const size_t bytes = 1024 + t.misc_off + misc;
-    if (bytes > GR_SMEM_MAX) continue;
+    if (bytes > GR_SMEM + 8192) continue;
     const long long cost = (long long)kts * (cols * 128 + t.ar * 64) + (S > 1 ? 40000 : 0);
     if (best < 0 || cost < best) { best = cost; *sh = t; *smem = bytes; }
   }
   return sh->S != 0;
-}
-
-template <int EPI, bool NORM>
-bool rows_shape(int M, int N, int K, RowsShape* sh, size_t* smem) {
-  return M <= 64 ? rows_shape_of<EPI, NORM, 64>(M, N, K, sh, smem) : rows_shape_of<EPI, NORM, 128>(M, N, K, sh, smem);
 }
 
 template <int EPI, bool NORM>
@@ -573,16 +563,15 @@ int launch_rows(const void* x, const void* w_tc, void* out, float* ss_out, const
   const cuuint32_t box[2] = {64, (cuuint32_t)sh.ar};
   int rc = tc_encode(&map, x, 2, dim, stride, box, CU_TENSOR_MAP_SWIZZLE_128B, who);
   if (rc) return rc;
-  static size_t done[2][64] = {{0}};
-  auto kern = M <= 64 ? k_gemm_rows<EPI, NORM, 64> : k_gemm_rows<EPI, NORM, 128>;
-  Q_CHECK_CUDA(q_ensure_smem(kern, GR_SMEM_MAX, done[M <= 64 ? 0 : 1]));
+  static size_t done[64] = {0};
+  Q_CHECK_CUDA(q_ensure_smem(k_gemm_rows<EPI, NORM>, smem, done));
   const dim3 grid(sh.clusters * sh.S), block(GR_THREADS);
   if (sh.S > 1)
-    Q_CHECK_CUDA(q_launch_cluster(kern, grid, block, smem, (cudaStream_t)stream, (unsigned)sh.S, map,
+    Q_CHECK_CUDA(q_launch_cluster(k_gemm_rows<EPI, NORM>, grid, block, smem, (cudaStream_t)stream, (unsigned)sh.S, map,
                                   (const unsigned char*)w_tc, out, ss_out, sh, nm, status, q_tl_next(Q_TL_GEMM_TC)));
   else
-    Q_CHECK_CUDA(q_launch(kern, grid, block, smem, (cudaStream_t)stream, map, (const unsigned char*)w_tc, out, ss_out,
-                          sh, nm, status, q_tl_next(Q_TL_GEMM_TC)));
+    Q_CHECK_CUDA(q_launch(k_gemm_rows<EPI, NORM>, grid, block, smem, (cudaStream_t)stream, map,
+                          (const unsigned char*)w_tc, out, ss_out, sh, nm, status, q_tl_next(Q_TL_GEMM_TC)));
   return Q_OK;
 }
 

@@ -1,4 +1,4 @@
-"""Projections of 1-128 rows with norm, residual add and SwiGLU inside (q_gemm_rows_*), against the
+"""Projections of 1-64 rows with norm, residual add and SwiGLU inside (q_gemm_rows_*), against the
 same rounding points in plain torch: fp64 products, everything else as the oracle rounds it."""
 import ctypes as C
 
@@ -56,7 +56,7 @@ def _close_add(got, want, branch):
 
 # rows at the edges of the 8-row slices, the 16-row warps and the clusters' row runs; widths of one atom,
 # of runs that cross a 128-row block, and the benchmark's
-ROWS = [1, 3, 8, 9, 16, 17, 33, 64, 65, 100, 128]
+ROWS = [1, 3, 8, 9, 16, 17, 33, 64]
 
 
 @pytest.mark.parametrize("rows", ROWS)
@@ -111,6 +111,6 @@ def test_swiglu(rows, inter, K):
 
 def test_refused():
     z = torch.zeros(4096, dtype=torch.bfloat16, device="cuda")
-    for rows, N, K in ((0, 64, 64), (129, 64, 64), (4, 12, 64), (4, 64, 96)):
+    for rows, N, K in ((0, 64, 64), (65, 64, 64), (4, 12, 64), (4, 64, 96)):
         assert lib.q_gemm_rows_parts(rows, N, K) == 0
         assert lib.q_gemm_rows_add(_p(z), _p(z), _p(z), _p(z), rows, N, K, _stream()) == ERR_ARG
