@@ -153,7 +153,7 @@ int* q_peer_status_addr();
 static int status_addrs(int* addr[4]) {
   addr[0] = q_attn_status_addr();   // attention: 1 producer wait ran out, 2 consumer wait ran out (prompt kernel: 7, 8 MMA issuer, 9 softmax)
   addr[1] = q_gemm_status_addr();   // stream-K GEMM: 1 ring wait ran out
-  addr[2] = q_tc_status_addr();     // tcgen05 GEMM: 1 producer, 2 MMA issuer, 3 epilogue wait ran out (CTA pairs: 5, 6, 7; 4 / 8 a copy did not land)
+  addr[2] = q_tc_status_addr();     // tcgen05 GEMM: 1 producer, 2 MMA issuer, 3 epilogue wait ran out (CTA pairs: 5, 6, 7; whole projections: 10, 11, 12; 4 / 8 / 13 a copy did not land)
   addr[3] = q_peer_status_addr();   // tensor parallel over peer memory: 1 = a peer's arrival word never came
   for (int i = 0; i < 4; ++i)
     if (!addr[i]) { q_set_error("could not locate the device status words"); return Q_ERR_CUDA; }

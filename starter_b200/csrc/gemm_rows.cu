@@ -43,6 +43,7 @@ constexpr int GR_TILE = 16 * GR_ATOM;             // one 128 x 64 tile
 constexpr int GR_MAX_COLS = 256;                  // accumulator columns of a CTA
 constexpr int GR_MAX_STAGES = 12;
 constexpr size_t GR_SMEM = 224 * 1024;            // one CTA per SM
+constexpr size_t GR_SMEM_MAX = 227 * 1024;        // what a kernel is allowed (always the same: no launch lowers another's)
 
 enum { EPI_F32 = 0, EPI_RESID = 1, EPI_SWIGLU = 2 };
 
@@ -486,7 +487,7 @@ int rows_clusters(int S, int sms) {
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     cfg.attrs = at; cfg.numAttrs = 1;
-    cudaError_t e = q_ensure_smem(k_gemm_rows<EPI, NORM>, cfg.dynamicSmemBytes, done);
+    cudaError_t e = q_ensure_smem(k_gemm_rows<EPI, NORM>, GR_SMEM_MAX, done);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&got, k_gemm_rows<EPI, NORM>, &cfg);
     if (e != cudaSuccess) { cudaGetLastError(); got = sms / S; }
     n = got < sms / S ? got : sms / S;
@@ -538,7 +539,7 @@ bool rows_shape(int M, int N, int K, RowsShape* sh, size_t* smem) {
     t.recv_off = S > 1 ? (int)ring : 0;
     t.misc_off = (int)((ring + (S > 1 ? recv : 0) + 15) / 16 * 16);
     const size_t bytes = 1024 + t.misc_off + misc;
-    if (bytes > GR_SMEM + 8192) continue;
+    if (bytes > GR_SMEM_MAX) continue;
     const long long cost = (long long)kts * (cols * 128 + t.ar * 64) + (S > 1 ? 40000 : 0);
     if (best < 0 || cost < best) { best = cost; *sh = t; *smem = bytes; }
   }
@@ -564,7 +565,7 @@ int launch_rows(const void* x, const void* w_tc, void* out, float* ss_out, const
   int rc = tc_encode(&map, x, 2, dim, stride, box, CU_TENSOR_MAP_SWIZZLE_128B, who);
   if (rc) return rc;
   static size_t done[64] = {0};
-  Q_CHECK_CUDA(q_ensure_smem(k_gemm_rows<EPI, NORM>, smem, done));
+  Q_CHECK_CUDA(q_ensure_smem(k_gemm_rows<EPI, NORM>, GR_SMEM_MAX, done));
   const dim3 grid(sh.clusters * sh.S), block(GR_THREADS);
   if (sh.S > 1)
     Q_CHECK_CUDA(q_launch_cluster(k_gemm_rows<EPI, NORM>, grid, block, smem, (cudaStream_t)stream, (unsigned)sh.S, map,

@@ -1,6 +1,6 @@
 // Weight-streaming GEMM on the 5th-generation tensor cores (tcgen05.mma, accumulators in
-// tensor memory) for 9 .. 256 activation rows (more run as row chunks of 256; the prompt pass uses
-// gemm_prompt.cu from 257 rows on).
+// tensor memory) for 9 .. 256 activation rows (more run as row chunks of 256): lm_head, prompts of 65 .. 256 rows
+// and tensor parallelism. gemm_rows.cu has the layers of steps and shorter prompts, gemm_prompt.cu those of longer ones.
 //
 // Y[M,N] = X[M,K] . W[N,K]^T, bf16 operands, fp32 accumulation, written as the same fp32
 // split-K partial slots that the stream-K kernel of gemm_streamk.cu produces, so the fused

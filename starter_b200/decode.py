@@ -259,8 +259,9 @@ class DecodeState:
     # ---- prefill: the prompt pass ----
     PREFILL_ROWS = 8192        # prompt rows processed together (bounds the activation scratch)
     # Rows from which the projections run on the CTA-pair kernel: the first that k_gemm_tc cannot hold in
-    # one pass over the weight (256). Prompt pass of 12 layers, k_gemm_tc / pairs, us: 64 rows 1133 / 2091,
-    # 192 1615 / 2058, 256 1856 / 2064, but 257 2232 / 2128, 300 2336 / 2118, 512 2641 / 2220, 1024 4548 / 3230.
+    # one pass over the weight (256; up to 64 rows the projections are k_gemm_rows). Prompt pass of 12 layers,
+    # below / pairs, us: 65 rows 1101 / 2025, 128 1300 / 1934, 192 1589 / 1972, 256 1823 / 1993; above, when the
+    # attention was slower for both: 257 2232 / 2128, 512 2641 / 2220, 1024 4548 / 3230.
     PROMPT_GEMM_ROWS = 257
     PROMPT_TICKET_BYTES = 16384    # leading bytes of q_gemm_prompt_*'s scratch that have to be zero
 
@@ -318,7 +319,8 @@ class DecodeState:
         The prompt pass of the reference (engine/prefill.py:26-62) on this library's own
         kernels: from PROMPT_GEMM_ROWS rows on every projection on the CTA-pair tcgen05 kernel with
         the residual add, SwiGLU or head norm + RoPE + page write (engine/kernels/prefill.py:19-63)
-        as its epilogue, below that on the decode step's projections and consumers; the causal
+        as its epilogue, below that on the decode step's projections (up to 64 rows whole ones, then split-K
+        with their consumers); the causal
         attention over the prompt as q_attention_prefill reading the pages just written, lm_head
         and argmax as in the step; no library kernel runs. Sequences are processed PREFILL_ROWS prompt
         rows at a time (one q_prompt_pass call each). Under tensor
