@@ -399,11 +399,19 @@ k_attn_prompt(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ 
       for (int j = 0; j < it.n; ++j, ++step) {
         wait(bar(B_SF, i), step & 1);
         float v[COLS];
+        if constexpr (TILES == 2) {
+          tc_ld32(s_addr, v);
+          tc_ld32(s_addr + 32, v + 32);
+          tc_wait_ld();
+          tc_pin32(v);
+          tc_pin32(v + 32);
+        } else {
+          float lo[16], hi[16];
+          tc_ld16(s_addr, lo);
+          tc_ld16(s_addr + 16, hi);
 #pragma unroll
-        for (int k = 0; k < COLS; k += 32) tc_ld32(s_addr + k, v + k);
-        tc_wait_ld();
-#pragma unroll
-        for (int k = 0; k < COLS; k += 32) tc_pin32(v + k);
+          for (int k = 0; k < 16; ++k) { v[k] = lo[k]; v[k + 16] = hi[k]; }
+        }
         const int key_base = j * AP_KEYS;
         if (!plain) {
 #pragma unroll
