@@ -471,7 +471,7 @@ k_gemm_rows(const __grid_constant__ CUtensorMap xmap, const unsigned char* __res
 // GPC); without a device what the SM count alone would allow.
 template <int EPI, bool NORM>
 int rows_clusters(int S, int sms) {
-  static int cached[64][5];
+  static int cached[64][9];
   if (S == 1) return sms;
   const int dev = q_device_index();
   if (dev < 0) return sms / S;
@@ -510,14 +510,17 @@ bool rows_shape(int M, int N, int K, RowsShape* sh, size_t* smem) {
   sh->ldo = N;
   sh->ar = (M + 7) / 8 * 8;
   sh->S = 0;
-  // K is split as far as it takes to give every SM a share of whole atoms that is not small beside the
-  // activation slice that comes with it; the exchange is charged like 40 KB of weights.
+  // K is split so that a CTA's time comes out least, in bytes at the HBM rate of an SM: its weights, half of its
+  // activation slices (from L2), 11 KB a ring stage (250 ns) and 40 KB for the exchange. Clusters of 8 leave a quarter of
+  // the SMs idle and still win by the stages and, since O and down then leave half as many sums of squares, in the next
+  // norm; above 32 rows their receive area does not fit. Step of 12 layers, at most 4 / 8 CTAs a cluster, us: 9 x 300
+  // keys 790 / 771, 16 x 1024 896 / 883, 32 x 500 904 / 902.
   long long best = -1;
-  for (int S = 1; S <= 4; S *= 2) {
+  for (int S = 1; S <= 8; S *= 2) {
     RowsShape t = *sh;
     const int ncl = rows_clusters<EPI, NORM>(S, sms);
     t.S = S;
-    t.log_s = S == 4 ? 2 : S - 1;
+    t.log_s = S == 8 ? 3 : S == 4 ? 2 : S - 1;
     t.clusters = t.units < ncl ? t.units : ncl;
     t.each = t.units / t.clusters;
     t.more = t.units - t.each * t.clusters;
@@ -540,7 +543,7 @@ bool rows_shape(int M, int N, int K, RowsShape* sh, size_t* smem) {
     t.misc_off = (int)((ring + (S > 1 ? recv : 0) + 15) / 16 * 16);
     const size_t bytes = 1024 + t.misc_off + misc;
     if (bytes > GR_SMEM_MAX) continue;
-    const long long cost = (long long)kts * (cols * 128 + t.ar * 64) + (S > 1 ? 40000 : 0);
+    const long long cost = (long long)kts * (cols * 128 + t.ar * 64) + (kts + 1) / 2 * 11000 + (S > 1 ? 40000 : 0);
     if (best < 0 || cost < best) { best = cost; *sh = t; *smem = bytes; }
   }
   return sh->S != 0;
