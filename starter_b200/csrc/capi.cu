@@ -751,10 +751,10 @@ extern "C" int q_prompt_pass(const q_prompt_t* p, const q_layer_weights_t* layer
                           p->rms_eps, p->split, stream));
     TRY(q_attention_prefill(p->q, &kv, p->pos, p->attended, batch, T, nq, p->attn_scale, stream));
     TRY(q_gemm_prompt_add(p->attended, w.wo_tc, p->x, rows, H, nq * 128, p->split, stream));
-    TRY(q_rmsnorm(p->x, w.ln_post, p->normed, rows, H, p->rms_eps, stream));
+    TRY(q_rmsnorm_weights(p->x, w.ln_post, p->normed, rows, H, p->rms_eps, stream));
     TRY(q_gemm_prompt_swiglu(p->normed, w.wgu_tc, p->act, rows, I, H, p->split, stream));
     TRY(q_gemm_prompt_add(p->act, w.wdown_tc, p->x, rows, H, I, p->split, stream));
-    if (!last) TRY(q_rmsnorm(p->x, gain, p->normed, rows, H, p->rms_eps, stream));
+    if (!last) TRY(q_rmsnorm_weights(p->x, gain, p->normed, rows, H, p->rms_eps, stream));
   }
   // the last position of every sequence (only these rows need the final norm)
   TRY(q_rmsnorm_strided((const char*)p->x + (size_t)(T - 1) * H * 2, (long long)T * H, p->ln_final, d_last, batch, H,

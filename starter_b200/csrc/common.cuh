@@ -132,7 +132,9 @@ int q_gemm_launch_planned(const void* d_x, const void* d_w_tiled, float* d_parti
 int q_gemm_tc_launch(const void* d_x, const void* d_w_tc, float* d_partials, const q_gemm_plan_t* plan,
                      void* stream);
 
-// RMSNorm of `rows` rows that lie `stride` elements apart, into consecutive rows.
+// q_rmsnorm with a gain that is a model's weight (it may be read before the kernels ahead in the stream
+// have ended), and the same of `rows` rows that lie `stride` elements apart, into consecutive rows.
+int q_rmsnorm_weights(const void* d_x, const void* d_gain, void* d_out, int rows, int cols, float eps, void* stream);
 int q_rmsnorm_strided(const void* d_x, long long stride, const void* d_gain, void* d_out, int rows, int cols,
                       float eps, void* stream);
 

@@ -44,9 +44,10 @@ k_rmsnorm(const bf16* __restrict__ X, const bf16* __restrict__ G, bf16* __restri
 
 // The same for whole matrices (the prompt pass): one warp per row, the row in registers, all of
 // its 16-byte loads in flight together and no block barrier. cols a multiple of 8, at most
-// 256 * VECS, 16-byte aligned rows. EARLY: the gains, which are weights, are asked for before the dependency
-// wait and held (they are cold in a step that streams all weights between two uses): where an SM has no second
-// CTA to run those registers cost nothing.
+// 256 * VECS, 16-byte aligned rows. EARLY: the gains are asked for before the dependency wait and held (they are
+// cold in a step that streams all weights between two uses): where an SM has no second CTA to run those registers
+// cost nothing. Only for gains that no kernel of the stream writes - a model's weights; a caller's gain may
+// come from the launch right before, which lets this kernel start before it has written it.
 template <int VECS, bool EARLY>
 __global__ void __launch_bounds__(256)
 k_rmsnorm_rows(const bf16* __restrict__ X, const bf16* __restrict__ G, bf16* __restrict__ O,
@@ -759,32 +760,17 @@ __global__ void k_argmax_merge(const float* __restrict__ val, const int32_t* __r
 
 #define S(x) ((cudaStream_t)(x))
 
-extern "C" int q_rmsnorm(const void* d_x, const void* d_gain, void* d_out, int rows, int cols,
-                         float eps, void* stream) {
-  Q_CHECK_ARG(d_x && d_gain && d_out && rows >= 1 && cols >= 1, "q_rmsnorm: bad argument");
-  Q_CHECK_ALIGN(d_x, 2, "q_rmsnorm"); Q_CHECK_ALIGN(d_gain, 2, "q_rmsnorm"); Q_CHECK_ALIGN(d_out, 2, "q_rmsnorm");
-  // Many rows: a warp each (k_rmsnorm_rows); odd widths and unaligned rows keep a CTA per row. So do up
-  // to two rows per SM, not for speed - CTA / warp, 2560 columns, us: 16 rows 4.9 / 3.8, 256 6.5 / 4.0,
-  // 400 6.8 / 4.2, 2048 10.2 / 4.4 - but because the two forms add the squares in another order and few
-  // rows are the operator's own use, where there is about a microsecond in it.
-  const int sms = q_sm_count();
-  if (rows > 2 * (sms > 0 ? sms : 148)) return q_rmsnorm_strided(d_x, cols, d_gain, d_out, rows, cols, eps, stream);
-  Q_CHECK_CUDA(q_launch(k_rmsnorm, dim3(rows), dim3(256), 0, S(stream), (const bf16*)d_x,
-                        (const bf16*)d_gain, (bf16*)d_out, cols, (long long)cols, eps));
-  return Q_OK;
-}
-
-// (the prompt pass norms one row per sequence with it: 16-byte loads in one round trip, where the
-// CTA per row of k_rmsnorm took 10 us for one cold row of 2560)
-int q_rmsnorm_strided(const void* d_x, long long stride, const void* d_gain, void* d_out, int rows, int cols,
-                      float eps, void* stream) {
+// RMSNorm of rows `stride` elements apart with a warp per row where width and alignment allow it (16-byte loads
+// in one round trip: the CTA per row of k_rmsnorm took 10 us for one cold row of 2560).
+static int rmsnorm_by_warps(const void* d_x, long long stride, const void* d_gain, void* d_out, int rows, int cols,
+                            float eps, bool weights, void* stream) {
   const bool vec = cols % 8 == 0 && stride % 8 == 0 && cols <= 4096 &&
                    (((uintptr_t)d_x | (uintptr_t)d_gain | (uintptr_t)d_out) & 15) == 0;
   const dim3 grid((rows + 7) / 8);
   // Gains held from before the wait / fetched after the sum, cols 2560, us: 300 rows 3.0 / 4.3, 1024 3.4 / 4.8, but
   // 2048 (256 CTAs) 6.2 / 5.3, 8192 20.5 / 16.4; the one norm of a 64-row decode step 4.1 / 8.7.
   const int sms = q_sm_count();
-  const bool early = (int)grid.x <= (sms > 0 ? sms : 148);
+  const bool early = weights && (int)grid.x <= (sms > 0 ? sms : 148);
   if (vec) {
     auto kern = cols <= 2560 ? (early ? k_rmsnorm_rows<10, true> : k_rmsnorm_rows<10, false>)
                              : (early ? k_rmsnorm_rows<16, true> : k_rmsnorm_rows<16, false>);
@@ -795,6 +781,35 @@ int q_rmsnorm_strided(const void* d_x, long long stride, const void* d_gain, voi
                           (bf16*)d_out, cols, stride, eps));
   }
   return Q_OK;
+}
+
+static int rmsnorm(const void* d_x, const void* d_gain, void* d_out, int rows, int cols, float eps, bool weights,
+                   void* stream) {
+  // Many rows: a warp each (k_rmsnorm_rows); odd widths and unaligned rows keep a CTA per row. So do up
+  // to two rows per SM, not for speed - CTA / warp, 2560 columns, us: 16 rows 4.9 / 3.8, 256 6.5 / 4.0,
+  // 400 6.8 / 4.2, 2048 10.2 / 4.4 - but because the two forms add the squares in another order and few
+  // rows are the operator's own use, where there is about a microsecond in it.
+  const int sms = q_sm_count();
+  if (rows > 2 * (sms > 0 ? sms : 148)) return rmsnorm_by_warps(d_x, cols, d_gain, d_out, rows, cols, eps, weights, stream);
+  Q_CHECK_CUDA(q_launch(k_rmsnorm, dim3(rows), dim3(256), 0, S(stream), (const bf16*)d_x,
+                        (const bf16*)d_gain, (bf16*)d_out, cols, (long long)cols, eps));
+  return Q_OK;
+}
+
+extern "C" int q_rmsnorm(const void* d_x, const void* d_gain, void* d_out, int rows, int cols,
+                         float eps, void* stream) {
+  Q_CHECK_ARG(d_x && d_gain && d_out && rows >= 1 && cols >= 1, "q_rmsnorm: bad argument");
+  Q_CHECK_ALIGN(d_x, 2, "q_rmsnorm"); Q_CHECK_ALIGN(d_gain, 2, "q_rmsnorm"); Q_CHECK_ALIGN(d_out, 2, "q_rmsnorm");
+  return rmsnorm(d_x, d_gain, d_out, rows, cols, eps, false, stream);
+}
+
+int q_rmsnorm_weights(const void* d_x, const void* d_gain, void* d_out, int rows, int cols, float eps, void* stream) {
+  return rmsnorm(d_x, d_gain, d_out, rows, cols, eps, true, stream);
+}
+
+int q_rmsnorm_strided(const void* d_x, long long stride, const void* d_gain, void* d_out, int rows, int cols,
+                      float eps, void* stream) {
+  return rmsnorm_by_warps(d_x, stride, d_gain, d_out, rows, cols, eps, true, stream);
 }
 
 extern "C" int q_embed_rmsnorm(const int64_t* d_tokens, const void* d_embed, const void* d_gain,

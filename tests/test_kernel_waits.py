@@ -59,6 +59,18 @@ def test_prompt_attention_reads_its_inputs_after_the_dependency_wait():
     assert not re.search(r"pos_ptr|block_table|table\[", before)
 
 
+def test_the_public_norm_reads_its_gain_after_the_dependency_wait():
+    """The gain of q_rmsnorm is the caller's and may be what the launch before computes; only the engine, whose
+    gains are weights, may have it fetched before the wait."""
+    text = source("fused_ops.cu")
+    kernel = between(text, "k_rmsnorm_rows(const bf16*", "\n}\n")
+    before = kernel[:kernel.index("pdl_wait();")]
+    assert before.count("__ldg(") == 1 and re.search(r"if \(EARLY\) \{[^}]*__ldg\(", before)
+    assert re.search(r"const bool early = weights && ", text)
+    public = between(text, 'extern "C" int q_rmsnorm(', "\n}\n")
+    assert "return rmsnorm(d_x, d_gain, d_out, rows, cols, eps, false, stream);" in public and "true" not in public
+
+
 def test_the_wait_on_an_mbarrier_is_one_loop_bounded_by_the_clock():
     """Every role of the tcgen05 kernels inlines it: a second loop for flag and clock cost a prompt of 64
     tokens 2 %. Its limit counts cycles, since a try may itself sleep."""

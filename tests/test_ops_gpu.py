@@ -330,6 +330,21 @@ def test_rms_norm_plain(ops):
     assert bit_equal_fraction(got, ref) > 0.99
 
 
+@pytest.mark.parametrize("rows", [7, 297, 1184, 1185])
+def test_rms_norm_with_a_gain_from_the_launch_before(ops, rows):
+    """A conditional gain: the projection that computes it lets its dependents start before it has written
+    anything, so a norm that fetched its gain early would take what the buffer held before."""
+    from starter_b200.weights import TiledWeight
+    x, w = randx(rows, H, 43).cuda(), TiledWeight.pack(randw(2 * H, H, 44).cuda(), interleave8=True)
+    for seed in range(45, 49):
+        condition = randx(1, H, seed).cuda()
+        torch.cuda.synchronize()
+        got = ops.rms_norm(x, ops.linear_silu_mul(condition, w).view(H), 1e-6)
+        gain = ops.linear_silu_mul(condition, w).view(H)
+        torch.cuda.synchronize()
+        assert torch.equal(got, ops.rms_norm(x, gain, 1e-6))
+
+
 @pytest.mark.parametrize("B,T,nq,nkv", [(1, 1, 32, 8), (4, 1, 8, 2), (2, 4, 8, 2), (3, 2, 4, 2)])
 def test_qkv_norm_rope_cache(ops, B, T, nq, nkv):
     """Q, K within one ulp of the oracle, V exact; only the slots position..position+T-1
