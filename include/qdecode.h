@@ -280,8 +280,11 @@ typedef struct q_kv_layout_t {
  * d_scratch: q_gemm_prompt_scratch_bytes() bytes, 16-byte aligned, the first 16 KB zeroed by the
  * caller before the first launch and after one that gave up (device status word 2; every other
  * launch leaves them zero), for the parts of tiles that several SM pairs share; one per stream,
- * since calls that overlap on the GPU may not share it. Null: whole tiles only. */
+ * since calls that overlap on the GPU may not share it. Null: whole tiles only.
+ * q_gemm_prompt_columns: the output columns of a tile (256 or 160) that q_gemm_prompt_add (residual
+ * != 0) or q_gemm_prompt_f32 takes with scratch; 0 for a shape they refuse. */
 int64_t q_gemm_prompt_scratch_bytes(void);
+int q_gemm_prompt_columns(int M, int N, int K, int residual);
 int q_gemm_prompt_f32(const void* d_x, const void* d_w_tc, float* d_out, int M, int N, int K,
                       void* d_scratch, void* stream);
 int q_gemm_prompt_add(const void* d_x, const void* d_w_tc, void* d_resid, int M, int N, int K,

@@ -115,6 +115,7 @@ SIGNATURES = {
     "q_gemm_rows_add": (_I, [_P, _P, _P, _P, _I, _I, _I, _P]),
     "q_gemm_rows_swiglu": (_I, [_P, _P, _P, _I, _P, _P, _I, _I, _I, _F, _P]),
     "q_gemm_prompt_scratch_bytes": (C.c_int64, []),
+    "q_gemm_prompt_columns": (_I, [_I, _I, _I, _I]),
     "q_gemm_prompt_f32": (_I, [_P, _P, _P, _I, _I, _I, _P, _P]),
     "q_gemm_prompt_add": (_I, [_P, _P, _P, _I, _I, _I, _P, _P]),
     "q_gemm_prompt_swiglu": (_I, [_P, _P, _P, _I, _I, _I, _P, _P]),

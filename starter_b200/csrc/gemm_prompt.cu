@@ -50,7 +50,7 @@ constexpr int PG_EPI_WARPS = 8;
 constexpr int PG_TILE_K = 64;
 constexpr int PG_A_BYTES = 128 * PG_TILE_K * 2;            // 16 KB of activations per CTA and stage
 constexpr int PG_BN = 256, PG_HALF = 128;                  // columns of a tile, weight rows per CTA
-constexpr int PG_NARROW = 160;                             // ... of a narrow tile: weight rows in runs of 16, see launch_prompt
+constexpr int PG_NARROW = 160;                             // ... of a narrow tile: weight rows in runs of 16, see prompt_plan
 __host__ __device__ constexpr uint32_t pg_stage(int bn) { return PG_A_BYTES + bn / 2 * PG_TILE_K * 2; }
 __host__ __device__ constexpr int pg_stages(int bn) { return bn == PG_BN ? 7 : 8; }                     // 224 KB, 208 KB
 constexpr size_t pg_smem(int bn) { return 1024 + pg_stages(bn) * pg_stage(bn) + (2 * pg_stages(bn) + 4) * 8 + 16; }
@@ -686,7 +686,70 @@ int pair_count() {
   return pairs < PG_MAX_PAIRS ? pairs : PG_MAX_PAIRS;
 }
 
-// `N` as in PromptShape; the weight has `wN` rows.
+// `N` as in PromptShape; the weight has `wN` rows. Tiles and their split for a shape; `pairs` in: of the device, out: of the launch. False: too many tiles.
+bool prompt_plan(int epi, int M, int N, int wN, int K, bool scratch, PromptShape* plan, int* pairs_io, bool* narrow) {
+  PromptShape& sh = *plan;
+  sh.M = M; sh.N = N;
+  // A raster group reads the whole weight once. Where the weight does not stay in L2 from one group to the next,
+  // fewer and taller groups: gate|up (100 MB) in groups of 4 / 8 / 16 / 32 row tiles 609 / 597 / 586 / 580 us at
+  // 8192 rows, 534 / 527 / 516 / 512 at 7000 (in a loop under the power cap), but down (50 MB) 328 / 333 / 335 / 351
+  // and O (21 MB) 143 / 141 / 143 / 152.
+  sh.group = (long long)wN * K * 2 > (64ll << 20) ? 32 : 8;
+  sh.KT = (K + PG_TILE_K - 1) / PG_TILE_K;
+  sh.mt = (M + 255) / 256;
+  const int cols = epi == EPI_SWIGLU ? PG_HALF : PG_BN;
+  sh.nt = (N + cols - 1) / cols;
+  const long long tiles = (long long)sh.mt * sh.nt;
+  if (tiles * sh.KT >= (1ll << 30)) return false;
+  sh.wrows = 128;
+  while (epi == EPI_SWIGLU && N % sh.wrows) sh.wrows >>= 1;
+  const int pairs = *pairs_io;
+  *narrow = false;
+  // Whole tiles only, or the last wave and the remainder cut evenly: the split saves the idle part of
+  // a wave (k steps of ~0.4 us each) and costs parts through L2, tickets, the merge and a late epilogue.
+  // Split / whole, us: QKV at 1024 rows (52 against 80 steps) 39.3 / 34.9, O at 400 (9 against 64)
+  // 29.4 / 25.3, down at 1500 (123 against 152) 70.2 / 58.8, but down at 1024 (83 against 152) 50.3 / 57.0.
+  const int full = (int)(tiles / pairs), rest = (int)(tiles % pairs);
+  sh.waves = full;
+  sh.share = sh.KT;
+  if (scratch && rest) {
+    const int whole = full > 0 ? full - 1 : 0;
+    const int left = (int)(tiles - (long long)whole * pairs);
+    const int share = (left * sh.KT + pairs - 1) / pairs;
+    if (share + PG_SPLIT_STEPS < (full - whole + 1) * sh.KT) {
+      sh.waves = whole;
+      sh.share = share;
+    }
+  }
+  if (epi == EPI_RESID || epi == EPI_F32) {
+    // Narrow tiles (whole ones) where they leave less of a wave idle. Both sides in k steps of a wide tile: a narrow
+    // step takes 0.71 (0.63 the columns, the same activations); a nearly empty wave down to 0.5 of a full one, a narrow
+    // one 0.7; a split 3 steps for each part of a tile and 31 (17 with fp32 sums, which wait for no residual), behind
+    // whole waves 5. Wide / narrow, us, weights cold: O at 257 rows 26.3 / 20.3, 1024 27.8 / 21.4, 2048 49.6 / 40.3, but
+    // 1280 27.8 / 34.7, 4096 80.0 / 81.7, 8192 143 / 154; down at 600 45.4 / 42.2, 1024 54.7 / 45.4, 2103 105 / 101, but
+    // 1900 96.1 / 100.3, 2500 117 / 150; down's fp32 sums at 1024 51.1 / 47.6, but 600 39.9 / 44.1, 2048 88.0 / 101. Of
+    // 780 shapes (N 896 - 5120, K 512 - 17408, 257 - 8192 rows, both epilogues) two lose more than 1 % (28.3 / 28.8, 2.4 %).
+    PromptShape nr = sh;
+    nr.nt = (N + PG_NARROW - 1) / PG_NARROW;
+    const long long nt = (long long)nr.mt * nr.nt;
+    const double busy = (double)rest / pairs, nbusy = (double)(nt % pairs) / pairs;
+    const double tail = sh.share != sh.KT ? sh.share + (sh.waves ? 5.0 : (epi == EPI_F32 ? 17 : 31) + 3.0 * sh.KT / sh.share)
+                        : rest ? sh.KT * (0.5 + 0.5 * busy) : 0;
+    const double wide = (double)sh.waves * sh.KT + tail;
+    const double cost = 0.71 * sh.KT * ((double)(nt / pairs) + (nt % pairs ? 0.7 + 0.3 * nbusy : 0.0));
+    if (cost < wide) {
+      nr.waves = (int)(nt / pairs);
+      nr.share = nr.KT;
+      if (nt < pairs) *pairs_io = (int)nt;
+      sh = nr;
+      *narrow = true;
+      return true;
+    }
+  }
+  if (sh.share == sh.KT && tiles < pairs) *pairs_io = (int)tiles;
+  return true;
+}
+
 template <int EPI, int BN>
 int launch_tiles(const void* x, const void* w_tc, void* out, int M, int wN, int K, PromptShape sh, int pairs,
                  const RopeArgs& ra, void* scratch, int* status, void* stream, const char* who) {
@@ -727,60 +790,12 @@ int launch_prompt(const void* x, const void* w_tc, void* out, int M, int N, int 
   int* status = q_tc_status_addr();
   if (!status) { q_set_error("%s: could not locate the device status word", who); return Q_ERR_CUDA; }
   PromptShape sh;
-  sh.M = M; sh.N = N;
-  // A raster group reads the whole weight once. Where the weight does not stay in L2 from one group to the next,
-  // fewer and taller groups: gate|up (100 MB) in groups of 4 / 8 / 16 / 32 row tiles 609 / 597 / 586 / 580 us at
-  // 8192 rows, 534 / 527 / 516 / 512 at 7000 (in a loop under the power cap), but down (50 MB) 328 / 333 / 335 / 351
-  // and O (21 MB) 143 / 141 / 143 / 152.
-  sh.group = (long long)wN * K * 2 > (64ll << 20) ? 32 : 8;
-  sh.KT = (K + PG_TILE_K - 1) / PG_TILE_K;
-  sh.mt = (M + 255) / 256;
-  const int cols = EPI == EPI_SWIGLU ? PG_HALF : PG_BN;
-  sh.nt = (N + cols - 1) / cols;
-  const long long tiles = (long long)sh.mt * sh.nt;
-  Q_CHECK_ARG(tiles * sh.KT < (1ll << 30), "%s: too many tiles", who);
-  sh.wrows = 128;
-  while (EPI == EPI_SWIGLU && N % sh.wrows) sh.wrows >>= 1;
   int pairs = pair_count();
-  // Whole tiles only, or the last wave and the remainder cut evenly: the split saves the idle part of
-  // a wave (k steps of ~0.4 us each) and costs parts through L2, tickets, the merge and a late epilogue.
-  // Split / whole, us: QKV at 1024 rows (52 against 80 steps) 39.3 / 34.9, O at 400 (9 against 64)
-  // 29.4 / 25.3, down at 1500 (123 against 152) 70.2 / 58.8, but down at 1024 (83 against 152) 50.3 / 57.0.
-  const int full = (int)(tiles / pairs), rest = (int)(tiles % pairs);
-  sh.waves = full;
-  sh.share = sh.KT;
-  if (scratch && rest) {
-    const int whole = full > 0 ? full - 1 : 0;
-    const int left = (int)(tiles - (long long)whole * pairs);
-    const int share = (left * sh.KT + pairs - 1) / pairs;
-    if (share + PG_SPLIT_STEPS < (full - whole + 1) * sh.KT) {
-      sh.waves = whole;
-      sh.share = share;
-    }
+  bool narrow = false;
+  Q_CHECK_ARG(prompt_plan(EPI, M, N, wN, K, scratch != nullptr, &sh, &pairs, &narrow), "%s: too many tiles", who);
+  if constexpr (EPI == EPI_RESID || EPI == EPI_F32) {
+    if (narrow) return launch_tiles<EPI, PG_NARROW>(x, w_tc, out, M, wN, K, sh, pairs, ra, scratch, status, stream, who);
   }
-  constexpr bool can_be_narrow = EPI == EPI_RESID || EPI == EPI_F32;
-  if (can_be_narrow) {
-    // Narrow tiles where they leave less of a wave idle: whole, in units of one k step x one column. A narrow step
-    // takes 0.69 of a wide one (0.63 the columns, the same activations), a split 45 steps here, 25 behind whole
-    // waves; the tiles of a wave that is nearly empty run faster, down to 0.6 of the time. Wide / narrow, us: O at 257 rows 25.5 / 19.1, 1024 27.1 / 20.4, 2048 44.0 / 36.2, but 1280 27.3 / 33.8,
-    // 4096 66.8 / 70.7, 8192 126 / 130; down at 512 41.0 / 39.6, 1024 51.7 / 42.7, 2103 100 / 90, but 2560
-    // 108 / 117, 8192 298 / 356.
-    PromptShape nr = sh;
-    nr.nt = (N + PG_NARROW - 1) / PG_NARROW;
-    const long long nt = (long long)nr.mt * nr.nt;
-    const int tail = sh.share != sh.KT ? sh.share + (sh.waves ? 25 : 45)
-                     : rest ? sh.KT * (6 * pairs + 4 * rest) / (10 * pairs) : 0;
-    const long long wide = (long long)(sh.waves * sh.KT + tail) * PG_BN;
-    const long long narrow = (nt + pairs - 1) / pairs * sh.KT * 175;
-    if (narrow < wide) {
-      nr.waves = (int)(nt / pairs);
-      nr.share = nr.KT;
-      if (nt < pairs) pairs = (int)nt;
-      return launch_tiles<EPI, can_be_narrow ? PG_NARROW : PG_BN>(x, w_tc, out, M, wN, K, nr, pairs, ra, scratch, status,
-                                                                  stream, who);
-    }
-  }
-  if (sh.share == sh.KT && tiles < pairs) pairs = (int)tiles;
   return launch_tiles<EPI, PG_BN>(x, w_tc, out, M, wN, K, sh, pairs, ra, scratch, status, stream, who);
 }
 
@@ -790,6 +805,15 @@ int64_t q_gemm_prompt_ticket_bytes() { return (int64_t)PG_TICKET_BYTES; }
 
 extern "C" int64_t q_gemm_prompt_scratch_bytes(void) {
   return (int64_t)(PG_TICKET_BYTES + (size_t)pair_count() * 2 * PG_PART_FLOATS * 4);
+}
+
+extern "C" int q_gemm_prompt_columns(int M, int N, int K, int residual) {
+  PromptShape sh;
+  int pairs = pair_count();
+  bool narrow = false;
+  if (M < 1 || N < 32 || N % 32 || K < 32 || K % 32 ||
+      !prompt_plan(residual ? EPI_RESID : EPI_F32, M, N, N, K, true, &sh, &pairs, &narrow)) return 0;
+  return narrow ? PG_NARROW : PG_BN;
 }
 
 extern "C" int q_gemm_prompt_f32(const void* d_x, const void* d_w_tc, float* d_out, int M, int N, int K,

@@ -81,6 +81,15 @@ def test_narrow_tiles(ops, scratch, M, N, K):
     test_sums_and_residual(ops, scratch, M, N, K)
 
 
+# The same edges where the rule takes narrow tiles for either epilogue (q_gemm_prompt_columns): one wave with idle
+# pairs, two waves, last tiles of 32 and 96 columns, a K that is no multiple of 64.
+@pytest.mark.parametrize("M,N,K", [(512, 2592, 512), (1800, 2592, 96), (8000, 576, 9728), (7000, 672, 160), (1000, 2560, 4096)])
+def test_narrow_tiles_where_the_rule_takes_them(ops, scratch, M, N, K):
+    from starter_b200._lib import lib
+    assert lib.q_gemm_prompt_columns(M, N, K, 0) == lib.q_gemm_prompt_columns(M, N, K, 1) == 160
+    test_sums_and_residual(ops, scratch, M, N, K)
+
+
 @pytest.mark.parametrize("M,inter,K", [(1, 32, 32), (300, 96, 128), (257, 1184, 416), (600, 9728, 256), (600, 1312, 9728)])
 def test_swiglu(ops, scratch, M, inter, K):
     """Within one bf16 rounding of the oracle's SwiGLU of the fp32 sums (inter not a multiple of 128
