@@ -437,8 +437,12 @@ k_attn_merge(const float* __restrict__ part_o, const float* __restrict__ part_ml
 // distributed shared memory: every CTA parks its (max, sum, O) rows in its own shared
 // memory, the cluster synchronises once, and CTA r of the cluster combines 1/S of the
 // (row, dim) outputs from all S CTAs in split order. No global round trips, no tickets.
-template <bool CL, int DG>
-__global__ void __launch_bounds__((4 * DG + 1) * 32, CL && DG == 1 ? 4 : 1)
+// BLOCKS: CTAs an SM must have registers for. Four only in the form for one split, which has nothing to merge and is
+// the only one launched with four on an SM: held to 96 registers the clustered form spilled (12 bytes stored, 44
+// loaded; 136 registers and none without, and steps of 12 layers, held / not, us: 9 x 300 keys 770 / 764, 12 x 1000 837 /
+// 827, 16 x 1000 876 / 871, 24 x 1000 949 / 947).
+template <bool CL, int DG, int BLOCKS = DG == 1 ? 3 : 1>
+__global__ void __launch_bounds__((4 * DG + 1) * 32, BLOCKS)
 k_attn_decode(const float* __restrict__ PQ, PlanView pv, const bf16* __restrict__ QG,
               const bf16* __restrict__ KG, const bf16* __restrict__ COS, const bf16* __restrict__ SIN,
               const int32_t* __restrict__ pos_ptr, char* __restrict__ kpool, char* __restrict__ vpool,
@@ -1084,11 +1088,12 @@ extern "C" int q_attention_decode(const float* d_qkv_partials, const q_gemm_plan
   const bool wide = splits > 1 && ctas <= sms && ring == 3 && NS == 3;
   const int dc = wide ? 12 : 4;
   const dim3 block((dc + 1) * 32);
-  static size_t done[4][64] = {{0}};
+  static size_t done[5][64] = {{0}};
   Q_CHECK_CUDA(q_ensure_smem(k_attn_decode<false, 1>, attn_decode_smem(NS), done[0]));
   Q_CHECK_CUDA(q_ensure_smem(k_attn_decode<true, 1>, attn_decode_smem(NS), done[1]));
   Q_CHECK_CUDA(q_ensure_smem(k_attn_decode<false, 3>, attn_decode_smem(NS), done[2]));
   Q_CHECK_CUDA(q_ensure_smem(k_attn_decode<true, 3>, attn_decode_smem(NS), done[3]));
+  Q_CHECK_CUDA(q_ensure_smem(k_attn_decode<true, 1, 4>, attn_decode_smem(NS), done[4]));
   // the merge scratch (consumer states, then the CTA's own rows) reuses the ring
   const int scratch_stages = (G * (dc + 1) * (MO_LD + 2) * 4 + STAGE_BYTES - 1) / STAGE_BYTES;
   if (ring < scratch_stages) ring = scratch_stages;
@@ -1136,8 +1141,8 @@ extern "C" int q_attention_decode(const float* d_qkv_partials, const q_gemm_plan
     if (wide) Q_CHECK_CUDA(q_launch_cluster(k_attn_decode<true, 3>, grid, block, smem, st, (unsigned)splits, Q_ATTN_DECODE_ARGS));
     else Q_CHECK_CUDA(q_launch_cluster(k_attn_decode<true, 1>, grid, block, smem, st, (unsigned)splits, Q_ATTN_DECODE_ARGS));
   } else if (splits == 1) {
-    // nothing to merge: the form without the merge through memory, which needs fewer registers (96, not 128)
-    Q_CHECK_CUDA(q_launch(k_attn_decode<true, 1>, grid, block, smem, st, Q_ATTN_DECODE_ARGS));
+    // nothing to merge: the form without the merge through memory, which does with 96 registers
+    Q_CHECK_CUDA(q_launch(k_attn_decode<true, 1, 4>, grid, block, smem, st, Q_ATTN_DECODE_ARGS));
   } else {
     if (wide) Q_CHECK_CUDA(q_launch(k_attn_decode<false, 3>, grid, block, smem, st, Q_ATTN_DECODE_ARGS));
     else Q_CHECK_CUDA(q_launch(k_attn_decode<false, 1>, grid, block, smem, st, Q_ATTN_DECODE_ARGS));

@@ -71,6 +71,17 @@ def test_the_public_norm_reads_its_gain_after_the_dependency_wait():
     assert "return rmsnorm(d_x, d_gain, d_out, rows, cols, eps, false, stream);" in public and "true" not in public
 
 
+def test_only_the_one_split_attention_is_held_to_four_ctas_on_an_sm():
+    """96 registers make the clustered form spill; what is launched with splits to merge keeps its registers."""
+    text = source("attention.cu")
+    assert "__launch_bounds__((4 * DG + 1) * 32, BLOCKS)" in text
+    held = between(text, "} else if (splits == 1) {", "} else {")
+    assert held.count("k_attn_decode<true, 1, 4>") == 1
+    assert text.count("k_attn_decode<true, 1, 4>") == 2            # ... and its shared-memory limit
+    clustered = text[text.index("if (cluster) {\n    if (wide)"):text.index("} else if (splits == 1) {")]
+    assert "k_attn_decode<true, 1>," in clustered
+
+
 def test_the_wait_on_an_mbarrier_is_one_loop_bounded_by_the_clock():
     """Every role of the tcgen05 kernels inlines it: a second loop for flag and clock cost a prompt of 64
     tokens 2 %. Its limit counts cycles, since a try may itself sleep."""
