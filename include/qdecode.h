@@ -86,8 +86,8 @@ int q_debug_tc_trace(unsigned long long* out, int n_ctas);
  * of the most recent execution, re-arms the records and returns the count (or a negative
  * q_status). At most 4096 launches are recorded after the option is set.
  * q_debug_timeline_kinds gives the kernel kind of each record: 1 stream-K projection,
- * 2 tcgen05 projection, 3 decode attention, 4 add+norm, 5 SwiGLU, 6 embedding + norm,
- * 7 logits + argmax, 8 add+norm over peer memory. */
+ * 2 tcgen05 projection with split-K slots (and the prompt's), 3 decode attention, 4 add+norm, 5 SwiGLU, 6 embedding + norm,
+ * 7 logits + argmax, 8 add+norm over peer memory, 9 whole projection (q_gemm_rows_*). */
 int q_debug_timeline(unsigned long long* out, int max_records);
 int q_debug_timeline_kinds(int32_t* out, int max_records);
 

@@ -150,7 +150,7 @@ int q_swiglu_layout(const float* d_branch, const q_gemm_plan_t* plan, void* d_ou
 // wait, last warp end, last CTA start} in %globaltimer ns. Launchers pass q_tl_next(kind) as
 // the kernel's last argument: null unless option "timeline" is on, else the next record.
 enum q_tl_kind { Q_TL_GEMM = 1, Q_TL_GEMM_TC = 2, Q_TL_ATTENTION = 3, Q_TL_ADD_NORM = 4, Q_TL_SWIGLU = 5,
-                 Q_TL_EMBED = 6, Q_TL_ARGMAX = 7, Q_TL_PEER_ADD_NORM = 8 };
+                 Q_TL_EMBED = 6, Q_TL_ARGMAX = 7, Q_TL_PEER_ADD_NORM = 8, Q_TL_GEMM_ROWS = 9 };
 unsigned long long* q_tl_next(int kind);
 
 // This rank's view of the tensor-parallel peers (q_peers_t with the pointers checked).

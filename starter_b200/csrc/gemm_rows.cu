@@ -572,10 +572,10 @@ int launch_rows(const void* x, const void* w_tc, void* out, float* ss_out, const
   const dim3 grid(sh.clusters * sh.S), block(GR_THREADS);
   if (sh.S > 1)
     Q_CHECK_CUDA(q_launch_cluster(k_gemm_rows<EPI, NORM>, grid, block, smem, (cudaStream_t)stream, (unsigned)sh.S, map,
-                                  (const unsigned char*)w_tc, out, ss_out, sh, nm, status, q_tl_next(Q_TL_GEMM_TC)));
+                                  (const unsigned char*)w_tc, out, ss_out, sh, nm, status, q_tl_next(Q_TL_GEMM_ROWS)));
   else
     Q_CHECK_CUDA(q_launch(k_gemm_rows<EPI, NORM>, grid, block, smem, (cudaStream_t)stream, map,
-                          (const unsigned char*)w_tc, out, ss_out, sh, nm, status, q_tl_next(Q_TL_GEMM_TC)));
+                          (const unsigned char*)w_tc, out, ss_out, sh, nm, status, q_tl_next(Q_TL_GEMM_ROWS)));
   return Q_OK;
 }
 

@@ -298,6 +298,51 @@ def test_steps_above_8_rows_match_native(cuda, golden_dir, tmp_path, route):
     assert device_status() == [0, 0, 0, 0]
 
 
+def _launch_kinds(state):
+    """How many launches of each kind (q_debug_timeline_kinds) one step makes."""
+    import ctypes as C
+    from collections import Counter
+    from starter_b200 import _lib
+    lib, check = _lib.lib, _lib.check
+    stamps, kinds = (C.c_uint64 * (4 * 256))(), (C.c_int32 * 256)()
+    check(lib.q_set_option(b"timeline", 1))
+    try:
+        state.step()
+        torch.cuda.synchronize()
+        n = lib.q_debug_timeline(stamps, 256)
+        lib.q_debug_timeline_kinds(kinds, 256)
+    finally:
+        check(lib.q_set_option(b"timeline", 0))
+    return Counter(kinds[:n])
+
+
+STREAMK, TCGEN05, ADD_NORM, SWIGLU, WHOLE = 1, 2, 4, 5, 9
+
+
+@pytest.mark.parametrize("hidden,batch,whole", [
+    (640, 9, True), (640, 64, True),         # five launches a layer
+    (160, 9, False), (160, 40, False),       # no multiple of 64: split-K slots and their consumers, eight
+])
+def test_routes_of_steps_above_8_rows(cuda, tmp_path, hidden, batch, whole):
+    """Which projections a step of 9-64 rows launches, each named in the time stamps, and both routes against
+    native Hugging Face."""
+    from starter_b200 import Engine
+    from starter_b200.ops import device_status
+    path, layers = _live_model(tmp_path, 4, 1, hidden, 256, 500, 2, 79), 2
+    engine, native = Engine(path, keep_logits=True), O.native_model(path)
+    prompt = torch.randint(0, 500, (batch, 21), generator=torch.Generator().manual_seed(batch)).tolist()
+    tokens, logits = stepwise_logits(engine, prompt, 4)
+    assert_parity(native, prompt, tokens, logits)
+    with torch.inference_mode():
+        kinds = _launch_kinds(stepwise_logits.last_state)
+    assert kinds[STREAMK] == 0
+    if whole:
+        assert (kinds[WHOLE], kinds[TCGEN05], kinds[ADD_NORM], kinds[SWIGLU]) == (4 * layers, 1, 0, 0)
+    else:
+        assert (kinds[WHOLE], kinds[TCGEN05], kinds[ADD_NORM], kinds[SWIGLU]) == (0, 4 * layers + 1, 2 * layers, layers)
+    assert device_status() == [0, 0, 0, 0]
+
+
 def test_both_routes_above_8_rows_agree(cuda, golden_dir):
     """tcgen05 route against the stream-K route at 32 rows: same tokens, logits equal up to the
     fp32 summation order of the projections (one bf16 ulp)."""
