@@ -382,7 +382,7 @@ def kernels_per_step(state) -> int:
         from starter_b200._lib import lib
         c = state.cfg
         q = c.n_q_heads * 128
-        if lib.q_gemm_rows_supported(rows, c.hidden, c.inter, q, q + 2 * c.n_kv_heads * 128):
+        if (rows > 16 or c.hidden > 512) and lib.q_gemm_rows_supported(rows, c.hidden, c.inter, q, q + 2 * c.n_kv_heads * 128):
             # embed | QKV, attention, O, gate|up, down (norm, add and SwiGLU inside) | final norm, lm_head, argmax
             return 1 + 5 * L + 3
         # embed | QKV, attention, O, add+norm, gate|up, SwiGLU, down, add+norm | lm_head, argmax

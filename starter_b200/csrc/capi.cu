@@ -384,8 +384,14 @@ static bool peer_exchange_in_gemm(const q_engine* e) {
          e->cfg.hidden <= 3072 && e->p_o.slots <= 2 && e->p_down.slots <= 2 && e->cfg.tp_size <= g_peer_in_gemm;
 }
 
-// Up to 64 rows on one GPU behind the tcgen05 tiling: five launches a layer (gemm_rows.cu).
-static bool rows_path(const q_config_t& c, int rows) {
+// Up to 64 rows on one GPU behind the tcgen05 tiling: five launches a layer (gemm_rows.cu). Not for few rows of a
+// very narrow model, whose weights take no time: what is left is what a launch costs, and a whole projection (one
+// CTA an SM, tensor memory, a cluster's exchange) costs more than the two it replaces. Decode step of 4 layers, 300
+// keys, eight launches / five, us: hidden 512, inter 1024, 9 rows 113 / 120, 16 115 / 122, but 33 134 / 132; hidden
+// 256, inter 512, 9 rows 100 / 110, 33 121 / 121; hidden 640, inter 1792, 9 rows 126.7 / 127.3, 24 143 / 137; hidden 1024,
+// inter 2048, 9 rows 133 / 129. (Verification and short prompts, with more launches around them: 0.92 - 1.04 of the time.)
+static bool rows_path(const q_config_t& c, int rows, int T) {
+  if (T == 1 && rows <= 16 && c.hidden <= 512) return false;
   return c.tp_size == 1 && q_gemm_rows_supported(rows, c.hidden, c.inter, c.n_q_heads * 128,
                                                  (c.n_q_heads + 2 * c.n_kv_heads) * 128);
 }
@@ -631,7 +637,7 @@ static int run_layers(q_engine* e, bool advance, void* stream) {
     }
     return head_argmax(e, advance, stream);
   }
-  if (e->tc && rows_path(c, e->rows)) {
+  if (e->tc && rows_path(c, e->rows, e->T)) {
     // The sums of squares of the residual's rows lie behind the QKV sums: their buffer holds two slots of them,
     // and a row has fewer parts than QKV columns (q_gemm_rows_supported).
     const int rows = e->rows, q_cols = c.n_q_heads * 128, qkv_cols = e->p_qkv.N;

@@ -322,6 +322,7 @@ STREAMK, TCGEN05, ADD_NORM, SWIGLU, WHOLE = 1, 2, 4, 5, 9
 @pytest.mark.parametrize("hidden,batch,whole", [
     (640, 9, True), (640, 64, True),         # five launches a layer
     (160, 9, False), (160, 40, False),       # no multiple of 64: split-K slots and their consumers, eight
+    (512, 16, False), (512, 17, True), (576, 16, True),      # few rows of a narrow model keep the eight
 ])
 def test_routes_of_steps_above_8_rows(cuda, tmp_path, hidden, batch, whole):
     """Which projections a step of 9-64 rows launches, each named in the time stamps, and both routes against
