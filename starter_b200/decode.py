@@ -257,10 +257,11 @@ class DecodeState:
         return weights + kv_token * self.batch * visible_keys + kv_token * self.batch
 
     # ---- prefill: the prompt pass ----
-    # Prompt rows processed together: launches, last waves and weights (203 MB a layer) are paid for once per so many
-    # rows, against 46 KB of activation scratch a row (1.1 GB). 12 x 2048 tokens, 12 layers, 8192 / 24576 rows at a
-    # time: 54.9 / 53.7 ms.
-    PREFILL_ROWS = 24576
+    # Prompt rows processed together, which bounds the activation scratch: 46 KB a row at hidden 2560, 0.38 GB, kept for
+    # the life of the state beside its pages. Launches, last waves and weights (203 MB a layer) are paid for once per so
+    # many rows: 12 x 2048 tokens at 2048 / 4096 / 8192 rows at a time 64.2 / 59.1 / 55.8 ms (12 layers). Three times the
+    # rows gained 2 % more there and took three times the scratch.
+    PREFILL_ROWS = 8192
     # Rows from which the projections run on the CTA-pair kernel: the first that k_gemm_tc cannot hold in
     # one pass over the weight (256; up to 64 rows the projections are k_gemm_rows). Prompt pass of 12 layers,
     # below / pairs, us: 65 rows 1101 / 2025, 128 1300 / 1934, 192 1589 / 1972, 256 1823 / 1993; above, when the

@@ -165,6 +165,20 @@ def test_prompt_pass_in_several_chunks(cuda, tmp_path, batch, length, budget):
         assert_parity(native, prompt.tolist(), [t.tolist()], lg[None])
 
 
+def test_prompt_scratch_is_bounded(cuda, golden_dir):
+    """A batch of long prompts takes the activation scratch of 8192 rows, not of all of its rows: what it takes stays
+    allocated beside the pages, and a context that fits must keep fitting."""
+    from starter_b200 import Engine
+    from starter_b200.decode import DecodeState
+    engine = Engine(str(golden_dir / "tiny_qwen3"))
+    ids = torch.randint(0, 127, (13, 1000), generator=torch.Generator().manual_seed(3)).cuda()
+    with torch.inference_mode():
+        state = DecodeState(engine.weights, 13, 1000, 1)
+        state.prefill(ids)
+    rows = [t.shape[0] for t in state._pf.values() if isinstance(t, torch.Tensor) and t.dtype == torch.bfloat16]
+    assert state._pf["rows"] == max(rows) == 8000
+
+
 def test_generate_contract_and_graph_replay(cuda, golden_dir):
     """N yields of B ids, none for N<=0, state reused across calls, stable
     addresses, graph replay equals eager stepping (reference tests/test_decode.py:94-118,
