@@ -65,7 +65,7 @@ struct RowsNorm {
   const bf16* gain;    // [K]
   const float* ss;     // [parts][M] sums of squares
   int parts;
-  float inv_k, eps;
+  float k, eps;
 };
 
 __device__ __forceinline__ void gr_cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
@@ -293,7 +293,7 @@ k_gemm_rows(const __grid_constant__ CUtensorMap xmap, const unsigned char* __res
       if (et < sh.M) {
         float t = 0.f;
         for (int j = 0; j < groups; ++j) t += inv_s[64 + j * mp + et];
-        inv_s[et] = rsqrtf(t * nm.inv_k + nm.eps);
+        inv_s[et] = rsqrtf(t / nm.k + nm.eps);            // (rounded as the row norm rounds it)
       }
       epi_sync();
       // A thread has one 16-byte chunk of rows r0, r0 + 16, ...: r0 % 8 is r % 8 of all of them, so that the
@@ -584,7 +584,7 @@ int norm_args(const void* gain, const float* ss, int parts, int K, float eps, Ro
   nm->gain = (const bf16*)gain;
   nm->ss = ss;
   nm->parts = parts;
-  nm->inv_k = 1.0f / (float)K;
+  nm->k = (float)K;
   nm->eps = eps;
   return Q_OK;
 }

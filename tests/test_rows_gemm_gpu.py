@@ -109,6 +109,19 @@ def test_swiglu(rows, inter, K):
     assert ops.device_status() == [0, 0, 0, 0]
 
 
+@pytest.mark.parametrize("K", [896, 2560])
+def test_norm_is_rounded_as_the_row_norm(K):
+    """Through an identity weight every normalised value comes out exactly, and it is the one that
+    bf16(x * rsqrt(sum / K + eps)) * gain gives: same division, same roundings."""
+    tc = ops.pack_weight_tc(torch.eye(K, dtype=torch.bfloat16, device="cuda"))
+    for seed in range(8):
+        x, gain = _bf16((64, K), seed), _bf16((K,), 100 + seed)
+        ss = _parts(x, 1)
+        out = torch.full((64, K), float("nan"), device="cuda")
+        check(lib.q_gemm_rows_f32(_p(x), _p(gain), _p(ss), 1, _p(tc), _p(out), 64, K, K, EPS, _stream()))
+        assert torch.equal(out, _rms(x, ss[0], gain).float())
+
+
 def test_refused():
     z = torch.zeros(4096, dtype=torch.bfloat16, device="cuda")
     for rows, N, K in ((0, 64, 64), (65, 64, 64), (4, 12, 64), (4, 64, 96)):
