@@ -193,9 +193,11 @@ int q_gemm_tc(const void* d_x, const void* d_w_tc, float* d_partials, int M, int
  * (engine/kernels/decode_fused.py:19-44 split between the two projections around it); a null gain
  * takes x as it is (q_gemm_rows_f32 only).
  * q_gemm_rows_supported: 1 if the four projections of a layer are all taken at this row count;
- * q_gemm_rows_parts: 0 if the shape is not. */
+ * q_gemm_rows_parts: 0 if the shape is not. q_gemm_rows_splits: the CTAs of a cluster, among which K
+ * is split, of q_gemm_rows_add (add != 0) or q_gemm_rows_f32 without gain; 0 if not taken. */
 int q_gemm_rows_supported(int M, int hidden, int inter, int q_cols, int qkv_cols);
 int q_gemm_rows_parts(int M, int N, int K);
+int q_gemm_rows_splits(int M, int N, int K, int add);
 int q_gemm_rows_f32(const void* d_x, const void* d_gain, const float* d_ss, int parts,
                     const void* d_w_tc, float* d_out, int M, int N, int K, float eps, void* stream);
 int q_gemm_rows_add(const void* d_x, const void* d_w_tc, void* d_resid, float* d_ss, int M, int N, int K,

@@ -111,6 +111,7 @@ SIGNATURES = {
     "q_gemm_tc": (_I, [_P, _P, _P, _I, _I, _I, _P]),
     "q_gemm_rows_supported": (_I, [_I, _I, _I, _I, _I]),
     "q_gemm_rows_parts": (_I, [_I, _I, _I]),
+    "q_gemm_rows_splits": (_I, [_I, _I, _I, _I]),
     "q_gemm_rows_f32": (_I, [_P, _P, _P, _I, _P, _P, _I, _I, _I, _F, _P]),
     "q_gemm_rows_add": (_I, [_P, _P, _P, _P, _I, _I, _I, _P]),
     "q_gemm_rows_swiglu": (_I, [_P, _P, _P, _I, _P, _P, _I, _I, _I, _F, _P]),

@@ -597,6 +597,12 @@ extern "C" int q_gemm_rows_parts(int M, int N, int K) {
   return rows_shape<EPI_RESID, false>(M, N, K, &sh, &smem) ? sh.clusters : 0;
 }
 
+extern "C" int q_gemm_rows_splits(int M, int N, int K, int add) {
+  RowsShape sh;
+  size_t smem = 0;
+  return (add ? rows_shape<EPI_RESID, false>(M, N, K, &sh, &smem) : rows_shape<EPI_F32, false>(M, N, K, &sh, &smem)) ? sh.S : 0;
+}
+
 extern "C" int q_gemm_rows_supported(int M, int hidden, int inter, int q_cols, int qkv_cols) {
   RowsShape sh;
   size_t smem = 0;

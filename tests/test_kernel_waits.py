@@ -24,6 +24,26 @@ def test_mma_roles_start_their_limit_after_the_dependency_wait():
         assert role.index("pdl_wait();") < role.index("mbar_wait("), f"{name}: a bounded wait comes before it"
 
 
+def test_whole_projections_touch_nothing_before_the_dependency_wait():
+    """Every role of k_gemm_rows passes the dependency wait before its first bounded wait (the limit of which would
+    otherwise run while a kernel ahead is still polling), and before what the kernels ahead write: the activations,
+    the rows' sums of squares, the residual. Only weights and gains are asked for earlier."""
+    text = source("gemm_rows.cu")
+    kernel = between(text, "k_gemm_rows(const __grid_constant__", "int rows_clusters(")
+    roles = kernel[kernel.index("auto warp_wait"):]
+    weights = between(roles, "if (warp == 0) {", "} else if (warp == 2) {")
+    assert weights.index("if (issued < n_fill) pdl_wait();") < weights.index("warp_wait(")
+    activations = between(roles, "} else if (warp == 2) {", "} else if (warp == 1) {")
+    assert activations.index("pdl_wait();") < min(activations.index("warp_wait("), activations.index("tma_load_2d("))
+    mma = between(roles, "} else if (warp == 1) {", "} else if (warp >= 4) {")
+    assert mma.index("pdl_wait();") < min(mma.index("warp_wait("), mma.index("tc_mma("))
+    rest = roles[roles.index("} else if (warp >= 4) {"):]
+    for touched in ("warp_wait(", "nm.ss[", "res[j] = ", "tc_ld16("):
+        assert rest.index("pdl_wait();") < rest.index(touched), touched
+    early = kernel[:kernel.index("auto warp_wait")]
+    assert not re.search(r"nm\.ss\b|tma_load_2d\(|ss_out\[", early) and "bulk_g2s(" in early
+
+
 def test_prompt_attention_commits_nothing_that_nobody_waits_for():
     """The softmax warps wait for the last products' B_OF commit and then the CTA leaves: a commit issued
     after it would arrive in shared memory that may be another CTA's by then. The stage releases come
@@ -39,7 +59,7 @@ def test_prompt_attention_commits_nothing_that_nobody_waits_for():
 def test_tensor_memory_loads_are_tied_to_their_wait():
     """A memory clobber does not order register arithmetic: the registers of a tensor-memory load are
     safe only if the wait is part of the same statement, or if they are pinned after it."""
-    statements = [s.split(");\n")[0] for name in ("tc.cuh", "gemm_tc.cu", "gemm_prompt.cu", "attn_prompt.cu")
+    statements = [s.split(");\n")[0] for name in ("tc.cuh", "gemm_tc.cu", "gemm_rows.cu", "gemm_prompt.cu", "attn_prompt.cu")
                   for s in source(name).split("asm volatile(")[1:]]
     loads = [s for s in statements if "tcgen05.ld." in s]
     waiting = [s for s in loads if "tcgen05.wait::ld" in s]

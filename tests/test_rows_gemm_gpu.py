@@ -109,6 +109,18 @@ def test_swiglu(rows, inter, K):
     assert ops.device_status() == [0, 0, 0, 0]
 
 
+# K of 14, 41 and 172 tiles of 64: clusters whose CTAs have different, odd and even, numbers of k tiles, with rows
+# that leave the last CTAs of a cluster none to finish.
+@pytest.mark.parametrize("rows", [1, 9, 17, 33, 64])
+@pytest.mark.parametrize("N,K", [(896, 896), (2048, 2624), (4096, 2624), (896, 11008), (2560, 11008)])
+def test_uneven_splits(rows, N, K):
+    splits = [lib.q_gemm_rows_splits(rows, N, K, add) for add in (0, 1)]
+    assert all(s > 1 and (K // 64) % s for s in splits), splits
+    test_f32(rows, N, K, False)
+    test_f32(rows, N, K, True)
+    test_add(rows, N, K)
+
+
 @pytest.mark.parametrize("K", [896, 2560])
 def test_norm_is_rounded_as_the_row_norm(K):
     """Through an identity weight every normalised value comes out exactly, and it is the one that
@@ -120,6 +132,25 @@ def test_norm_is_rounded_as_the_row_norm(K):
         out = torch.full((64, K), float("nan"), device="cuda")
         check(lib.q_gemm_rows_f32(_p(x), _p(gain), _p(ss), 1, _p(tc), _p(out), 64, K, K, EPS, _stream()))
         assert torch.equal(out, _rms(x, ss[0], gain).float())
+
+
+@pytest.mark.parametrize("rows", [9, 33, 64])
+@pytest.mark.parametrize("inter,K", [(264, 128), (9728, 2560)])
+def test_swiglu_of_each_element(rows, inter, K):
+    """With the row's sum in one part the normalised values are those of the oracle bit for bit; then g and u can
+    only round the other way (one ulp of each, rarely), and so can silu(g) (whose slope is at most 1.1) and the product."""
+    x, w, gain = _bf16((rows, K), 1), _bf16((2 * inter, K), 2, 0.05), _bf16((K,), 3)
+    ss = _parts(x, 1)
+    act = torch.full((rows, inter), float("nan"), dtype=torch.bfloat16, device="cuda")
+    check(lib.q_gemm_rows_swiglu(_p(x), _p(gain), _p(ss), 1, _p(ops.pack_weight_tc(w)), _p(act), rows, inter, K, EPS,
+                                 _stream()))
+    y = (_rms(x, ss[0], gain).double() @ w.double().T).bfloat16().float()
+    g, u = y[:, :inter], y[:, inter:]
+    want = (torch.nn.functional.silu(g).bfloat16().float() * u).bfloat16().float()
+    diff = (act.float() - want).abs()
+    assert bool((diff <= BF16_ULP * (1.1 * g.abs() * u.abs() + 3 * want.abs()) + 1e-4).all())
+    assert float((diff > 0).float().mean()) < 0.02
+    assert ops.device_status() == [0, 0, 0, 0]
 
 
 def test_refused():
