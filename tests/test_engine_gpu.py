@@ -165,12 +165,12 @@ def test_prompt_pass_in_several_chunks(cuda, tmp_path, batch, length, budget):
         assert_parity(native, prompt.tolist(), [t.tolist()], lg[None])
 
 
-def test_prompt_scratch_is_bounded(cuda, golden_dir):
+def test_prompt_scratch_is_bounded(cuda, tmp_path):
     """A batch of long prompts takes the activation scratch of 8192 rows, not of all of its rows: what it takes stays
     allocated beside the pages, and a context that fits must keep fitting."""
     from starter_b200 import Engine
     from starter_b200.decode import DecodeState
-    engine = Engine(str(golden_dir / "tiny_qwen3"))
+    engine = Engine(_live_model(tmp_path, 4, 1, 128, 128, 127, 1, 80, positions=1024))
     ids = torch.randint(0, 127, (13, 1000), generator=torch.Generator().manual_seed(3)).cuda()
     with torch.inference_mode():
         state = DecodeState(engine.weights, 13, 1000, 1)
