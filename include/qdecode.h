@@ -185,6 +185,10 @@ int q_gemm_tc(const void* d_x, const void* d_w_tc, float* d_partials, int M, int
 /* ---- whole projections of 1..64 rows with the layer's element-wise work inside -------------
  * Same weight tiling as q_gemm_tc; N and K multiples of 8 and 64, x, gain and outputs 16-byte
  * aligned. No partial slots: K is split inside a thread-block cluster and added there.
+ * The weight and the gain are a model's: they are read before the kernels ahead in the stream have
+ * ended, so no launch right before may write them. x, d_ss and d_resid may come from one.
+ * Limits on 148 SMs: a CTA per SM has at most 256 output columns and needs a ring of three stages,
+ * which ends q_gemm_rows_swiglu at inter 18944, and at inter 17408 at 40 rows.
  *   q_gemm_rows_f32     out = n @ W^T in fp32                          (W [N][K])
  *   q_gemm_rows_add     resid = bf16(resid + bf16(x @ W^T)) in place, and into
  *                       d_ss[q_gemm_rows_parts(M, N, K)][M] the sums of squares of parts of its rows
@@ -413,7 +417,9 @@ typedef struct q_layer_weights_t {
   void* kpool;
   void* vpool;
   /* optional: the four matrices in q_pack_weight_tc's tiling (wgu_tc = [gate rows | up rows],
-   * not interleaved). All four set = steps with tc_min_rows rows or more use q_gemm_tc. */
+   * not interleaved). All four set = steps with tc_min_rows rows or more use q_gemm_rows_* where it
+   * takes all four projections (not for 16 rows and fewer of hidden 512 and less, nor under tensor
+   * parallelism), else q_gemm_tc. */
   const void* wqkv_tc;
   const void* wo_tc;
   const void* wgu_tc;
@@ -423,8 +429,9 @@ typedef struct q_layer_weights_t {
 /* The prompt pass of one GPU in one call (engine/prefill.py:26-62): batch * T prompt tokens through
  * all layers, K and V rows of positions *pos .. *pos+T-1 into the pages, the final norm of every
  * sequence's last position into d_last [batch][hidden]. From few_rows rows on the projections are
- * q_gemm_prompt_*, below that q_gemm_tc and its consumers (partials: enough for every plan of up to
- * few_rows - 1 rows). x, normed [rows][hidden], q, attended [rows][n_q*128], act [rows][inter] are
+ * q_gemm_prompt_*, below that q_gemm_tc and its consumers (partials: enough for every q_gemm_tc plan of
+ * up to few_rows - 1 rows), and where q_gemm_rows_supported says so q_gemm_rows_*: the QKV sums in
+ * the first slot of partials, the rows' sums of squares behind them in the second. x, normed [rows][hidden], q, attended [rows][n_q*128], act [rows][inter] are
  * scratch of the caller (32-byte aligned), split as in q_gemm_prompt_* (its tickets are cleared by
  * every call; null if no call has few_rows rows).
  * layers: wqkv_tc .. wdown_tc, gains and pools are read; only enqueues on `stream`. */
@@ -570,9 +577,10 @@ int64_t q_engine_peer_floats(const q_engine* e, int rows);
 int q_bind_peers(q_engine* e, const q_peers_t* peers);
 int q_decode_step_peers(q_engine* e, void* stream);
 
-/* One full step for T=1 on a single GPU: embed .. argmax, tokens and pos updated:
- * 2 + 5 per layer + 1 kernels up to 8 rows (add+norm and SwiGLU folded into the projections),
- * 1 + 8 per layer + 2 above, all with programmatic dependent launch. */
+/* One full step for T=1 on a single GPU: embed .. argmax, tokens and pos updated, all with
+ * programmatic dependent launch. Kernels of L layers: 3 + 5 L for 1-2 rows (add+norm and SwiGLU folded
+ * into the projections; needs hidden % 4 == 0 and at most 3072), 3 + 7 L up to 8 (add+norm of their own),
+ * 4 + 5 L for 9-64 on q_gemm_rows_*, 3 + 8 L on q_gemm_tc. */
 int q_decode_step(q_engine* e, void* stream);
 
 /* The same step in pieces, for tensor parallelism: the caller all-reduces
@@ -604,7 +612,7 @@ int q_verify_step(q_engine* e, void* stream);
  * not capturable). A non-zero word means a bounded wait inside a kernel ran out and the
  * results since then are not to be trusted: out[0] attention (1 producer, 2 consumer),
  * out[1] stream-K GEMM ring (1), out[2] tcgen05 GEMM (1 producer, 2 MMA issuer, 3 epilogue,
- * 4 drain), out[3] tensor parallel over peer memory (1 = a peer's arrival word never came).
+ * 4 drain; prompt 5-8, whole projections 10-13 in the same order), out[3] tensor parallel over peer memory (1 = a peer's arrival word never came).
  * The words are sticky; q_clear_status zeroes them (synchronises too). */
 int q_device_status(int32_t out[4]);
 int q_clear_status(void);

@@ -956,7 +956,9 @@ extern "C" int q_attention_decode_splits(int batch, int n_kv_heads, int capacity
   // One sequence of a very long context: every SM takes a split (merged through global memory).
   // 8 kv heads, 18 splits / 8: 247 / 248 at 8 K, 299 / 345 at 30 K, but 226 / 224 at 4 K.
   if (tiles > 96 && sms / vh > MAX_CLUSTER) return sms / vh < 32 ? sms / vh : 32;
-  // From 9 rows on the projections run on k_gemm_tc, whose CTAs leave no room on their SM: all of the
+  // From 9 rows on the projections run on the tcgen05 kernels, whose CTAs leave no room on their SM (the figures are
+  // behind k_gemm_tc; k_gemm_rows takes a whole SM for a CTA as well, and behind it no size has been measured
+  // slower with this rule than behind k_gemm_tc, but other counts were not tried): all of the
   // attention starts at once when they end, and clusters of three and more need a tenth of the places
   // to spare (44 clusters of 3, 45 would fit an idle GPU: 389 at 4 K; of 6 narrow CTAs, 45 again: 348; of 5: 310).
   const bool after_tc = batch >= 9;
@@ -975,7 +977,7 @@ extern "C" int q_attention_decode_splits(int batch, int n_kv_heads, int capacity
     if (tiles > 20 * s && 2 * sms / vh > MAX_CLUSTER) return 2 * sms / vh;
     // Behind the stream-K projections, whose CTAs leave room, the wide CTAs start early and win up to 8
     // sequences - 5 of 8 kv heads, 3 / 7 splits: 231 / 243 at 700, 256 / 292 at 2 K, 335 / 399 at 8 K. Behind
-    // k_gemm_tc they win while a split's tiles go around the three groups once (9 sequences of 4 kv heads,
+    // tcgen05 projections they win while a split's tiles go around the three groups once (9 sequences of 4 kv heads,
     // 3 / 7 splits: 251 / 253 at 400, but 3 / 6 splits 283 / 280 at 2 K, 311 / 301 at 4 K) or where they
     // fill the SMs (9 sequences of 8 kv heads, 2 / 3 splits: 300 / 304 at 1 K).
     if (!after_tc || tiles < 3 * s || (s * vh * 10 >= sms * 9 && tiles >= 6 * s)) return s;

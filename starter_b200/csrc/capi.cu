@@ -686,7 +686,8 @@ extern "C" int q_verify_step(q_engine* e, void* stream) {
   return run_layers(e, false, stream);
 }
 
-// The prompt pass: the same launches as the steps above, seven a layer (eight on split-K partials),
+// The prompt pass: the same launches as the steps above, seven a layer (up to 64 rows six: whole projections; then up to
+// few_rows - 1 nine, on split-K partials),
 // enqueued from here because a host loop over the ABI costs more than the kernels of a short prompt.
 extern "C" int q_prompt_pass(const q_prompt_t* p, const q_layer_weights_t* layers, const int64_t* d_tokens,
                              const int32_t* d_block_table, int pages_per_seq, int batch, int T, void* d_last,

@@ -21,13 +21,14 @@
 // needed), warp 1 MMA issuer, warp 2 activation slices by TMA after the dependency wait, warps 4-11 norm of the
 // slices (four warps to each of a stage's two k tiles), then the epilogue. What each role's loop costs per stage
 // is what limits short tiles - 250 ns a stage with nothing to copy and nothing to multiply -, hence two k tiles a
-// stage (down at 16 rows 13.9 -> 10.9 us), whole warps that walk their loop and elect the lane that issues (the
-// loop inside one lane's branch: 14.3 us, with polls by one lane 12.6), and a hardware barrier, not an mbarrier
-// that eight warps poll, to wake the epilogue. With a ring of half an SM the next kernel's CTA could start beside
-// this one, but at 64 rows it has too little in flight (12 layers 1228 against 1044 us; 922 / 908 at 16).
-// Decode step of 12 layers, gemm_tc.cu and its consumers / this, us: 16 x 1024 keys 1040 / 908, 32 x 2048
-// 1430 / 1281, 64 x 333 1254 / 1044; a layer's QKV, O, gate|up, down at 16 rows 10.5, 7.5, 18.7, 11.5 us, of
-// which the weights take 4.8, 3.2, 15.2, 7.6.
+// stage, whole warps that walk their loop and elect the lane that issues, and a hardware barrier, not an mbarrier
+// that eight warps poll, to wake the epilogue. (While it was built, with clusters of at most four, down alone at 16 rows:
+// one k tile a stage 13.9 us, two 10.9; the loop inside one lane's branch 14.3, polls by one lane 12.6. With a ring of
+// half an SM, so that the next kernel's CTA could start beside this one, there is too little in flight at 64 rows: 12
+// layers 1228 against 1044 us; 922 / 908 at 16.)
+// Decode step of 12 layers, gemm_tc.cu and its consumers / this, us: 16 x 1000 keys 1032 / 870, 32 x 2000
+// 1402 / 1249, 64 x 333 1251 / 1004; inside the step a layer's QKV, O, gate|up, down at 16 rows 8.8, 7.4, 18.8, 11.4 us,
+// of which the weights take 4.8, 3.2, 15.2, 7.6.
 // Every wait is bounded as in gemm_tc.cu and reports in the same status word (codes 10-13).
 #include "tc.cuh"
 
@@ -119,7 +120,7 @@ k_gemm_rows(const __grid_constant__ CUtensorMap xmap, const unsigned char* __res
   uint32_t off[PIECES], bytes[PIECES];
   int issued = 0, kt = rot;                                  // ring stages filled, next k tile
   // weights of the next stage; sources move on (the whole warp keeps the addresses, so that they stay in uniform
-  // registers, and one elected lane issues: with the loop inside one lane's branch down took 14.3 us, now 12.2)
+  // registers, and one elected lane issues)
   auto weights = [&](uint32_t dst, uint32_t full, uint64_t policy) {
     const bool two = issued * 2 + 1 < nk;
     const ptrdiff_t next = kt + 1 == nk ? GR_TILE - (ptrdiff_t)nk * GR_TILE : GR_TILE;
@@ -513,8 +514,8 @@ bool rows_shape(int M, int N, int K, RowsShape* sh, size_t* smem) {
   // K is split so that a CTA's time comes out least, in bytes at the HBM rate of an SM: its weights, half of its
   // activation slices (from L2), 11 KB a ring stage (250 ns) and 40 KB for the exchange. Clusters of 8 leave a quarter of
   // the SMs idle and still win by the stages and, since O and down then leave half as many sums of squares, in the next
-  // norm; above 32 rows their receive area does not fit. Step of 12 layers, at most 4 / 8 CTAs a cluster, us: 9 x 300
-  // keys 790 / 771, 16 x 1024 896 / 883, 32 x 500 904 / 902.
+  // norm; towards 64 rows their receive area does not fit (33 rows still take them). Step of 12 layers, at most 4 / 8 CTAs
+  // a cluster, when that was chosen, us: 9 x 300 keys 790 / 771, 16 x 1024 896 / 883, 32 x 500 904 / 902.
   long long best = -1;
   for (int S = 1; S <= 8; S *= 2) {
     RowsShape t = *sh;
