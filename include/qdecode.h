@@ -187,8 +187,8 @@ int q_gemm_tc(const void* d_x, const void* d_w_tc, float* d_partials, int M, int
  * aligned. No partial slots: K is split inside a thread-block cluster and added there.
  * The weight and the gain are a model's: they are read before the kernels ahead in the stream have
  * ended, so no launch right before may write them. x, d_ss and d_resid may come from one.
- * Limits on 148 SMs: a CTA per SM has at most 256 output columns and needs a ring of three stages,
- * which ends q_gemm_rows_swiglu at inter 18944, and at inter 17408 at 40 rows.
+ * Limits on 148 SMs: a CTA per SM has at most 256 output columns and needs a ring of three stages;
+ * q_gemm_rows_swiglu takes 64 rows up to inter 16384, 48 at 17408, 32 at 18944 and none above.
  *   q_gemm_rows_f32     out = n @ W^T in fp32                          (W [N][K])
  *   q_gemm_rows_add     resid = bf16(resid + bf16(x @ W^T)) in place, and into
  *                       d_ss[q_gemm_rows_parts(M, N, K)][M] the sums of squares of parts of its rows
